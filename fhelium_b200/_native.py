@@ -72,6 +72,7 @@ SIGNATURES: dict[str, tuple] = {
     "fhb_rns_binary": (_I, [_P, _I, _P, _P, _P, _I64, _I, _I, _I, _P]),
     "fhb_rns_lift_signed": (_I, [_P, _P, _P, _I64, _I, _I, _P]),
     "fhb_ckks_keyswitch_scratch_bytes": (_I64, [_P, _I64, _I]),
+    "fhb_ckks_keyswitch_workspace_bytes": (_I64, [_P, _I64, _I]),
     "fhb_ckks_relinearize": (_I, [_P, _P, _P, _P, _P, _I64, _I64, _I, _I, _P]),
     "fhb_ckks_multiply_relinearize": (_I, [_P, _P, _P, _P, _P, _P, _I64, _I64, _I, _I, _P]),
     "fhb_ckks_rotate": (_I, [_P, _P, _P, _P, _P, _I64, _I64, _I, _U32, _P]),

@@ -187,7 +187,7 @@ class MixedBatchExecutor:
             self._streams.append(torch.cuda.Stream(eng.device))
         need = [0] * self.streams
         for g in self.groups:
-            nb = int(eng.ctx.lib.fhb_ckks_keyswitch_scratch_bytes(eng.ctx.handle, g.items, g.level))
+            nb = int(eng.ctx.lib.fhb_ckks_keyswitch_workspace_bytes(eng.ctx.handle, g.items, g.level))
             need[g.stream] = max(need[g.stream], nb)
         self._scratch = [torch.empty(max(nb, 16), dtype=torch.uint8, device=eng.device) for nb in need]
 

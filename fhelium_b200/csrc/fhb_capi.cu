@@ -116,6 +116,10 @@ int ks_core(const Context& c, const void* digits, const void* key, void* acc0, v
             bool pre = false, int64_t ct3_pitch = 0) {
   FHB_DISPATCH(run_ks_core, c, digits, key, acc0, acc1, batch, level, st, item_keys, ct3, pre, ct3_pitch);
 }
+int ks_pass(const Context& c, const void* digits, void* y, int64_t y_words, const void* key, void* acc0, void* acc1,
+            int64_t batch, int level, cudaStream_t st, const uint64_t* item_keys, const void* ct3, bool pre) {
+  FHB_DISPATCH(run_ks_pass, c, digits, y, y_words, key, acc0, acc1, batch, level, st, item_keys, ct3, pre, 0);
+}
 int ks_sum(const Context& c, const void* digits, const uint64_t* key_ptrs, void* acc0, void* acc1, int giants,
            int64_t batch, int level, cudaStream_t st, bool pre = false) {
   FHB_DISPATCH(run_ks_sum, c, digits, key_ptrs, acc0, acc1, giants, batch, level, st, pre);
@@ -285,9 +289,19 @@ struct Scratch {
   char* t0;      // [B, L+P, N]
   char* t1;      // [B, L+P, N]
   char* ext;     // tensor-core form only: [D_l, B, L+P, N] digit extensions
+  char* y;       // CUDA-core form: what the caller's buffer holds beyond the above
+  int64_t y_words;
 };
 
-Scratch carve(const Context& c, void* base, int64_t batch, int level) {
+// Words of one ciphertext's digits of one row: the least the key-switch
+// core's column and block launches can work with.
+int64_t ks_pass_min_words(const Context& c, int level) {
+  return int64_t(c.level_digits[level].size()) * c.n();
+}
+
+// scratch_bytes: the size of the caller's buffer; what it holds beyond the
+// regions every form needs is the intermediate of the key-switch core.
+Scratch carve(const Context& c, void* base, int64_t batch, int level, int64_t scratch_bytes = 0) {
   const int64_t w = word_bytes(c), n = c.n(), l = c.num_q - level, lp = l + c.num_p;
   char* p = static_cast<char*>(base);
   Scratch s;
@@ -296,6 +310,8 @@ Scratch carve(const Context& c, void* base, int64_t batch, int level) {
   s.t0 = s.digits + batch * l * n * w;
   s.t1 = s.t0 + batch * lp * n * w;
   s.ext = s.t1 + batch * lp * n * w;
+  s.y = s.ext;
+  s.y_words = c.basis_tc ? 0 : std::max<int64_t>(0, (scratch_bytes - (s.y - p)) / w);
   return s;
 }
 
@@ -721,6 +737,17 @@ int64_t fhb_ckks_keyswitch_scratch_bytes(const fhb_context* ctx, int64_t batch, 
   return per_ct * batch;
 }
 
+int64_t fhb_ckks_keyswitch_workspace_bytes(const fhb_context* ctx, int64_t batch, int level) {
+  const int64_t need = fhb_ckks_keyswitch_scratch_bytes(ctx, batch, level);
+  if (need < 0) return -1;
+  const Context& c = *ctx->impl;
+  if (c.basis_tc || batch == 0) return need;
+  const int64_t row = fhb::ks_pass_min_words(c, level) * fhb::word_bytes(c);
+  const int64_t rows = c.num_q - level + c.num_p;
+  const int64_t all = batch > INT64_MAX / (row * rows) ? INT64_MAX : row * rows * batch;
+  return need + std::min(all, std::max(row, fhb::kKsPassRoom));
+}
+
 // Scratch check shared by the entry points that take a caller scratch buffer:
 // a negative batch, an invalid level or a size that overflows is an invalid
 // argument, not a small buffer.
@@ -732,14 +759,25 @@ static int check_scratch(const fhb_context* ctx, int64_t batch, int level, int64
   return 0;
 }
 
+// Whether the caller's buffer has room for the key-switch core's column and
+// block launches; without it (exactly fhb_ckks_keyswitch_scratch_bytes) the
+// one-launch cluster core runs.
+static bool ks_passes(const Context& c, const fhb::Scratch& s, int level) {
+  return c.basis_tc || s.y_words >= fhb::ks_pass_min_words(c, level);
+}
+
 // Key-switch core on the ModUp digits in s.digits: with the tensor-core
 // basis conversion the extensions are materialised first (own-digit rows
 // skipped when the core reuses c2 there) and the core only transforms.
 static int ks_core_from_digits(const Context& c, const fhb::Scratch& s, const void* key, int64_t batch, int level,
                                cudaStream_t st, const uint64_t* item_keys = nullptr, const void* ct3 = nullptr) {
-  if (!c.basis_tc) return fhb::ks_core(c, s.digits, key, s.t0, s.t1, batch, level, st, item_keys, ct3);
-  TRY(fhb::tc_extend(const_cast<Context&>(c), s.digits, s.ext, batch, level, ct3 != nullptr, st));
-  return fhb::ks_core(c, s.ext, key, s.t0, s.t1, batch, level, st, item_keys, ct3, true);
+  if (c.basis_tc) {
+    TRY(fhb::tc_extend(const_cast<Context&>(c), s.digits, s.ext, batch, level, ct3 != nullptr, st));
+    return fhb::ks_pass(c, s.digits, s.ext, 0, key, s.t0, s.t1, batch, level, st, item_keys, ct3, true);
+  }
+  if (ks_passes(c, s, level))
+    return fhb::ks_pass(c, s.digits, s.y, s.y_words, key, s.t0, s.t1, batch, level, st, item_keys, ct3, false);
+  return fhb::ks_core(c, s.digits, key, s.t0, s.t1, batch, level, st, item_keys, ct3);
 }
 
 static int keyswitch_tail(const Context& c, const fhb::Scratch& s, const void* key, const void* add0,
@@ -770,7 +808,7 @@ int fhb_ckks_relinearize(const fhb_context* ctx, const void* ct3, const void* ke
   TRY(check_scratch(ctx, batch, level, scratch_bytes));
   if (rescale && level + 1 >= c.num_q) return fail(-4, "cannot rescale at the last level");
   const int limbs = c.num_q - level;
-  const fhb::Scratch s = fhb::carve(c, scratch, batch, level);
+  const fhb::Scratch s = fhb::carve(c, scratch, batch, level, scratch_bytes);
   const int64_t comp = batch * limbs * c.n() * fhb::word_bytes(c);
   TRY(fhb::inverse(c, static_cast<const char*>(ct3) + 2 * comp, s.t0, batch * limbs, limbs, level,
                    fhb::kInvStandard, st));
@@ -910,11 +948,11 @@ int fhb_ckks_multiply_relinearize(const fhb_context* ctx, const void* a, const v
   const int64_t in_bytes = 2 * batch * limbs * c.n() * fhb::word_bytes(c);
   const int64_t out_bytes = 2 * batch * (limbs - (rescale ? 1 : 0)) * c.n() * fhb::word_bytes(c);
   const bool alias = ranges_overlap(out, out_bytes, a, in_bytes) || ranges_overlap(out, out_bytes, b, in_bytes);
-  if (k > 1 && cap == cudaStreamCaptureStatusNone && !(c.basis_tc && c.tc_moddown) && !alias)
+  const fhb::Scratch s = fhb::carve(c, scratch, batch, level, scratch_bytes);
+  if (k > 1 && cap == cudaStreamCaptureStatusNone && !ks_passes(c, s, level) && !alias)
     return multiply_relinearize_chunked(ctx, static_cast<const char*>(a), static_cast<const char*>(b), key,
                                         static_cast<char*>(out), static_cast<char*>(scratch), batch, level, rescale,
                                         st, k);
-  const fhb::Scratch s = fhb::carve(c, scratch, batch, level);
   const int64_t comp = batch * limbs * c.n() * fhb::word_bytes(c);
   // ct3 = a x b into the scratch (elementwise, every SM), then the
   // relinearisation of an NTT-domain ct3
@@ -1012,7 +1050,7 @@ int fhb_ckks_rotate_multi(const fhb_context* ctx, const void* ct, const uint64_t
   TRY(fhb::check_level(c, level));
   TRY(check_scratch(ctx, batch, level, scratch_bytes));
   const int limbs = c.num_q - level;
-  const fhb::Scratch s = fhb::carve(c, scratch, batch, level);
+  const fhb::Scratch s = fhb::carve(c, scratch, batch, level, scratch_bytes);
   const int64_t comp = batch * limbs * c.n() * fhb::word_bytes(c);
   TRY(FHB_WORD(fhb::modup, c, static_cast<const char*>(ct) + comp, s.digits, batch, level, 1u, st, galois));
   TRY(ks_core_from_digits(c, s, nullptr, batch, level, st, key_ptrs));
@@ -1086,11 +1124,11 @@ int fhb_ckks_rotate(const fhb_context* ctx, const void* ct, const void* key, voi
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
   TRY(fhb::cuda_status(cudaStreamIsCapturing(st, &cap), "capture status"));
   const int64_t ct_bytes = 2 * batch * limbs * c.n() * fhb::word_bytes(c);
-  if (k > 1 && cap == cudaStreamCaptureStatusNone && !(c.basis_tc && c.tc_moddown) &&
+  const fhb::Scratch s = fhb::carve(c, scratch, batch, level, scratch_bytes);
+  if (k > 1 && cap == cudaStreamCaptureStatusNone && !ks_passes(c, s, level) &&
       !ranges_overlap(out, ct_bytes, ct, ct_bytes))
     return rotate_chunked(ctx, static_cast<const char*>(ct), key, static_cast<char*>(out),
                           static_cast<char*>(scratch), batch, level, galois, st, k);
-  const fhb::Scratch s = fhb::carve(c, scratch, batch, level);
   const int64_t comp = batch * limbs * c.n() * fhb::word_bytes(c);
   TRY(FHB_WORD(fhb::modup, c, static_cast<const char*>(ct) + comp, s.digits, batch, level, galois, st));
   return keyswitch_tail(c, s, key, ct, nullptr, galois, out, batch, level, 0, st);

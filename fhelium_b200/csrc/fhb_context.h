@@ -12,6 +12,9 @@
 namespace fhb {
 
 constexpr int kMaxDigitWidth = 8;  // hybrid digit width bound (= P count)
+// Room for the key-switch core's intermediate that fhb_ckks_keyswitch_workspace_bytes
+// asks for at most (rows are processed in groups that fit it).
+constexpr int64_t kKsPassRoom = int64_t{1} << 30;
 constexpr int kMaxOverlapChunks = 8;  // chunks of the overlapped fused HMult
 
 // One active hybrid digit at one level.

@@ -711,7 +711,7 @@ struct U64RowSource {
   template <int C>
   __device__ __forceinline__ void column(int m, int stride, double (&x)[C]) const {
 #pragma unroll
-    for (int k = 0; k < C; ++k) x[k] = __ull2double_rn(in[k * stride + m]);
+    for (int k = 0; k < C; ++k) x[k] = Word<double>::from_word(in[k * stride + m]);
   }
 };
 
@@ -740,12 +740,12 @@ struct ExtSourceF64 {
 #pragma unroll
         for (int k = 0; k < C; ++k) {
           const uint64_t w = row[k * stride];
-          x[k] += W::shoup_bal(__ull2double_rn(w >> 30), hi.w, hi.wp, q);
-          x[k] += W::shoup_bal(__ull2double_rn(w & ((uint64_t{1} << 30) - 1)), lo.w, lo.wp, q);
+          x[k] += W::shoup_bal(W::from_word(w >> 30), hi.w, hi.wp, q);
+          x[k] += W::shoup_bal(W::from_word(w & ((uint64_t{1} << 30) - 1)), lo.w, lo.wp, q);
         }
       } else {
 #pragma unroll
-        for (int k = 0; k < C; ++k) x[k] += W::shoup_bal(__ull2double_rn(row[k * stride]), lo.w, lo.wp, q);
+        for (int k = 0; k < C; ++k) x[k] += W::shoup_bal(W::from_word(row[k * stride]), lo.w, lo.wp, q);
       }
     }
   }
@@ -757,7 +757,7 @@ struct F64InvEpilogue {
   double q, c, cs;
   __device__ __forceinline__ void operator()(int pos, double v) const {
     v = Word<double>::shoup_bal(v, c, cs, q);
-    dst[pos] = __double2ull_rz(v < 0.0 ? v + q : v);
+    dst[pos] = Word<double>::to_word(v < 0.0 ? v + q : v);
   }
 };
 

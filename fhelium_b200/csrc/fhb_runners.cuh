@@ -5,6 +5,7 @@
 #include <algorithm>
 #include "fhb_items.cuh"
 #include "fhb_kernels.cuh"
+#include "fhb_pass.cuh"
 
 namespace fhb {
 
@@ -141,6 +142,88 @@ int run_ks_core(const Context& c, const void* digits, const void* key, void* acc
   return launch_int(k_keyswitch_core<T, LOGN>);
 }
 
+template <typename... KArgs, typename... Args>
+int launch_blocks(void (*kernel)(KArgs...), int64_t blocks, int threads, size_t smem, cudaStream_t stream,
+                  Args... args) {
+  if (blocks <= 0) return 0;
+  if (blocks > 0x7fffffffLL) return fail(-6, "too many blocks for one launch");
+  if (smem > 48 * 1024) {
+    const int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(kernel), int(smem));
+    if (rc != 0) return rc;
+  }
+  kernel<<<unsigned(blocks), unsigned(threads), smem, stream>>>(static_cast<KArgs>(args)...);
+  return cuda_status(cudaGetLastError(), "pass launch");
+}
+
+// The three launches of one group of rows.
+template <typename T, int LOGN, bool SPLIT>
+int launch_ks_pass(const KsPass<T>& k, int digits, bool pre, cudaStream_t st) {
+  using G = ColGeom<T, LOGN>;
+  const int64_t polys = int64_t(digits) * k.batch * k.rows;
+  int rc = pre ? launch_blocks(k_ks_columns<T, LOGN, true, SPLIT>, polys * G::kTiles, G::kThreads, G::smem_bytes(), st, k)
+               : launch_blocks(k_ks_columns<T, LOGN, false, SPLIT>, polys * G::kTiles, G::kThreads, G::smem_bytes(), st, k);
+  if (rc != 0) return rc;
+  const int64_t slots = (int64_t(k.batch) << (LOGN - kBlkLog));
+  rc = launch_blocks(k_ks_rows<T, LOGN, SPLIT>, (slots + kRowSlots - 1) / kRowSlots * k.rows, kRowThreads, 0, st, k);
+  if (rc != 0) return rc;
+  return launch_blocks(k_ks_columns_inverse<T, LOGN, SPLIT>, int64_t(2) * k.batch * k.rows * G::kTiles, G::kThreads,
+                       G::smem_bytes(), st, k);
+}
+
+template <typename T, int LOGN>
+int run_ks_pass(const Context& c, const void* digits, void* y, int64_t y_words, const void* key, void* acc0,
+                void* acc1, int64_t batch, int level, cudaStream_t st, const uint64_t* item_keys, const void* ct3,
+                bool pre, int64_t ct3_pitch) {
+  const int ql = c.num_q - level, qpl = ql + c.num_p;
+  const int64_t n = c.n();
+  const int nd = level_tables<T>(c, level).num_digits;
+  if (ct3_pitch <= 0) ct3_pitch = batch * ql * n;
+  KsPass<T> k = {};
+  k.digits = static_cast<const T*>(digits);
+  k.y = static_cast<T*>(y);
+  k.key = static_cast<const T*>(key);
+  k.item_keys = reinterpret_cast<const unsigned long long*>(item_keys);
+  k.ct3_stride = ct3_pitch;
+  k.q_limbs = ql, k.qp_limbs = qpl, k.level = level, k.qp0 = c.qp();
+  k.f64_rows = sizeof(T) == 8 ? f64_rows(c, level, ql) : 0;
+  k.ext_digits = c.ext64f_digits, k.f64_end = c.f64_prime_end;
+  k.tabs = tables<T>(c), k.lt = level_tables<T>(c, level);
+  k.tabs64f = c.t64f, k.ext64f = c.ext64f;
+  // ciphertexts per group: all of them, unless the room holds fewer or the
+  // launch would pass the grid's limit
+  constexpr int64_t kMaxGroup = 4096;
+  const int64_t per_row = nd * n;  // words of one ciphertext's row
+  int64_t group = std::min(batch, kMaxGroup);
+  if (!pre) {
+    group = std::min(group, y_words / per_row);
+    if (group < 1) return fail(-8, "no room for the transform's intermediate");
+  }
+  for (int64_t b0 = 0; b0 < batch; b0 += group) {
+    k.batch = int(std::min(group, batch - b0));
+    k.y_batch = pre ? int(batch) : k.batch;
+    if (pre) k.y = static_cast<T*>(y) + b0 * qpl * n;
+    k.digits = static_cast<const T*>(digits) + b0 * ql * n;
+    k.acc0 = static_cast<T*>(acc0) + b0 * qpl * n;
+    k.acc1 = static_cast<T*>(acc1) + b0 * qpl * n;
+    k.ct3 = ct3 ? static_cast<const T*>(ct3) + b0 * ql * n : nullptr;
+    if (item_keys) k.item_keys = reinterpret_cast<const unsigned long long*>(item_keys) + b0;
+    const int step = pre ? qpl : int(std::min<int64_t>(qpl, y_words / (per_row * k.batch)));
+    for (int hi = qpl; hi > 0; hi -= step) {
+      k.rows = std::min(step, hi);
+      k.row_lo = hi - k.rows;
+      int rc = 0;
+      if constexpr (sizeof(T) == 8) {
+        rc = k.f64_rows > 0 ? launch_ks_pass<T, LOGN, true>(k, nd, pre, st) : launch_ks_pass<T, LOGN, false>(k, nd, pre, st);
+      } else {
+        if (pre) return fail(-7, "the tensor-core basis conversion needs an int64 context");
+        rc = launch_ks_pass<T, LOGN, false>(k, nd, false, st);
+      }
+      if (rc != 0) return rc;
+    }
+  }
+  return 0;
+}
+
 template <typename T, int LOGN>
 int run_ks_sum(const Context& c, const void* digits, const uint64_t* key_ptrs, void* acc0, void* acc1, int giants,
                int64_t batch, int level, cudaStream_t st, bool pre) {
@@ -253,6 +336,8 @@ int run_items(const Context& c, int stage, const void* items, int item_count, in
   template int run_inverse<T, LOGN>(const Context&, const void*, void*, int64_t, int, int, int, cudaStream_t);    \
   template int run_mul_coef<T, LOGN>(const Context&, const void*, const void*, void*, int64_t, int, cudaStream_t); \
   template int run_ks_core<T, LOGN>(const Context&, const void*, const void*, void*, void*, int64_t, int,        \
+                                    cudaStream_t, const uint64_t*, const void*, bool, int64_t);                 \
+  template int run_ks_pass<T, LOGN>(const Context&, const void*, void*, int64_t, const void*, void*, void*, int64_t, int, \
                                     cudaStream_t, const uint64_t*, const void*, bool, int64_t);                 \
   template int run_ks_sum<T, LOGN>(const Context&, const void*, const uint64_t*, void*, void*, int, int64_t, int, \
                                    cudaStream_t, bool);                                                         \

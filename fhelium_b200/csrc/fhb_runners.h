@@ -19,6 +19,15 @@ template <typename T, int LOGN>
 int run_ks_core(const Context& c, const void* digits, const void* key, void* acc0, void* acc1, int64_t batch,
                 int level, cudaStream_t st, const uint64_t* item_keys, const void* ct3, bool pre,
                 int64_t ct3_pitch = 0);
+// The key-switch core as launches of column and block stages (fhb_pass.cuh).
+// pre: `y` holds the extensions [D_l][B][QP_l][N] already (all rows in one
+// go).  Otherwise `y` has room for y_words words (at least one ciphertext's
+// digits of one row, ks_pass_min_words) and rows are processed in as few
+// groups as that allows.
+template <typename T, int LOGN>
+int run_ks_pass(const Context& c, const void* digits, void* y, int64_t y_words, const void* key, void* acc0,
+                void* acc1, int64_t batch, int level, cudaStream_t st, const uint64_t* item_keys, const void* ct3,
+                bool pre, int64_t ct3_pitch = 0);
 template <typename T, int LOGN>
 int run_ks_sum(const Context& c, const void* digits, const uint64_t* key_ptrs, void* acc0, void* acc1, int giants,
                int64_t batch, int level, cudaStream_t st, bool pre);

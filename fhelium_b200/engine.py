@@ -152,7 +152,7 @@ class CkksEngine:
         return torch.empty(shape, dtype=self.dtype, device=self.device)
 
     def _scratch_for(self, batch: int, level: int) -> tuple[torch.Tensor, int]:
-        nbytes = int(self.ctx.lib.fhb_ckks_keyswitch_scratch_bytes(self.ctx.handle, batch, level))
+        nbytes = int(self.ctx.lib.fhb_ckks_keyswitch_workspace_bytes(self.ctx.handle, batch, level))
         if self._scratch is None or self._scratch.numel() < nbytes:
             self._scratch = torch.empty(nbytes, dtype=torch.uint8, device=self.device)
         return self._scratch, nbytes

@@ -327,6 +327,14 @@ int fhb_rns_add_constant(const fhb_context* ctx, void* data, const void* constan
 /* Scratch bytes needed by fhb_ckks_relinearize / fhb_ckks_rotate. */
 int64_t fhb_ckks_keyswitch_scratch_bytes(const fhb_context* ctx, int64_t batch, int level);
 
+/* Scratch bytes with which they run fastest: fhb_ckks_keyswitch_scratch_bytes
+ * plus room (at most 1 GiB) for the intermediate of the key-switch core's
+ * transforms, which then run as column and block launches on every SM.  With
+ * less (down to fhb_ckks_keyswitch_scratch_bytes) the calls give the same
+ * results through smaller groups of rows or the one-launch cluster core.
+ * -1 for an invalid batch or level. */
+int64_t fhb_ckks_keyswitch_workspace_bytes(const fhb_context* ctx, int64_t batch, int level);
+
 /* HMult-result relinearisation (optionally fused with the rescale):
  * ct3 [3, batch, L, N] NTT/Montgomery -> out [2, batch, L (- 1), N]
  * coefficient/standard canonical.  Replaces CkksEngine.relinearize

@@ -1,0 +1,101 @@
+"""The key-switch core as column and block launches (fhb_pass.cuh), against the
+oracle, at every ring degree (each has its own split of the stages), with
+every amount of scratch the calls accept: exactly the required size (the
+one-launch cluster core), room for one ciphertext's digits of one row (groups
+of one ciphertext and one row), room for a few rows (an uneven last group)
+and the recommended size.  Whole numbers, no tolerance."""
+
+import numpy as np
+import pytest
+import torch
+
+from fhelium_b200 import _native as nat
+from fhelium_b200.config import CkksConfig, Preset
+from fhelium_b200.engine import CkksEngine
+from tests.helpers import oracle_for, random_key, reduced_ring, to_dev, to_np, uniform_residues
+
+pytestmark = pytest.mark.gpu
+
+# (preset, logN, level, batch): FP64 + integer rows, integer rows only, int32;
+# odd batches leave spare half warps in the last block
+CASES = [
+    ("slots8192_scale40_levels7_int64", 12, 4, 3),
+    ("slots8192_scale40_levels7_int64", 13, 0, 1),
+    ("slots8192_scale40_levels7_int64", 14, 6, 5),
+    ("slots16384_scale30_levels21_int64", 15, 18, 2),
+    ("slots16384_scale50_levels12_int64", 15, 10, 3),
+    ("slots32768_scale40_levels34_int64", 16, 33, 9),
+    ("slots65536_scale40_levels72_int64", 17, 70, 1),
+    ("slots65536_scale50_levels58_int64", 17, 57, 1),
+    ("slots8192_scale25_levels14_int32", 12, 10, 3),
+    ("slots16384_scale25_levels29_int32", 13, 27, 1),
+    ("slots16384_scale25_levels29_int32", 15, 26, 7),
+    ("slots32768_scale25_levels24_int32", 16, 22, 3),
+    ("slots65536_scale25_levels14_int32", 17, 12, 1),
+]
+
+
+def _engine(preset, log_n):
+    cfg = CkksConfig.parse(Preset[preset])
+    if log_n != cfg.logN:
+        cfg = reduced_ring(cfg, log_n)
+    return cfg, CkksEngine(cfg, basis_conversion="cuda_cores"), oracle_for(cfg, log_n)
+
+
+def _rooms(eng, cfg, level, batch):
+    lib, word = eng.ctx.lib, 8 if cfg.buffer_bit_length == 62 else 4
+    need = int(lib.fhb_ckks_keyswitch_scratch_bytes(eng.ctx.handle, batch, level))
+    full = int(lib.fhb_ckks_keyswitch_workspace_bytes(eng.ctx.handle, batch, level))
+    row = len(eng.level_digits[level]) * cfg.N * word
+    return [need, need + row, need + 3 * batch * row - 16, full]
+
+
+@pytest.mark.parametrize("preset,log_n,level,batch", CASES)
+def test_relinearize_every_ring_and_room(preset, log_n, level, batch):
+    cfg, eng, orc = _engine(preset, log_n)
+    rng = np.random.default_rng(log_n * 100 + level)
+    rows = orc.q_rows(level)
+    ct3 = uniform_residues(rng, cfg.moduli, rows, (3, batch), cfg.N, lazy=True)
+    key = random_key(rng, cfg, cfg.N)
+    want = np.stack([orc.relinearize(ct3[:, b], key, level) for b in range(batch)], axis=1)
+    d_ct3, d_key = to_dev(ct3, cfg), to_dev(key, cfg)
+    for room in _rooms(eng, cfg, level, batch):
+        out = torch.full((2, batch, len(rows), cfg.N), -1, dtype=cfg.torch_dtype, device="cuda")
+        scratch = torch.empty(room, dtype=torch.uint8, device="cuda")
+        eng.ctx.call("fhb_ckks_relinearize", nat.ptr(d_ct3), nat.ptr(d_key), nat.ptr(out), nat.ptr(scratch), room,
+                     batch, level, 0, eng._stream())
+        np.testing.assert_array_equal(to_np(out), want, err_msg=f"scratch {room}")
+
+
+@pytest.mark.parametrize("preset,log_n,level,batch", [CASES[2], CASES[4], CASES[10]])
+def test_rotations_with_their_own_keys_every_room(preset, log_n, level, batch):
+    cfg, eng, orc = _engine(preset, log_n)
+    rng = np.random.default_rng(5)
+    rows = orc.q_rows(level)
+    ct = uniform_residues(rng, cfg.moduli, rows, (2, batch), cfg.N)
+    steps = [1 + 3 * b for b in range(batch)]
+    keys = [random_key(rng, cfg, cfg.N) for _ in steps]
+    want = np.stack([orc.rotate(ct[:, b], steps[b], keys[b], level) for b in range(batch)], axis=1)
+    d_ct, d_keys = to_dev(ct, cfg), [to_dev(k, cfg) for k in keys]
+    ptrs = torch.tensor([k.data_ptr() for k in d_keys], dtype=torch.int64, device="cuda")
+    galois = torch.tensor([eng.galois_element_for_step(s) for s in steps], dtype=torch.int32, device="cuda")
+    for room in _rooms(eng, cfg, level, batch):
+        out = torch.full_like(d_ct, -1)
+        scratch = torch.empty(room, dtype=torch.uint8, device="cuda")
+        eng.ctx.call("fhb_ckks_rotate_multi", nat.ptr(d_ct), nat.ptr(ptrs), nat.ptr(galois), nat.ptr(out),
+                     nat.ptr(scratch), room, batch, level, eng._stream())
+        np.testing.assert_array_equal(to_np(out), want, err_msg=f"scratch {room}")
+
+
+def test_workspace_holds_the_required_scratch():
+    """The recommended size is never below the required one, and at most 1 GiB
+    (or one row of one ciphertext) above it."""
+    _, eng, _ = _engine("slots8192_scale40_levels7_int64", 14)
+    lib = eng.ctx.lib
+    for batch in (0, 1, 7, 64):
+        for level in range(eng.num_q):
+            need = int(lib.fhb_ckks_keyswitch_scratch_bytes(eng.ctx.handle, batch, level))
+            full = int(lib.fhb_ckks_keyswitch_workspace_bytes(eng.ctx.handle, batch, level))
+            assert need <= full <= need + (1 << 30)
+    assert int(lib.fhb_ckks_keyswitch_workspace_bytes(eng.ctx.handle, -1, 0)) == -1
+    assert int(lib.fhb_ckks_keyswitch_workspace_bytes(eng.ctx.handle, 1, eng.num_q)) == -1
