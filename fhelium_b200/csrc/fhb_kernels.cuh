@@ -932,338 +932,6 @@ k_keyswitch_sum(const T* __restrict__ digits, const unsigned long long* __restri
   tw.inverse(s, p, v, e1);
 }
 
-// Hoisting stage 1: materialise NTT-domain extended digits once
-// (fhelium/engine/hybrid_keyswitch.py:373-417).  prepared: [D_l, B, QP_l, N]
-// standard NTT-domain values in [0, 2p).  SPLIT (int64 chains with FP64
-// tables): the units of the leading f64_rows rows (primes below 2^42) run
-// the extension and the transform in balanced FP64 arithmetic, the others
-// the integer body, in one launch; both store lazy words in [0, 2p) (equal
-// modulo p, not word for word).
-template <typename T, int LOGN>
-__device__ __forceinline__ void prepare_unit(const T* __restrict__ digits, T* __restrict__ prepared, int64_t batch,
-                                             int q_limbs, int qp_limbs, int level, int qp0, const ChainTables<T>& tabs,
-                                             const LevelTables<T>& lt, int64_t bi, int jrow, unsigned char* smem_raw,
-                                             int rank) {
-  using G = NttGeom<T, LOGN>;
-  T* s = reinterpret_cast<T*>(smem_raw);
-  const int64_t poly = bi * qp_limbs + jrow;
-  const int pid = level + jrow;
-  const PrimeInfo<T> p = tabs.prime[pid];
-  const T* dig = digits + bi * q_limbs * int64_t(G::kN);
-  const int64_t own = int64_t(rank) * G::kM + threadIdx.x * G::kE;
-  KsTw<T, LOGN> tw(smem_raw, tabs.tw_fwd + int64_t(pid) * G::kN, tabs.tw_inv + int64_t(pid) * G::kN, rank);
-  tw.stage(false);
-  for (int a = 0; a < lt.num_digits; ++a) {
-    const DigitDesc d = lt.digits[a];
-    ExtSource<T> src{dig + (int64_t(d.prime0 - level) << LOGN), lt.ext + int64_t(a) * kMaxDigitWidth * qp0 + pid,
-                     qp0, d.alpha, LOGN, p.q, p.twice_q};
-    T v[G::kE];
-    tw.forward_from(src, s, p, v);
-#pragma unroll
-    for (int e = 0; e < G::kE; ++e) v[e] = csub(v[e], p.twice_q);
-    store16(prepared + (int64_t(a) * batch * qp_limbs + poly) * G::kN + own, v);
-  }
-}
-
-template <int LOGN>
-__device__ __forceinline__ void prepare_unit_f64(const uint64_t* __restrict__ digits, uint64_t* __restrict__ prepared,
-                                                 int64_t batch, int q_limbs, int qp_limbs, int level, int qp0,
-                                                 const ChainTables<double>& tabs, const LevelTables<uint64_t>& lt,
-                                                 const TwPair<double>* __restrict__ ext64f, int ext_digits,
-                                                 int f64_end, int64_t bi, int jrow, unsigned char* smem_raw,
-                                                 int rank) {
-  using G = NttGeom<double, LOGN>;
-  double* s = reinterpret_cast<double*>(smem_raw);
-  const int64_t poly = bi * qp_limbs + jrow;
-  const int pid = level + jrow;
-  const PrimeInfo<double> p = tabs.prime[pid];
-  const int64_t own = int64_t(rank) * G::kM + threadIdx.x * G::kE;
-  KsTw<double, LOGN> tw(smem_raw, tabs.tw_fwd + int64_t(pid) * G::kN, tabs.tw_inv + int64_t(pid) * G::kN, rank);
-  tw.stage(false);
-  for (int a = 0; a < lt.num_digits; ++a) {
-    const DigitDesc d = lt.digits[a];
-    ExtSourceF64 src{digits + (bi * q_limbs + (d.prime0 - level)) * int64_t(G::kN),
-                     ext64f + (((int64_t(level) * ext_digits + a) * kMaxDigitWidth) * 2) * qp0 + pid, qp0, d.alpha,
-                     LOGN, d.prime0 + d.alpha > f64_end, p.q, p.twice_q};
-    double v[G::kE];
-    tw.forward_from(src, s, p, v);
-#pragma unroll
-    for (int e = 0; e < G::kE; ++e) v[e] = Word<double>::to_lazy(v[e], p.q, p.one_s);
-    store_words(prepared + (int64_t(a) * batch * qp_limbs + poly) * G::kN + own, v);
-  }
-}
-
-template <typename T, int LOGN, bool SPLIT = false>
-__global__ void __launch_bounds__(NttGeom<T, LOGN>::kThreads)
-k_prepare_rotation(const T* __restrict__ digits, T* __restrict__ prepared, int64_t batch, int q_limbs,
-                   int qp_limbs, int level, int qp0, int order, ChainTables<T> tabs, LevelTables<T> lt,
-                   ChainTables<double> tabs64f, int f64_rows, const TwPair<double>* __restrict__ ext64f,
-                   int ext_digits, int f64_end) {
-  using G = NttGeom<T, LOGN>;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  const int rank = cluster_rank<T, LOGN>();
-  int64_t poly, bi;  // poly over [B, QP_l]
-  int jrow;
-  ks_work(blockIdx.x / G::kC, qp_limbs, batch, order, poly, bi, jrow);
-  if constexpr (SPLIT) {
-    static_assert(sizeof(T) == 8, "FP64 rows exist in int64 chains only");
-    if (jrow < f64_rows) {
-      prepare_unit_f64<LOGN>(reinterpret_cast<const uint64_t*>(digits), reinterpret_cast<uint64_t*>(prepared), batch,
-                             q_limbs, qp_limbs, level, qp0, tabs64f, lt, ext64f, ext_digits, f64_end, bi, jrow,
-                             smem_raw, rank);
-      return;
-    }
-  }
-  prepare_unit<T, LOGN>(digits, prepared, batch, q_limbs, qp_limbs, level, qp0, tabs, lt, bi, jrow, smem_raw, rank);
-}
-
-// The NTT-domain automorphism keeps a CTA's block whole: destination k's
-// CTA is given by the low log C bits of br(k), and the low log C bits of the
-// source's natural index depend only on those.  So the M destinations of
-// CTA `rank` read one contiguous block of M source words, which the CTA
-// copies into shared memory with 16-byte loads before gathering from it.
-template <typename T, int LOGN>
-__device__ __forceinline__ int galois_source_block(int rank, uint32_t galois) {
-  using G = NttGeom<T, LOGN>;
-  return galois_ntt_source(rank * G::kM, LOGN, galois) >> G::kLogM;
-}
-
-template <typename T, int LOGN>
-__device__ __forceinline__ void stage_block(T* dst, const T* src) {
-  using G = NttGeom<T, LOGN>;
-  constexpr int kVec = G::kM * int(sizeof(T)) / 16;
-  static_assert(kVec % G::kThreads == 0, "whole 16-byte vectors per thread");
-#pragma unroll
-  for (int i = threadIdx.x; i < kVec; i += G::kThreads)
-    reinterpret_cast<uint4*>(dst)[i] = __ldg(reinterpret_cast<const uint4*>(src) + i);
-}
-
-// Hoisting stage 2 for rings whose key-switch accumulators live outside
-// shared memory (N = 2^17): per rotation step, NTT-domain automorphism of the
-// prepared digits + key inner product + inverse NTT of both accumulators
-// (fhelium/engine/hybrid_keyswitch.py:419-469).  The automorphism gathers
-// from a staged copy of the source block (galois_source_block) in the NTT
-// working area, which is free until the inverse transform.  SPLIT: the units
-// of the leading f64_rows rows in balanced FP64 arithmetic (the key used as
-// stored, k R, and R removed with N^{-1} R^{-1}), the same canonical outputs.
-template <typename T, int LOGN, bool SPLIT = false>
-__global__ void __launch_bounds__(NttGeom<T, LOGN>::kThreads)
-k_apply_prepared_rotation_staged(const T* __restrict__ prepared, const T* __restrict__ key, T* __restrict__ acc0,
-                          T* __restrict__ acc1, int64_t batch, int qp_limbs, int level, int qp0,
-                          uint32_t galois, int order, ChainTables<T> tabs, LevelTables<T> lt,
-                          ChainTables<double> tabs64f, int f64_rows) {
-  using G = NttGeom<T, LOGN>;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  const int rank = cluster_rank<T, LOGN>();
-  int64_t poly, bi;
-  int jrow;
-  ks_work(blockIdx.x / G::kC, qp_limbs, batch, order, poly, bi, jrow);
-  (void)bi;
-  const int pid = level + jrow;
-  const int own = rank * G::kM + threadIdx.x * G::kE;
-  const int blk = galois ? galois_source_block<T, LOGN>(rank, galois) : rank;
-  T* staged = reinterpret_cast<T*>(smem_raw);  // the NTT working area, M words
-  if constexpr (SPLIT) {
-    static_assert(sizeof(T) == 8, "FP64 rows exist in int64 chains only");
-    if (jrow < f64_rows) {
-      double* s = reinterpret_cast<double*>(smem_raw);
-      const PrimeInfo<double> p = tabs64f.prime[pid];
-      const double q = p.q, qinv = p.one_s;
-      KsAcc<double, LOGN> acc(s, nullptr, nullptr);
-      KsTw<double, LOGN> tw(smem_raw, tabs64f.tw_fwd + int64_t(pid) * G::kN, tabs64f.tw_inv + int64_t(pid) * G::kN,
-                            rank);
-      for (int a = 0; a < lt.num_digits; ++a) {
-        const DigitDesc d = lt.digits[a];
-        const T* pr = prepared + (int64_t(a) * batch * qp_limbs + poly) * G::kN;
-        const T* key0 = key + ((int64_t(d.key_digit) * 2 + 0) * qp0 + pid) * G::kN + own;
-        const T* key1 = key + ((int64_t(d.key_digit) * 2 + 1) * qp0 + pid) * G::kN + own;
-        if (galois) {
-          __syncthreads();  // the previous digit's gathers are done
-          stage_block<T, LOGN>(staged, pr + int64_t(blk) * G::kM);
-          __syncthreads();
-        }
-#pragma unroll 4
-        for (int e = 0; e < G::kE; ++e) {
-          const T x = galois ? staged[galois_ntt_source(own + e, LOGN, galois) - blk * G::kM] : __ldg(pr + own + e);
-          acc.mac_f64(e, __ull2double_rn(x), __ull2double_rn(__ldg(key0 + e)), __ull2double_rn(__ldg(key1 + e)), q,
-                      qinv);
-        }
-      }
-      if (galois) __syncthreads();  // the inverse transform reuses the working area
-      tw.stage(true);
-      for (int c = 0; c < 2; ++c) {
-        double v[G::kE];
-        acc.get(c, v);
-#pragma unroll
-        for (int e = 0; e < G::kE; ++e) v[e] = Word<double>::reduce_bal(v[e], q, qinv);
-        F64InvEpilogue epi{reinterpret_cast<uint64_t*>(c ? acc1 : acc0) + poly * G::kN, q, p.ninv_rinv,
-                           p.ninv_rinv_s};
-        tw.inverse(s, p, v, epi);
-      }
-      return;
-    }
-  }
-  T* s = reinterpret_cast<T*>(smem_raw);
-  const PrimeInfo<T> p = tabs.prime[pid];
-  KsAcc<T, LOGN> acc(s, acc0 + poly * G::kN + own, acc1 + poly * G::kN + own);
-  KsTw<T, LOGN> tw(smem_raw, tabs.tw_fwd + int64_t(pid) * G::kN, tabs.tw_inv + int64_t(pid) * G::kN, rank);
-  for (int a = 0; a < lt.num_digits; ++a) {
-    const DigitDesc d = lt.digits[a];
-    const T* pr = prepared + (int64_t(a) * batch * qp_limbs + poly) * G::kN;
-    const T* key0 = key + ((int64_t(d.key_digit) * 2 + 0) * qp0 + pid) * G::kN + own;
-    const T* key1 = key + ((int64_t(d.key_digit) * 2 + 1) * qp0 + pid) * G::kN + own;
-    if (galois) {
-      __syncthreads();
-      stage_block<T, LOGN>(staged, pr + int64_t(blk) * G::kM);
-      __syncthreads();
-    }
-#pragma unroll 4
-    for (int e = 0; e < G::kE; ++e) {
-      const T x = galois ? staged[galois_ntt_source(own + e, LOGN, galois) - blk * G::kM] : __ldg(pr + own + e);
-      acc.mac(e, x, __ldg(key0 + e), __ldg(key1 + e), p);
-    }
-  }
-  if (galois) __syncthreads();
-  tw.stage(true);
-  T v[G::kE];
-  acc.get(0, v);
-  InvEpilogue<T> e0 = make_inv_epilogue<T>(acc0 + poly * G::kN, p, kInvStandard, false);
-  tw.inverse(s, p, v, e0);
-  acc.get(1, v);
-  InvEpilogue<T> e1 = make_inv_epilogue<T>(acc1 + poly * G::kN, p, kInvStandard, false);
-  tw.inverse(s, p, v, e1);
-}
-
-// Hoisting stage 2 with the accumulators in registers (rings whose key-
-// switch accumulators fit in shared memory, 8 residues per thread): thread
-// t of CTA `rank` accumulates destinations base + j * threads + t, so a
-// warp covers 32 consecutive destinations, whose sources under the
-// NTT-domain automorphism are a permutation of one aligned group of 32
-// (the low five bits of k become the top bits of br(k), and the odd g
-// permutes them): the gathers, like the key loads, are 256-byte coalesced
-// global loads, with no staging and no barrier in the digit loop.  The sums
-// then pass through shared memory once (padded, conflict-free) into the
-// thread-contiguous layout of the inverse transform.
-template <typename T, int LOGN>
-struct ApplyRegs {
-  using G = NttGeom<T, LOGN>;
-  static constexpr bool kOk = KsAcc<T, LOGN>::kSmem && G::kE == 8;
-};
-
-template <typename T, int LOGN>
-__device__ __forceinline__ void apply_transpose(unsigned char* smem_raw, const T (&a0)[NttGeom<T, LOGN>::kE],
-                                                const T (&a1)[NttGeom<T, LOGN>::kE], T* r1) {
-  using G = NttGeom<T, LOGN>;
-  T* w = reinterpret_cast<T*>(smem_raw);
-#pragma unroll
-  for (int j = 0; j < G::kE; ++j) {
-    w[G::sidx(j * G::kThreads + threadIdx.x)] = a0[j];
-    r1[G::sidx(j * G::kThreads + threadIdx.x)] = a1[j];
-  }
-  __syncthreads();
-}
-
-// Hoisting stage 2: per rotation step, NTT-domain automorphism of the
-// prepared digits + key inner product + inverse NTT of both accumulators
-// (fhelium/engine/hybrid_keyswitch.py:419-469).  SPLIT: the units of the
-// leading f64_rows rows in balanced FP64 arithmetic (the key used as stored,
-// k R, and R removed with N^{-1} R^{-1}), the same canonical outputs.
-template <typename T, int LOGN, bool SPLIT = false>
-__global__ void __launch_bounds__(NttGeom<T, LOGN>::kThreads)
-k_apply_prepared_rotation(const T* __restrict__ prepared, const T* __restrict__ key, T* __restrict__ acc0,
-                          T* __restrict__ acc1, int64_t batch, int qp_limbs, int level, int qp0,
-                          uint32_t galois, int order, ChainTables<T> tabs, LevelTables<T> lt,
-                          ChainTables<double> tabs64f, int f64_rows) {
-  using G = NttGeom<T, LOGN>;
-  static_assert(ApplyRegs<T, LOGN>::kOk, "register accumulators need the shared-memory accumulator room");
-  constexpr int E = G::kE;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  const int rank = cluster_rank<T, LOGN>();
-  int64_t poly, bi;
-  int jrow;
-  ks_work(blockIdx.x / G::kC, qp_limbs, batch, order, poly, bi, jrow);
-  (void)bi;
-  const int pid = level + jrow;
-  const int base = rank * G::kM;
-  // the second sum's transpose area: the key-switch accumulator room
-  T* r1 = reinterpret_cast<T*>(smem_raw) + G::kSmemElems;
-  if constexpr (SPLIT) {
-    static_assert(sizeof(T) == 8, "FP64 rows exist in int64 chains only");
-    if (jrow < f64_rows) {
-      const PrimeInfo<double> p = tabs64f.prime[pid];
-      const double q = p.q, qinv = p.one_s;
-      double a0[E], a1[E];
-#pragma unroll
-      for (int j = 0; j < E; ++j) a0[j] = a1[j] = 0.0;
-      for (int a = 0; a < lt.num_digits; ++a) {
-        const DigitDesc d = lt.digits[a];
-        const T* pr = prepared + (int64_t(a) * batch * qp_limbs + poly) * G::kN;
-        const T* key0 = key + ((int64_t(d.key_digit) * 2 + 0) * qp0 + pid) * G::kN;
-        const T* key1 = key + ((int64_t(d.key_digit) * 2 + 1) * qp0 + pid) * G::kN;
-#pragma unroll
-        for (int j = 0; j < E; ++j) {
-          const int dst = base + j * G::kThreads + int(threadIdx.x);
-          const int src = galois ? galois_ntt_source(dst, LOGN, galois) : dst;
-          const double x = __ull2double_rn(__ldg(pr + src));
-          a0[j] += Word<double>::mul_qinv_bal(x, __ull2double_rn(__ldg(key0 + dst)), q, qinv);
-          a1[j] += Word<double>::mul_qinv_bal(x, __ull2double_rn(__ldg(key1 + dst)), q, qinv);
-        }
-      }
-#pragma unroll
-      for (int j = 0; j < E; ++j) {
-        a0[j] = Word<double>::reduce_bal(a0[j], q, qinv);
-        a1[j] = Word<double>::reduce_bal(a1[j], q, qinv);
-      }
-      double* w = reinterpret_cast<double*>(smem_raw);
-      double* r1d = reinterpret_cast<double*>(r1);
-      apply_transpose<double, LOGN>(smem_raw, a0, a1, r1d);
-      KsTw<double, LOGN> tw(smem_raw, tabs64f.tw_fwd + int64_t(pid) * G::kN, tabs64f.tw_inv + int64_t(pid) * G::kN,
-                            rank);
-      tw.stage(true);
-      for (int c = 0; c < 2; ++c) {
-        double v[E];
-#pragma unroll
-        for (int e = 0; e < E; ++e) v[e] = (c ? r1d : w)[G::sidx(int(threadIdx.x) * E + e)];
-        if (c == 0) __syncthreads();  // every thread has its values before the transform reuses the area
-        F64InvEpilogue epi{reinterpret_cast<uint64_t*>(c ? acc1 : acc0) + poly * G::kN, q, p.ninv_rinv,
-                           p.ninv_rinv_s};
-        tw.inverse(w, p, v, epi);
-      }
-      return;
-    }
-  }
-  const PrimeInfo<T> p = tabs.prime[pid];
-  T a0[E], a1[E];
-#pragma unroll
-  for (int j = 0; j < E; ++j) a0[j] = a1[j] = 0;
-  for (int a = 0; a < lt.num_digits; ++a) {
-    const DigitDesc d = lt.digits[a];
-    const T* pr = prepared + (int64_t(a) * batch * qp_limbs + poly) * G::kN;
-    const T* key0 = key + ((int64_t(d.key_digit) * 2 + 0) * qp0 + pid) * G::kN;
-    const T* key1 = key + ((int64_t(d.key_digit) * 2 + 1) * qp0 + pid) * G::kN;
-#pragma unroll
-    for (int j = 0; j < E; ++j) {
-      const int dst = base + j * G::kThreads + int(threadIdx.x);
-      const int src = galois ? galois_ntt_source(dst, LOGN, galois) : dst;
-      const T x = __ldg(pr + src);
-      a0[j] = csub(a0[j] + Word<T>::mont(x, __ldg(key0 + dst), p.q, p.neg_inv), p.twice_q);
-      a1[j] = csub(a1[j] + Word<T>::mont(x, __ldg(key1 + dst), p.q, p.neg_inv), p.twice_q);
-    }
-  }
-  T* w = reinterpret_cast<T*>(smem_raw);
-  apply_transpose<T, LOGN>(smem_raw, a0, a1, r1);
-  KsTw<T, LOGN> tw(smem_raw, tabs.tw_fwd + int64_t(pid) * G::kN, tabs.tw_inv + int64_t(pid) * G::kN, rank);
-  tw.stage(true);
-  for (int c = 0; c < 2; ++c) {
-    T v[E];
-#pragma unroll
-    for (int e = 0; e < E; ++e) v[e] = (c ? r1 : w)[G::sidx(int(threadIdx.x) * E + e)];
-    if (c == 0) __syncthreads();
-    InvEpilogue<T> epi = make_inv_epilogue<T>((c ? acc1 : acc0) + poly * G::kN, p, kInvStandard, false);
-    tw.inverse(w, p, v, epi);
-  }
-}
-
 // ---------------------------------------------------------------------------
 // ModDown by P fused with the final addition and, optionally, the rescale by
 // the leading prime.  t0/t1: [B, QP_l, N] canonical coefficient rows;

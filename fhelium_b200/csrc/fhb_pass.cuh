@@ -76,6 +76,17 @@ struct ColGeom {
   static constexpr size_t smem_bytes() { return kPasses > 1 ? size_t(kTile) * sizeof(T) : 0; }
 };
 
+// Blocks per SM the column kernels are compiled for: two of 256 threads where
+// a thread holds the words of two rows (128 registers), otherwise 768 threads
+// (80 registers) for 64-bit words and 1024 for 32-bit words.  (Left to itself
+// the compiler takes 150 registers and the kernel 1.4 times as long.)
+template <typename T, int LOGN>
+constexpr int col_blocks(bool pairs) {
+  constexpr int kThreads = ColGeom<T, LOGN>::kThreads;
+  if (sizeof(T) == 4) return 1024 / kThreads;
+  return pairs ? 512 / kThreads : (kThreads > 256 ? 1 : 3);
+}
+
 template <typename T, int LOGN, class TW>
 struct Cols {
   using G = ColGeom<T, LOGN>;
@@ -92,10 +103,21 @@ struct Cols {
     row0 = (hi << (K + R)) | (rest & ((1 << R) - 1));
   }
 
+  template <int A, int K>
+  __device__ __forceinline__ static void fwd_stages(T (&x)[1 << K], const TW& tw, T q, T m2, int hi) {
+#pragma unroll
+    for (int b = 0; b < K; ++b) {
+      const int h = (1 << K) >> (b + 1);
+#pragma unroll
+      for (int i = 0; i < (1 << K); ++i)
+        if (!(i & h)) B::fwd_bfly(x[i], x[i + h], tw.at((1 << (A + b)) + (hi << b) + (i >> (K - b))), q, m2);
+    }
+  }
+
+  // Pass J: words from `src` (J = 0) or shared memory, to shared memory or (the last pass) to `sink`.
   template <int J, class Src, class Sink>
-  __device__ __forceinline__ static void fwd(Src& src, Sink& sink, T* s, const TW& tw, T q, T m2, int col0) {
+  __device__ __forceinline__ static void fwd_pass(Src& src, Sink& sink, T* s, const TW& tw, T q, T m2, int col0) {
     constexpr int K = G::pass_k(J), A = G::pass_a(J), R = G::kA - A - K, kGs = 1 << K;
-    constexpr bool kLast = J == G::kPasses - 1;
 #pragma unroll
     for (int u = 0; u < (16 >> K); ++u) {
       int row0, hi, col;
@@ -107,21 +129,20 @@ struct Cols {
 #pragma unroll
         for (int k = 0; k < kGs; ++k) x[k] = s[(row0 + (k << R)) * G::kCols + col];
       }
-#pragma unroll
-      for (int b = 0; b < K; ++b) {
-        const int h = kGs >> (b + 1);
-#pragma unroll
-        for (int i = 0; i < kGs; ++i)
-          if (!(i & h)) B::fwd_bfly(x[i], x[i + h], tw.at((1 << (A + b)) + (hi << b) + (i >> (K - b))), q, m2);
-      }
-      if constexpr (kLast) {
+      fwd_stages<A, K>(x, tw, q, m2, hi);
+      if constexpr (J == G::kPasses - 1) {
         sink.template column<kGs>(row0 * kBlk + col0 + col, kBlk << R, x);
       } else {
 #pragma unroll
         for (int k = 0; k < kGs; ++k) s[(row0 + (k << R)) * G::kCols + col] = x[k];
       }
     }
-    if constexpr (!kLast) {
+  }
+
+  template <int J, class Src, class Sink>
+  __device__ __forceinline__ static void fwd(Src& src, Sink& sink, T* s, const TW& tw, T q, T m2, int col0) {
+    fwd_pass<J>(src, sink, s, tw, q, m2, col0);
+    if constexpr (J + 1 < G::kPasses) {
       __syncthreads();
       fwd<J + 1>(src, sink, s, tw, q, m2, col0);
     }
@@ -265,6 +286,40 @@ struct RowX {
   }
 };
 
+// The next row of 256 words on its way into shared memory (cp.async, 16 bytes
+// a thread and piece) while the current one is transformed: half a warp owns
+// 256 words here, read back in the strided layout without bank conflicts.
+template <typename T>
+struct RowStage {
+  unsigned char* w;
+  int half, t;
+  __device__ __forceinline__ explicit RowStage(unsigned char* smem)
+      : w(smem + (threadIdx.x >> 5) * (2 * kBlk * sizeof(T))), half((threadIdx.x >> 4) & 1), t(threadIdx.x & 15) {}
+  __device__ __forceinline__ unsigned char* at(int word) const {
+    if constexpr (sizeof(T) == 8) return w + half * 2048 + word * 8;
+    return w + (word >> 4) * 128 + half * 64 + (word & 15) * 4;
+  }
+  __device__ __forceinline__ void request(const T* row) const {
+    constexpr int V = 16 / int(sizeof(T));
+#pragma unroll
+    for (int i = 0; i < 16 / V; ++i) {
+      const int word = (i * 16 + t) * V;
+      const unsigned dst = unsigned(__cvta_generic_to_shared(at(word)));
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(row + word) : "memory");
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  }
+  // Every thread's words of the requested row, strided layout.  The caller
+  // may request the next row afterwards.
+  __device__ __forceinline__ void take(T (&v)[16]) const {
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncwarp();
+#pragma unroll
+    for (int k = 0; k < 16; ++k) v[k] = *reinterpret_cast<const T*>(at(16 * k + t));
+    __syncwarp();
+  }
+};
+
 template <typename T, int LOGN, class TW>
 struct Rows {
   using B = Ntt<T, LOGN, TW>;
@@ -340,9 +395,12 @@ struct Rows {
 };
 
 // ---------------------------------------------------------------------------
-// Key switch.  Y holds, per (digit a, ciphertext b, row j) of the rows
-// [row_lo, row_lo + rows) in flight, the polynomial between the launches:
-// Y[(a y_batch + b) rows + j - row_lo][N].
+// Key switch.  The rows in flight are f_cnt FP64 rows from f_lo and i_cnt
+// integer rows from i_lo, dealt out evenly over the blocks (row_at), so that
+// blocks of both kinds share the SMs: the FP64 and the integer pipe then work
+// side by side.  Y holds, per (digit a, ciphertext b, row), the polynomial
+// between the launches: Y[(a y_batch + b) y_rows + slot][N], slot the row
+// itself (by_row: Y covers every row) or its place among the rows in flight.
 template <typename T>
 struct KsPass {
   const T* digits;      // ModUp digits [B, L, N]
@@ -353,12 +411,26 @@ struct KsPass {
   T* acc1;
   const T* ct3;         // relinearisation addends (nullable), components ct3_stride words apart
   int64_t ct3_stride;
-  int batch, y_batch, q_limbs, qp_limbs, level, qp0, row_lo, rows, f64_rows, ext_digits, f64_end;
+  int batch, y_batch, y_rows, by_row, q_limbs, qp_limbs, level, qp0, ext_digits, f64_end;
+  int f_lo, f_cnt, i_lo, i_cnt;
   ChainTables<T> tabs;
   LevelTables<T> lt;
   ChainTables<double> tabs64f;
   const TwPair<double>* ext64f;
+  __host__ __device__ int rows() const { return f_cnt + i_cnt; }
+  __device__ __forceinline__ T* y_poly(int a, int bi, int jrow, bool f64, int log_n) const {
+    const int slot = by_row ? jrow : (f64 ? jrow - f_lo : f_cnt + jrow - i_lo);
+    return y + (((int64_t(a) * y_batch + bi) * y_rows + slot) << log_n);
+  }
 };
+
+// Unit p of `total` of which `ints` are integer ones, spread evenly: true and
+// the index among the integer ones, or false and the index among the others.
+__device__ __forceinline__ bool ks_unit(int p, int total, int ints, int& index) {
+  const int before = int(unsigned(p * ints) / unsigned(total)), after = int(unsigned((p + 1) * ints) / unsigned(total));
+  index = after > before ? before : p - before;
+  return after > before;
+}
 
 // True when row pid's own digit residue replaces the transform (relinearisation).
 template <typename T>
@@ -367,50 +439,179 @@ __device__ __forceinline__ bool ks_own(const KsPass<T>& k, const DigitDesc& d, i
   return k.ct3 != nullptr && jrow < k.q_limbs && pid >= d.prime0 && pid < d.prime0 + d.alpha;
 }
 
+// Exact extension of a digit of at most four primes below 2^42 to a prime
+// p < 2^42, in FP64: d_0 + sum_{r >= 1} d_r M_r (M_0 = 1) with one reduction.
+// The products are summed in T on top of 1.5 2^88, so every T is a multiple
+// of 2^36 in one binade (the sum stays below 2^87): the differences of
+// successive T are exact, and d_r M_r minus that difference, at most 2^35 in
+// magnitude, is exact too (fma).  With H the sum of the differences,
+// H - rint(H / p) p lies in (-0.51 p, 0.51 p) and the result below
+// 0.51 p + 2^42 + 2^37.  14 operations for four primes, where a reduction per
+// product takes 27.
+template <int ALPHA>
+__device__ __forceinline__ double ext_chain(const double (&d)[ALPHA], const double (&m)[4], double q, double qinv) {
+  if constexpr (ALPHA == 1) return d[0];
+  constexpr double kBig = 1.5 * 309485009821345068724781056.0;  // 1.5 2^88
+  double t = kBig, low = d[0];
+#pragma unroll
+  for (int r = 1; r < ALPHA; ++r) {
+    const double next = fma(d[r], m[r], t);
+    low += fma(d[r], m[r], t - next);
+    t = next;
+  }
+  const double h = t - kBig;
+  return fma(-Word<double>::mul_round(h, qinv), q, h) + low;
+}
+
+// The extensions to two primes of 16 words `stride` apart.
+template <int ALPHA, int LOGN>
+__device__ __forceinline__ void ext_pair(const uint64_t* __restrict__ p, int stride, const double (&m0)[4],
+                                         const double (&m1)[4], double q0, double qi0, double q1, double qi1,
+                                         double (&x0)[16], double (&x1)[16]) {
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    uint64_t w[ALPHA][8];
+#pragma unroll
+    for (int r = 0; r < ALPHA; ++r)
+#pragma unroll
+      for (int e = 0; e < 8; ++e) w[r][e] = __ldg(p + (int64_t(r) << LOGN) + (h * 8 + e) * stride);
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      double d[ALPHA];
+#pragma unroll
+      for (int r = 0; r < ALPHA; ++r) d[r] = Word<double>::from_word(w[r][e]);
+      x0[h * 8 + e] = ext_chain<ALPHA>(d, m0, q0, qi0);
+      x1[h * 8 + e] = ext_chain<ALPHA>(d, m1, q1, qi1);
+    }
+  }
+}
+
+// A column source that hands out 16 words already in registers.
+struct RegSource {
+  const double (&v)[16];
+  template <int C>
+  __device__ __forceinline__ void column(int, int, double (&x)[C]) const {
+    static_assert(C == 16, "one group of 16 words per thread");
+#pragma unroll
+    for (int k = 0; k < C; ++k) x[k] = v[k];
+  }
+};
+
+// Two FP64 rows of one (digit, ciphertext, column tile): the digit's words
+// are loaded and converted once for both.  Rows not live (own-digit rows, the
+// missing partner of an odd row) are not transformed.
+template <int LOGN>
+__device__ __forceinline__ void ks_columns_pair(const KsPass<uint64_t>& k, const DigitDesc& d, int a, int bi, int col0,
+                                                int j0, int j1, bool live0, bool live1, double* s) {
+  using G = ColGeom<uint64_t, LOGN>;
+  using C = Cols<double, LOGN, TwAtQ>;
+  constexpr int64_t kN = int64_t(1) << LOGN;
+  if (!live0) j0 = j1;
+  if (!live1) j1 = j0;
+  const int p0 = k.level + j0, p1 = k.level + j1;
+  const double q0 = k.tabs64f.prime[p0].q, qi0 = k.tabs64f.prime[p0].one_s;
+  const double q1 = k.tabs64f.prime[p1].q, qi1 = k.tabs64f.prime[p1].one_s;
+  const TwPair<double>* ext = k.ext64f + (((int64_t(k.level) * k.ext_digits + a) * kMaxDigitWidth) * 2 + 1) * k.qp0;
+  double m0[4], m1[4];
+#pragma unroll
+  for (int r = 1; r < 4; ++r) {
+    m0[r] = r < d.alpha ? ext[int64_t(2 * r) * k.qp0 + p0].w : 0.0;
+    m1[r] = r < d.alpha ? ext[int64_t(2 * r) * k.qp0 + p1].w : 0.0;
+  }
+  m0[0] = m1[0] = 1.0;
+  int row0, hi, col;
+  C::template group<4, G::kA - 4>(0, row0, hi, col);
+  const uint64_t* p = k.digits + (int64_t(bi) * k.q_limbs + (d.prime0 - k.level)) * kN + row0 * kBlk + col0 + col;
+  constexpr int kStride = kBlk << (G::kA - 4);
+  double x0[16], x1[16];
+  if (d.alpha == 4) {
+    ext_pair<4, LOGN>(p, kStride, m0, m1, q0, qi0, q1, qi1, x0, x1);
+  } else if (d.alpha == 3) {
+    ext_pair<3, LOGN>(p, kStride, m0, m1, q0, qi0, q1, qi1, x0, x1);
+  } else if (d.alpha == 2) {
+    ext_pair<2, LOGN>(p, kStride, m0, m1, q0, qi0, q1, qi1, x0, x1);
+  } else {
+    ext_pair<1, LOGN>(p, kStride, m0, m1, q0, qi0, q1, qi1, x0, x1);
+  }
+  const TwAtQ tw0{k.tabs64f.twv_fwd + int64_t(p0) * kN, qi0}, tw1{k.tabs64f.twv_fwd + int64_t(p1) * kN, qi1};
+  ColSink<double> sink0{reinterpret_cast<double*>(k.y_poly(a, bi, j0, true, LOGN))};
+  ColSink<double> sink1{reinterpret_cast<double*>(k.y_poly(a, bi, j1, true, LOGN))};
+  RegSource r0{x0}, r1{x1};
+  double* s1 = s + G::kTile;
+  if (live0) C::template fwd_pass<0>(r0, sink0, s, tw0, q0, qi0, col0);
+  if (live1) C::template fwd_pass<0>(r1, sink1, s1, tw1, q1, qi1, col0);
+  if constexpr (G::kPasses > 1) {
+    __syncthreads();
+    if (live0) C::template fwd_pass<1>(r0, sink0, s, tw0, q0, qi0, col0);
+    if (live1) C::template fwd_pass<1>(r1, sink1, s1, tw1, q1, qi1, col0);
+  }
+}
+
+template <typename T, int LOGN>
+constexpr size_t ks_columns_smem(bool split) {
+  return ColGeom<T, LOGN>::smem_bytes() * (split && ColGeom<T, LOGN>::kPasses <= 2 ? 2 : 1);
+}
+
 // Launch 1: extension of a digit to a row's prime and the column stages of
-// its forward transform.  One block per (digit, ciphertext, column tile, row),
-// rows fastest, so the blocks in flight share the digit's words in L2.  PRE:
-// Y already holds the extensions (tensor-core basis conversion), transformed
-// in place.
+// its forward transform.  One block per (digit, ciphertext, column tile, two
+// FP64 rows or one integer row), rows fastest, so the blocks in flight share
+// the digit's words in L2.  PRE: Y already holds the extensions (tensor-core
+// basis conversion), transformed in place.
 template <typename T, int LOGN, bool PRE, bool SPLIT>
-__global__ void __launch_bounds__(ColGeom<T, LOGN>::kThreads)
+__global__ void __launch_bounds__(ColGeom<T, LOGN>::kThreads, col_blocks<T, LOGN>(SPLIT && !PRE))
 k_ks_columns(const __grid_constant__ KsPass<T> k) {
   using G = ColGeom<T, LOGN>;
   constexpr int64_t kN = int64_t(1) << LOGN;
   extern __shared__ __align__(16) unsigned char smem_raw[];
+  const int units = (k.f_cnt + 1) / 2 + k.i_cnt;
   unsigned idx = blockIdx.x;
-  const int jrow = k.row_lo + k.rows - 1 - int(idx % unsigned(k.rows));
-  idx /= unsigned(k.rows);
+  int at;
+  const bool is_int = ks_unit(int(idx % unsigned(units)), units, k.i_cnt, at);
+  idx /= unsigned(units);
   const int col0 = int(idx % G::kTiles) * G::kCols;
   idx /= G::kTiles;
   const int bi = int(idx % unsigned(k.batch)), a = int(idx / unsigned(k.batch));
   const DigitDesc d = k.lt.digits[a];
-  if (ks_own(k, d, jrow)) return;
-  const int pid = k.level + jrow;
-  T* y = k.y + ((int64_t(a) * k.y_batch + bi) * k.rows + (jrow - k.row_lo)) * kN;
-  const T* dig = k.digits + (int64_t(bi) * k.q_limbs + (d.prime0 - k.level)) * kN;
   if constexpr (SPLIT) {
     static_assert(sizeof(T) == 8, "FP64 rows exist in int64 chains only");
-    if (jrow < k.f64_rows) {
-      using C = Cols<double, LOGN, TwAtQ>;
-      const double q = k.tabs64f.prime[pid].q, qinv = k.tabs64f.prime[pid].one_s;
-      ColSink<double> sink{reinterpret_cast<double*>(y)};
+    if (!is_int) {
+      const int j0 = k.f_lo + 2 * at, j1 = j0 + 1;
+      const bool live0 = !ks_own(k, d, j0), live1 = 2 * at + 1 < k.f_cnt && !ks_own(k, d, j1);
+      if (!live0 && !live1) return;
       double* s = reinterpret_cast<double*>(smem_raw);
-      const TwAtQ tw{k.tabs64f.twv_fwd + int64_t(pid) * kN, qinv};
-      if constexpr (PRE) {
-        U64RowSource src{reinterpret_cast<const uint64_t*>(y)};
-        C::template fwd<0>(src, sink, s, tw, q, qinv, col0);
-      } else {
-        ExtSourceF64 src{reinterpret_cast<const uint64_t*>(dig),
-                         k.ext64f + (((int64_t(k.level) * k.ext_digits + a) * kMaxDigitWidth) * 2) * k.qp0 + pid,
-                         k.qp0, d.alpha, LOGN, d.prime0 + d.alpha > k.f64_end, q, qinv};
-        C::template fwd<0>(src, sink, s, tw, q, qinv, col0);
+      if constexpr (!PRE && G::kPasses <= 2) {
+        if (d.alpha <= 4 && d.prime0 + d.alpha <= k.f64_end) {
+          ks_columns_pair<LOGN>(k, d, a, bi, col0, j0, j1, live0, live1, s);
+          return;
+        }
+      }
+      using C = Cols<double, LOGN, TwAtQ>;
+      for (int i = 0; i < 2; ++i) {
+        const int jrow = i ? j1 : j0, pid = k.level + jrow;
+        if (!(i ? live1 : live0)) continue;
+        if (i) __syncthreads();  // the first row's words have been read
+        const double q = k.tabs64f.prime[pid].q, qinv = k.tabs64f.prime[pid].one_s;
+        uint64_t* y = k.y_poly(a, bi, jrow, true, LOGN);
+        ColSink<double> sink{reinterpret_cast<double*>(y)};
+        const TwAtQ tw{k.tabs64f.twv_fwd + int64_t(pid) * kN, qinv};
+        if constexpr (PRE) {
+          U64RowSource src{y};
+          C::template fwd<0>(src, sink, s, tw, q, qinv, col0);
+        } else {
+          ExtSourceF64 src{k.digits + (int64_t(bi) * k.q_limbs + (d.prime0 - k.level)) * kN,
+                           k.ext64f + (((int64_t(k.level) * k.ext_digits + a) * kMaxDigitWidth) * 2) * k.qp0 + pid,
+                           k.qp0, d.alpha, LOGN, d.prime0 + d.alpha > k.f64_end, q, qinv};
+          C::template fwd<0>(src, sink, s, tw, q, qinv, col0);
+        }
       }
       return;
     }
   }
+  const int jrow = k.i_lo + at, pid = k.level + jrow;
+  if (ks_own(k, d, jrow)) return;
   using C = Cols<T, LOGN, TwAt<T>>;
   const T q = k.tabs.prime[pid].q, twoq = k.tabs.prime[pid].twice_q;
+  T* y = k.y_poly(a, bi, jrow, false, LOGN);
   ColSink<T> sink{y};
   T* s = reinterpret_cast<T*>(smem_raw);
   const TwAt<T> tw{k.tabs.tw_fwd + int64_t(pid) * kN};
@@ -418,9 +619,28 @@ k_ks_columns(const __grid_constant__ KsPass<T> k) {
     ColSource<T> src{y};
     C::template fwd<0>(src, sink, s, tw, q, twoq, col0);
   } else {
-    ExtSource<T> src{dig, k.lt.ext + int64_t(a) * kMaxDigitWidth * k.qp0 + pid, k.qp0, d.alpha, LOGN, q, twoq};
+    ExtSource<T> src{k.digits + (int64_t(bi) * k.q_limbs + (d.prime0 - k.level)) * kN,
+                     k.lt.ext + int64_t(a) * kMaxDigitWidth * k.qp0 + pid, k.qp0, d.alpha, LOGN, q, twoq};
     C::template fwd<0>(src, sink, s, tw, q, twoq, col0);
   }
+}
+
+// x k 2^-W mod q (W the word's bits) in (0, 2q) for x < 4q, k < 2q: one
+// high product and a subtraction instead of the masked carries of a
+// reduction by R = 2^(W - 2); qi = q^{-1} mod 2^W.
+__device__ __forceinline__ uint64_t redc_word(uint64_t x, uint64_t k, uint64_t q, uint64_t qi) {
+  const unsigned __int128 p = static_cast<unsigned __int128>(x) * k;
+  return uint64_t(p >> 64) - __umul64hi(uint64_t(p) * qi, q) + q;
+}
+__device__ __forceinline__ uint32_t redc_word(uint32_t x, uint32_t k, uint32_t q, uint32_t qi) {
+  const uint64_t p = static_cast<uint64_t>(x) * k;
+  return uint32_t(p >> 32) - __umulhi(uint32_t(p) * qi, q) + q;
+}
+// q^{-1} mod 2^W from -q^{-1} mod 2^(W - 2) (one Newton step doubles the bits)
+template <typename T>
+__device__ __forceinline__ T inverse_pow2(T q, T neg_inv) {
+  const T x = T(0) - neg_inv;
+  return x * (T(2) - q * x);
 }
 
 // Launch 2: for one row of 256 words of (ciphertext, row j): the block stages
@@ -442,6 +662,12 @@ __device__ __forceinline__ void ks_rows_f64(const KsPass<uint64_t>& k, int jrow,
   const uint64_t* key = k.item_keys ? reinterpret_cast<const uint64_t*>(k.item_keys[bi]) : k.key;
   const uint64_t* ct3 = k.ct3 ? k.ct3 + (int64_t(bi) * k.q_limbs + jrow) * kN + vec : nullptr;
   const TwAtQ twf{k.tabs64f.twv_fwd + int64_t(pid) * kN, qinv};
+  const RowStage<double> stage(smem + kRowSlots * kBlk * sizeof(double));
+  auto request = [&](int a) {  // digit a's row, unless its residue is the ciphertext's own
+    if (a < k.lt.num_digits && !ks_own(k, k.lt.digits[a], jrow))
+      stage.request(reinterpret_cast<const double*>(k.y_poly(a, bi, jrow, true, LOGN)) + blk * kBlk);
+  };
+  request(0);
   double a0[16], a1[16];
 #pragma unroll
   for (int e = 0; e < 16; ++e) a0[e] = a1[e] = 0.0;
@@ -455,11 +681,10 @@ __device__ __forceinline__ void ks_rows_f64(const KsPass<uint64_t>& k, int jrow,
         v[2 * e] = W::shoup_bal(W::from_word(w.x), p.rinv, p.rinv_s, q);
         v[2 * e + 1] = W::shoup_bal(W::from_word(w.y), p.rinv, p.rinv_s, q);
       }
+      request(a + 1);
     } else {
-      const double* y = reinterpret_cast<const double*>(k.y) +
-                        ((int64_t(a) * k.y_batch + bi) * k.rows + (jrow - k.row_lo)) * kN + blk * kBlk + x.t;
-#pragma unroll
-      for (int e = 0; e < 16; ++e) v[e] = __ldg(y + 16 * e);
+      stage.take(v);
+      request(a + 1);
       R::fwd(v, x, twf, q, qinv, blk);
       R::contiguous_to_vector(v, x);
     }
@@ -521,6 +746,13 @@ __device__ __forceinline__ void ks_rows_int(const KsPass<T>& k, int jrow, int bi
     return r;
   };
   const TwAt<T> twf{k.tabs.tw_fwd + int64_t(pid) * kN};
+  const RowStage<T> stage(smem + kRowSlots * kBlk * sizeof(T));
+  auto request = [&](int a) {
+    if (a < k.lt.num_digits && !ks_own(k, k.lt.digits[a], jrow))
+      stage.request(k.y_poly(a, bi, jrow, false, LOGN) + blk * kBlk);
+  };
+  request(0);
+  const T qi = inverse_pow2(q, ni);
   T a0[16], a1[16];
 #pragma unroll
   for (int e = 0; e < 16; ++e) a0[e] = a1[e] = 0;
@@ -534,11 +766,10 @@ __device__ __forceinline__ void ks_rows_int(const KsPass<T>& k, int jrow, int bi
 #pragma unroll
         for (int i = 0; i < X::V; ++i) v[e * X::V + i] = W::shoup(w.v[i], p.rinv, p.rinv_s, q);
       }
+      request(a + 1);
     } else {
-      const T* y =
-          k.y + ((int64_t(a) * k.y_batch + bi) * k.rows + (jrow - k.row_lo)) * kN + blk * kBlk + x.t;
-#pragma unroll
-      for (int e = 0; e < 16; ++e) v[e] = __ldg(y + 16 * e);
+      stage.take(v);
+      request(a + 1);
       R::fwd(v, x, twf, q, twoq, blk);
       R::contiguous_to_vector(v, x);
     }
@@ -550,14 +781,18 @@ __device__ __forceinline__ void ks_rows_int(const KsPass<T>& k, int jrow, int bi
 #pragma unroll
       for (int i = 0; i < X::V; ++i) {
         const int at = e * X::V + i;
-        const T y = csub(v[at], twoq);
-        a0[at] = csub(a0[at] + W::mont(y, u0.v[i], q, ni), twoq);
-        a1[at] = csub(a1[at] + W::mont(y, u1.v[i], q, ni), twoq);
+        a0[at] = csub(a0[at] + redc_word(v[at], u0.v[i], q, qi), twoq);
+        a1[at] = csub(a1[at] + redc_word(v[at], u1.v[i], q, qi), twoq);
       }
     }
   }
   const TwAt<T> twi{k.tabs.tw_inv + int64_t(pid) * kN};
   auto finish = [&](T (&v)[16], const T* add, T* out) {
+#pragma unroll
+    for (int e = 0; e < 16; ++e) {  // x 4: the products were reduced by 2^W, not by R = 2^(W - 2)
+      v[e] = csub(v[e] + v[e], twoq);
+      v[e] = csub(v[e] + v[e], twoq);
+    }
     if (add) {
       const TwPair<T> ps = k.tabs.p_rinv[pid];
 #pragma unroll
@@ -584,24 +819,28 @@ __device__ __forceinline__ void ks_rows_int(const KsPass<T>& k, int jrow, int bi
 
 template <typename T>
 constexpr size_t row_smem() {
-  return size_t(kRowSlots) * kBlk * sizeof(T);
+  return size_t(2 * kRowSlots) * kBlk * sizeof(T);  // exchanges and the next rows
 }
 
 template <typename T, int LOGN, bool SPLIT>
-__global__ void __launch_bounds__(kRowThreads, 4)
+__global__ void __launch_bounds__(kRowThreads, sizeof(T) == 8 ? 3 : 4)
 k_ks_rows(const __grid_constant__ KsPass<T> k) {
   __shared__ __align__(16) unsigned char smem[row_smem<T>()];
   constexpr int kBlks = 1 << (LOGN - kBlkLog);
   const unsigned slots = unsigned(kBlks) * unsigned(k.batch);
+  // rows one after the other: the blocks in flight share a row's keys and
+  // twiddles (all rows side by side measured 6 % slower)
   const unsigned per_row = (slots + kRowSlots - 1) / kRowSlots;
-  const int jrow = k.row_lo + k.rows - 1 - int(blockIdx.x / per_row);
-  unsigned slot = (blockIdx.x % per_row) * kRowSlots + (threadIdx.x >> 4);
+  int at;
+  const bool is_int = ks_unit(int(blockIdx.x / per_row), k.rows(), k.i_cnt, at);
+  const int jrow = at + (is_int ? k.i_lo : k.f_lo);
+  unsigned slot = blockIdx.x % per_row * kRowSlots + (threadIdx.x >> 4);
   const bool live = slot < slots;
   if (!live) slot = slots - 1;  // the last block's spare half warps repeat a row and store nothing
   const int bi = int(slot % unsigned(k.batch)), blk = int(slot / unsigned(k.batch));
   if constexpr (SPLIT) {
     static_assert(sizeof(T) == 8, "FP64 rows exist in int64 chains only");
-    if (jrow < k.f64_rows) {
+    if (!is_int) {
       ks_rows_f64<LOGN>(k, jrow, bi, blk, live, smem);
       return;
     }
@@ -613,7 +852,7 @@ k_ks_rows(const __grid_constant__ KsPass<T> k) {
 // accumulator rows, to canonical coefficients.  One block per (component,
 // ciphertext, row, column tile).
 template <typename T, int LOGN, bool SPLIT>
-__global__ void __launch_bounds__(ColGeom<T, LOGN>::kThreads)
+__global__ void __launch_bounds__(ColGeom<T, LOGN>::kThreads, col_blocks<T, LOGN>(false))
 k_ks_columns_inverse(const __grid_constant__ KsPass<T> k) {
   using G = ColGeom<T, LOGN>;
   constexpr int64_t kN = int64_t(1) << LOGN;
@@ -621,13 +860,15 @@ k_ks_columns_inverse(const __grid_constant__ KsPass<T> k) {
   unsigned idx = blockIdx.x;
   const int col0 = int(idx % G::kTiles) * G::kCols;
   idx /= G::kTiles;
-  const int jrow = k.row_lo + k.rows - 1 - int(idx % unsigned(k.rows));
-  idx /= unsigned(k.rows);
+  int at;
+  const bool is_int = ks_unit(int(idx % unsigned(k.rows())), k.rows(), k.i_cnt, at);
+  const int jrow = at + (is_int ? k.i_lo : k.f_lo);
+  idx /= unsigned(k.rows());
   const int bi = int(idx % unsigned(k.batch));
   T* z = (idx / unsigned(k.batch) ? k.acc1 : k.acc0) + (int64_t(bi) * k.qp_limbs + jrow) * kN;
   const int pid = k.level + jrow;
   if constexpr (SPLIT) {
-    if (jrow < k.f64_rows) {
+    if (!is_int) {
       const PrimeInfo<double>& p = k.tabs64f.prime[pid];
       ColSource<double> src{reinterpret_cast<double*>(z)};
       F64InvEpilogue epi{reinterpret_cast<uint64_t*>(z), p.q, p.ninv_rinv, p.ninv_rinv_s};
@@ -642,6 +883,311 @@ k_ks_columns_inverse(const __grid_constant__ KsPass<T> k) {
   InvEpilogue<T> epi{z, p.q, p.ninv, p.ninv_s, kInvStandard};
   Cols<T, LOGN, TwAt<T>>::template inv<0>(src, epi, reinterpret_cast<T*>(smem_raw),
                                           TwAt<T>{k.tabs.tw_inv + int64_t(pid) * kN}, p.q, p.twice_q, col0);
+}
+
+// ---------------------------------------------------------------------------
+// Standalone transforms of polynomials [polys][N], poly p of row p mod rows
+// (prime row_start + row); the leading f64_rows rows of every group in FP64.
+// Both directions hold the intermediate in `out`.
+template <bool TO_MONT>
+struct WordSource {  // 64-bit words of a prime below 2^42 as balanced doubles
+  const uint64_t* in;
+  double c, cs, q;
+  template <int C>
+  __device__ __forceinline__ void column(int m, int stride, double (&x)[C]) const {
+#pragma unroll
+    for (int k = 0; k < C; ++k) {
+      x[k] = Word<double>::from_word(in[k * stride + m]);
+      if constexpr (TO_MONT) x[k] = Word<double>::shoup_bal(x[k], c, cs, q);
+    }
+  }
+};
+
+template <typename T, int LOGN, bool TO_MONT, bool SPLIT>
+__global__ void __launch_bounds__(ColGeom<T, LOGN>::kThreads, col_blocks<T, LOGN>(false))
+k_ntt_columns(const T* in, T* out, int rows, int row_start, ChainTables<T> tabs, ChainTables<double> tabs64f,
+              int f64_rows) {
+  using G = ColGeom<T, LOGN>;
+  constexpr int64_t kN = int64_t(1) << LOGN;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const int col0 = int(blockIdx.x % G::kTiles) * G::kCols;
+  const int64_t poly = blockIdx.x / G::kTiles;
+  const int row = int(poly % rows), pid = row_start + row;
+  if constexpr (SPLIT) {
+    if (row < f64_rows) {
+      const PrimeInfo<double>& p = tabs64f.prime[pid];
+      WordSource<TO_MONT> src{in + poly * kN, p.rmod, p.rmod_s, p.q};
+      ColSink<double> sink{reinterpret_cast<double*>(out + poly * kN)};
+      Cols<double, LOGN, TwAtQ>::template fwd<0>(src, sink, reinterpret_cast<double*>(smem_raw),
+                                                 TwAtQ{tabs64f.twv_fwd + int64_t(pid) * kN, p.one_s}, p.q, p.one_s,
+                                                 col0);
+      return;
+    }
+  }
+  const PrimeInfo<T>& p = tabs.prime[pid];
+  RowSource<T, TO_MONT> src{in + poly * kN, p.rmod, p.rmod_s, p.q};
+  ColSink<T> sink{out + poly * kN};
+  Cols<T, LOGN, TwAt<T>>::template fwd<0>(src, sink, reinterpret_cast<T*>(smem_raw),
+                                          TwAt<T>{tabs.tw_fwd + int64_t(pid) * kN}, p.q, p.twice_q, col0);
+}
+
+template <typename T>
+constexpr size_t exchange_smem() {
+  return size_t(kRowSlots) * kBlk * sizeof(T);
+}
+
+// The block stages of the forward transform, in place, to lazy words in
+// [0, 2q).  Half a warp per row of 256 words.
+template <typename T, int LOGN, bool SPLIT>
+__global__ void __launch_bounds__(kRowThreads, sizeof(T) == 8 ? 5 : 8)
+k_ntt_rows(T* out, int64_t slots, int rows, int row_start, ChainTables<T> tabs, ChainTables<double> tabs64f,
+           int f64_rows) {
+  using X = RowX<T>;
+  constexpr int64_t kN = int64_t(1) << LOGN;
+  constexpr int kBlks = 1 << (LOGN - kBlkLog);
+  __shared__ __align__(16) unsigned char smem[exchange_smem<T>()];
+  const int64_t slot = int64_t(blockIdx.x) * kRowSlots + (threadIdx.x >> 4);
+  if (slot >= slots) return;  // a whole warp: a polynomial has an even number of rows of 256 words
+  const int blk = int(slot % kBlks);
+  const int64_t poly = slot / kBlks;
+  const int row = int(poly % rows), pid = row_start + row;
+  const X x(smem);
+  T* at = out + poly * kN + blk * kBlk;
+  T* dst = at + X::V * x.t;
+  if constexpr (SPLIT) {
+    if (row < f64_rows) {
+      const double q = tabs64f.prime[pid].q, qinv = tabs64f.prime[pid].one_s;
+      const double* src = reinterpret_cast<const double*>(at) + x.t;
+      const RowX<double> xd(smem);
+      using R = Rows<double, LOGN, TwAtQ>;
+      double v[16];
+#pragma unroll
+      for (int e = 0; e < 16; ++e) v[e] = src[16 * e];
+      R::fwd(v, xd, TwAtQ{tabs64f.twv_fwd + int64_t(pid) * kN, qinv}, q, qinv, blk);
+      R::contiguous_to_vector(v, xd);
+#pragma unroll
+      for (int e = 0; e < 8; ++e)
+        reinterpret_cast<ulonglong2*>(dst)[16 * e] =
+            make_ulonglong2(Word<double>::to_word(Word<double>::to_lazy(v[2 * e], q, qinv)),
+                            Word<double>::to_word(Word<double>::to_lazy(v[2 * e + 1], q, qinv)));
+      return;
+    }
+  }
+  const T q = tabs.prime[pid].q, twoq = tabs.prime[pid].twice_q;
+  using R = Rows<T, LOGN, TwAt<T>>;
+  T v[16];
+#pragma unroll
+  for (int e = 0; e < 16; ++e) v[e] = at[x.t + 16 * e];
+  R::fwd(v, x, TwAt<T>{tabs.tw_fwd + int64_t(pid) * kN}, q, twoq, blk);
+  R::contiguous_to_vector(v, x);
+#pragma unroll
+  for (int e = 0; e < X::kVec; ++e) {
+    typename X::Piece w;
+#pragma unroll
+    for (int i = 0; i < X::V; ++i) w.v[i] = csub(v[e * X::V + i], twoq);
+    reinterpret_cast<typename X::Piece*>(dst)[16 * e] = w;
+  }
+}
+
+// The block stages of the inverse transform, `in` to `out` (which may be the
+// same buffer).
+template <typename T, int LOGN, bool SPLIT>
+__global__ void __launch_bounds__(kRowThreads, sizeof(T) == 8 ? 5 : 8)
+k_ntt_rows_inverse(const T* in, T* out, int64_t slots, int rows, int row_start, ChainTables<T> tabs,
+                   ChainTables<double> tabs64f, int f64_rows) {
+  using X = RowX<T>;
+  constexpr int64_t kN = int64_t(1) << LOGN;
+  constexpr int kBlks = 1 << (LOGN - kBlkLog);
+  __shared__ __align__(16) unsigned char smem[exchange_smem<T>()];
+  const int64_t slot = int64_t(blockIdx.x) * kRowSlots + (threadIdx.x >> 4);
+  if (slot >= slots) return;
+  const int blk = int(slot % kBlks);
+  const int64_t poly = slot / kBlks;
+  const int row = int(poly % rows), pid = row_start + row;
+  const X x(smem);
+  const typename X::Piece* src =
+      reinterpret_cast<const typename X::Piece*>(in + poly * kN + blk * kBlk + X::V * x.t);
+  T* dst = out + poly * kN + blk * kBlk + x.t;
+  if constexpr (SPLIT) {
+    if (row < f64_rows) {
+      const double q = tabs64f.prime[pid].q, qinv = tabs64f.prime[pid].one_s;
+      const RowX<double> xd(smem);
+      using R = Rows<double, LOGN, TwAtQ>;
+      double v[16];
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        const typename X::Piece w = src[16 * e];
+        v[2 * e] = Word<double>::from_word(w.v[0]);
+        v[2 * e + 1] = Word<double>::from_word(w.v[1]);
+      }
+      R::vector_to_contiguous(v, xd);
+      R::inv(v, xd, TwAtQ{tabs64f.twv_inv + int64_t(pid) * kN, qinv}, q, qinv, blk);
+#pragma unroll
+      for (int e = 0; e < 16; ++e) reinterpret_cast<double*>(dst)[16 * e] = v[e];
+      return;
+    }
+  }
+  using R = Rows<T, LOGN, TwAt<T>>;
+  T v[16];
+#pragma unroll
+  for (int e = 0; e < X::kVec; ++e) {
+    const typename X::Piece w = src[16 * e];
+#pragma unroll
+    for (int i = 0; i < X::V; ++i) v[e * X::V + i] = w.v[i];
+  }
+  R::vector_to_contiguous(v, x);
+  R::inv(v, x, TwAt<T>{tabs.tw_inv + int64_t(pid) * kN}, tabs.prime[pid].q, tabs.prime[pid].twice_q, blk);
+#pragma unroll
+  for (int e = 0; e < 16; ++e) dst[16 * e] = v[e];
+}
+
+// Canonical (centred: signed) word of a balanced inverse transform's output.
+// The lazy kinds get the canonical word too: their range is [0, 2q).
+struct WordOutEpilogue {
+  uint64_t* dst;
+  double q, c, cs;
+  bool centred;
+  __device__ __forceinline__ void operator()(int pos, double v) const {
+    v = Word<double>::shoup_bal(v, c, cs, q);  // (-0.6 q, 0.6 q)
+    if (v < 0.0) v += q;
+    const uint64_t w = Word<double>::to_word(v);
+    dst[pos] = centred && v > floor(0.5 * q) ? w - uint64_t(q) : w;
+  }
+};
+
+template <typename T, int LOGN, bool SPLIT>
+__global__ void __launch_bounds__(ColGeom<T, LOGN>::kThreads, col_blocks<T, LOGN>(false))
+k_ntt_columns_inverse(T* out, int rows, int row_start, int kind, ChainTables<T> tabs, ChainTables<double> tabs64f,
+                      int f64_rows) {
+  using G = ColGeom<T, LOGN>;
+  constexpr int64_t kN = int64_t(1) << LOGN;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const int col0 = int(blockIdx.x % G::kTiles) * G::kCols;
+  const int64_t poly = blockIdx.x / G::kTiles;
+  const int row = int(poly % rows), pid = row_start + row;
+  if constexpr (SPLIT) {
+    if (row < f64_rows) {
+      const PrimeInfo<double>& p = tabs64f.prime[pid];
+      const bool std_out = kind != kInvMontgomery;  // N^-1 R^-1 unless the output stays Montgomery
+      ColSource<double> src{reinterpret_cast<const double*>(out + poly * kN)};
+      WordOutEpilogue epi{out + poly * kN, p.q, std_out ? p.ninv_rinv : p.ninv, std_out ? p.ninv_rinv_s : p.ninv_s,
+                          kind == kInvCentered};
+      Cols<double, LOGN, TwAtQ>::template inv<0>(src, epi, reinterpret_cast<double*>(smem_raw),
+                                                 TwAtQ{tabs64f.twv_inv + int64_t(pid) * kN, p.one_s}, p.q, p.one_s,
+                                                 col0);
+      return;
+    }
+  }
+  const PrimeInfo<T>& p = tabs.prime[pid];
+  ColSource<T> src{out + poly * kN};
+  InvEpilogue<T> epi = make_inv_epilogue<T>(out + poly * kN, p, kind, true);
+  Cols<T, LOGN, TwAt<T>>::template inv<0>(src, epi, reinterpret_cast<T*>(smem_raw),
+                                          TwAt<T>{tabs.tw_inv + int64_t(pid) * kN}, p.q, p.twice_q, col0);
+}
+
+// ---------------------------------------------------------------------------
+// Hoisting stage 2, per rotation step: NTT-domain automorphism of the prepared
+// digits, products with both key components, block stages of both inverse
+// transforms (fhelium/engine/hybrid_keyswitch.py:419-469); the column stages
+// follow in k_ks_columns_inverse.  The sources of 16 aligned destinations
+// under the NTT-domain automorphism are a permutation of 16 aligned words
+// (the low bits of k are the top bits of br(k), which the odd g permutes), so
+// in the strided layout the gathers, like the key loads, are whole 128-byte
+// lines.  y: the prepared digits [D_l, B, QP_l, N].
+template <int LOGN>
+__device__ __forceinline__ void apply_sources(int (&src)[16], int blk, int t, uint32_t galois) {
+#pragma unroll
+  for (int e = 0; e < 16; ++e) {
+    const int dst = blk * kBlk + t + 16 * e;
+    src[e] = galois ? galois_ntt_source(dst, LOGN, galois) : dst;
+  }
+}
+
+template <typename T, int LOGN, bool SPLIT>
+__global__ void __launch_bounds__(kRowThreads, sizeof(T) == 8 ? 3 : 4)
+k_apply_rows(const __grid_constant__ KsPass<T> k, uint32_t galois) {
+  using X = RowX<T>;
+  constexpr int64_t kN = int64_t(1) << LOGN;
+  constexpr int kBlks = 1 << (LOGN - kBlkLog);
+  __shared__ __align__(16) unsigned char smem[exchange_smem<T>()];
+  const unsigned slots = unsigned(kBlks) * unsigned(k.batch);  // even: whole warps
+  const unsigned per_row = (slots + kRowSlots - 1) / kRowSlots;
+  int at;
+  const bool is_int = ks_unit(int(blockIdx.x / per_row), k.rows(), k.i_cnt, at);
+  const int jrow = at + (is_int ? k.i_lo : k.f_lo), pid = k.level + jrow;
+  const unsigned slot = blockIdx.x % per_row * kRowSlots + (threadIdx.x >> 4);
+  if (slot >= slots) return;
+  const int bi = int(slot % unsigned(k.batch)), blk = int(slot / unsigned(k.batch));
+  const X x(smem);
+  int src[16];
+  apply_sources<LOGN>(src, blk, x.t, galois);
+  const T* key = k.key + int64_t(pid) * kN + blk * kBlk + x.t;
+  const int64_t o = (int64_t(bi) * k.qp_limbs + jrow) * kN + blk * kBlk + x.t;
+  if constexpr (SPLIT) {
+    if (!is_int) {
+      using W = Word<double>;
+      using R = Rows<double, LOGN, TwAtQ>;
+      const RowX<double> xd(smem);
+      const double q = k.tabs64f.prime[pid].q, qinv = k.tabs64f.prime[pid].one_s;
+      double a0[16], a1[16];
+#pragma unroll
+      for (int e = 0; e < 16; ++e) a0[e] = a1[e] = 0.0;
+      for (int a = 0; a < k.lt.num_digits; ++a) {
+        const T* y = k.y_poly(a, bi, jrow, true, LOGN);
+        const T* key0 = key + int64_t(k.lt.digits[a].key_digit) * 2 * k.qp0 * kN;
+        const T* key1 = key0 + k.qp0 * kN;
+#pragma unroll
+        for (int e = 0; e < 16; ++e) {
+          const double v = W::from_word(__ldg(y + src[e]));
+          a0[e] += W::mul_qinv_bal(v, W::from_word(__ldg(key0 + 16 * e)), q, qinv);
+          a1[e] += W::mul_qinv_bal(v, W::from_word(__ldg(key1 + 16 * e)), q, qinv);
+        }
+      }
+      const TwAtQ tw{k.tabs64f.twv_inv + int64_t(pid) * kN, qinv};
+      auto finish = [&](double (&v)[16], T* out) {
+#pragma unroll
+        for (int e = 0; e < 16; ++e) v[e] = W::reduce_bal(v[e], q, qinv);
+        R::strided_to_contiguous(v, xd);
+        R::inv(v, xd, tw, q, qinv, blk);
+#pragma unroll
+        for (int e = 0; e < 16; ++e) reinterpret_cast<double*>(out + o)[16 * e] = v[e];
+      };
+      finish(a0, k.acc0);
+      finish(a1, k.acc1);
+      return;
+    }
+  }
+  using R = Rows<T, LOGN, TwAt<T>>;
+  const T q = k.tabs.prime[pid].q, twoq = k.tabs.prime[pid].twice_q;
+  const T qi = inverse_pow2(q, k.tabs.prime[pid].neg_inv);
+  T a0[16], a1[16];
+#pragma unroll
+  for (int e = 0; e < 16; ++e) a0[e] = a1[e] = 0;
+  for (int a = 0; a < k.lt.num_digits; ++a) {
+    const T* y = k.y_poly(a, bi, jrow, false, LOGN);
+    const T* key0 = key + int64_t(k.lt.digits[a].key_digit) * 2 * k.qp0 * kN;
+    const T* key1 = key0 + k.qp0 * kN;
+#pragma unroll
+    for (int e = 0; e < 16; ++e) {
+      const T v = __ldg(y + src[e]);
+      a0[e] = csub(a0[e] + redc_word(v, __ldg(key0 + 16 * e), q, qi), twoq);
+      a1[e] = csub(a1[e] + redc_word(v, __ldg(key1 + 16 * e), q, qi), twoq);
+    }
+  }
+  const TwAt<T> tw{k.tabs.tw_inv + int64_t(pid) * kN};
+  auto finish = [&](T (&v)[16], T* out) {
+#pragma unroll
+    for (int e = 0; e < 16; ++e) {  // x 4, as in ks_rows_int
+      v[e] = csub(v[e] + v[e], twoq);
+      v[e] = csub(v[e] + v[e], twoq);
+    }
+    R::strided_to_contiguous(v, x);
+    R::inv(v, x, tw, q, twoq, blk);
+#pragma unroll
+    for (int e = 0; e < 16; ++e) out[o + 16 * e] = v[e];
+  };
+  finish(a0, k.acc0);
+  finish(a1, k.acc1);
 }
 
 }  // namespace fhb

@@ -39,6 +39,19 @@ int launch_cluster(void (*kernel)(KArgs...), int64_t polys, size_t smem, cudaStr
   return cuda_status(cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...), "cluster launch");
 }
 
+template <typename... KArgs, typename... Args>
+int launch_blocks(void (*kernel)(KArgs...), int64_t blocks, int threads, size_t smem, cudaStream_t stream,
+                  Args... args) {
+  if (blocks <= 0) return 0;
+  if (blocks > 0x7fffffffLL) return fail(-6, "too many blocks for one launch");
+  if (smem > 48 * 1024) {
+    const int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(kernel), int(smem));
+    if (rc != 0) return rc;
+  }
+  kernel<<<unsigned(blocks), unsigned(threads), smem, stream>>>(static_cast<KArgs>(args)...);
+  return cuda_status(cudaGetLastError(), "pass launch");
+}
+
 template <typename T, int LOGN>
 constexpr size_t ntt_smem() {
   return size_t(NttGeom<T, LOGN>::kSmemElems) * sizeof(T);
@@ -64,9 +77,45 @@ int run_forward_e(const Context& c, const void* in, void* out, int64_t polys, in
   return mont ? launch(k_ntt_forward<T, LOGN, false, EPT>) : launch(k_ntt_forward<T, LOGN, true, EPT>);
 }
 
+// By default (no tuning value) both directions run as two launches, columns
+// then rows of 256 words or the reverse (fhb_pass.cuh), the intermediate in `out`.
+template <typename T, int LOGN, bool SPLIT>
+int run_forward_passes(const Context& c, const void* in, void* out, int64_t polys, int rows, int row_start, bool mont,
+                       int k, cudaStream_t st) {
+  using G = ColGeom<T, LOGN>;
+  auto columns = [&](auto kern) {
+    return launch_blocks(kern, polys * G::kTiles, G::kThreads, G::smem_bytes(), st, (const T*)in, (T*)out, rows,
+                         row_start, tables<T>(c), c.t64f, k);
+  };
+  const int rc = mont ? columns(k_ntt_columns<T, LOGN, false, SPLIT>) : columns(k_ntt_columns<T, LOGN, true, SPLIT>);
+  if (rc != 0) return rc;
+  const int64_t slots = polys << (LOGN - kBlkLog);
+  return launch_blocks(k_ntt_rows<T, LOGN, SPLIT>, (slots + kRowSlots - 1) / kRowSlots, kRowThreads, 0, st, (T*)out,
+                       slots, rows, row_start, tables<T>(c), c.t64f, k);
+}
+
+template <typename T, int LOGN, bool SPLIT>
+int run_inverse_passes(const Context& c, const void* in, void* out, int64_t polys, int rows, int row_start, int kind,
+                       int k, cudaStream_t st) {
+  using G = ColGeom<T, LOGN>;
+  const int64_t slots = polys << (LOGN - kBlkLog);
+  const int rc = launch_blocks(k_ntt_rows_inverse<T, LOGN, SPLIT>, (slots + kRowSlots - 1) / kRowSlots, kRowThreads, 0,
+                               st, (const T*)in, (T*)out, slots, rows, row_start, tables<T>(c), c.t64f, k);
+  if (rc != 0) return rc;
+  return launch_blocks(k_ntt_columns_inverse<T, LOGN, SPLIT>, polys * G::kTiles, G::kThreads, G::smem_bytes(), st,
+                       (T*)out, rows, row_start, kind, tables<T>(c), c.t64f, k);
+}
+
 template <typename T, int LOGN>
 int run_forward(const Context& c, const void* in, void* out, int64_t polys, int rows, int row_start,
                 bool mont, cudaStream_t st) {
+  if (c.ntt_ept_fwd == 0) {
+    if constexpr (sizeof(T) == 8) {
+      const int k = f64_rows(c, row_start, rows);
+      if (k > 0) return run_forward_passes<T, LOGN, true>(c, in, out, polys, rows, row_start, mont, k, st);
+    }
+    return run_forward_passes<T, LOGN, false>(c, in, out, polys, rows, row_start, mont, 0, st);
+  }
   if (c.ntt_ept_fwd == 16) return run_forward_e<T, LOGN, 16>(c, in, out, polys, rows, row_start, mont, st);
   return run_forward_e<T, LOGN, 0>(c, in, out, polys, rows, row_start, mont, st);
 }
@@ -88,6 +137,13 @@ int run_inverse_e(const Context& c, const void* in, void* out, int64_t polys, in
 template <typename T, int LOGN>
 int run_inverse(const Context& c, const void* in, void* out, int64_t polys, int rows, int row_start, int kind,
                 cudaStream_t st) {
+  if (c.ntt_ept_inv == 0) {
+    if constexpr (sizeof(T) == 8) {
+      const int k = f64_rows(c, row_start, rows);
+      if (k > 0) return run_inverse_passes<T, LOGN, true>(c, in, out, polys, rows, row_start, kind, k, st);
+    }
+    return run_inverse_passes<T, LOGN, false>(c, in, out, polys, rows, row_start, kind, 0, st);
+  }
   if (c.ntt_ept_inv == 16) return run_inverse_e<T, LOGN, 16>(c, in, out, polys, rows, row_start, kind, st);
   return run_inverse_e<T, LOGN, 0>(c, in, out, polys, rows, row_start, kind, st);
 }
@@ -142,31 +198,34 @@ int run_ks_core(const Context& c, const void* digits, const void* key, void* acc
   return launch_int(k_keyswitch_core<T, LOGN>);
 }
 
-template <typename... KArgs, typename... Args>
-int launch_blocks(void (*kernel)(KArgs...), int64_t blocks, int threads, size_t smem, cudaStream_t stream,
-                  Args... args) {
-  if (blocks <= 0) return 0;
-  if (blocks > 0x7fffffffLL) return fail(-6, "too many blocks for one launch");
-  if (smem > 48 * 1024) {
-    const int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(kernel), int(smem));
-    if (rc != 0) return rc;
-  }
-  kernel<<<unsigned(blocks), unsigned(threads), smem, stream>>>(static_cast<KArgs>(args)...);
-  return cuda_status(cudaGetLastError(), "pass launch");
+constexpr int64_t kMaxPassGroup = 4096;  // ciphertexts per launch (grid limit)
+
+// What the pass kernels of one level share; all rows in flight.
+template <typename T>
+KsPass<T> ks_pass_args(const Context& c, int level) {
+  KsPass<T> k = {};
+  k.q_limbs = c.num_q - level, k.qp_limbs = k.q_limbs + c.num_p, k.level = level, k.qp0 = c.qp();
+  k.f_cnt = sizeof(T) == 8 ? f64_rows(c, level, k.q_limbs) : 0;
+  k.i_lo = k.f_cnt, k.i_cnt = k.qp_limbs - k.f_cnt;
+  k.ext_digits = c.ext64f_digits, k.f64_end = c.f64_prime_end;
+  k.tabs = tables<T>(c), k.lt = level_tables<T>(c, level);
+  k.tabs64f = c.t64f, k.ext64f = c.ext64f;
+  return k;
 }
 
 // The three launches of one group of rows.
 template <typename T, int LOGN, bool SPLIT>
 int launch_ks_pass(const KsPass<T>& k, int digits, bool pre, cudaStream_t st) {
   using G = ColGeom<T, LOGN>;
-  const int64_t polys = int64_t(digits) * k.batch * k.rows;
-  int rc = pre ? launch_blocks(k_ks_columns<T, LOGN, true, SPLIT>, polys * G::kTiles, G::kThreads, G::smem_bytes(), st, k)
-               : launch_blocks(k_ks_columns<T, LOGN, false, SPLIT>, polys * G::kTiles, G::kThreads, G::smem_bytes(), st, k);
+  const int64_t units = (k.f_cnt + 1) / 2 + k.i_cnt, blocks = int64_t(digits) * k.batch * units * G::kTiles;
+  int rc = pre ? launch_blocks(k_ks_columns<T, LOGN, true, SPLIT>, blocks, G::kThreads, G::smem_bytes(), st, k)
+               : launch_blocks(k_ks_columns<T, LOGN, false, SPLIT>, blocks, G::kThreads,
+                               ks_columns_smem<T, LOGN>(SPLIT), st, k);
   if (rc != 0) return rc;
   const int64_t slots = (int64_t(k.batch) << (LOGN - kBlkLog));
-  rc = launch_blocks(k_ks_rows<T, LOGN, SPLIT>, (slots + kRowSlots - 1) / kRowSlots * k.rows, kRowThreads, 0, st, k);
+  rc = launch_blocks(k_ks_rows<T, LOGN, SPLIT>, (slots + kRowSlots - 1) / kRowSlots * k.rows(), kRowThreads, 0, st, k);
   if (rc != 0) return rc;
-  return launch_blocks(k_ks_columns_inverse<T, LOGN, SPLIT>, int64_t(2) * k.batch * k.rows * G::kTiles, G::kThreads,
+  return launch_blocks(k_ks_columns_inverse<T, LOGN, SPLIT>, int64_t(2) * k.batch * k.rows() * G::kTiles, G::kThreads,
                        G::smem_bytes(), st, k);
 }
 
@@ -174,26 +233,18 @@ template <typename T, int LOGN>
 int run_ks_pass(const Context& c, const void* digits, void* y, int64_t y_words, const void* key, void* acc0,
                 void* acc1, int64_t batch, int level, cudaStream_t st, const uint64_t* item_keys, const void* ct3,
                 bool pre, int64_t ct3_pitch) {
-  const int ql = c.num_q - level, qpl = ql + c.num_p;
+  KsPass<T> k = ks_pass_args<T>(c, level);
+  const int ql = k.q_limbs, qpl = k.qp_limbs, nd = k.lt.num_digits, f64 = k.f_cnt, ints = k.i_cnt;
   const int64_t n = c.n();
-  const int nd = level_tables<T>(c, level).num_digits;
   if (ct3_pitch <= 0) ct3_pitch = batch * ql * n;
-  KsPass<T> k = {};
-  k.digits = static_cast<const T*>(digits);
   k.y = static_cast<T*>(y);
   k.key = static_cast<const T*>(key);
-  k.item_keys = reinterpret_cast<const unsigned long long*>(item_keys);
   k.ct3_stride = ct3_pitch;
-  k.q_limbs = ql, k.qp_limbs = qpl, k.level = level, k.qp0 = c.qp();
-  k.f64_rows = sizeof(T) == 8 ? f64_rows(c, level, ql) : 0;
-  k.ext_digits = c.ext64f_digits, k.f64_end = c.f64_prime_end;
-  k.tabs = tables<T>(c), k.lt = level_tables<T>(c, level);
-  k.tabs64f = c.t64f, k.ext64f = c.ext64f;
+  k.by_row = pre;
   // ciphertexts per group: all of them, unless the room holds fewer or the
   // launch would pass the grid's limit
-  constexpr int64_t kMaxGroup = 4096;
   const int64_t per_row = nd * n;  // words of one ciphertext's row
-  int64_t group = std::min(batch, kMaxGroup);
+  int64_t group = std::min(batch, kMaxPassGroup);
   if (!pre) {
     group = std::min(group, y_words / per_row);
     if (group < 1) return fail(-8, "no room for the transform's intermediate");
@@ -208,12 +259,15 @@ int run_ks_pass(const Context& c, const void* digits, void* y, int64_t y_words, 
     k.ct3 = ct3 ? static_cast<const T*>(ct3) + b0 * ql * n : nullptr;
     if (item_keys) k.item_keys = reinterpret_cast<const unsigned long long*>(item_keys) + b0;
     const int step = pre ? qpl : int(std::min<int64_t>(qpl, y_words / (per_row * k.batch)));
-    for (int hi = qpl; hi > 0; hi -= step) {
-      k.rows = std::min(step, hi);
-      k.row_lo = hi - k.rows;
+    for (int lo = 0; lo < qpl; lo += step) {
+      // rows lo .. hi of the order that spreads the integer rows evenly
+      const int hi = std::min(qpl, lo + step);
+      k.i_lo = f64 + lo * ints / qpl, k.i_cnt = f64 + hi * ints / qpl - k.i_lo;
+      k.f_lo = lo - (k.i_lo - f64), k.f_cnt = hi - lo - k.i_cnt;
+      k.y_rows = pre ? qpl : hi - lo;
       int rc = 0;
       if constexpr (sizeof(T) == 8) {
-        rc = k.f64_rows > 0 ? launch_ks_pass<T, LOGN, true>(k, nd, pre, st) : launch_ks_pass<T, LOGN, false>(k, nd, pre, st);
+        rc = f64 > 0 ? launch_ks_pass<T, LOGN, true>(k, nd, pre, st) : launch_ks_pass<T, LOGN, false>(k, nd, pre, st);
       } else {
         if (pre) return fail(-7, "the tensor-core basis conversion needs an int64 context");
         rc = launch_ks_pass<T, LOGN, false>(k, nd, false, st);
@@ -244,55 +298,64 @@ int run_ks_sum(const Context& c, const void* digits, const uint64_t* key_ptrs, v
                                  level_tables<T>(c, level));
 }
 
-// Rows [0, k) of Q_l (primes below 2^42) of a key-switch kernel at `level`
-// that run in FP64 arithmetic (int64 chains with FP64 tables, N <= 2^16).
-template <typename T, int LOGN>
-int ks_f64_rows(const Context& c, int level) {
-  if constexpr (sizeof(T) == 8 && KsAcc<double, LOGN>::kSmem) {
-    static_assert(KsAcc<double, LOGN>::smem_bytes() == KsAcc<T, LOGN>::smem_bytes(), "one smem size for both");
-    return c.f64_core && c.f64_tables_ok ? std::max(0, std::min(c.num_q - level, c.f64_prime_end - level)) : 0;
-  }
-  return 0;
-}
-
+// Hoisting stage 1 (fhelium/engine/hybrid_keyswitch.py:373-417): the digits'
+// extensions transformed once, [D_l, B, QP_l, N] standard NTT-domain values
+// in [0, 2p), as the column launch of the key switch and the row launch of
+// the plain transform.
 template <typename T, int LOGN>
 int run_prepare(const Context& c, const void* digits, void* prepared, int64_t batch, int level,
                 cudaStream_t st) {
-  const int ql = c.num_q - level, qpl = ql + c.num_p;
-  const int k = ks_f64_rows<T, LOGN>(c, level);
-  auto launch = [&](auto kern) {
-    return launch_cluster<T, LOGN>(kern, batch * qpl, KsAcc<T, LOGN>::smem_bytes(), st, (const T*)digits,
-                                   (T*)prepared, batch, ql, qpl, level, c.qp(), c.ks_order, tables<T>(c),
-                                   level_tables<T>(c, level), c.t64f, k, c.ext64f, c.ext64f_digits, c.f64_prime_end);
+  KsPass<T> k = ks_pass_args<T>(c, level);
+  const int f64 = k.f_cnt, nd = k.lt.num_digits, qpl = k.qp_limbs;
+  const int64_t n = c.n(), units = (k.f_cnt + 1) / 2 + k.i_cnt, polys = int64_t(nd) * batch * qpl;
+  k.by_row = 1, k.y_rows = qpl, k.y_batch = int(batch);
+  using G = ColGeom<T, LOGN>;
+  auto run = [&](auto columns, auto rows, bool split) {
+    for (int64_t b0 = 0; b0 < batch; b0 += k.batch) {
+      k.batch = int(std::min(batch - b0, kMaxPassGroup));
+      k.digits = static_cast<const T*>(digits) + b0 * k.q_limbs * n;
+      k.y = static_cast<T*>(prepared) + b0 * qpl * n;
+      const int rc = launch_blocks(columns, int64_t(nd) * k.batch * units * G::kTiles, G::kThreads,
+                                   ks_columns_smem<T, LOGN>(split), st, k);
+      if (rc != 0) return rc;
+    }
+    const int64_t slots = polys << (LOGN - kBlkLog);
+    return launch_blocks(rows, (slots + kRowSlots - 1) / kRowSlots, kRowThreads, 0, st, (T*)prepared, slots, qpl,
+                         level, tables<T>(c), c.t64f, f64);
   };
   if constexpr (sizeof(T) == 8) {
-    if (k > 0) return launch(k_prepare_rotation<T, LOGN, true>);
+    if (f64 > 0) return run(k_ks_columns<T, LOGN, false, true>, k_ntt_rows<T, LOGN, true>, true);
   }
-  return launch(k_prepare_rotation<T, LOGN>);
+  return run(k_ks_columns<T, LOGN, false, false>, k_ntt_rows<T, LOGN, false>, false);
 }
 
 template <typename T, int LOGN>
 int run_apply_prepared(const Context& c, const void* prepared, const void* key, void* acc0, void* acc1,
                        int64_t batch, int level, uint32_t galois, cudaStream_t st) {
-  const int ql = c.num_q - level, qpl = ql + c.num_p;
-  const int k = ks_f64_rows<T, LOGN>(c, level);
-  auto launch = [&](auto kern) {
-    return launch_cluster<T, LOGN>(kern, batch * qpl, KsAcc<T, LOGN>::smem_bytes(), st, (const T*)prepared,
-                                   (const T*)key, (T*)acc0, (T*)acc1, batch, qpl, level, c.qp(),
-                                   galois == 1 ? 0u : galois, c.ks_order, tables<T>(c), level_tables<T>(c, level),
-                                   c.t64f, k);
+  KsPass<T> k = ks_pass_args<T>(c, level);
+  const int64_t n = c.n();
+  k.by_row = 1, k.y_rows = k.qp_limbs, k.y_batch = int(batch);
+  k.key = static_cast<const T*>(key);
+  using G = ColGeom<T, LOGN>;
+  auto run = [&](auto rows, auto columns) {
+    for (int64_t b0 = 0; b0 < batch; b0 += k.batch) {
+      k.batch = int(std::min(batch - b0, kMaxPassGroup));
+      k.y = static_cast<T*>(const_cast<void*>(prepared)) + b0 * k.qp_limbs * n;
+      k.acc0 = static_cast<T*>(acc0) + b0 * k.qp_limbs * n;
+      k.acc1 = static_cast<T*>(acc1) + b0 * k.qp_limbs * n;
+      const int64_t slots = int64_t(k.batch) << (LOGN - kBlkLog);
+      int rc = launch_blocks(rows, (slots + kRowSlots - 1) / kRowSlots * k.rows(), kRowThreads, 0, st, k,
+                             galois == 1 ? 0u : galois);
+      if (rc != 0) return rc;
+      rc = launch_blocks(columns, int64_t(2) * k.batch * k.rows() * G::kTiles, G::kThreads, G::smem_bytes(), st, k);
+      if (rc != 0) return rc;
+    }
+    return 0;
   };
-  if constexpr (ApplyRegs<T, LOGN>::kOk) {
-    if constexpr (sizeof(T) == 8) {
-      if (k > 0) return launch(k_apply_prepared_rotation<T, LOGN, true>);
-    }
-    return launch(k_apply_prepared_rotation<T, LOGN>);
-  } else {
-    if constexpr (sizeof(T) == 8) {
-      if (k > 0) return launch(k_apply_prepared_rotation_staged<T, LOGN, true>);
-    }
-    return launch(k_apply_prepared_rotation_staged<T, LOGN>);
+  if constexpr (sizeof(T) == 8) {
+    if (k.f_cnt > 0) return run(k_apply_rows<T, LOGN, true>, k_ks_columns_inverse<T, LOGN, true>);
   }
+  return run(k_apply_rows<T, LOGN, false>, k_ks_columns_inverse<T, LOGN, false>);
 }
 
 // ---- mixed-level item stages (fhb_items.cuh): one cluster per unit ----------
