@@ -78,6 +78,8 @@ SIGNATURES: dict[str, tuple] = {
     "fhb_ckks_rotate": (_I, [_P, _P, _P, _P, _P, _I64, _I64, _I, _U32, _P]),
     "fhb_ckks_rotate_multi": (_I, [_P, _P, _P, _P, _P, _P, _I64, _I64, _I, _P]),
     "fhb_ckks_keyswitch_sum": (_I, [_P, _P, _P, _P, _P, _I, _I64, _I, _P]),
+    "fhb_ckks_keyswitch_sum_workspace_bytes": (_I64, [_P, _I, _I64, _I]),
+    "fhb_ckks_keyswitch_sum_work": (_I, [_P, _P, _P, _P, _P, _P, _I64, _I, _I64, _I, _P]),
     "fhb_ckks_keyswitch_sum_extended": (_I, [_P, _P, _P, _P, _P, _I, _I64, _I, _P]),
     "fhb_ckks_decrypt_tail": (_I, [_P, _P, _P, _I64, _I, _P]),
     "fhb_ckks_items_plan_info": (_I, [_P, ctypes.POINTER(KsItem), _I, ctypes.POINTER(ItemsPlanInfo)]),

@@ -124,6 +124,10 @@ int ks_sum(const Context& c, const void* digits, const uint64_t* key_ptrs, void*
            int64_t batch, int level, cudaStream_t st, bool pre = false) {
   FHB_DISPATCH(run_ks_sum, c, digits, key_ptrs, acc0, acc1, giants, batch, level, st, pre);
 }
+int ks_sum_pass(const Context& c, const void* digits, void* y, int64_t y_words, const uint64_t* key_ptrs, void* acc0,
+                void* acc1, int terms, int64_t batch, int level, cudaStream_t st, bool pre) {
+  FHB_DISPATCH(run_ks_sum_pass, c, digits, y, y_words, key_ptrs, acc0, acc1, terms, batch, level, st, pre);
+}
 int prepare(const Context& c, const void* digits, void* prepared, int64_t batch, int level, cudaStream_t st) {
   FHB_DISPATCH(run_prepare, c, digits, prepared, batch, level, st);
 }
@@ -971,6 +975,39 @@ int fhb_ckks_keyswitch_sum(const fhb_context* ctx, const void* digits, const uin
   if (giants < 1 || batch < 0) return fail(-2, "need giants >= 1 and batch >= 0");
   TRY(fhb::check_level(c, level));
   return fhb::ks_sum(c, digits, key_ptrs, acc0, acc1, giants, batch, level, st);
+}
+
+int64_t fhb_ckks_keyswitch_sum_workspace_bytes(const fhb_context* ctx, int giants, int64_t batch, int level) {
+  if (!ctx || !ctx->impl || giants < 1 || batch < 0 || level < 0 || level >= ctx->impl->num_q) return -1;
+  const Context& c = *ctx->impl;
+  if (batch > INT64_MAX / giants) return -1;
+  const int64_t cts = batch * giants, word = fhb::word_bytes(c);
+  if (c.basis_tc) return fhb::tc_ext_words(c, cts, level) * word;
+  const int64_t one = fhb::ks_pass_min_words(c, level) * word, rows = c.num_q - level + c.num_p;
+  if (cts > INT64_MAX / (one * rows)) return -1;
+  return std::min(one * rows * cts, std::max(one * cts, fhb::kKsPassRoom));
+}
+
+int fhb_ckks_keyswitch_sum_work(const fhb_context* ctx, const void* digits, const uint64_t* key_ptrs, void* acc0,
+                                void* acc1, void* work, int64_t work_bytes, int giants, int64_t batch, int level,
+                                fhb_stream stream) {
+  CTX_OR_FAIL();
+  TRY(fhb::check_ptr(digits, "digits"));
+  TRY(fhb::check_ptr(acc0, "acc0"));
+  TRY(fhb::check_ptr(acc1, "acc1"));
+  TRY(fhb::check_ptr(work, "work"));
+  TRY(fhb::check_level(c, level));
+  if (!key_ptrs) return fail(-2, "key_ptrs is NULL");
+  if (giants < 1 || batch < 0) return fail(-2, "need giants >= 1 and batch >= 0");
+  if (batch == 0) return 0;
+  const int64_t cts = batch * giants, words = work_bytes / fhb::word_bytes(c);
+  if (words < (c.basis_tc ? fhb::tc_ext_words(c, cts, level) : fhb::ks_pass_min_words(c, level) * cts))
+    return fail(-8, "work buffer too small");
+  if (c.basis_tc) {  // the giants' digits as one batch of giants x batch ciphertexts
+    TRY(fhb::tc_extend(*ctx->impl, digits, work, cts, level, false, st));
+    return fhb::ks_sum_pass(c, digits, work, words, key_ptrs, acc0, acc1, giants, batch, level, st, true);
+  }
+  return fhb::ks_sum_pass(c, digits, work, words, key_ptrs, acc0, acc1, giants, batch, level, st, false);
 }
 
 int fhb_ckks_decrypt_tail(const fhb_context* ctx, const void* phase, double* out, int64_t batch, int level,

@@ -413,6 +413,8 @@ struct KsPass {
   int64_t ct3_stride;
   int batch, y_batch, y_rows, by_row, q_limbs, qp_limbs, level, qp0, ext_digits, f64_end;
   int f_lo, f_cnt, i_lo, i_cnt;
+  int terms;            // > 1: accumulator bi sums the key switches of ciphertexts g batch + bi of Y
+                        // (g < terms), each with the key item_keys[g]
   ChainTables<T> tabs;
   LevelTables<T> lt;
   ChainTables<double> tabs64f;
@@ -552,68 +554,58 @@ constexpr size_t ks_columns_smem(bool split) {
   return ColGeom<T, LOGN>::smem_bytes() * (split && ColGeom<T, LOGN>::kPasses <= 2 ? 2 : 1);
 }
 
-// Launch 1: extension of a digit to a row's prime and the column stages of
-// its forward transform.  One block per (digit, ciphertext, column tile, two
-// FP64 rows or one integer row), rows fastest, so the blocks in flight share
-// the digit's words in L2.  PRE: Y already holds the extensions (tensor-core
-// basis conversion), transformed in place.
-template <typename T, int LOGN, bool PRE, bool SPLIT>
-__global__ void __launch_bounds__(ColGeom<T, LOGN>::kThreads, col_blocks<T, LOGN>(SPLIT && !PRE))
-k_ks_columns(const __grid_constant__ KsPass<T> k) {
-  using G = ColGeom<T, LOGN>;
+// Launch 1, one column tile: extension of digit a of ciphertext bi to the
+// primes of FP64 rows j0, j1 (each if live) and the column stages of their
+// forward transforms.  PRE: Y already holds the extensions (tensor-core basis
+// conversion), transformed in place.
+template <int LOGN, bool PRE>
+__device__ __forceinline__ void ks_columns_f64(const KsPass<uint64_t>& k, int a, int bi, int col0, int j0, int j1,
+                                               bool live0, bool live1, unsigned char* smem) {
+  using G = ColGeom<uint64_t, LOGN>;
+  using C = Cols<double, LOGN, TwAtQ>;
   constexpr int64_t kN = int64_t(1) << LOGN;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  const int units = (k.f_cnt + 1) / 2 + k.i_cnt;
-  unsigned idx = blockIdx.x;
-  int at;
-  const bool is_int = ks_unit(int(idx % unsigned(units)), units, k.i_cnt, at);
-  idx /= unsigned(units);
-  const int col0 = int(idx % G::kTiles) * G::kCols;
-  idx /= G::kTiles;
-  const int bi = int(idx % unsigned(k.batch)), a = int(idx / unsigned(k.batch));
+  if (!live0 && !live1) return;
   const DigitDesc d = k.lt.digits[a];
-  if constexpr (SPLIT) {
-    static_assert(sizeof(T) == 8, "FP64 rows exist in int64 chains only");
-    if (!is_int) {
-      const int j0 = k.f_lo + 2 * at, j1 = j0 + 1;
-      const bool live0 = !ks_own(k, d, j0), live1 = 2 * at + 1 < k.f_cnt && !ks_own(k, d, j1);
-      if (!live0 && !live1) return;
-      double* s = reinterpret_cast<double*>(smem_raw);
-      if constexpr (!PRE && G::kPasses <= 2) {
-        if (d.alpha <= 4 && d.prime0 + d.alpha <= k.f64_end) {
-          ks_columns_pair<LOGN>(k, d, a, bi, col0, j0, j1, live0, live1, s);
-          return;
-        }
-      }
-      using C = Cols<double, LOGN, TwAtQ>;
-      for (int i = 0; i < 2; ++i) {
-        const int jrow = i ? j1 : j0, pid = k.level + jrow;
-        if (!(i ? live1 : live0)) continue;
-        if (i) __syncthreads();  // the first row's words have been read
-        const double q = k.tabs64f.prime[pid].q, qinv = k.tabs64f.prime[pid].one_s;
-        uint64_t* y = k.y_poly(a, bi, jrow, true, LOGN);
-        ColSink<double> sink{reinterpret_cast<double*>(y)};
-        const TwAtQ tw{k.tabs64f.twv_fwd + int64_t(pid) * kN, qinv};
-        if constexpr (PRE) {
-          U64RowSource src{y};
-          C::template fwd<0>(src, sink, s, tw, q, qinv, col0);
-        } else {
-          ExtSourceF64 src{k.digits + (int64_t(bi) * k.q_limbs + (d.prime0 - k.level)) * kN,
-                           k.ext64f + (((int64_t(k.level) * k.ext_digits + a) * kMaxDigitWidth) * 2) * k.qp0 + pid,
-                           k.qp0, d.alpha, LOGN, d.prime0 + d.alpha > k.f64_end, q, qinv};
-          C::template fwd<0>(src, sink, s, tw, q, qinv, col0);
-        }
-      }
+  double* s = reinterpret_cast<double*>(smem);
+  if constexpr (!PRE && G::kPasses <= 2) {
+    if (d.alpha <= 4 && d.prime0 + d.alpha <= k.f64_end) {
+      ks_columns_pair<LOGN>(k, d, a, bi, col0, j0, j1, live0, live1, s);
       return;
     }
   }
-  const int jrow = k.i_lo + at, pid = k.level + jrow;
-  if (ks_own(k, d, jrow)) return;
+  for (int i = 0; i < 2; ++i) {
+    const int jrow = i ? j1 : j0, pid = k.level + jrow;
+    if (!(i ? live1 : live0)) continue;
+    if (i) __syncthreads();  // the first row's words have been read
+    const double q = k.tabs64f.prime[pid].q, qinv = k.tabs64f.prime[pid].one_s;
+    uint64_t* y = k.y_poly(a, bi, jrow, true, LOGN);
+    ColSink<double> sink{reinterpret_cast<double*>(y)};
+    const TwAtQ tw{k.tabs64f.twv_fwd + int64_t(pid) * kN, qinv};
+    if constexpr (PRE) {
+      U64RowSource src{y};
+      C::template fwd<0>(src, sink, s, tw, q, qinv, col0);
+    } else {
+      ExtSourceF64 src{k.digits + (int64_t(bi) * k.q_limbs + (d.prime0 - k.level)) * kN,
+                       k.ext64f + (((int64_t(k.level) * k.ext_digits + a) * kMaxDigitWidth) * 2) * k.qp0 + pid, k.qp0,
+                       d.alpha, LOGN, d.prime0 + d.alpha > k.f64_end, q, qinv};
+      C::template fwd<0>(src, sink, s, tw, q, qinv, col0);
+    }
+  }
+}
+
+// The same for one integer row.
+template <typename T, int LOGN, bool PRE>
+__device__ __forceinline__ void ks_columns_int(const KsPass<T>& k, int a, int bi, int col0, int jrow,
+                                               unsigned char* smem) {
   using C = Cols<T, LOGN, TwAt<T>>;
+  constexpr int64_t kN = int64_t(1) << LOGN;
+  const DigitDesc d = k.lt.digits[a];
+  if (ks_own(k, d, jrow)) return;
+  const int pid = k.level + jrow;
   const T q = k.tabs.prime[pid].q, twoq = k.tabs.prime[pid].twice_q;
   T* y = k.y_poly(a, bi, jrow, false, LOGN);
   ColSink<T> sink{y};
-  T* s = reinterpret_cast<T*>(smem_raw);
+  T* s = reinterpret_cast<T*>(smem);
   const TwAt<T> tw{k.tabs.tw_fwd + int64_t(pid) * kN};
   if constexpr (PRE) {
     ColSource<T> src{y};
@@ -623,6 +615,34 @@ k_ks_columns(const __grid_constant__ KsPass<T> k) {
                      k.lt.ext + int64_t(a) * kMaxDigitWidth * k.qp0 + pid, k.qp0, d.alpha, LOGN, q, twoq};
     C::template fwd<0>(src, sink, s, tw, q, twoq, col0);
   }
+}
+
+// One block per (digit, ciphertext, column tile, two FP64 rows or one integer
+// row), rows fastest, so the blocks in flight share the digit's words in L2.
+template <typename T, int LOGN, bool PRE, bool SPLIT>
+__global__ void __launch_bounds__(ColGeom<T, LOGN>::kThreads, col_blocks<T, LOGN>(SPLIT && !PRE))
+k_ks_columns(const __grid_constant__ KsPass<T> k) {
+  using G = ColGeom<T, LOGN>;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const int units = (k.f_cnt + 1) / 2 + k.i_cnt;
+  unsigned idx = blockIdx.x;
+  int at;
+  const bool is_int = ks_unit(int(idx % unsigned(units)), units, k.i_cnt, at);
+  idx /= unsigned(units);
+  const int col0 = int(idx % G::kTiles) * G::kCols;
+  idx /= G::kTiles;
+  const int bi = int(idx % unsigned(k.batch)), a = int(idx / unsigned(k.batch));
+  if constexpr (SPLIT) {
+    static_assert(sizeof(T) == 8, "FP64 rows exist in int64 chains only");
+    if (!is_int) {
+      const DigitDesc d = k.lt.digits[a];
+      const int j0 = k.f_lo + 2 * at, j1 = j0 + 1;
+      ks_columns_f64<LOGN, PRE>(k, a, bi, col0, j0, j1, !ks_own(k, d, j0),
+                                2 * at + 1 < k.f_cnt && !ks_own(k, d, j1), smem_raw);
+      return;
+    }
+  }
+  ks_columns_int<T, LOGN, PRE>(k, a, bi, col0, k.i_lo + at, smem_raw);
 }
 
 // x k 2^-W mod q (W the word's bits) in (0, 2q) for x < 4q, k < 2q: one
@@ -659,45 +679,56 @@ __device__ __forceinline__ void ks_rows_f64(const KsPass<uint64_t>& k, int jrow,
   const double q = p.q, qinv = p.one_s;
   const RowX<double> x(smem);
   const int vec = blk * kBlk + 2 * x.t;  // this thread's first word, vector layout
-  const uint64_t* key = k.item_keys ? reinterpret_cast<const uint64_t*>(k.item_keys[bi]) : k.key;
   const uint64_t* ct3 = k.ct3 ? k.ct3 + (int64_t(bi) * k.q_limbs + jrow) * kN + vec : nullptr;
   const TwAtQ twf{k.tabs64f.twv_fwd + int64_t(pid) * kN, qinv};
   const RowStage<double> stage(smem + kRowSlots * kBlk * sizeof(double));
+  int next = 0;  // the term whose row is requested next
   auto request = [&](int a) {  // digit a's row, unless its residue is the ciphertext's own
+    if (a == k.lt.num_digits && ++next < k.terms) a = 0;
     if (a < k.lt.num_digits && !ks_own(k, k.lt.digits[a], jrow))
-      stage.request(reinterpret_cast<const double*>(k.y_poly(a, bi, jrow, true, LOGN)) + blk * kBlk);
+      stage.request(reinterpret_cast<const double*>(k.y_poly(a, next * k.batch + bi, jrow, true, LOGN)) + blk * kBlk);
   };
   request(0);
   double a0[16], a1[16];
 #pragma unroll
   for (int e = 0; e < 16; ++e) a0[e] = a1[e] = 0.0;
-  for (int a = 0; a < k.lt.num_digits; ++a) {
-    const DigitDesc d = k.lt.digits[a];
-    double v[16];
-    if (ks_own(k, d, jrow)) {
+  for (int g = 0; g < k.terms; ++g) {
+    const uint64_t* key = k.item_keys ? reinterpret_cast<const uint64_t*>(k.item_keys[k.terms > 1 ? g : bi]) : k.key;
+    for (int a = 0; a < k.lt.num_digits; ++a) {
+      const DigitDesc d = k.lt.digits[a];
+      double v[16];
+      if (ks_own(k, d, jrow)) {
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+          const ulonglong2 w = __ldg(reinterpret_cast<const ulonglong2*>(ct3 + 2 * k.ct3_stride + 32 * e));
+          v[2 * e] = W::shoup_bal(W::from_word(w.x), p.rinv, p.rinv_s, q);
+          v[2 * e + 1] = W::shoup_bal(W::from_word(w.y), p.rinv, p.rinv_s, q);
+        }
+        request(a + 1);
+      } else {
+        stage.take(v);
+        request(a + 1);
+        R::fwd(v, x, twf, q, qinv, blk);
+        R::contiguous_to_vector(v, x);
+      }
+      const uint64_t* key0 = key + ((int64_t(d.key_digit) * 2) * k.qp0 + pid) * kN + vec;
+      const uint64_t* key1 = key0 + k.qp0 * kN;
 #pragma unroll
       for (int e = 0; e < 8; ++e) {
-        const ulonglong2 w = __ldg(reinterpret_cast<const ulonglong2*>(ct3 + 2 * k.ct3_stride + 32 * e));
-        v[2 * e] = W::shoup_bal(W::from_word(w.x), p.rinv, p.rinv_s, q);
-        v[2 * e + 1] = W::shoup_bal(W::from_word(w.y), p.rinv, p.rinv_s, q);
+        const ulonglong2 u0 = __ldg(reinterpret_cast<const ulonglong2*>(key0 + 32 * e));
+        const ulonglong2 u1 = __ldg(reinterpret_cast<const ulonglong2*>(key1 + 32 * e));
+        a0[2 * e] += W::mul_qinv_bal(v[2 * e], W::from_word(u0.x), q, qinv);
+        a0[2 * e + 1] += W::mul_qinv_bal(v[2 * e + 1], W::from_word(u0.y), q, qinv);
+        a1[2 * e] += W::mul_qinv_bal(v[2 * e], W::from_word(u1.x), q, qinv);
+        a1[2 * e + 1] += W::mul_qinv_bal(v[2 * e + 1], W::from_word(u1.y), q, qinv);
       }
-      request(a + 1);
-    } else {
-      stage.take(v);
-      request(a + 1);
-      R::fwd(v, x, twf, q, qinv, blk);
-      R::contiguous_to_vector(v, x);
     }
-    const uint64_t* key0 = key + ((int64_t(d.key_digit) * 2) * k.qp0 + pid) * kN + vec;
-    const uint64_t* key1 = key0 + k.qp0 * kN;
+    if (k.terms > 1) {  // at most 17 digits a term: the sums stay below 2^48
 #pragma unroll
-    for (int e = 0; e < 8; ++e) {
-      const ulonglong2 u0 = __ldg(reinterpret_cast<const ulonglong2*>(key0 + 32 * e));
-      const ulonglong2 u1 = __ldg(reinterpret_cast<const ulonglong2*>(key1 + 32 * e));
-      a0[2 * e] += W::mul_qinv_bal(v[2 * e], W::from_word(u0.x), q, qinv);
-      a0[2 * e + 1] += W::mul_qinv_bal(v[2 * e + 1], W::from_word(u0.y), q, qinv);
-      a1[2 * e] += W::mul_qinv_bal(v[2 * e], W::from_word(u1.x), q, qinv);
-      a1[2 * e + 1] += W::mul_qinv_bal(v[2 * e + 1], W::from_word(u1.y), q, qinv);
+      for (int e = 0; e < 16; ++e) {
+        a0[e] = W::reduce_bal(a0[e], q, qinv);
+        a1[e] = W::reduce_bal(a1[e], q, qinv);
+      }
     }
   }
   const TwAtQ twi{k.tabs64f.twv_inv + int64_t(pid) * kN, qinv};
@@ -738,7 +769,6 @@ __device__ __forceinline__ void ks_rows_int(const KsPass<T>& k, int jrow, int bi
   const T q = p.q, twoq = p.twice_q, ni = p.neg_inv;
   const X x(smem);
   const int vec = blk * kBlk + X::V * x.t;
-  const T* key = k.item_keys ? reinterpret_cast<const T*>(k.item_keys[bi]) : k.key;
   const T* ct3 = k.ct3 && jrow < k.q_limbs ? k.ct3 + (int64_t(bi) * k.q_limbs + jrow) * kN + vec : nullptr;
   auto piece = [](const T* at) {
     Piece r;
@@ -747,42 +777,47 @@ __device__ __forceinline__ void ks_rows_int(const KsPass<T>& k, int jrow, int bi
   };
   const TwAt<T> twf{k.tabs.tw_fwd + int64_t(pid) * kN};
   const RowStage<T> stage(smem + kRowSlots * kBlk * sizeof(T));
+  int next = 0;
   auto request = [&](int a) {
+    if (a == k.lt.num_digits && ++next < k.terms) a = 0;
     if (a < k.lt.num_digits && !ks_own(k, k.lt.digits[a], jrow))
-      stage.request(k.y_poly(a, bi, jrow, false, LOGN) + blk * kBlk);
+      stage.request(k.y_poly(a, next * k.batch + bi, jrow, false, LOGN) + blk * kBlk);
   };
   request(0);
   const T qi = inverse_pow2(q, ni);
   T a0[16], a1[16];
 #pragma unroll
   for (int e = 0; e < 16; ++e) a0[e] = a1[e] = 0;
-  for (int a = 0; a < k.lt.num_digits; ++a) {
-    const DigitDesc d = k.lt.digits[a];
-    T v[16];
-    if (ks_own(k, d, jrow)) {
+  for (int g = 0; g < k.terms; ++g) {
+    const T* key = k.item_keys ? reinterpret_cast<const T*>(k.item_keys[k.terms > 1 ? g : bi]) : k.key;
+    for (int a = 0; a < k.lt.num_digits; ++a) {
+      const DigitDesc d = k.lt.digits[a];
+      T v[16];
+      if (ks_own(k, d, jrow)) {
+#pragma unroll
+        for (int e = 0; e < X::kVec; ++e) {
+          const Piece w = piece(ct3 + 2 * k.ct3_stride + 16 * X::V * e);
+#pragma unroll
+          for (int i = 0; i < X::V; ++i) v[e * X::V + i] = W::shoup(w.v[i], p.rinv, p.rinv_s, q);
+        }
+        request(a + 1);
+      } else {
+        stage.take(v);
+        request(a + 1);
+        R::fwd(v, x, twf, q, twoq, blk);
+        R::contiguous_to_vector(v, x);
+      }
+      const T* key0 = key + ((int64_t(d.key_digit) * 2) * k.qp0 + pid) * kN + vec;
+      const T* key1 = key0 + k.qp0 * kN;
 #pragma unroll
       for (int e = 0; e < X::kVec; ++e) {
-        const Piece w = piece(ct3 + 2 * k.ct3_stride + 16 * X::V * e);
+        const Piece u0 = piece(key0 + 16 * X::V * e), u1 = piece(key1 + 16 * X::V * e);
 #pragma unroll
-        for (int i = 0; i < X::V; ++i) v[e * X::V + i] = W::shoup(w.v[i], p.rinv, p.rinv_s, q);
-      }
-      request(a + 1);
-    } else {
-      stage.take(v);
-      request(a + 1);
-      R::fwd(v, x, twf, q, twoq, blk);
-      R::contiguous_to_vector(v, x);
-    }
-    const T* key0 = key + ((int64_t(d.key_digit) * 2) * k.qp0 + pid) * kN + vec;
-    const T* key1 = key0 + k.qp0 * kN;
-#pragma unroll
-    for (int e = 0; e < X::kVec; ++e) {
-      const Piece u0 = piece(key0 + 16 * X::V * e), u1 = piece(key1 + 16 * X::V * e);
-#pragma unroll
-      for (int i = 0; i < X::V; ++i) {
-        const int at = e * X::V + i;
-        a0[at] = csub(a0[at] + redc_word(v[at], u0.v[i], q, qi), twoq);
-        a1[at] = csub(a1[at] + redc_word(v[at], u1.v[i], q, qi), twoq);
+        for (int i = 0; i < X::V; ++i) {
+          const int at = e * X::V + i;
+          a0[at] = csub(a0[at] + redc_word(v[at], u0.v[i], q, qi), twoq);
+          a1[at] = csub(a1[at] + redc_word(v[at], u1.v[i], q, qi), twoq);
+        }
       }
     }
   }
@@ -848,14 +883,36 @@ k_ks_rows(const __grid_constant__ KsPass<T> k) {
   ks_rows_int<T, LOGN>(k, jrow, bi, blk, live, smem);
 }
 
-// Launch 3: the column stages of the inverse transforms, in place over the
-// accumulator rows, to canonical coefficients.  One block per (component,
-// ciphertext, row, column tile).
+// Launch 3: one column tile of the inverse transform of the accumulator row z
+// of prime pid, in place, to canonical coefficients.
+template <typename T, int LOGN, bool SPLIT>
+__device__ __forceinline__ void ks_columns_inverse(T* z, int pid, bool f64, const ChainTables<T>& tabs,
+                                                   const ChainTables<double>& tabs64f, int col0,
+                                                   unsigned char* smem) {
+  constexpr int64_t kN = int64_t(1) << LOGN;
+  if constexpr (SPLIT) {
+    if (f64) {
+      const PrimeInfo<double>& p = tabs64f.prime[pid];
+      ColSource<double> src{reinterpret_cast<double*>(z)};
+      F64InvEpilogue epi{reinterpret_cast<uint64_t*>(z), p.q, p.ninv_rinv, p.ninv_rinv_s};
+      Cols<double, LOGN, TwAtQ>::template inv<0>(src, epi, reinterpret_cast<double*>(smem),
+                                                 TwAtQ{tabs64f.twv_inv + int64_t(pid) * kN, p.one_s}, p.q, p.one_s,
+                                                 col0);
+      return;
+    }
+  }
+  const PrimeInfo<T>& p = tabs.prime[pid];
+  ColSource<T> src{z};
+  InvEpilogue<T> epi{z, p.q, p.ninv, p.ninv_s, kInvStandard};
+  Cols<T, LOGN, TwAt<T>>::template inv<0>(src, epi, reinterpret_cast<T*>(smem),
+                                          TwAt<T>{tabs.tw_inv + int64_t(pid) * kN}, p.q, p.twice_q, col0);
+}
+
+// One block per (component, ciphertext, row, column tile).
 template <typename T, int LOGN, bool SPLIT>
 __global__ void __launch_bounds__(ColGeom<T, LOGN>::kThreads, col_blocks<T, LOGN>(false))
 k_ks_columns_inverse(const __grid_constant__ KsPass<T> k) {
   using G = ColGeom<T, LOGN>;
-  constexpr int64_t kN = int64_t(1) << LOGN;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   unsigned idx = blockIdx.x;
   const int col0 = int(idx % G::kTiles) * G::kCols;
@@ -865,24 +922,8 @@ k_ks_columns_inverse(const __grid_constant__ KsPass<T> k) {
   const int jrow = at + (is_int ? k.i_lo : k.f_lo);
   idx /= unsigned(k.rows());
   const int bi = int(idx % unsigned(k.batch));
-  T* z = (idx / unsigned(k.batch) ? k.acc1 : k.acc0) + (int64_t(bi) * k.qp_limbs + jrow) * kN;
-  const int pid = k.level + jrow;
-  if constexpr (SPLIT) {
-    if (!is_int) {
-      const PrimeInfo<double>& p = k.tabs64f.prime[pid];
-      ColSource<double> src{reinterpret_cast<double*>(z)};
-      F64InvEpilogue epi{reinterpret_cast<uint64_t*>(z), p.q, p.ninv_rinv, p.ninv_rinv_s};
-      Cols<double, LOGN, TwAtQ>::template inv<0>(src, epi, reinterpret_cast<double*>(smem_raw),
-                                                 TwAtQ{k.tabs64f.twv_inv + int64_t(pid) * kN, p.one_s}, p.q, p.one_s,
-                                                 col0);
-      return;
-    }
-  }
-  const PrimeInfo<T>& p = k.tabs.prime[pid];
-  ColSource<T> src{z};
-  InvEpilogue<T> epi{z, p.q, p.ninv, p.ninv_s, kInvStandard};
-  Cols<T, LOGN, TwAt<T>>::template inv<0>(src, epi, reinterpret_cast<T*>(smem_raw),
-                                          TwAt<T>{k.tabs.tw_inv + int64_t(pid) * kN}, p.q, p.twice_q, col0);
+  T* z = (idx / unsigned(k.batch) ? k.acc1 : k.acc0) + ((int64_t(bi) * k.qp_limbs + jrow) << LOGN);
+  ks_columns_inverse<T, LOGN, SPLIT>(z, k.level + jrow, !is_int, k.tabs, k.tabs64f, col0, smem_raw);
 }
 
 // ---------------------------------------------------------------------------
@@ -903,31 +944,27 @@ struct WordSource {  // 64-bit words of a prime below 2^42 as balanced doubles
   }
 };
 
+// One column tile of the forward transform of the polynomial `in` of prime
+// pid into `out` (f64: FP64 arithmetic, the intermediate in doubles).
 template <typename T, int LOGN, bool TO_MONT, bool SPLIT>
-__global__ void __launch_bounds__(ColGeom<T, LOGN>::kThreads, col_blocks<T, LOGN>(false))
-k_ntt_columns(const T* in, T* out, int rows, int row_start, ChainTables<T> tabs, ChainTables<double> tabs64f,
-              int f64_rows) {
-  using G = ColGeom<T, LOGN>;
+__device__ __forceinline__ void ntt_columns(const T* in, T* out, int pid, bool f64, const ChainTables<T>& tabs,
+                                            const ChainTables<double>& tabs64f, int col0, unsigned char* smem) {
   constexpr int64_t kN = int64_t(1) << LOGN;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  const int col0 = int(blockIdx.x % G::kTiles) * G::kCols;
-  const int64_t poly = blockIdx.x / G::kTiles;
-  const int row = int(poly % rows), pid = row_start + row;
   if constexpr (SPLIT) {
-    if (row < f64_rows) {
+    if (f64) {
       const PrimeInfo<double>& p = tabs64f.prime[pid];
-      WordSource<TO_MONT> src{in + poly * kN, p.rmod, p.rmod_s, p.q};
-      ColSink<double> sink{reinterpret_cast<double*>(out + poly * kN)};
-      Cols<double, LOGN, TwAtQ>::template fwd<0>(src, sink, reinterpret_cast<double*>(smem_raw),
+      WordSource<TO_MONT> src{in, p.rmod, p.rmod_s, p.q};
+      ColSink<double> sink{reinterpret_cast<double*>(out)};
+      Cols<double, LOGN, TwAtQ>::template fwd<0>(src, sink, reinterpret_cast<double*>(smem),
                                                  TwAtQ{tabs64f.twv_fwd + int64_t(pid) * kN, p.one_s}, p.q, p.one_s,
                                                  col0);
       return;
     }
   }
   const PrimeInfo<T>& p = tabs.prime[pid];
-  RowSource<T, TO_MONT> src{in + poly * kN, p.rmod, p.rmod_s, p.q};
-  ColSink<T> sink{out + poly * kN};
-  Cols<T, LOGN, TwAt<T>>::template fwd<0>(src, sink, reinterpret_cast<T*>(smem_raw),
+  RowSource<T, TO_MONT> src{in, p.rmod, p.rmod_s, p.q};
+  ColSink<T> sink{out};
+  Cols<T, LOGN, TwAt<T>>::template fwd<0>(src, sink, reinterpret_cast<T*>(smem),
                                           TwAt<T>{tabs.tw_fwd + int64_t(pid) * kN}, p.q, p.twice_q, col0);
 }
 
@@ -936,26 +973,18 @@ constexpr size_t exchange_smem() {
   return size_t(kRowSlots) * kBlk * sizeof(T);
 }
 
-// The block stages of the forward transform, in place, to lazy words in
-// [0, 2q).  Half a warp per row of 256 words.
+// The block stages of the forward transform of row blk of `poly`, in place,
+// to lazy words in [0, 2q).  Half a warp per row of 256 words.
 template <typename T, int LOGN, bool SPLIT>
-__global__ void __launch_bounds__(kRowThreads, sizeof(T) == 8 ? 5 : 8)
-k_ntt_rows(T* out, int64_t slots, int rows, int row_start, ChainTables<T> tabs, ChainTables<double> tabs64f,
-           int f64_rows) {
+__device__ __forceinline__ void ntt_rows(T* poly, int pid, bool f64, const ChainTables<T>& tabs,
+                                         const ChainTables<double>& tabs64f, int blk, unsigned char* smem) {
   using X = RowX<T>;
   constexpr int64_t kN = int64_t(1) << LOGN;
-  constexpr int kBlks = 1 << (LOGN - kBlkLog);
-  __shared__ __align__(16) unsigned char smem[exchange_smem<T>()];
-  const int64_t slot = int64_t(blockIdx.x) * kRowSlots + (threadIdx.x >> 4);
-  if (slot >= slots) return;  // a whole warp: a polynomial has an even number of rows of 256 words
-  const int blk = int(slot % kBlks);
-  const int64_t poly = slot / kBlks;
-  const int row = int(poly % rows), pid = row_start + row;
   const X x(smem);
-  T* at = out + poly * kN + blk * kBlk;
+  T* at = poly + blk * kBlk;
   T* dst = at + X::V * x.t;
   if constexpr (SPLIT) {
-    if (row < f64_rows) {
+    if (f64) {
       const double q = tabs64f.prime[pid].q, qinv = tabs64f.prime[pid].one_s;
       const double* src = reinterpret_cast<const double*>(at) + x.t;
       const RowX<double> xd(smem);
@@ -989,27 +1018,18 @@ k_ntt_rows(T* out, int64_t slots, int rows, int row_start, ChainTables<T> tabs, 
   }
 }
 
-// The block stages of the inverse transform, `in` to `out` (which may be the
-// same buffer).
+// The block stages of the inverse transform of row blk, `in` to `out` (which
+// may be the same buffer).
 template <typename T, int LOGN, bool SPLIT>
-__global__ void __launch_bounds__(kRowThreads, sizeof(T) == 8 ? 5 : 8)
-k_ntt_rows_inverse(const T* in, T* out, int64_t slots, int rows, int row_start, ChainTables<T> tabs,
-                   ChainTables<double> tabs64f, int f64_rows) {
+__device__ __forceinline__ void ntt_rows_inverse(const T* in, T* out, int pid, bool f64, const ChainTables<T>& tabs,
+                                                 const ChainTables<double>& tabs64f, int blk, unsigned char* smem) {
   using X = RowX<T>;
   constexpr int64_t kN = int64_t(1) << LOGN;
-  constexpr int kBlks = 1 << (LOGN - kBlkLog);
-  __shared__ __align__(16) unsigned char smem[exchange_smem<T>()];
-  const int64_t slot = int64_t(blockIdx.x) * kRowSlots + (threadIdx.x >> 4);
-  if (slot >= slots) return;
-  const int blk = int(slot % kBlks);
-  const int64_t poly = slot / kBlks;
-  const int row = int(poly % rows), pid = row_start + row;
   const X x(smem);
-  const typename X::Piece* src =
-      reinterpret_cast<const typename X::Piece*>(in + poly * kN + blk * kBlk + X::V * x.t);
-  T* dst = out + poly * kN + blk * kBlk + x.t;
+  const typename X::Piece* src = reinterpret_cast<const typename X::Piece*>(in + blk * kBlk + X::V * x.t);
+  T* dst = out + blk * kBlk + x.t;
   if constexpr (SPLIT) {
-    if (row < f64_rows) {
+    if (f64) {
       const double q = tabs64f.prime[pid].q, qinv = tabs64f.prime[pid].one_s;
       const RowX<double> xd(smem);
       using R = Rows<double, LOGN, TwAtQ>;
@@ -1055,34 +1075,82 @@ struct WordOutEpilogue {
   }
 };
 
+// One column tile of the inverse transform, in place.
 template <typename T, int LOGN, bool SPLIT>
-__global__ void __launch_bounds__(ColGeom<T, LOGN>::kThreads, col_blocks<T, LOGN>(false))
-k_ntt_columns_inverse(T* out, int rows, int row_start, int kind, ChainTables<T> tabs, ChainTables<double> tabs64f,
-                      int f64_rows) {
-  using G = ColGeom<T, LOGN>;
+__device__ __forceinline__ void ntt_columns_inverse(T* out, int pid, bool f64, int kind, const ChainTables<T>& tabs,
+                                                    const ChainTables<double>& tabs64f, int col0,
+                                                    unsigned char* smem) {
   constexpr int64_t kN = int64_t(1) << LOGN;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  const int col0 = int(blockIdx.x % G::kTiles) * G::kCols;
-  const int64_t poly = blockIdx.x / G::kTiles;
-  const int row = int(poly % rows), pid = row_start + row;
   if constexpr (SPLIT) {
-    if (row < f64_rows) {
+    if (f64) {
       const PrimeInfo<double>& p = tabs64f.prime[pid];
       const bool std_out = kind != kInvMontgomery;  // N^-1 R^-1 unless the output stays Montgomery
-      ColSource<double> src{reinterpret_cast<const double*>(out + poly * kN)};
-      WordOutEpilogue epi{out + poly * kN, p.q, std_out ? p.ninv_rinv : p.ninv, std_out ? p.ninv_rinv_s : p.ninv_s,
+      ColSource<double> src{reinterpret_cast<const double*>(out)};
+      WordOutEpilogue epi{out, p.q, std_out ? p.ninv_rinv : p.ninv, std_out ? p.ninv_rinv_s : p.ninv_s,
                           kind == kInvCentered};
-      Cols<double, LOGN, TwAtQ>::template inv<0>(src, epi, reinterpret_cast<double*>(smem_raw),
+      Cols<double, LOGN, TwAtQ>::template inv<0>(src, epi, reinterpret_cast<double*>(smem),
                                                  TwAtQ{tabs64f.twv_inv + int64_t(pid) * kN, p.one_s}, p.q, p.one_s,
                                                  col0);
       return;
     }
   }
   const PrimeInfo<T>& p = tabs.prime[pid];
-  ColSource<T> src{out + poly * kN};
-  InvEpilogue<T> epi = make_inv_epilogue<T>(out + poly * kN, p, kind, true);
-  Cols<T, LOGN, TwAt<T>>::template inv<0>(src, epi, reinterpret_cast<T*>(smem_raw),
+  ColSource<T> src{out};
+  InvEpilogue<T> epi = make_inv_epilogue<T>(out, p, kind, true);
+  Cols<T, LOGN, TwAt<T>>::template inv<0>(src, epi, reinterpret_cast<T*>(smem),
                                           TwAt<T>{tabs.tw_inv + int64_t(pid) * kN}, p.q, p.twice_q, col0);
+}
+
+template <typename T, int LOGN, bool TO_MONT, bool SPLIT>
+__global__ void __launch_bounds__(ColGeom<T, LOGN>::kThreads, col_blocks<T, LOGN>(false))
+k_ntt_columns(const T* in, T* out, int rows, int row_start, ChainTables<T> tabs, ChainTables<double> tabs64f,
+              int f64_rows) {
+  using G = ColGeom<T, LOGN>;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const int64_t poly = blockIdx.x / G::kTiles, at = poly << LOGN;
+  const int row = int(poly % rows);
+  ntt_columns<T, LOGN, TO_MONT, SPLIT>(in + at, out + at, row_start + row, row < f64_rows, tabs, tabs64f,
+                                       int(blockIdx.x % G::kTiles) * G::kCols, smem_raw);
+}
+
+template <typename T, int LOGN, bool SPLIT>
+__global__ void __launch_bounds__(kRowThreads, sizeof(T) == 8 ? 5 : 8)
+k_ntt_rows(T* out, int64_t slots, int rows, int row_start, ChainTables<T> tabs, ChainTables<double> tabs64f,
+           int f64_rows) {
+  constexpr int kBlks = 1 << (LOGN - kBlkLog);
+  __shared__ __align__(16) unsigned char smem[exchange_smem<T>()];
+  const int64_t slot = int64_t(blockIdx.x) * kRowSlots + (threadIdx.x >> 4);
+  if (slot >= slots) return;  // a whole warp: a polynomial has an even number of rows of 256 words
+  const int64_t poly = slot / kBlks;
+  const int row = int(poly % rows);
+  ntt_rows<T, LOGN, SPLIT>(out + (poly << LOGN), row_start + row, row < f64_rows, tabs, tabs64f, int(slot % kBlks),
+                           smem);
+}
+
+template <typename T, int LOGN, bool SPLIT>
+__global__ void __launch_bounds__(kRowThreads, sizeof(T) == 8 ? 5 : 8)
+k_ntt_rows_inverse(const T* in, T* out, int64_t slots, int rows, int row_start, ChainTables<T> tabs,
+                   ChainTables<double> tabs64f, int f64_rows) {
+  constexpr int kBlks = 1 << (LOGN - kBlkLog);
+  __shared__ __align__(16) unsigned char smem[exchange_smem<T>()];
+  const int64_t slot = int64_t(blockIdx.x) * kRowSlots + (threadIdx.x >> 4);
+  if (slot >= slots) return;
+  const int64_t poly = slot / kBlks, at = poly << LOGN;
+  const int row = int(poly % rows);
+  ntt_rows_inverse<T, LOGN, SPLIT>(in + at, out + at, row_start + row, row < f64_rows, tabs, tabs64f,
+                                   int(slot % kBlks), smem);
+}
+
+template <typename T, int LOGN, bool SPLIT>
+__global__ void __launch_bounds__(ColGeom<T, LOGN>::kThreads, col_blocks<T, LOGN>(false))
+k_ntt_columns_inverse(T* out, int rows, int row_start, int kind, ChainTables<T> tabs, ChainTables<double> tabs64f,
+                      int f64_rows) {
+  using G = ColGeom<T, LOGN>;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const int64_t poly = blockIdx.x / G::kTiles;
+  const int row = int(poly % rows);
+  ntt_columns_inverse<T, LOGN, SPLIT>(out + (poly << LOGN), row_start + row, row < f64_rows, kind, tabs, tabs64f,
+                                      int(blockIdx.x % G::kTiles) * G::kCols, smem_raw);
 }
 
 // ---------------------------------------------------------------------------

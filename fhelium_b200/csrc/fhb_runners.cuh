@@ -207,6 +207,7 @@ KsPass<T> ks_pass_args(const Context& c, int level) {
   k.q_limbs = c.num_q - level, k.qp_limbs = k.q_limbs + c.num_p, k.level = level, k.qp0 = c.qp();
   k.f_cnt = sizeof(T) == 8 ? f64_rows(c, level, k.q_limbs) : 0;
   k.i_lo = k.f_cnt, k.i_cnt = k.qp_limbs - k.f_cnt;
+  k.terms = 1;
   k.ext_digits = c.ext64f_digits, k.f64_end = c.f64_prime_end;
   k.tabs = tables<T>(c), k.lt = level_tables<T>(c, level);
   k.tabs64f = c.t64f, k.ext64f = c.ext64f;
@@ -227,6 +228,59 @@ int launch_ks_pass(const KsPass<T>& k, int digits, bool pre, cudaStream_t st) {
   if (rc != 0) return rc;
   return launch_blocks(k_ks_columns_inverse<T, LOGN, SPLIT>, int64_t(2) * k.batch * k.rows() * G::kTiles, G::kThreads,
                        G::smem_bytes(), st, k);
+}
+
+// Launch 1 over the ciphertexts of all terms, then launches 2 and 3 over the sums.
+template <typename T, int LOGN, bool SPLIT>
+int launch_ks_sum(KsPass<T> k, int digits, int terms, bool pre, cudaStream_t st) {
+  using G = ColGeom<T, LOGN>;
+  const int batch = k.batch;
+  k.batch = batch * terms;
+  const int64_t units = (k.f_cnt + 1) / 2 + k.i_cnt, blocks = int64_t(digits) * k.batch * units * G::kTiles;
+  int rc = pre ? launch_blocks(k_ks_columns<T, LOGN, true, SPLIT>, blocks, G::kThreads, G::smem_bytes(), st, k)
+               : launch_blocks(k_ks_columns<T, LOGN, false, SPLIT>, blocks, G::kThreads,
+                               ks_columns_smem<T, LOGN>(SPLIT), st, k);
+  if (rc != 0) return rc;
+  k.batch = batch, k.terms = terms;
+  const int64_t slots = (int64_t(batch) << (LOGN - kBlkLog));
+  rc = launch_blocks(k_ks_rows<T, LOGN, SPLIT>, (slots + kRowSlots - 1) / kRowSlots * k.rows(), kRowThreads, 0, st, k);
+  if (rc != 0) return rc;
+  return launch_blocks(k_ks_columns_inverse<T, LOGN, SPLIT>, int64_t(2) * batch * k.rows() * G::kTiles, G::kThreads,
+                       G::smem_bytes(), st, k);
+}
+
+// Sum of the key switches of `terms` x batch ciphertexts, each term with its
+// own key, in the groups of rows that `y` has room for (pre: the extensions).
+template <typename T, int LOGN>
+int run_ks_sum_pass(const Context& c, const void* digits, void* y, int64_t y_words, const uint64_t* key_ptrs,
+                    void* acc0, void* acc1, int terms, int64_t batch, int level, cudaStream_t st, bool pre) {
+  KsPass<T> k = ks_pass_args<T>(c, level);
+  const int qpl = k.qp_limbs, nd = k.lt.num_digits, f64 = k.f_cnt, ints = k.i_cnt;
+  const int64_t per_row = int64_t(nd) * terms * batch * c.n();
+  if (batch * terms > kMaxPassGroup) return fail(-6, "too many ciphertexts for one launch");
+  k.digits = static_cast<const T*>(digits);
+  k.y = static_cast<T*>(y);
+  k.item_keys = reinterpret_cast<const unsigned long long*>(key_ptrs);
+  k.acc0 = static_cast<T*>(acc0), k.acc1 = static_cast<T*>(acc1);
+  k.by_row = pre, k.batch = int(batch), k.y_batch = int(batch) * terms;
+  const int step = pre ? qpl : int(std::min<int64_t>(qpl, y_words / per_row));
+  if (step < 1) return fail(-8, "no room for the transform's intermediate");
+  for (int lo = 0; lo < qpl; lo += step) {
+    const int hi = std::min(qpl, lo + step);
+    k.i_lo = f64 + lo * ints / qpl, k.i_cnt = f64 + hi * ints / qpl - k.i_lo;
+    k.f_lo = lo - (k.i_lo - f64), k.f_cnt = hi - lo - k.i_cnt;
+    k.y_rows = pre ? qpl : hi - lo;
+    int rc = 0;
+    if constexpr (sizeof(T) == 8) {
+      rc = f64 > 0 ? launch_ks_sum<T, LOGN, true>(k, nd, terms, pre, st)
+                   : launch_ks_sum<T, LOGN, false>(k, nd, terms, pre, st);
+    } else {
+      if (pre) return fail(-7, "the tensor-core basis conversion needs an int64 context");
+      rc = launch_ks_sum<T, LOGN, false>(k, nd, terms, false, st);
+    }
+    if (rc != 0) return rc;
+  }
+  return 0;
 }
 
 template <typename T, int LOGN>
@@ -402,6 +456,8 @@ int run_items(const Context& c, int stage, const void* items, int item_count, in
                                     cudaStream_t, const uint64_t*, const void*, bool, int64_t);                 \
   template int run_ks_pass<T, LOGN>(const Context&, const void*, void*, int64_t, const void*, void*, void*, int64_t, int, \
                                     cudaStream_t, const uint64_t*, const void*, bool, int64_t);                 \
+  template int run_ks_sum_pass<T, LOGN>(const Context&, const void*, void*, int64_t, const uint64_t*, void*, void*, \
+                                        int, int64_t, int, cudaStream_t, bool);                                 \
   template int run_ks_sum<T, LOGN>(const Context&, const void*, const uint64_t*, void*, void*, int, int64_t, int, \
                                    cudaStream_t, bool);                                                         \
   template int run_prepare<T, LOGN>(const Context&, const void*, void*, int64_t, int, cudaStream_t);            \

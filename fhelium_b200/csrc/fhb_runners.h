@@ -31,6 +31,10 @@ int run_ks_pass(const Context& c, const void* digits, void* y, int64_t y_words, 
 template <typename T, int LOGN>
 int run_ks_sum(const Context& c, const void* digits, const uint64_t* key_ptrs, void* acc0, void* acc1, int giants,
                int64_t batch, int level, cudaStream_t st, bool pre);
+// The sum as launches of column and block stages; `y` as for run_ks_pass.
+template <typename T, int LOGN>
+int run_ks_sum_pass(const Context& c, const void* digits, void* y, int64_t y_words, const uint64_t* key_ptrs,
+                    void* acc0, void* acc1, int terms, int64_t batch, int level, cudaStream_t st, bool pre);
 // Mixed-level item stages: 0 = forward NTT of the HMult operands, 1 =
 // inverse NTT of d2, 2 = key-switch core; `count` units of `units`, of
 // which the leading `f64_units` (stage 2) may run in FP64 arithmetic.

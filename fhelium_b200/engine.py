@@ -528,7 +528,7 @@ class CkksEngine:
     def rotate_and_sum(self, cts: Sequence[Ciphertext], keys: Sequence[RotationKey]) -> Ciphertext:
         """sum_i rotate_with_key(cts[i], keys[i]) with one ModDown for the
         whole sum: ModUp of every sigma_g(c1), the key switches accumulated
-        in the NTT domain (fhb_ckks_keyswitch_sum), one inverse NTT and one
+        in the NTT domain (fhb_ckks_keyswitch_sum_work), one inverse NTT and one
         ModDown with sum_i sigma_g(c0_i) added.  The sum is rounded once
         instead of once per term, so it is within len(cts) units of the sum
         of separately rounded rotations (not bit-identical to it)."""
@@ -547,13 +547,12 @@ class CkksEngine:
             self.ctx.call("fhb_ckks_modup_digits", nat.ptr(ct.c1), nat.ptr(digits[i]), b, level, key.galois_element, st)
         key_ptrs = torch.tensor([k.data.data_ptr() for k in keys], dtype=torch.int64, device=self.device)
         t = self._empty(2, b, limbs + self.num_p, self.n)
-        if self.basis_conversion == "tensor_cores":
-            # the giants' digits as one batch of len(cts) x b ciphertexts
-            words = int(self.ctx.lib.fhb_tc_basis_extend_words(self.ctx.handle, len(cts) * b, level))
-            ext = torch.empty(words, dtype=self.dtype, device=self.device)
-            self.ctx.call("fhb_tc_basis_extend", nat.ptr(digits), nat.ptr(ext), len(cts) * b, level, st)
-            self.ctx.call("fhb_ckks_keyswitch_sum_extended", nat.ptr(ext), nat.ptr(key_ptrs), nat.ptr(t[0]),
-                          nat.ptr(t[1]), len(cts), b, level, st)
+        # (a batch beyond the work buffer's launches takes the cluster kernel)
+        if len(cts) * b <= 4096:
+            nbytes = int(self.ctx.lib.fhb_ckks_keyswitch_sum_workspace_bytes(self.ctx.handle, len(cts), b, level))
+            work = torch.empty(nbytes, dtype=torch.uint8, device=self.device)
+            self.ctx.call("fhb_ckks_keyswitch_sum_work", nat.ptr(digits), nat.ptr(key_ptrs), nat.ptr(t[0]),
+                          nat.ptr(t[1]), nat.ptr(work), nbytes, len(cts), b, level, st)
         else:
             self.ctx.call("fhb_ckks_keyswitch_sum", nat.ptr(digits), nat.ptr(key_ptrs), nat.ptr(t[0]),
                           nat.ptr(t[1]), len(cts), b, level, st)

@@ -398,6 +398,16 @@ int fhb_ckks_keyswitch_sum(const fhb_context* ctx, const void* digits, const uin
 int fhb_ckks_keyswitch_sum_extended(const fhb_context* ctx, const void* ext, const uint64_t* key_ptrs, void* acc0,
                                     void* acc1, int giants, int64_t batch, int level, fhb_stream stream);
 
+/* fhb_ckks_keyswitch_sum with a work buffer, as column and block launches on
+ * every SM, in the context's basis-conversion form (the extensions of the
+ * tensor-core form are written to `work`).  Same result, faster.  work_bytes:
+ * fhb_ckks_keyswitch_sum_workspace_bytes; in the CUDA-core form a smaller
+ * buffer is accepted down to one row's transforms.  -1 for invalid sizes. */
+int64_t fhb_ckks_keyswitch_sum_workspace_bytes(const fhb_context* ctx, int giants, int64_t batch, int level);
+int fhb_ckks_keyswitch_sum_work(const fhb_context* ctx, const void* digits, const uint64_t* key_ptrs, void* acc0,
+                                void* acc1, void* work, int64_t work_bytes, int giants, int64_t batch, int level,
+                                fhb_stream stream);
+
 /* ---- mixed-level batches: one launch per stage over every item ----------
  * One item is one ciphertext (batch 1) with its own operation and level:
  * HMult + relinearise + rescale of a and b (kind 0), or a rotation of a by

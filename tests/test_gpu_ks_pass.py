@@ -99,3 +99,39 @@ def test_workspace_holds_the_required_scratch():
             assert need <= full <= need + (1 << 30)
     assert int(lib.fhb_ckks_keyswitch_workspace_bytes(eng.ctx.handle, -1, 0)) == -1
     assert int(lib.fhb_ckks_keyswitch_workspace_bytes(eng.ctx.handle, 1, eng.num_q)) == -1
+
+
+@pytest.mark.parametrize("form", ["cuda_cores", "tensor_cores"])
+@pytest.mark.parametrize("preset,log_n,level,batch,giants", [
+    ("slots8192_scale40_levels7_int64", 12, 2, 3, 5),
+    ("slots16384_scale50_levels12_int64", 15, 9, 1, 3),
+    ("slots8192_scale25_levels14_int32", 14, 11, 2, 2),
+])
+def test_key_switch_sum_equals_the_cluster_kernel(preset, log_n, level, batch, giants, form):
+    """Whole numbers: the canonical sums of the launches over a work buffer
+    equal the one-launch kernel's, in both forms, with one row's room and more."""
+    cfg, eng, orc = _engine(preset, log_n)
+    if form == "tensor_cores" and cfg.buffer_bit_length != 62:
+        pytest.skip("the tensor-core form needs an int64 chain")
+    rng = np.random.default_rng(9)
+    rows = orc.q_rows(level)
+    digits = to_dev(uniform_residues(rng, cfg.moduli, rows, (giants, batch), cfg.N), cfg)
+    keys = [to_dev(random_key(rng, cfg, cfg.N), cfg) for _ in range(giants)]
+    ptrs = torch.tensor([k.data_ptr() for k in keys], dtype=torch.int64, device="cuda")
+    shape = (2, batch, len(rows) + cfg.num_p_primes, cfg.N)
+    want = torch.empty(shape, dtype=cfg.torch_dtype, device="cuda")
+    eng.ctx.call("fhb_ckks_keyswitch_sum", nat.ptr(digits), nat.ptr(ptrs), nat.ptr(want[0]), nat.ptr(want[1]),
+                 giants, batch, level, eng._stream())
+    eng.basis_conversion = form
+    full = int(eng.ctx.lib.fhb_ckks_keyswitch_sum_workspace_bytes(eng.ctx.handle, giants, batch, level))
+    rows_all = len(rows) + cfg.num_p_primes
+    rooms = [full] if form == "tensor_cores" else [full // rows_all, 2 * (full // rows_all), full]
+    for room in rooms:
+        got = torch.full(shape, -1, dtype=cfg.torch_dtype, device="cuda")
+        work = torch.empty(room, dtype=torch.uint8, device="cuda")
+        eng.ctx.call("fhb_ckks_keyswitch_sum_work", nat.ptr(digits), nat.ptr(ptrs), nat.ptr(got[0]), nat.ptr(got[1]),
+                     nat.ptr(work), room, giants, batch, level, eng._stream())
+        assert torch.equal(got, want), room
+    with pytest.raises(nat.NativeCallError):
+        eng.ctx.call("fhb_ckks_keyswitch_sum_work", nat.ptr(digits), nat.ptr(ptrs), nat.ptr(got[0]), nat.ptr(got[1]),
+                     nat.ptr(work), rooms[0] - 16, giants, batch, level, eng._stream())
