@@ -550,7 +550,7 @@ def mixed_batch_leg(dev, stream, count=512, steps=3):
     torch.cuda.synchronize(dev)
     items_ms = _time_events(items.run, max(3, steps), stream)
     bad = {"items": mismatches(items)}
-    item_chunks, item_launches = len(items.chunks), items.launches_per_run
+    item_chunks, item_launches = len(items.chunks), items.kernel_launches_per_run
     peak_gb = {"items": torch.cuda.max_memory_allocated(dev) / 1e9}
     del items
     torch.cuda.empty_cache()

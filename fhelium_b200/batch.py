@@ -269,7 +269,7 @@ class MixedBatchExecutor:
 
 
 class MixedItemsExecutor:
-    """A fixed mixed batch as six library launches, whatever its levels.
+    """A fixed mixed batch as six stages, whatever its levels.
 
     Every ciphertext's operation becomes one item descriptor (level, Galois
     element, operand, key and output addresses) in a device plan, and each
@@ -278,9 +278,9 @@ class MixedItemsExecutor:
     ONE launch over all items, with work lists that map clusters to
     (item, row) units.  The operands are read in place (no gathers), so
     updating the ciphertexts' tensors between runs is seen.  Every item in
-    flight holds its own scratch (ModUp digits, two Q_l P accumulators, and
-    for HMult the operands' NTTs and ct3), so a batch whose scratch would
-    pass ``max_scratch_bytes`` runs as several such six-launch chunks in
+    flight holds its own scratch (ModUp digits, two Q_l P accumulators, the
+    core's intermediate, and for HMult the operands' NTTs and ct3), so a batch whose scratch would
+    pass ``max_scratch_bytes`` runs as several such six-stage chunks in
     stream order over one shared scratch.  Results are integer-equal to
     :class:`MixedBatchExecutor` and to :func:`run_per_ciphertext`.
     """
@@ -397,8 +397,13 @@ class MixedItemsExecutor:
 
     @property
     def launches_per_run(self) -> int:
-        """Library kernels one run launches."""
+        """Stages one run goes through (six a chunk, three without HMult items)."""
         return sum(6 if info.hmult_items else 3 for info, _ in self.chunks)
+
+    @property
+    def kernel_launches_per_run(self) -> int:
+        """Library kernels one run launches: two per transform stage, three for the key-switch core."""
+        return sum(10 if info.hmult_items else 5 for info, _ in self.chunks)
 
     def status(self) -> int:
         """First error the kernels raised since the last call (0: none), after

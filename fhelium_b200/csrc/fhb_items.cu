@@ -3,10 +3,10 @@
 // A plan is built once on the host from the caller's item descriptors and
 // uploaded into a caller-provided device buffer: the device descriptors (with
 // each item's scratch regions resolved), the list of HMult items, and the
-// (item, row) work lists of the three cluster stages.  A run then issues six
-// launches over all items, whatever their levels - forward NTT of the HMult
+// (item, row) work lists of the three transform stages.  A run then takes six
+// stages over all items, whatever their levels - forward NTT of the HMult
 // operands, tensor product, inverse NTT of d2, ModUp digits, key-switch core,
-// ModDown - and makes no host calls, so it can be captured in a CUDA graph
+// ModDown; two launches per transform, three for the core - and makes no host calls, so it can be captured in a CUDA graph
 // and replayed.  The reference runs such a batch as one engine call sequence
 // per ciphertext (fhelium/engine/ckks_engine.py:1530-1675, 2183-2300).
 #include <algorithm>
@@ -33,7 +33,7 @@ static_assert(sizeof(KsItem) == 88 && offsetof(KsItem, level) == 4, "device desc
 int64_t align_up(int64_t x) { return (x + kRegionAlign - 1) / kRegionAlign * kRegionAlign; }
 
 struct PlanLayout {
-  int64_t items_off, hmult_off, fwd_off, inv_off, core_off, status_off, plan_bytes;
+  int64_t items_off, hmult_off, fwd_off, inv_off, core_off, pair_off, pairs, status_off, plan_bytes;
 };
 
 PlanLayout layout_of(const fhb_items_plan_info& info) {
@@ -43,7 +43,11 @@ PlanLayout layout_of(const fhb_items_plan_info& info) {
   l.fwd_off = l.hmult_off + align_up(int64_t(info.hmult_items) * 4);
   l.inv_off = l.fwd_off + align_up(int64_t(info.forward_units) * int64_t(sizeof(ItemUnit)));
   l.core_off = l.inv_off + align_up(int64_t(info.inverse_units) * int64_t(sizeof(ItemUnit)));
-  l.status_off = l.core_off + align_up(int64_t(info.core_units) * int64_t(sizeof(ItemUnit)));
+  // the core's column launch: two FP64 rows or one other row per unit (every
+  // item leaves at most one FP64 row over; spare entries name no item)
+  l.pairs = int64_t(info.core_units - info.core_f64_units) + (int64_t(info.core_f64_units) + info.items + 1) / 2;
+  l.pair_off = l.core_off + align_up(int64_t(info.core_units) * int64_t(sizeof(ItemUnit)));
+  l.status_off = l.pair_off + align_up(l.pairs * int64_t(sizeof(ItemUnit)));
   l.plan_bytes = l.status_off + kRegionAlign;
   return l;
 }
@@ -65,18 +69,26 @@ class ItemsDeviceGuard {  // makes the context's device current for the call
   int prev_ = 0, dev_ = 0;
 };
 
-// Scratch words of one item: HMult ab (4 L) + ct3 (3 L); every item digits
-// (L) and the two accumulators (2 (L + P)).
+// Bytes of an item's `ab` region: the core's intermediate (digits x (L + P)
+// rows), which for HMult first holds the operands' transforms (4 L rows).
+int64_t item_ab_bytes(const Context& c, const fhb_ks_item& it) {
+  const int64_t l = c.num_q - it.level, row = int64_t(c.n()) * (c.bits / 8);
+  const int64_t core = int64_t(c.level_digits[it.level].size()) * (l + c.num_p);
+  return align_up(std::max(core, it.kind == FHB_ITEM_HMULT_RELIN_RESCALE ? 4 * l : 0) * row);
+}
+
+// Scratch bytes of one item: HMult ct3 (3 L); every item digits (L), the two
+// accumulators (2 (L + P)) and `ab`.
 int64_t item_scratch_bytes(const Context& c, const fhb_ks_item& it) {
   const int64_t l = c.num_q - it.level, lp = l + c.num_p, row = int64_t(c.n()) * (c.bits / 8);
-  int64_t b = align_up(l * row) + 2 * align_up(lp * row);
-  if (it.kind == FHB_ITEM_HMULT_RELIN_RESCALE) b += align_up(4 * l * row) + align_up(3 * l * row);
+  int64_t b = align_up(l * row) + 2 * align_up(lp * row) + item_ab_bytes(c, it);
+  if (it.kind == FHB_ITEM_HMULT_RELIN_RESCALE) b += align_up(3 * l * row);
   return b;
 }
 
 // Leading rows of an item's Q_l whose primes are below 2^42: the key-switch
 // core runs them in FP64 arithmetic (int64 chains with FP64 tables, unless
-// the FP64 core is switched off).
+// the FP64 core is switched off: the integer body then takes them).
 int f64_item_rows(const Context& c, int level) {
   if (c.bits != 64 || !c.f64_tables_ok) return 0;
   return std::max(0, std::min(c.num_q - level, c.f64_prime_end - level));
@@ -98,13 +110,15 @@ int check_item(const Context& c, const fhb_ks_item& it, int i) {
 }
 
 int run_stage(const Context& c, int stage, const ItemsView& iv, const void* units, int64_t count, cudaStream_t st,
-              int64_t f64_units = 0) {
+              const void* pairs = nullptr, int64_t pair_count = 0, int max_digits = 0) {
   if (count == 0) return 0;
 #define FHB_ITEMS_CASE(L)                                                                                       \
   case L:                                                                                                       \
     return c.bits == 64                                                                                         \
-               ? run_items<uint64_t, L>(c, stage, iv.items, iv.count, iv.status, units, count, st, f64_units) \
-               : run_items<uint32_t, L>(c, stage, iv.items, iv.count, iv.status, units, count, st);
+               ? run_items<uint64_t, L>(c, stage, iv.items, iv.count, iv.status, units, count, st, pairs, pair_count, \
+                                        max_digits)                                                              \
+               : run_items<uint32_t, L>(c, stage, iv.items, iv.count, iv.status, units, count, st, pairs, pair_count, \
+                                        max_digits);
   switch (c.log_n) {
     FHB_ITEMS_CASE(12)
     FHB_ITEMS_CASE(13)
@@ -138,7 +152,9 @@ int run_elementwise(const Context& c, const char* plan, const PlanLayout& l, con
   k_items_modup<T, V><<<dim3(xb, unsigned(info.max_digits), unsigned(info.items)), kEwThreads, 0, st>>>(
       iv, level_tables_dev<T>(c), c.num_q, c.log_n, tables<T>(c));
   if (int e = cuda_status(cudaGetLastError(), "k_items_modup")) return e;
-  if (int rc = run_stage(c, 2, iv, plan + l.core_off, info.core_units, st, info.core_f64_units)) return rc;
+  if (int rc = run_stage(c, 2, iv, plan + l.core_off, info.core_units, st, plan + l.pair_off, l.pairs,
+                         info.max_digits))
+    return rc;
   k_items_moddown<T><<<dim3(unsigned((n + 255) / 256), unsigned(info.items)), 256, 0, st>>>(
       iv, level_tables_dev<T>(c), c.num_q, c.num_p, c.log_n, tables<T>(c));
   return cuda_status(cudaGetLastError(), "k_items_moddown");
@@ -211,9 +227,9 @@ int fhb_ckks_items_plan(const fhb_context* ctx, const fhb_ks_item* items, int co
     sp += fhb::align_up(lp * row);
     d.t1 = sp;
     sp += fhb::align_up(lp * row);
+    d.ab = sp;
+    sp += fhb::item_ab_bytes(c, src);
     if (src.kind == FHB_ITEM_HMULT_RELIN_RESCALE) {
-      d.ab = sp;
-      sp += fhb::align_up(4 * ll * row);
       d.coef = sp;
       sp += fhb::align_up(3 * ll * row);
       hmult[nh++] = i;
@@ -226,7 +242,7 @@ int fhb_ckks_items_plan(const fhb_context* ctx, const fhb_ks_item* items, int co
   // Core work list: items of one (level, key) back to back; within such a
   // group, the context's key-switch work order picks one destination row
   // across the group's items (orders 1 and 2: concurrently resident
-  // clusters share key rows in L2) or the rows of one item back to back
+  // blocks share key rows in L2) or the rows of one item back to back
   // (order 0: an item's digit rows stay in L2).
   std::vector<int> order(count);
   for (int i = 0; i < count; ++i) order[i] = i;
@@ -250,6 +266,16 @@ int fhb_ckks_items_plan(const fhb_context* ctx, const fhb_ks_item* items, int co
     }
     g0 = g1;
   }
+  // The core's column launch: the rows of one item back to back (its digit
+  // rows stay in L2), FP64 rows in pairs.
+  auto* pairs = reinterpret_cast<fhb::ItemUnit*>(host.data() + l.pair_off);
+  int64_t np = 0;
+  for (int i : order) {
+    const int f = fhb::f64_item_rows(c, items[i].level), lp = c.num_q - items[i].level + c.num_p;
+    for (int r = 0; r < f; r += 2) pairs[np++] = fhb::ItemUnit{i, r + 1 < f ? r + fhb::kItemPair : r};
+    for (int r = f; r < lp; ++r) pairs[np++] = fhb::ItemUnit{i, r};
+  }
+  while (np < l.pairs) pairs[np++] = fhb::ItemUnit{fhb::kItemNone, fhb::kItemNone};
   fhb::ItemsDeviceGuard guard(c.device);
   return fhb::cuda_status(cudaMemcpy(plan, host.data(), host.size(), cudaMemcpyHostToDevice), "plan upload");
 }

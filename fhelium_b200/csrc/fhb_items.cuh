@@ -12,10 +12,11 @@
 // with c0, c1 folded in for relinearisation, ModDown with the rescale or
 // with sigma_g(c0)), and use the same building blocks, so every result is
 // integer-equal to the per-level batch calls.  Work lists of (item, row)
-// units map the cluster kernels' clusters to items; the element-wise kernels
+// units map the transform kernels' blocks to items; the element-wise kernels
 // take the item from the grid's z dimension.
 #pragma once
 #include "fhb_kernels.cuh"
+#include "fhb_pass.cuh"
 
 namespace fhb {
 
@@ -28,7 +29,8 @@ struct KsItem {
   const void* b;        // HMult rhs [2, L, N] coefficient/standard; null for a rotation
   const void* key;      // [D, 2, QP0, N] NTT/Montgomery key
   void* out;            // HMult [2, L - 1, N]; rotation [2, L, N]; coefficient/standard
-  void* ab;             // scratch: HMult [2 operands][2][L][N] NTT/Montgomery
+  void* ab;             // scratch: HMult [2 operands][2][L][N] NTT/Montgomery, then (and for rotations)
+                        // the core's intermediate [D][L + P][N]
   void* coef;           // scratch: HMult ct3 [3, L, N] NTT/Montgomery
   void* digits;         // scratch: [L, N] ModUp digits
   void* t0;             // scratch: [L + P, N] (d2 in the coefficient domain, then accumulator 0)
@@ -255,171 +257,218 @@ __global__ void k_items_moddown(ItemsView iv, const LevelTables<T>* __restrict__
   }
 }
 
-// Forward NTT of the HMult operands (k_ntt_forward per row): one cluster per
-// unit (item, operand 2 L + component L + row), coefficient/standard ->
-// NTT/Montgomery (x R), lazy [0, 2q), into the item's `ab`.  SPLIT (int64
-// chains with FP64 tables): the rows whose primes are below 2^42 (prime id
-// < f64_end) run the transform in FP64 arithmetic (as k_ntt_forward's SPLIT
-// form does); their lazy words may differ from the integer transform's by q,
-// which the later stages (all modular, canonical at the end) do not see.
-template <typename T, int LOGN, bool SPLIT = false>
-__global__ void __launch_bounds__(NttGeom<T, LOGN>::kThreads)
-k_items_ntt_forward(ItemsView iv, const ItemUnit* __restrict__ units, int num_q, ChainTables<T> tabs,
-                    ChainTables<double> tabs64f, int f64_end) {
-  using G = NttGeom<T, LOGN>;
-  static_assert(!SPLIT || (sizeof(T) == 8 && NttGeom<double, LOGN>::kC == G::kC &&
-                           NttGeom<double, LOGN>::kThreads == G::kThreads),
-                "the FP64 rows share the integer transform's geometry");
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  const int rank = cluster_rank<T, LOGN>();
-  // every CTA of the cluster reads the same unit, so an early return is cluster-uniform
-  const ItemUnit u = units[blockIdx.x / G::kC];
-  KsItem it;
-  if (!items_fetch(iv, u.item, it)) return;
+// The transform stages take their (item, row) from a work list.  Every thread
+// of a block reads the same unit in the column kernels, every half warp its
+// own in the row kernels (all warps of one unit have an even number of rows
+// of 256 words, so a warp never splits).  Rows of primes below 2^42 (prime id
+// < f64_end) run in FP64 arithmetic; their lazy words may differ from the
+// integer transform's by q, which the later stages (all modular, canonical at
+// the end) do not see.
+
+// Forward NTT of the HMult operands, unit row operand * 2 L + component * L +
+// row: coefficient/standard -> NTT/Montgomery (x R), into the item's `ab`.
+template <typename T>
+__device__ __forceinline__ bool items_forward_unit(const ItemsView& iv, const ItemUnit& u, int num_q, int64_t n,
+                                                   KsItem& it, const T*& in, T*& out, int& pid) {
+  if (!items_fetch(iv, u.item, it)) return false;
   const int limbs = num_q - it.level;
   if (it.kind != 0) {
     items_raise(iv.status, kItemsBadKind);
-    return;
+    return false;
   }
   if (u.row < 0 || u.row >= 4 * limbs) {
     items_raise(iv.status, kItemsBadRow);
-    return;
+    return false;
   }
   const int op = u.row / (2 * limbs), rem = u.row - op * 2 * limbs;  // rem = component L + row
-  const int pid = it.level + rem % limbs;
-  const T* in = static_cast<const T*>(op == 0 ? it.a : it.b) + int64_t(rem) * G::kN;
-  T* out = static_cast<T*>(it.ab) + int64_t(u.row) * G::kN + int64_t(rank) * G::kM + threadIdx.x * G::kE;
-  if constexpr (SPLIT) {
-    if (pid < f64_end) {
-      const PrimeInfo<double> p = tabs64f.prime[pid];
-      U64MontSource<true> src{reinterpret_cast<const uint64_t*>(in), p.rmod, p.rmod_s, p.q};
-      double v[G::kE];
-      Ntt<double, LOGN, TwGlobalQ<LOGN>>::forward_from(src, reinterpret_cast<double*>(smem_raw),
-                                                       TwGlobalQ<LOGN>{tabs64f.twv_fwd + int64_t(pid) * G::kN, p.one_s},
-                                                       p.q, p.one_s, rank, v);
-#pragma unroll
-      for (int e = 0; e < G::kE; ++e) v[e] = Word<double>::to_lazy(v[e], p.q, p.one_s);
-      store_words(reinterpret_cast<uint64_t*>(out), v);
-      return;
-    }
-  }
-  const PrimeInfo<T> p = tabs.prime[pid];
-  RowSource<T, true> src{in, p.rmod, p.rmod_s, p.q};
-  T v[G::kE];
-  Ntt<T, LOGN>::forward_from(src, reinterpret_cast<T*>(smem_raw), TwGlobal<T, LOGN>(tabs.tw_fwd + int64_t(pid) * G::kN),
-                             p.q, p.twice_q, rank, v);
-#pragma unroll
-  for (int e = 0; e < G::kE; ++e) v[e] = csub(v[e], p.twice_q);
-  store16(out, v);
+  pid = it.level + rem % limbs;
+  in = static_cast<const T*>(op == 0 ? it.a : it.b) + int64_t(rem) * n;
+  out = static_cast<T*>(it.ab) + int64_t(u.row) * n;
+  return true;
 }
 
-// Inverse NTT of d2 of the HMult items (k_ntt_inverse per row): one cluster
-// per unit (item, row), NTT/Montgomery -> coefficient/standard canonical,
-// into the item's t0.  SPLIT: rows of primes below 2^42 in FP64 arithmetic
-// (as k_ntt_inverse's SPLIT form), the same canonical words.
-template <typename T, int LOGN, bool SPLIT = false>
-__global__ void __launch_bounds__(NttGeom<T, LOGN>::kThreads)
-k_items_ntt_inverse(ItemsView iv, const ItemUnit* __restrict__ units, int num_q, ChainTables<T> tabs,
-                    ChainTables<double> tabs64f, int f64_end) {
-  using G = NttGeom<T, LOGN>;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  const int rank = cluster_rank<T, LOGN>();
-  const ItemUnit u = units[blockIdx.x / G::kC];
-  KsItem it;
-  if (!items_fetch(iv, u.item, it)) return;
+// Inverse NTT of d2 of the HMult items, unit row a Q_l row: NTT/Montgomery ->
+// coefficient/standard canonical, into the item's t0.
+template <typename T>
+__device__ __forceinline__ bool items_inverse_unit(const ItemsView& iv, const ItemUnit& u, int num_q, int64_t n,
+                                                   KsItem& it, const T*& in, T*& out, int& pid) {
+  if (!items_fetch(iv, u.item, it)) return false;
   const int limbs = num_q - it.level;
   if (it.kind != 0) {
     items_raise(iv.status, kItemsBadKind);
-    return;
+    return false;
   }
   if (u.row < 0 || u.row >= limbs) {
     items_raise(iv.status, kItemsBadRow);
-    return;
+    return false;
   }
-  const int pid = it.level + u.row;
-  const T* in = static_cast<const T*>(it.coef) + int64_t(2 * limbs + u.row) * G::kN + int64_t(rank) * G::kM +
-                threadIdx.x * G::kE;
-  T* out = static_cast<T*>(it.t0) + int64_t(u.row) * G::kN;
-  T w[G::kE];
-  load16(in, w);
-  if constexpr (SPLIT) {
-    if (pid < f64_end) {
-      const PrimeInfo<double> p = tabs64f.prime[pid];
-      double v[G::kE];
-#pragma unroll
-      for (int e = 0; e < G::kE; ++e) v[e] = __ull2double_rn(w[e]);
-      F64OutEpilogue epi{reinterpret_cast<uint64_t*>(out), p.q, p.ninv_rinv, p.ninv_rinv_s, kInvStandard};
-      Ntt<double, LOGN, TwGlobalQ<LOGN>>::inverse(reinterpret_cast<double*>(smem_raw),
-                                                  TwGlobalQ<LOGN>{tabs64f.twv_inv + int64_t(pid) * G::kN, p.one_s},
-                                                  p.q, p.one_s, rank, v, epi);
-      return;
-    }
-  }
-  const PrimeInfo<T> p = tabs.prime[pid];
-  InvEpilogue<T> epi = make_inv_epilogue<T>(out, p, kInvStandard, true);
-  Ntt<T, LOGN>::inverse(reinterpret_cast<T*>(smem_raw), TwGlobal<T, LOGN>(tabs.tw_inv + int64_t(pid) * G::kN), p.q,
-                        p.twice_q, rank, w, epi);
+  pid = it.level + u.row;
+  in = static_cast<const T*>(it.coef) + int64_t(2 * limbs + u.row) * n;
+  out = static_cast<T*>(it.t0) + int64_t(u.row) * n;
+  return true;
 }
 
-// Key-switch core of every item (k_keyswitch_core per (ciphertext, row)):
-// one cluster per unit (item, destination row of Q_l P).  For HMult items
-// the NTT-domain ct3 is folded in (c0, c1 as P c_k, own-digit rows from c2).
-// Returns false (status raised) for a unit outside its item's rows.
-__device__ __forceinline__ bool items_core_unit(const ItemsView& iv, const ItemUnit& u, int num_q, int num_p,
-                                                KsItem& it) {
-  if (!items_fetch(iv, u.item, it)) return false;
-  if (u.row < 0 || u.row >= num_q - it.level + num_p) {
+template <typename T, int LOGN, bool INVERSE, bool SPLIT>
+__global__ void __launch_bounds__(ColGeom<T, LOGN>::kThreads, col_blocks<T, LOGN>(false))
+k_items_ntt_columns(ItemsView iv, const ItemUnit* __restrict__ units, int num_q, ChainTables<T> tabs,
+                    ChainTables<double> tabs64f, int f64_end) {
+  using G = ColGeom<T, LOGN>;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  KsItem it;
+  const T* in;
+  T* out;
+  int pid;
+  const ItemUnit u = units[blockIdx.x / G::kTiles];
+  const int col0 = int(blockIdx.x % G::kTiles) * G::kCols;
+  if constexpr (INVERSE) {
+    if (!items_inverse_unit<T>(iv, u, num_q, int64_t(1) << LOGN, it, in, out, pid)) return;
+    ntt_columns_inverse<T, LOGN, SPLIT>(out, pid, pid < f64_end, kInvStandard, tabs, tabs64f, col0, smem_raw);
+  } else {
+    if (!items_forward_unit<T>(iv, u, num_q, int64_t(1) << LOGN, it, in, out, pid)) return;
+    ntt_columns<T, LOGN, true, SPLIT>(in, out, pid, pid < f64_end, tabs, tabs64f, col0, smem_raw);
+  }
+}
+
+template <typename T, int LOGN, bool INVERSE, bool SPLIT>
+__global__ void __launch_bounds__(kRowThreads, sizeof(T) == 8 ? 5 : 8)
+k_items_ntt_rows(ItemsView iv, const ItemUnit* __restrict__ units, int64_t slots, int num_q, ChainTables<T> tabs,
+                 ChainTables<double> tabs64f, int f64_end) {
+  constexpr int kBlks = 1 << (LOGN - kBlkLog);
+  __shared__ __align__(16) unsigned char smem[exchange_smem<T>()];
+  const int64_t slot = int64_t(blockIdx.x) * kRowSlots + (threadIdx.x >> 4);
+  if (slot >= slots) return;
+  KsItem it;
+  const T* in;
+  T* out;
+  int pid;
+  const ItemUnit u = units[slot / kBlks];
+  const int blk = int(slot % kBlks);
+  if constexpr (INVERSE) {
+    if (!items_inverse_unit<T>(iv, u, num_q, int64_t(1) << LOGN, it, in, out, pid)) return;
+    ntt_rows_inverse<T, LOGN, SPLIT>(in, out, pid, pid < f64_end, tabs, tabs64f, blk, smem);
+  } else {
+    if (!items_forward_unit<T>(iv, u, num_q, int64_t(1) << LOGN, it, in, out, pid)) return;
+    ntt_rows<T, LOGN, SPLIT>(out, pid, pid < f64_end, tabs, tabs64f, blk, smem);
+  }
+}
+
+// Key-switch core of every item: the three launches of fhb_pass.cuh over
+// units (item, destination row of Q_l P); the column launch's units name two
+// adjacent rows with kItemPair (both in FP64 arithmetic when the form is on).
+// For HMult items the NTT-domain ct3 is folded in (c0, c1 as P c_k, own-digit
+// rows from c2).
+constexpr int32_t kItemPair = 1 << 24;
+constexpr int32_t kItemNone = -1;  // fills the column launch's list
+
+// False (status raised) for a unit outside its item's rows.
+__device__ __forceinline__ bool items_core_unit(const ItemsView& iv, int item, int row, int rows_named, int num_q,
+                                                int num_p, KsItem& it) {
+  if (!items_fetch(iv, item, it)) return false;
+  if (row < 0 || row + rows_named > num_q - it.level + num_p) {
     items_raise(iv.status, kItemsBadRow);
     return false;
   }
   return true;
 }
 
-template <typename T, int LOGN>
-__global__ void __launch_bounds__(NttGeom<T, LOGN>::kThreads)
-k_items_core(ItemsView iv, const ItemUnit* __restrict__ units, const LevelTables<T>* __restrict__ levels, int num_q,
-             int num_p, ChainTables<T> tabs) {
-  using G = NttGeom<T, LOGN>;
+template <typename T>
+struct ItemsCore {
+  const LevelTables<T>* levels;
+  int num_q, num_p, ext_digits, f64_end;
+  ChainTables<T> tabs;
+  ChainTables<double> tabs64f;
+  const TwPair<double>* ext64f;
+  // The item as a batch of one, every row's intermediate in `ab`.
+  __device__ __forceinline__ KsPass<T> pass(const KsItem& it, int64_t n) const {
+    KsPass<T> k;
+    k.digits = static_cast<const T*>(it.digits);
+    k.y = static_cast<T*>(it.ab);
+    k.key = static_cast<const T*>(it.key);
+    k.item_keys = nullptr;
+    k.acc0 = static_cast<T*>(it.t0), k.acc1 = static_cast<T*>(it.t1);
+    k.q_limbs = num_q - it.level, k.qp_limbs = k.q_limbs + num_p, k.level = it.level, k.qp0 = num_q + num_p;
+    k.ct3 = it.kind == 0 ? static_cast<const T*>(it.coef) : nullptr;
+    k.ct3_stride = int64_t(k.q_limbs) * n;
+    k.batch = k.y_batch = k.by_row = k.terms = 1;
+    k.y_rows = k.qp_limbs;
+    k.f_lo = k.f_cnt = k.i_lo = k.i_cnt = 0;
+    k.ext_digits = ext_digits, k.f64_end = f64_end;
+    k.tabs = tabs, k.lt = levels[it.level], k.tabs64f = tabs64f, k.ext64f = ext64f;
+    return k;
+  }
+};
+
+// Blocks (unit, column tile, digit), digits fastest; digits past an item's level return.
+template <typename T, int LOGN, bool SPLIT>
+__global__ void __launch_bounds__(ColGeom<T, LOGN>::kThreads, col_blocks<T, LOGN>(SPLIT))
+k_items_core_columns(ItemsView iv, const ItemUnit* __restrict__ units, int max_digits,
+                     const __grid_constant__ ItemsCore<T> core) {
+  using G = ColGeom<T, LOGN>;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  const ItemUnit u = units[blockIdx.x / G::kC];  // the same unit on every CTA of the cluster
+  unsigned idx = blockIdx.x;
+  const int a = int(idx % unsigned(max_digits));
+  idx /= unsigned(max_digits);
+  const int col0 = int(idx % G::kTiles) * G::kCols;
+  const ItemUnit u = units[idx / G::kTiles];
+  if (u.item == kItemNone && u.row == kItemNone) return;
+  const int named = u.row >= kItemPair ? 2 : 1, j0 = u.row >= kItemPair ? u.row - kItemPair : u.row;
   KsItem it;
-  if (!items_core_unit(iv, u, num_q, num_p, it)) return;
-  const int q_limbs = num_q - it.level;
-  ks_core_unit<T, LOGN, false>(static_cast<const T*>(it.digits), static_cast<const T*>(it.key),
-                               static_cast<T*>(it.t0), static_cast<T*>(it.t1), 1, q_limbs, q_limbs + num_p, it.level,
-                               num_q + num_p, it.kind == 0 ? static_cast<const T*>(it.coef) : nullptr,
-                               int64_t(q_limbs) * G::kN, tabs, levels[it.level], 0, u.row, smem_raw,
-                               cluster_rank<T, LOGN>());
+  if (!items_core_unit(iv, u.item, j0, named, core.num_q, core.num_p, it)) return;
+  const KsPass<T> k = core.pass(it, int64_t(1) << LOGN);
+  if (a >= k.lt.num_digits) return;
+  if constexpr (SPLIT) {
+    if (it.level + j0 < core.f64_end) {
+      const bool two = named == 2 && it.level + j0 + 1 < core.f64_end;
+      const DigitDesc d = k.lt.digits[a];
+      ks_columns_f64<LOGN, false>(k, a, 0, col0, j0, j0 + 1, !ks_own(k, d, j0), two && !ks_own(k, d, j0 + 1),
+                                  smem_raw);
+      return;
+    }
+  }
+  for (int i = 0; i < named; ++i) {
+    if (i) __syncthreads();
+    ks_columns_int<T, LOGN, false>(k, a, 0, col0, j0 + i, smem_raw);
+  }
 }
 
-// The same for an int64 chain with FP64 tables: the units of rows whose
-// primes are below 2^42 run the FP64 body (k_keyswitch_core_split), the
-// others the integer body, in one launch.  ext64f [level][digit][r][2][QP]
-// of ext_digits digits per level.
-template <int LOGN>
-__global__ void __launch_bounds__(NttGeom<double, LOGN>::kThreads)
-k_items_core_split(ItemsView iv, const ItemUnit* __restrict__ units, const LevelTables<uint64_t>* __restrict__ levels,
-                   int num_q, int num_p, ChainTables<uint64_t> tabs, ChainTables<double> tabs64f,
-                   const TwPair<double>* __restrict__ ext64f, int ext_digits, int f64_end) {
-  using G = NttGeom<double, LOGN>;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  const ItemUnit u = units[blockIdx.x / G::kC];
+template <typename T, int LOGN, bool SPLIT>
+__global__ void __launch_bounds__(kRowThreads, sizeof(T) == 8 ? 3 : 4)
+k_items_core_rows(ItemsView iv, const ItemUnit* __restrict__ units, int64_t slots,
+                  const __grid_constant__ ItemsCore<T> core) {
+  constexpr int kBlks = 1 << (LOGN - kBlkLog);
+  __shared__ __align__(16) unsigned char smem[row_smem<T>()];
+  const int64_t slot = int64_t(blockIdx.x) * kRowSlots + (threadIdx.x >> 4);
+  if (slot >= slots) return;
+  const ItemUnit u = units[slot / kBlks];
+  const int blk = int(slot % kBlks);
   KsItem it;
-  if (!items_core_unit(iv, u, num_q, num_p, it)) return;
-  const int q_limbs = num_q - it.level, qp_limbs = q_limbs + num_p, qp0 = num_q + num_p;
-  const uint64_t* ct3 = it.kind == 0 ? static_cast<const uint64_t*>(it.coef) : nullptr;
-  const int rank = cluster_rank<double, LOGN>();
-  const LevelTables<uint64_t> lt = levels[it.level];
-  if (it.level + u.row < f64_end)
-    ks_core_unit_f64<LOGN, false>(static_cast<const uint64_t*>(it.digits), static_cast<const uint64_t*>(it.key),
-                                  static_cast<uint64_t*>(it.t0), static_cast<uint64_t*>(it.t1), 1, q_limbs, qp_limbs,
-                                  it.level, qp0, ct3, int64_t(q_limbs) * G::kN, tabs64f, lt, ext64f, ext_digits,
-                                  f64_end, 0, u.row, smem_raw, rank);
-  else
-    ks_core_unit<uint64_t, LOGN, false>(static_cast<const uint64_t*>(it.digits),
-                                        static_cast<const uint64_t*>(it.key), static_cast<uint64_t*>(it.t0),
-                                        static_cast<uint64_t*>(it.t1), 1, q_limbs, qp_limbs, it.level, qp0, ct3,
-                                        int64_t(q_limbs) * G::kN, tabs, lt, 0, u.row, smem_raw, rank);
+  if (!items_core_unit(iv, u.item, u.row, 1, core.num_q, core.num_p, it)) return;
+  const KsPass<T> k = core.pass(it, int64_t(1) << LOGN);
+  if constexpr (SPLIT) {
+    if (it.level + u.row < core.f64_end) {
+      ks_rows_f64<LOGN>(k, u.row, 0, blk, true, smem);
+      return;
+    }
+  }
+  ks_rows_int<T, LOGN>(k, u.row, 0, blk, true, smem);
+}
+
+// Blocks (unit, component, column tile).
+template <typename T, int LOGN, bool SPLIT>
+__global__ void __launch_bounds__(ColGeom<T, LOGN>::kThreads, col_blocks<T, LOGN>(false))
+k_items_core_columns_inverse(ItemsView iv, const ItemUnit* __restrict__ units,
+                             const __grid_constant__ ItemsCore<T> core) {
+  using G = ColGeom<T, LOGN>;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  unsigned idx = blockIdx.x;
+  const int col0 = int(idx % G::kTiles) * G::kCols;
+  idx /= G::kTiles;
+  const ItemUnit u = units[idx / 2];
+  KsItem it;
+  if (!items_core_unit(iv, u.item, u.row, 1, core.num_q, core.num_p, it)) return;
+  T* z = static_cast<T*>(idx & 1 ? it.t1 : it.t0) + (int64_t(u.row) << LOGN);
+  const int pid = it.level + u.row;
+  ks_columns_inverse<T, LOGN, SPLIT>(z, pid, SPLIT && pid < core.f64_end, core.tabs, core.tabs64f, col0, smem_raw);
 }
 
 }  // namespace fhb

@@ -412,39 +412,51 @@ int run_apply_prepared(const Context& c, const void* prepared, const void* key, 
   return run(k_apply_rows<T, LOGN, false>, k_ks_columns_inverse<T, LOGN, false>);
 }
 
-// ---- mixed-level item stages (fhb_items.cuh): one cluster per unit ----------
+// ---- mixed-level item stages (fhb_items.cuh) ---------------------------------
+template <typename T, int LOGN, bool SPLIT>
+int run_items_form(const Context& c, int stage, const ItemsView& iv, const ItemUnit* un, int64_t count,
+                   const ItemUnit* column_units, int64_t column_count, int max_digits, cudaStream_t st) {
+  using G = ColGeom<T, LOGN>;
+  const int64_t slots = count << (LOGN - kBlkLog), row_blocks = (slots + kRowSlots - 1) / kRowSlots;
+  auto columns = [&](auto kern, int64_t blocks, size_t smem, auto... args) {
+    return launch_blocks(kern, blocks, G::kThreads, smem, st, iv, args...);
+  };
+  auto rows = [&](auto kern, auto... args) {
+    return launch_blocks(kern, row_blocks, kRowThreads, 0, st, iv, un, slots, args...);
+  };
+  if (stage == 0) {
+    const int rc = columns(k_items_ntt_columns<T, LOGN, false, SPLIT>, count * G::kTiles, G::smem_bytes(), un, c.num_q,
+                           tables<T>(c), c.t64f, c.f64_prime_end);
+    return rc ? rc : rows(k_items_ntt_rows<T, LOGN, false, SPLIT>, c.num_q, tables<T>(c), c.t64f, c.f64_prime_end);
+  }
+  if (stage == 1) {
+    const int rc = rows(k_items_ntt_rows<T, LOGN, true, SPLIT>, c.num_q, tables<T>(c), c.t64f, c.f64_prime_end);
+    return rc ? rc
+              : columns(k_items_ntt_columns<T, LOGN, true, SPLIT>, count * G::kTiles, G::smem_bytes(), un, c.num_q,
+                        tables<T>(c), c.t64f, c.f64_prime_end);
+  }
+  const ItemsCore<T> core{level_tables_dev<T>(c), c.num_q, c.num_p, c.ext64f_digits, c.f64_prime_end, tables<T>(c),
+                          c.t64f, c.ext64f};
+  int rc = columns(k_items_core_columns<T, LOGN, SPLIT>, column_count * G::kTiles * max_digits,
+                   ks_columns_smem<T, LOGN>(SPLIT), column_units, max_digits, core);
+  if (rc != 0) return rc;
+  rc = rows(k_items_core_rows<T, LOGN, SPLIT>, core);
+  if (rc != 0) return rc;
+  return columns(k_items_core_columns_inverse<T, LOGN, SPLIT>, 2 * count * G::kTiles, G::smem_bytes(), un, core);
+}
+
 template <typename T, int LOGN>
 int run_items(const Context& c, int stage, const void* items, int item_count, int* status, const void* units,
-              int64_t count, cudaStream_t st, int64_t f64_units) {
+              int64_t count, cudaStream_t st, const void* column_units, int64_t column_count, int max_digits) {
   const ItemsView iv{static_cast<const KsItem*>(items), item_count, status};
   const auto* un = static_cast<const ItemUnit*>(units);
+  const auto* cu = static_cast<const ItemUnit*>(column_units);
   // int64 chains with FP64 tables: the rows of primes below 2^42 in FP64 arithmetic
-  const bool split = sizeof(T) == 8 && c.f64_core && c.f64_tables_ok && c.f64_prime_end > 0;
-  if (stage < 2) {
-    auto launch = [&](auto kern) {
-      return launch_cluster<T, LOGN>(kern, count, ntt_smem<T, LOGN>(), st, iv, un, c.num_q, tables<T>(c), c.t64f,
-                                     c.f64_prime_end);
-    };
-    if constexpr (sizeof(T) == 8) {
-      if (split)
-        return stage == 0 ? launch(k_items_ntt_forward<T, LOGN, true>) : launch(k_items_ntt_inverse<T, LOGN, true>);
-    }
-    return stage == 0 ? launch(k_items_ntt_forward<T, LOGN>) : launch(k_items_ntt_inverse<T, LOGN>);
-  }
-  // stage 2, the key-switch core; on an int64 chain with FP64 tables the
-  // units of rows whose primes are below 2^42 run in FP64 arithmetic
   if constexpr (sizeof(T) == 8) {
-    if constexpr (KsAcc<double, LOGN>::kSmem) {
-      static_assert(KsAcc<double, LOGN>::smem_bytes() == KsAcc<T, LOGN>::smem_bytes(), "one smem size for both");
-      if (split && f64_units > 0)
-        return launch_cluster<double, LOGN>(k_items_core_split<LOGN>, count, KsAcc<double, LOGN>::smem_bytes(), st,
-                                            iv, un, level_tables_dev<uint64_t>(c), c.num_q, c.num_p,
-                                            tables<uint64_t>(c), c.t64f, c.ext64f, c.ext64f_digits,
-                                            c.f64_prime_end);
-    }
+    if (c.f64_core && c.f64_tables_ok && c.f64_prime_end > 0)
+      return run_items_form<T, LOGN, true>(c, stage, iv, un, count, cu, column_count, max_digits, st);
   }
-  return launch_cluster<T, LOGN>(k_items_core<T, LOGN>, count, KsAcc<T, LOGN>::smem_bytes(), st, iv, un,
-                                 level_tables_dev<T>(c), c.num_q, c.num_p, tables<T>(c));
+  return run_items_form<T, LOGN, false>(c, stage, iv, un, count, cu, column_count, max_digits, st);
 }
 
 // Explicit instantiation of every runner for one (T, LOGN).
@@ -462,7 +474,7 @@ int run_items(const Context& c, int stage, const void* items, int item_count, in
                                    cudaStream_t, bool);                                                         \
   template int run_prepare<T, LOGN>(const Context&, const void*, void*, int64_t, int, cudaStream_t);            \
   template int run_items<T, LOGN>(const Context&, int, const void*, int, int*, const void*, int64_t, cudaStream_t, \
-                                  int64_t);                                                                     \
+                                  const void*, int64_t, int);                                                                     \
   template int run_apply_prepared<T, LOGN>(const Context&, const void*, const void*, void*, void*, int64_t, int, \
                                            uint32_t, cudaStream_t);
 
