@@ -7,6 +7,7 @@
 
 #include "../../include/fhb200.h"
 #include "fhb_kernels.cuh"
+#include "fhb_moddown.cuh"
 #include "fhb_runners.h"
 
 struct fhb_context {
@@ -165,19 +166,47 @@ int moddown(const Context& c, const void* t0, const void* t1, const void* a0, co
     if (c.basis_tc && c.tc_moddown)  // P -> Q conversion on the int8 tensor cores
       return tc_moddown(const_cast<Context&>(c), t0, t1, a0, a1, out, batch, level, ginv, item_galois, rescale, st);
   }
+  if (batch == 0) return 0;
   if (out_pitch <= 0) out_pitch = batch * (c.num_q - level - (rescale ? 1 : 0)) * c.n();
-  k_moddown<T><<<elementwise_grid(batch << c.log_n), 256, 0, st>>>(
-      (const T*)t0, (const T*)t1, (const T*)a0, (const T*)a1, (T*)out, batch, c.log_n, level, c.num_q, c.num_p,
-      ginv, item_galois, rescale, tables<T>(c), level_tables<T>(c, level), out_pitch);
-  return cuda_status(cudaGetLastError(), "k_moddown");
+  const MdArgs<T> args = moddown_args<T>(c, level, rescale);
+  const int64_t tiles = (int64_t(c.n()) >> 9) * 2 * batch;
+  const int groups = moddown_groups(tiles, c.num_q - level);
+  if (tiles * groups > 0x7fffffffLL) return fail(-6, "too many blocks for one launch");
+  auto run = [&](auto kern) {
+    kern<<<unsigned(tiles * groups), kMdThreads, 0, st>>>(args, (const T*)t0, (const T*)t1, (const T*)a0,
+                                                          (const T*)a1, (T*)out, out_pitch, groups, ginv, item_galois);
+    return cuda_status(cudaGetLastError(), "k_moddown");
+  };
+  auto width = [&](auto split) {
+    constexpr bool S = decltype(split)::value;
+    switch (c.num_p) {
+      case 1: return run(k_moddown<T, 1, S>);
+      case 2: return run(k_moddown<T, 2, S>);
+      case 4: return run(k_moddown<T, 4, S>);
+      default: return run(k_moddown<T, kMaxDigitWidth, S>);
+    }
+  };
+  if constexpr (sizeof(T) == 8) {
+    if (args.f64_end > level) return width(std::true_type{});
+  }
+  return width(std::false_type{});
 }
 
 template <typename T>
 int rescale(const Context& c, const void* in, void* out, int64_t polys, int level, int nearest, cudaStream_t st) {
-  const int limbs = c.num_q - level;
-  k_rescale<T><<<elementwise_grid(polys * (limbs - 1) << c.log_n), 256, 0, st>>>(
-      (const T*)in, (T*)out, polys, limbs, c.log_n, level, nearest, tables<T>(c), level_tables<T>(c, level));
-  return cuda_status(cudaGetLastError(), "k_rescale");
+  const int groups = (c.num_q - level - 1 + kRescaleRows - 1) / kRescaleRows;
+  const int64_t blocks = (int64_t(c.n()) >> 9) * polys * groups;
+  if (blocks <= 0) return 0;
+  if (blocks > 0x7fffffffLL) return fail(-6, "too many blocks for one launch");
+  const MdArgs<T> args = moddown_args<T>(c, level, 1);
+  auto run = [&](auto kern) {
+    kern<<<unsigned(blocks), kMdThreads, 0, st>>>(args, (const T*)in, (T*)out, groups, nearest);
+    return cuda_status(cudaGetLastError(), "k_rescale");
+  };
+  if constexpr (sizeof(T) == 8) {
+    if (args.f64_end > level) return run(k_rescale<T, true>);
+  }
+  return run(k_rescale<T, false>);
 }
 
 template <typename T>

@@ -92,8 +92,50 @@ uint64_t prefix_product_mod(const std::vector<uint64_t>& mods, int k, uint64_t m
   return r;
 }
 
+// ModDown's row constants (fhb_moddown.cuh): C = 1 or q_l^{-1}, A = P^{-1} C,
+// D = -C, B_r = -M_r A.
 template <typename T>
-bool build_tables(Context& c, ChainTables<T>& t, std::vector<LevelTables<T>>& levels, LevelTables<T>*& levels_dev) {
+bool build_moddown(Context& c, MdTables<T>& md) {
+  const int qp = c.qp();
+  const int bits = int(8 * sizeof(T));
+  const std::vector<uint64_t> pm(c.moduli.begin() + c.num_q, c.moduli.end());
+  std::vector<T> words(size_t(c.num_q + 1) * qp * kMdWords, 0);
+  std::vector<double> doubles;
+  const bool f64 = sizeof(T) == 8 && c.f64_tables_ok;
+  if (f64) doubles.assign(size_t(c.num_q + 1) * qp * kMdDoubles, 0.0);
+  for (int pid = 0; pid < c.num_q; ++pid) {
+    const uint64_t q = c.moduli[pid], w = powmod(2, bits, q);
+    const uint64_t p_inv = invmod(prefix_product_mod(pm, c.num_p, q), q);
+    std::vector<uint64_t> mix(c.num_p);
+    for (int r = 0; r < c.num_p; ++r) mix[r] = prefix_product_mod(pm, r, q);
+    for (int table = 0; table <= c.num_q; ++table) {
+      const int level = table - 1;  // the rescale's, or none
+      if (level >= pid) continue;
+      const uint64_t cc = table == 0 ? 1 : invmod(c.moduli[level] % q, q);
+      const uint64_t a = mulmod(p_inv, cc, q);
+      const size_t row = size_t(table) * qp + pid;
+      std::vector<uint64_t> v = {a, cc, q - cc};
+      for (int r = 0; r < c.num_p; ++r) v.push_back((q - mulmod(mix[r], a, q)) % q);
+      for (size_t i = 0; i < v.size(); ++i) words[row * kMdWords + i] = T(mulmod(v[i], w, q));
+      if (f64 && pid < c.f64_prime_end) {
+        double* d = &doubles[row * kMdDoubles];
+        for (int i = 0; i < 3; ++i) d[i] = double(v[i]);
+        for (int r = 0; r < c.num_p; ++r) {
+          d[3 + 2 * r] = double(mulmod(v[3 + r], (uint64_t{1} << 30) % q, q));
+          d[4 + 2 * r] = double(v[3 + r]);
+        }
+      }
+    }
+  }
+  md.w = upload(c, words);
+  md.f = upload(c, doubles);
+  md.prime = c.t64f.prime;
+  return md.w && (!f64 || md.f);
+}
+
+template <typename T>
+bool build_tables(Context& c, ChainTables<T>& t, std::vector<LevelTables<T>>& levels, LevelTables<T>*& levels_dev,
+                  MdTables<T>& md) {
   const int qp = c.qp();
   const uint64_t n = c.n();
   const int radix_bits = sizeof(T) == 8 ? 62 : 30;
@@ -289,7 +331,7 @@ bool build_tables(Context& c, ChainTables<T>& t, std::vector<LevelTables<T>>& le
     c.ext64f_digits = d0;
     c.f64_tables_ok = c.f64_tables_ok && c.ext64f;
   }
-  return t.prime && t.tw_fwd && t.tw_inv && t.p_garner && t.p_mix && t.p_inv && t.p_rinv;
+  return t.prime && t.tw_fwd && t.tw_inv && t.p_garner && t.p_mix && t.p_inv && t.p_rinv && build_moddown(c, md);
 }
 
 }  // namespace
@@ -331,8 +373,8 @@ Context* build_context(int bits, int log_n, const uint64_t* moduli, int num_q, i
   c->num_p = num_p;
   c->device = device;
   c->moduli.assign(moduli, moduli + num_q + num_p);
-  bool ok = bits == 64 ? build_tables<uint64_t>(*c, c->t64, c->lv64, c->lv64_dev)
-                       : build_tables<uint32_t>(*c, c->t32, c->lv32, c->lv32_dev);
+  bool ok = bits == 64 ? build_tables<uint64_t>(*c, c->t64, c->lv64, c->lv64_dev, c->md64)
+                       : build_tables<uint32_t>(*c, c->t32, c->lv32, c->lv32_dev, c->md32);
   if (!ok) {
     cudaError_t e = cudaGetLastError();
     *status = e != cudaSuccess ? cuda_status(e, "context tables") : fail(-3, "no primitive 2N-th root for a modulus");

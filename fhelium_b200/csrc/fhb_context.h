@@ -12,6 +12,10 @@
 namespace fhb {
 
 constexpr int kMaxDigitWidth = 8;  // hybrid digit width bound (= P count)
+// Constants of one row of ModDown: A, C, D, B_0.. (words); A, C, D, then
+// (B_r 2^30 mod q, B_r) per digit (FP64).
+constexpr int kMdWords = 3 + kMaxDigitWidth;
+constexpr int kMdDoubles = 3 + 2 * kMaxDigitWidth;
 // Room for the key-switch core's intermediate that fhb_ckks_keyswitch_workspace_bytes
 // asks for at most (rows are processed in groups that fit it).
 constexpr int64_t kKsPassRoom = int64_t{1} << 30;
@@ -45,6 +49,16 @@ struct ChainTables {
   // the quotient from the product and 1/q (prime.one_s).
   T* twv_fwd = nullptr;
   T* twv_inv = nullptr;
+};
+
+// ModDown's constants per row (fhb_moddown.cuh): table 0 without rescale,
+// table 1 + l with the rescale of level l, each [QP] rows of kMdWords words
+// (times 2^W mod q) and of kMdDoubles doubles (FP64 rows).
+template <typename T>
+struct MdTables {
+  T* w = nullptr;
+  double* f = nullptr;
+  PrimeInfo<double>* prime = nullptr;
 };
 
 // Per-level key-switch / rescale tables (device).
@@ -88,6 +102,8 @@ struct Context {
   std::vector<uint64_t> roots;  // primitive 2N-th roots psi
   ChainTables<uint64_t> t64;
   ChainTables<uint32_t> t32;
+  MdTables<uint64_t> md64;
+  MdTables<uint32_t> md32;
   std::vector<LevelTables<uint64_t>> lv64;
   std::vector<LevelTables<uint32_t>> lv32;
   // the same per-level tables as a device array [num_q] (kernels over
@@ -152,6 +168,12 @@ template <>
 inline const ChainTables<uint64_t>& tables<uint64_t>(const Context& c) { return c.t64; }
 template <>
 inline const ChainTables<uint32_t>& tables<uint32_t>(const Context& c) { return c.t32; }
+template <typename T>
+inline const MdTables<T>& md_tables(const Context& c);
+template <>
+inline const MdTables<uint64_t>& md_tables<uint64_t>(const Context& c) { return c.md64; }
+template <>
+inline const MdTables<uint32_t>& md_tables<uint32_t>(const Context& c) { return c.md32; }
 template <typename T>
 inline const LevelTables<T>& level_tables(const Context& c, int level);
 template <>

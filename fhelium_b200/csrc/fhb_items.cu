@@ -155,9 +155,26 @@ int run_elementwise(const Context& c, const char* plan, const PlanLayout& l, con
   if (int rc = run_stage(c, 2, iv, plan + l.core_off, info.core_units, st, plan + l.pair_off, l.pairs,
                          info.max_digits))
     return rc;
-  k_items_moddown<T><<<dim3(unsigned((n + 255) / 256), unsigned(info.items)), 256, 0, st>>>(
-      iv, level_tables_dev<T>(c), c.num_q, c.num_p, c.log_n, tables<T>(c));
-  return cuda_status(cudaGetLastError(), "k_items_moddown");
+  const MdArgs<T> args = moddown_args<T>(c, 0, 0);
+  const int64_t tiles = (n >> 9) * 2;
+  const int groups = moddown_groups(tiles * info.items, info.max_limbs);
+  auto run = [&](auto kern) {
+    kern<<<dim3(unsigned(tiles * groups), unsigned(info.items)), kMdThreads, 0, st>>>(iv, args, groups);
+    return cuda_status(cudaGetLastError(), "k_items_moddown");
+  };
+  auto width = [&](auto split) {
+    constexpr bool S = decltype(split)::value;
+    switch (c.num_p) {
+      case 1: return run(k_items_moddown<T, 1, S>);
+      case 2: return run(k_items_moddown<T, 2, S>);
+      case 4: return run(k_items_moddown<T, 4, S>);
+      default: return run(k_items_moddown<T, kMaxDigitWidth, S>);
+    }
+  };
+  if constexpr (sizeof(T) == 8) {
+    if (args.f64_end > 0) return width(std::true_type{});
+  }
+  return width(std::false_type{});
 }
 
 }  // namespace

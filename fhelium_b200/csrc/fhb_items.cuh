@@ -16,6 +16,7 @@
 // take the item from the grid's z dimension.
 #pragma once
 #include "fhb_kernels.cuh"
+#include "fhb_moddown.cuh"
 #include "fhb_pass.cuh"
 
 namespace fhb {
@@ -188,73 +189,25 @@ __global__ void k_items_modup(ItemsView iv, const LevelTables<T>* __restrict__ l
 
 // ModDown of every item (k_moddown per item): HMult items rescale by the
 // leading prime (c0, c1 are already in the accumulators); rotations add
-// sigma_g(c0).  Grid (N / 256, items), one coefficient per thread.
-template <typename T>
-__global__ void k_items_moddown(ItemsView iv, const LevelTables<T>* __restrict__ levels, int num_q, int num_p,
-                                int log_n, ChainTables<T> tabs) {
-  using W = Word<T>;
+// sigma_g(c0).  Blocks (coefficients, component, group of rows) on x, items on y.
+template <typename T, int NP, bool SPLIT>
+__global__ void __launch_bounds__(kMdThreads, 2)
+k_items_moddown(ItemsView iv, const __grid_constant__ MdArgs<T> args, int groups) {
   KsItem it;
   if (!items_fetch(iv, int(blockIdx.y), it)) return;
-  const int64_t n = int64_t(1) << log_n;
-  const int k = int(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (k >= n) return;
-  const int level = it.level;
-  const int q_limbs = num_q - level, qp0 = num_q + num_p;
-  const int rescale = it.kind == 0 ? 1 : 0;
-  const int out_limbs = q_limbs - rescale;
-  const uint32_t gi = (it.kind == 0 || it.galois == 1) ? 0u : galois_inverse_dev(it.galois, log_n);
-  bool neg = false;
-  const int ak = gi ? galois_source(k, log_n, gi, neg) : k;
-  const LevelTables<T> lt = levels[level];
-  for (int c = 0; c < 2; ++c) {
-    const T* t = static_cast<const T*>(c == 0 ? it.t0 : it.t1);
-    const T* ad = (it.kind == 1 && c == 0) ? static_cast<const T*>(it.a) : nullptr;
-    T e[kMaxDigitWidth];
-    for (int r = 0; r < num_p; ++r) {
-      const PrimeInfo<T> p = tabs.prime[num_q + r];
-      T x = t[(q_limbs + r) * n + k];
-      T acc = 0;
-      for (int i = 0; i < r; ++i) {
-        const TwPair<T> g = tabs.p_garner[r * kMaxDigitWidth + i];
-        acc = csub(acc + csub(W::shoup(e[i], g.w, g.wp, p.q), p.q), p.q);
-      }
-      if (r > 0) {
-        const TwPair<T> inv = tabs.p_garner[r * kMaxDigitWidth + r];
-        x = csub(W::shoup(csub(x + p.q - acc, p.q), inv.w, inv.wp, p.q), p.q);
-      }
-      e[r] = x;
-    }
-    T* o = static_cast<T*>(it.out) + int64_t(c) * out_limbs * n;
-    T v0 = 0;
-    for (int i = 0; i < q_limbs; ++i) {
-      const int pid = level + i;
-      const PrimeInfo<T> p = tabs.prime[pid];
-      T sub = 0;
-      for (int r = 0; r < num_p; ++r) {
-        const TwPair<T> m = tabs.p_mix[r * qp0 + pid];
-        sub = csub(sub + csub(W::shoup(e[r], m.w, m.wp, p.q), p.q), p.q);
-      }
-      const TwPair<T> pinv = tabs.p_inv[pid];
-      T v = csub(t[i * n + k] + p.q - sub, p.q);
-      v = csub(W::shoup(v, pinv.w, pinv.wp, p.q), p.q);
-      if (ad) {
-        T x = csub(ad[i * n + ak], p.q);
-        if (neg && x) x = p.q - x;
-        v = csub(v + x, p.q);
-      }
-      if (!rescale) {
-        o[i * n + k] = v;
-      } else if (i == 0) {
-        v0 = v;
-      } else {
-        const T x0 = reduce_any(v0, p);
-        const TwPair<T> inv = lt.rescale_inv[pid];
-        T r = csub(W::shoup(csub(v + p.q - x0, p.q), inv.w, inv.wp, p.q), p.q);
-        r += (v0 > (tabs.prime[level].q >> 1)) ? 1 : 0;
-        o[(i - 1) * n + k] = csub(r, p.q);
-      }
-    }
-  }
+  unsigned idx = blockIdx.x;
+  const int g = int(idx % unsigned(groups));
+  idx /= unsigned(groups);
+  const int c = int(idx & 1), k0 = int((idx >> 1) * kMdThreads + threadIdx.x) * 2;
+  MdArgs<T> a = args;
+  a.level = it.level;
+  a.rescale = it.kind == 0 ? 1 : 0;
+  const int ql = a.num_q - a.level, out_limbs = ql - a.rescale;
+  const bool add = it.kind == 1 && c == 0;
+  const uint32_t gi = !add || it.galois == 1 ? 0u : galois_inverse_dev(it.galois, a.log_n);
+  moddown_rows<T, NP, SPLIT>(a, static_cast<const T*>(c ? it.t1 : it.t0), add ? static_cast<const T*>(it.a) : nullptr,
+                             gi, static_cast<T*>(it.out) + ((int64_t(c) * out_limbs) << a.log_n), k0,
+                             ql * g / groups, ql * (g + 1) / groups);
 }
 
 // The transform stages take their (item, row) from a work list.  Every thread

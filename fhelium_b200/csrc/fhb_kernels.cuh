@@ -933,121 +933,6 @@ k_keyswitch_sum(const T* __restrict__ digits, const unsigned long long* __restri
 }
 
 // ---------------------------------------------------------------------------
-// ModDown by P fused with the final addition and, optionally, the rescale by
-// the leading prime.  t0/t1: [B, QP_l, N] canonical coefficient rows;
-// add0/add1 (nullable): [B, Q_l, N] canonical, add0 optionally read through
-// sigma_g (rotation of c0).  Result per Q row i (prime q):
-//   v_i = (t_i - [t]_P) P^{-1} + add_i  (mod q)
-// which is exactly the sequential divide-by-p_j chain of
-// csrc/ops/ckks/cpu/ckks_cpu.cpp:474-601 (both compute (t - [t]_P)/P over
-// the integers), then (when rescale) the nearest-rounded division by the
-// leading prime of csrc/ops/ckks/cpu/ckks_cpu.cpp:203-262:
-//   out_i = (v_i - v_0) q_0^{-1} + [v_0 > q_0/2]  (mod q_i), i >= 1.
-// out: [2, B, Q_l (- 1 if rescale), N] canonical, components out_pitch
-// words apart (a slice of a larger batch when the pitch exceeds the slice).
-template <typename T>
-__global__ void k_moddown(const T* __restrict__ t0, const T* __restrict__ t1, const T* __restrict__ add0,
-                          const T* __restrict__ add1, T* __restrict__ out, int64_t batch, int log_n,
-                          int level, int num_q, int num_p, uint32_t add0_ginv,
-                          const uint32_t* __restrict__ item_galois, int rescale, ChainTables<T> tabs,
-                          LevelTables<T> lt, int64_t out_pitch) {
-  using W = Word<T>;
-  const int64_t n = int64_t(1) << log_n;
-  const int q_limbs = num_q - level;
-  const int qp_limbs = q_limbs + num_p;
-  const int out_limbs = q_limbs - (rescale ? 1 : 0);
-  const int64_t total = batch * n;
-  const int qp0 = num_q + num_p;
-  for (int64_t idx = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; idx < total;
-       idx += int64_t(gridDim.x) * blockDim.x) {
-    const int64_t bi = idx >> log_n;
-    const int k = int(idx & (n - 1));
-    bool neg = false;
-    const uint32_t gi =
-        item_galois ? (item_galois[bi] == 1 ? 0u : galois_inverse_dev(item_galois[bi], log_n)) : add0_ginv;
-    const int ak = gi ? galois_source(k, log_n, gi, neg) : k;
-    for (int c = 0; c < 2; ++c) {
-      const T* t = (c == 0 ? t0 : t1) + bi * qp_limbs * n;
-      const T* ad = c == 0 ? add0 : add1;
-      const int kk = c == 0 ? ak : k;
-      const bool nn = c == 0 ? neg : false;
-      // Garner digits of the P part
-      T e[kMaxDigitWidth];
-      for (int r = 0; r < num_p; ++r) {
-        const PrimeInfo<T> p = tabs.prime[num_q + r];
-        T x = t[(q_limbs + r) * n + k];
-        T acc = 0;
-        for (int i = 0; i < r; ++i) {
-          const TwPair<T> g = tabs.p_garner[r * kMaxDigitWidth + i];
-          acc = csub(acc + csub(W::shoup(e[i], g.w, g.wp, p.q), p.q), p.q);
-        }
-        if (r > 0) {
-          const TwPair<T> inv = tabs.p_garner[r * kMaxDigitWidth + r];
-          x = csub(W::shoup(csub(x + p.q - acc, p.q), inv.w, inv.wp, p.q), p.q);
-        }
-        e[r] = x;
-      }
-      T* o = out + int64_t(c) * out_pitch + bi * out_limbs * n;
-      T v0 = 0;
-      for (int i = 0; i < q_limbs; ++i) {
-        const int pid = level + i;
-        const PrimeInfo<T> p = tabs.prime[pid];
-        T sub = 0;
-        for (int r = 0; r < num_p; ++r) {
-          const TwPair<T> m = tabs.p_mix[r * qp0 + pid];
-          sub = csub(sub + csub(W::shoup(e[r], m.w, m.wp, p.q), p.q), p.q);
-        }
-        const TwPair<T> pinv = tabs.p_inv[pid];
-        T v = csub(t[i * n + k] + p.q - sub, p.q);
-        v = csub(W::shoup(v, pinv.w, pinv.wp, p.q), p.q);
-        if (ad) {
-          T x = csub(ad[(bi * q_limbs + i) * n + kk], p.q);
-          if (nn && x) x = p.q - x;
-          v = csub(v + x, p.q);
-        }
-        if (!rescale) {
-          o[i * n + k] = v;
-        } else if (i == 0) {
-          v0 = v;
-        } else {
-          const T x0 = reduce_any(v0, p);
-          const TwPair<T> inv = lt.rescale_inv[pid];
-          T r = csub(W::shoup(csub(v + p.q - x0, p.q), inv.w, inv.wp, p.q), p.q);
-          r += (v0 > (tabs.prime[level].q >> 1)) ? 1 : 0;
-          o[(i - 1) * n + k] = csub(r, p.q);
-        }
-      }
-    }
-  }
-}
-
-// Standalone rescale of coefficient/standard components: in [K, L, N] ->
-// out [K, L-1, N] (csrc/ops/ckks/cpu/ckks_cpu.cpp:203-262).
-template <typename T>
-__global__ void k_rescale(const T* __restrict__ in, T* __restrict__ out, int64_t polys, int limbs, int log_n,
-                          int level, int nearest, ChainTables<T> tabs, LevelTables<T> lt) {
-  using W = Word<T>;
-  const int64_t n = int64_t(1) << log_n;
-  const int64_t total = polys * (limbs - 1) * n;
-  const T half = tabs.prime[level].q >> 1;
-  for (int64_t idx = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; idx < total;
-       idx += int64_t(gridDim.x) * blockDim.x) {
-    const int k = int(idx & (n - 1));
-    const int64_t rowi = idx >> log_n;
-    const int i = int(rowi % (limbs - 1)) + 1;
-    const int64_t pl = rowi / (limbs - 1);
-    const int pid = level + i;
-    const PrimeInfo<T> p = tabs.prime[pid];
-    const T v0 = in[pl * limbs * n + k];
-    const T x0 = reduce_any(v0, p);
-    const T v = reduce_any(in[(pl * limbs + i) * n + k], p);
-    const TwPair<T> inv = lt.rescale_inv[pid];
-    T r = csub(W::shoup(csub(v + p.q - x0, p.q), inv.w, inv.wp, p.q), p.q);
-    if (nearest) r += (v0 > half) ? 1 : 0;
-    out[idx] = csub(r, p.q);
-  }
-}
-
 // Coefficient-domain automorphism: out = sigma_g(in), canonical
 // (csrc/ops/ckks/cpu/ckks_cpu.cpp:287-380).
 template <typename T>
