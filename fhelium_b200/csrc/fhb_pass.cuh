@@ -221,6 +221,11 @@ constexpr int kRowThreads = 128;                 // four warps, eight half warps
 constexpr int kRowSlots = kRowThreads / 16;
 
 template <typename T>
+constexpr size_t exchange_smem() {
+  return size_t(kRowSlots) * kBlk * sizeof(T);
+}
+
+template <typename T>
 struct RowX {
   static constexpr int V = 16 / int(sizeof(T));  // words per 16-byte piece
   static constexpr int kVec = 16 / V;            // pieces per thread
@@ -325,6 +330,16 @@ struct Rows {
   using B = Ntt<T, LOGN, TW>;
   static constexpr int kA = LOGN - kBlkLog;
 
+  // Twiddle j of row blk's stage b of the strided layout's four (a) and of
+  // thread t's stage b of the contiguous layout's four (b); the inverse
+  // stages mirror them (b = 3 first).
+  __device__ __forceinline__ static TwPair<T> tw_a(const TW& tw, int b, int blk, int j) {
+    return tw.at((1 << (kA + b)) + (blk << b) + j);
+  }
+  __device__ __forceinline__ static TwPair<T> tw_b(const TW& tw, int b, int blk, int t, int j) {
+    return tw.at((1 << (kA + 4 + b)) + ((blk * 16 + t) << b) + j);
+  }
+
   // strided -> contiguous
   __device__ __forceinline__ static void fwd(T (&v)[16], const RowX<T>& x, const TW& tw, T q, T m2, int blk) {
 #pragma unroll
@@ -332,7 +347,7 @@ struct Rows {
       const int h = 8 >> b;
 #pragma unroll
       for (int i = 0; i < 16; ++i)
-        if (!(i & h)) B::fwd_bfly(v[i], v[i + h], tw.at((1 << (kA + b)) + (blk << b) + (i >> (4 - b))), q, m2);
+        if (!(i & h)) B::fwd_bfly(v[i], v[i + h], tw_a(tw, b, blk, i >> (4 - b)), q, m2);
     }
     __syncwarp();
     x.put_strided(v);
@@ -343,8 +358,7 @@ struct Rows {
       const int h = 8 >> b;
 #pragma unroll
       for (int i = 0; i < 16; ++i)
-        if (!(i & h))
-          B::fwd_bfly(v[i], v[i + h], tw.at((1 << (kA + 4 + b)) + ((blk * 16 + x.t) << b) + (i >> (4 - b))), q, m2);
+        if (!(i & h)) B::fwd_bfly(v[i], v[i + h], tw_b(tw, b, blk, x.t, i >> (4 - b)), q, m2);
     }
   }
   __device__ __forceinline__ static void contiguous_to_vector(T (&v)[16], const RowX<T>& x) {
@@ -368,14 +382,12 @@ struct Rows {
 
   // contiguous -> strided
   __device__ __forceinline__ static void inv(T (&v)[16], const RowX<T>& x, const TW& tw, T q, T m2, int blk) {
-    constexpr int kN = 1 << LOGN;
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       const int h = 1 << j;
 #pragma unroll
       for (int i = 0; i < 16; ++i)
-        if (!(i & h))
-          B::inv_bfly(v[i], v[i + h], tw.at((kN >> (j + 1)) + ((blk * 16 + x.t) << (3 - j)) + (i >> (j + 1))), q, m2);
+        if (!(i & h)) B::inv_bfly(v[i], v[i + h], tw_b(tw, 3 - j, blk, x.t, i >> (j + 1)), q, m2);
     }
     reduce_grown<T, 4>(v, q, m2);
     __syncwarp();
@@ -387,8 +399,7 @@ struct Rows {
       const int h = 1 << j;
 #pragma unroll
       for (int i = 0; i < 16; ++i)
-        if (!(i & h))
-          B::inv_bfly(v[i], v[i + h], tw.at((kN >> (j + 5)) + (blk << (3 - j)) + (i >> (j + 1))), q, m2);
+        if (!(i & h)) B::inv_bfly(v[i], v[i + h], tw_a(tw, 3 - j, blk, i >> (j + 1)), q, m2);
     }
     reduce_grown<T, 4>(v, q, m2);
   }
@@ -694,6 +705,7 @@ __device__ __forceinline__ void ks_rows_f64(const KsPass<uint64_t>& k, int jrow,
   for (int e = 0; e < 16; ++e) a0[e] = a1[e] = 0.0;
   for (int g = 0; g < k.terms; ++g) {
     const uint64_t* key = k.item_keys ? reinterpret_cast<const uint64_t*>(k.item_keys[k.terms > 1 ? g : bi]) : k.key;
+#pragma unroll 1
     for (int a = 0; a < k.lt.num_digits; ++a) {
       const DigitDesc d = k.lt.digits[a];
       double v[16];
@@ -790,6 +802,7 @@ __device__ __forceinline__ void ks_rows_int(const KsPass<T>& k, int jrow, int bi
   for (int e = 0; e < 16; ++e) a0[e] = a1[e] = 0;
   for (int g = 0; g < k.terms; ++g) {
     const T* key = k.item_keys ? reinterpret_cast<const T*>(k.item_keys[k.terms > 1 ? g : bi]) : k.key;
+#pragma unroll 1
     for (int a = 0; a < k.lt.num_digits; ++a) {
       const DigitDesc d = k.lt.digits[a];
       T v[16];
@@ -966,11 +979,6 @@ __device__ __forceinline__ void ntt_columns(const T* in, T* out, int pid, bool f
   ColSink<T> sink{out};
   Cols<T, LOGN, TwAt<T>>::template fwd<0>(src, sink, reinterpret_cast<T*>(smem),
                                           TwAt<T>{tabs.tw_fwd + int64_t(pid) * kN}, p.q, p.twice_q, col0);
-}
-
-template <typename T>
-constexpr size_t exchange_smem() {
-  return size_t(kRowSlots) * kBlk * sizeof(T);
 }
 
 // The block stages of the forward transform of row blk of `poly`, in place,
@@ -1161,16 +1169,9 @@ k_ntt_columns_inverse(T* out, int rows, int row_start, int kind, ChainTables<T> 
 // under the NTT-domain automorphism are a permutation of 16 aligned words
 // (the low bits of k are the top bits of br(k), which the odd g permutes), so
 // in the strided layout the gathers, like the key loads, are whole 128-byte
-// lines.  y: the prepared digits [D_l, B, QP_l, N].
-template <int LOGN>
-__device__ __forceinline__ void apply_sources(int (&src)[16], int blk, int t, uint32_t galois) {
-#pragma unroll
-  for (int e = 0; e < 16; ++e) {
-    const int dst = blk * kBlk + t + 16 * e;
-    src[e] = galois ? galois_ntt_source(dst, LOGN, galois) : dst;
-  }
-}
-
+// lines.  y: the prepared digits [D_l, B, QP_l, N].  A thread takes its 16
+// words in two halves, so that a digit's 24 loads fit the registers and can
+// all be in flight.
 template <typename T, int LOGN, bool SPLIT>
 __global__ void __launch_bounds__(kRowThreads, sizeof(T) == 8 ? 3 : 4)
 k_apply_rows(const __grid_constant__ KsPass<T> k, uint32_t galois) {
@@ -1187,8 +1188,10 @@ k_apply_rows(const __grid_constant__ KsPass<T> k, uint32_t galois) {
   if (slot >= slots) return;
   const int bi = int(slot % unsigned(k.batch)), blk = int(slot / unsigned(k.batch));
   const X x(smem);
-  int src[16];
-  apply_sources<LOGN>(src, blk, x.t, galois);
+  auto source = [&](int e) {  // the word gathered for this thread's word t + 16 e
+    const int dst = blk * kBlk + x.t + 16 * e;
+    return galois ? galois_ntt_source(dst, LOGN, galois) : dst;
+  };
   const T* key = k.key + int64_t(pid) * kN + blk * kBlk + x.t;
   const int64_t o = (int64_t(bi) * k.qp_limbs + jrow) * kN + blk * kBlk + x.t;
   if constexpr (SPLIT) {
@@ -1199,16 +1202,24 @@ k_apply_rows(const __grid_constant__ KsPass<T> k, uint32_t galois) {
       const double q = k.tabs64f.prime[pid].q, qinv = k.tabs64f.prime[pid].one_s;
       double a0[16], a1[16];
 #pragma unroll
-      for (int e = 0; e < 16; ++e) a0[e] = a1[e] = 0.0;
-      for (int a = 0; a < k.lt.num_digits; ++a) {
-        const T* y = k.y_poly(a, bi, jrow, true, LOGN);
-        const T* key0 = key + int64_t(k.lt.digits[a].key_digit) * 2 * k.qp0 * kN;
-        const T* key1 = key0 + k.qp0 * kN;
+      for (int h = 0; h < 16; h += 8) {
+        int src[8];
 #pragma unroll
-        for (int e = 0; e < 16; ++e) {
-          const double v = W::from_word(__ldg(y + src[e]));
-          a0[e] += W::mul_qinv_bal(v, W::from_word(__ldg(key0 + 16 * e)), q, qinv);
-          a1[e] += W::mul_qinv_bal(v, W::from_word(__ldg(key1 + 16 * e)), q, qinv);
+        for (int e = 0; e < 8; ++e) src[e] = source(h + e), a0[h + e] = a1[h + e] = 0.0;
+#pragma unroll 1
+        for (int a = 0; a < k.lt.num_digits; ++a) {
+          const T* y = k.y_poly(a, bi, jrow, true, LOGN);
+          const T* key0 = key + int64_t(k.lt.digits[a].key_digit) * 2 * k.qp0 * kN + 16 * h;
+          const T* key1 = key0 + k.qp0 * kN;
+          T w[8], k0[8], k1[8];
+#pragma unroll
+          for (int e = 0; e < 8; ++e) w[e] = __ldg(y + src[e]), k0[e] = __ldg(key0 + 16 * e), k1[e] = __ldg(key1 + 16 * e);
+#pragma unroll
+          for (int e = 0; e < 8; ++e) {
+            const double v = W::from_word(w[e]);
+            a0[h + e] += W::mul_qinv_bal(v, W::from_word(k0[e]), q, qinv);
+            a1[h + e] += W::mul_qinv_bal(v, W::from_word(k1[e]), q, qinv);
+          }
         }
       }
       const TwAtQ tw{k.tabs64f.twv_inv + int64_t(pid) * kN, qinv};
@@ -1230,16 +1241,23 @@ k_apply_rows(const __grid_constant__ KsPass<T> k, uint32_t galois) {
   const T qi = inverse_pow2(q, k.tabs.prime[pid].neg_inv);
   T a0[16], a1[16];
 #pragma unroll
-  for (int e = 0; e < 16; ++e) a0[e] = a1[e] = 0;
-  for (int a = 0; a < k.lt.num_digits; ++a) {
-    const T* y = k.y_poly(a, bi, jrow, false, LOGN);
-    const T* key0 = key + int64_t(k.lt.digits[a].key_digit) * 2 * k.qp0 * kN;
-    const T* key1 = key0 + k.qp0 * kN;
+  for (int h = 0; h < 16; h += 8) {
+    int src[8];
 #pragma unroll
-    for (int e = 0; e < 16; ++e) {
-      const T v = __ldg(y + src[e]);
-      a0[e] = csub(a0[e] + redc_word(v, __ldg(key0 + 16 * e), q, qi), twoq);
-      a1[e] = csub(a1[e] + redc_word(v, __ldg(key1 + 16 * e), q, qi), twoq);
+    for (int e = 0; e < 8; ++e) src[e] = source(h + e), a0[h + e] = a1[h + e] = 0;
+#pragma unroll 1
+    for (int a = 0; a < k.lt.num_digits; ++a) {
+      const T* y = k.y_poly(a, bi, jrow, false, LOGN);
+      const T* key0 = key + int64_t(k.lt.digits[a].key_digit) * 2 * k.qp0 * kN + 16 * h;
+      const T* key1 = key0 + k.qp0 * kN;
+      T w[8], k0[8], k1[8];
+#pragma unroll
+      for (int e = 0; e < 8; ++e) w[e] = __ldg(y + src[e]), k0[e] = __ldg(key0 + 16 * e), k1[e] = __ldg(key1 + 16 * e);
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        a0[h + e] = csub(a0[h + e] + redc_word(w[e], k0[e], q, qi), twoq);
+        a1[h + e] = csub(a1[h + e] + redc_word(w[e], k1[e], q, qi), twoq);
+      }
     }
   }
   const TwAt<T> tw{k.tabs.tw_inv + int64_t(pid) * kN};
