@@ -116,6 +116,11 @@ struct Word<double> {
   __device__ __forceinline__ static T from_word(uint64_t u) {
     return __dadd_rn(__hiloint2double(int(uint32_t(u >> 32) | 0x43300000u), int(uint32_t(u))), -4503599627370496.0);
   }
+  // u - q (for q < 2^51), as cheap: the offset joins the addition
+  __device__ __forceinline__ static T from_word_minus(uint64_t u, T q) {
+    return __dadd_rn(__hiloint2double(int(uint32_t(u >> 32) | 0x43300000u), int(uint32_t(u))),
+                     -(4503599627370496.0 + q));
+  }
   __device__ __forceinline__ static uint64_t to_word(T x) {  // 0 <= x < 2^52, integer
     const T t = __dadd_rn(x, 4503599627370496.0);
     return (uint64_t(uint32_t(__double2hiint(t)) & 0xfffffu) << 32) | uint32_t(__double2loint(t));

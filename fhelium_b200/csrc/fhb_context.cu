@@ -228,6 +228,39 @@ bool build_tables(Context& c, ChainTables<T>& t, std::vector<LevelTables<T>>& le
     }
   }
 
+  // wide FP64 tables
+  if constexpr (sizeof(T) == 8) {
+    while (!f64 && c.wide_prime_end < c.num_q && c.moduli[c.wide_prime_end] < kWidePrimeEnd) ++c.wide_prime_end;
+    if (c.wide_prime_end > 0) {
+      const int end = c.wide_prime_end;
+      std::vector<PrimeInfo<double>> dinfo(qp);
+      std::vector<double> vfwd(size_t(end) * n), vinv(size_t(end) * n);
+      std::vector<TwPair<double>> dp(qp, TwPair<double>{0.0, 0.0});
+      const std::vector<uint64_t> pm(c.moduli.begin() + c.num_q, c.moduli.end());
+      for (int j = 0; j < end; ++j) {
+        const uint64_t q = c.moduli[j], p_mod = prefix_product_mod(pm, c.num_p, q);
+        auto balanced = [&](uint64_t w) { return w > q / 2 ? double(w) - double(q) : double(w); };
+        PrimeInfo<double>& d = dinfo[j];
+        d.q = double(q);
+        d.twice_q = 2.0 * double(q);
+        d.one_s = 1.0 / double(q);
+        d.ninv_rinv = double(uint64_t(info[j].ninv_rinv)), d.ninv_rinv_s = d.ninv_rinv / double(q);
+        d.ninv = double(uint64_t(info[j].ninv)), d.ninv_s = d.ninv / double(q);
+        d.rinv = double(uint64_t(info[j].rinv)), d.rinv_s = d.rinv / double(q);
+        dp[j] = TwPair<double>{double(p_mod), double(p_mod) / double(q)};
+        for (uint64_t k = 0; k < n; ++k) {
+          vfwd[size_t(j) * n + k] = balanced(uint64_t(fwd[size_t(j) * n + k].w));
+          vinv[size_t(j) * n + k] = balanced(uint64_t(inv[size_t(j) * n + k].w));
+        }
+      }
+      c.t64w.prime = upload(c, dinfo);
+      c.t64w.twv_fwd = upload(c, vfwd);
+      c.t64w.twv_inv = upload(c, vinv);
+      c.t64w.p_rinv = upload(c, dp);
+      c.wide_tables_ok = c.t64w.prime && c.t64w.twv_fwd && c.t64w.twv_inv && c.t64w.p_rinv;
+    }
+  }
+
   // ---- ModDown by P -------------------------------------------------------
   std::vector<uint64_t> pm(c.moduli.begin() + c.num_q, c.moduli.end());
   std::vector<TwPair<T>> pg(kMaxDigitWidth * kMaxDigitWidth, TwPair<T>{0, 0});

@@ -19,6 +19,7 @@ constexpr int kMdDoubles = 3 + 2 * kMaxDigitWidth;
 // Room for the key-switch core's intermediate that fhb_ckks_keyswitch_workspace_bytes
 // asks for at most (rows are processed in groups that fit it).
 constexpr int64_t kKsPassRoom = int64_t{1} << 30;
+constexpr uint64_t kWidePrimeEnd = (uint64_t{1} << 50) / 10 * 11;  // 1.1 2^50
 constexpr int kMaxOverlapChunks = 8;  // chunks of the overlapped fused HMult
 
 // One active hybrid digit at one level.
@@ -133,6 +134,12 @@ struct Context {
   int ext64f_digits = 0;  // digits per level in that layout (those of level 0)
   bool f64_tables_ok = false;
   int f64_prime_end = 0;  // Q primes [0, f64_prime_end) are below 2^42 (FP64 rows)
+  // FP64 tables of the wide form (fhb_pass.cuh), on chains without such
+  // primes whose leading Q primes are below 1.1 2^50: twiddle values balanced
+  // to (-q/2, q/2), p_rinv holds P mod q
+  ChainTables<double> t64w;
+  bool wide_tables_ok = false;
+  int wide_prime_end = 0;
   // tuning: the rows of primes below 2^42 run in FP64 arithmetic (1, default
   // when the tables exist: the NTTs and the key-switch kernels) or on the
   // integer pipe (0)

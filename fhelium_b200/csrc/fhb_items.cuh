@@ -373,7 +373,7 @@ k_items_core_columns(ItemsView iv, const ItemUnit* __restrict__ units, int max_d
     if (it.level + j0 < core.f64_end) {
       const bool two = named == 2 && it.level + j0 + 1 < core.f64_end;
       const DigitDesc d = k.lt.digits[a];
-      ks_columns_f64<LOGN, false>(k, a, 0, col0, j0, j0 + 1, !ks_own(k, d, j0), two && !ks_own(k, d, j0 + 1),
+      ks_columns_f64<LOGN, false, false>(k, a, 0, col0, j0, j0 + 1, !ks_own(k, d, j0), two && !ks_own(k, d, j0 + 1),
                                   smem_raw);
       return;
     }
@@ -399,7 +399,7 @@ k_items_core_rows(ItemsView iv, const ItemUnit* __restrict__ units, int64_t slot
   const KsPass<T> k = core.pass(it, int64_t(1) << LOGN);
   if constexpr (SPLIT) {
     if (it.level + u.row < core.f64_end) {
-      ks_rows_f64<LOGN>(k, u.row, 0, blk, true, smem);
+      ks_rows_f64<LOGN, false>(k, u.row, 0, blk, true, smem);
       return;
     }
   }

@@ -31,15 +31,57 @@ namespace fhb {
 template <typename T>
 struct TwAt {
   static constexpr bool kQFromProduct = false;
+  static constexpr bool kWide = false;
   const TwPair<T>* g;
   __device__ __forceinline__ TwPair<T> at(int i) const { return ldtw(g, i); }
 };
-struct TwAtQ {
+template <bool WIDE>
+struct TwQ {
   static constexpr bool kQFromProduct = true;
+  static constexpr bool kWide = WIDE;
   const double* g;
   double qinv;
   __device__ __forceinline__ TwPair<double> at(int i) const { return TwPair<double>{__ldg(g + i), qinv}; }
 };
+
+using TwAtQ = TwQ<false>;
+
+// Forms of the FP64 rows (the kernels' FORM): none; narrow, primes below
+// 2^42; or wide, primes below 1.1 2^50 (kWidePrimeEnd), on chains without
+// narrow rows (the 50-bit chains).  Wide rows use the same butterfly with
+// twiddles balanced to (-q/2, q/2) and keep less headroom: a product of x by
+// such a twiddle has a quotient below |x| / 2, whose estimate is off by at most
+// |x / q| / 8 besides the rounding, so it leaves (0.5 + |x / q| / 8) q, and
+// every value stays exact below 2^53 = 7.2 q as long as each pass of at most
+// four stages starts from reduced words: forward from 1.0 q, 1.63, 2.33, 3.1
+// to 4.0 q; inverse from 0.51 q, sums double, so the words that were sums
+// twice are reduced after two stages (2.0 q) and reach 3.0 q after four.
+// Operands stay below 3.1 q, quotients below 1.55 q < 2^51.  Words enter as
+// u - q (lazy words below 2q, so |x| <= q).
+constexpr int kNoF64 = 0, kNarrowF64 = 1, kWideF64 = 2;
+
+template <bool WIDE>
+__device__ __forceinline__ double f64_word(uint64_t u, double q) {
+  if constexpr (WIDE) return Word<double>::from_word_minus(u, q);
+  return Word<double>::from_word(u);
+}
+
+template <class TW, typename T, int COUNT>
+__device__ __forceinline__ void reduce_wide(T (&x)[COUNT], T q, T qinv) {
+  if constexpr (TW::kWide) {
+#pragma unroll
+    for (int i = 0; i < COUNT; ++i) x[i] = Word<double>::reduce_bal(x[i], q, qinv);
+  }
+}
+// after the second of an inverse pass's stages: the words summed in both
+template <class TW, typename T, int COUNT>
+__device__ __forceinline__ void reduce_wide_sums(T (&x)[COUNT], T q, T qinv) {
+  if constexpr (TW::kWide) {
+#pragma unroll
+    for (int i = 0; i < COUNT; ++i)
+      if ((i & 3) < 2) x[i] = Word<double>::reduce_bal(x[i], q, qinv);
+  }
+}
 
 constexpr int kBlkLog = 8;           // words per row: the block stages' length
 constexpr int kBlk = 1 << kBlkLog;
@@ -50,9 +92,10 @@ constexpr int kBlk = 1 << kBlkLog;
 // by 2^K, word 1 to 0.6 q 2^(K-1), words 2 and 3 to at most 2.4 q, the others
 // less.  Reducing words 0 and (K = 4) 1 keeps every pass's inputs below
 // 2.4 q and every product operand below 2 x 19.2 q < 2^48 (q < 2^42).
-template <typename T, int K>
+template <class TW, typename T, int K>
 __device__ __forceinline__ void reduce_grown(T (&x)[1 << K], T q, T qinv) {
-  if constexpr (std::is_same<T, double>::value) {
+  reduce_wide<TW>(x, q, qinv);
+  if constexpr (std::is_same<T, double>::value && !TW::kWide) {
     x[0] = Word<double>::reduce_bal(x[0], q, qinv);
     if constexpr (K >= 4) x[1] = Word<double>::reduce_bal(x[1], q, qinv);
   }
@@ -112,6 +155,7 @@ struct Cols {
       for (int i = 0; i < (1 << K); ++i)
         if (!(i & h)) B::fwd_bfly(x[i], x[i + h], tw.at((1 << (A + b)) + (hi << b) + (i >> (K - b))), q, m2);
     }
+    reduce_wide<TW>(x, q, m2);
   }
 
   // Pass J: words from `src` (J = 0) or shared memory, to shared memory or (the last pass) to `sink`.
@@ -172,12 +216,14 @@ struct Cols {
         for (int i = 0; i < kGs; ++i)
           if (!(i & h))
             B::inv_bfly(x[i], x[i + h], tw.at(((1 << LOGN) >> (j + 1)) + (hi << (K - 1 - b)) + (i >> (b + 1))), q, m2);
+        if (b == 1 && K > 2) reduce_wide_sums<TW>(x, q, m2);
       }
       if constexpr (kLast) {
+        reduce_wide<TW>(x, q, m2);
 #pragma unroll
         for (int k = 0; k < kGs; ++k) epi(at + k * (kBlk << R), x[k]);
       } else {
-        reduce_grown<T, K>(x, q, m2);
+        reduce_grown<TW, T, K>(x, q, m2);
 #pragma unroll
         for (int k = 0; k < kGs; ++k) s[(row0 + (k << R)) * G::kCols + col] = x[k];
       }
@@ -349,6 +395,7 @@ struct Rows {
       for (int i = 0; i < 16; ++i)
         if (!(i & h)) B::fwd_bfly(v[i], v[i + h], tw_a(tw, b, blk, i >> (4 - b)), q, m2);
     }
+    reduce_wide<TW>(v, q, m2);
     __syncwarp();
     x.put_strided(v);
     __syncwarp();
@@ -360,6 +407,7 @@ struct Rows {
       for (int i = 0; i < 16; ++i)
         if (!(i & h)) B::fwd_bfly(v[i], v[i + h], tw_b(tw, b, blk, x.t, i >> (4 - b)), q, m2);
     }
+    reduce_wide<TW>(v, q, m2);
   }
   __device__ __forceinline__ static void contiguous_to_vector(T (&v)[16], const RowX<T>& x) {
     __syncwarp();
@@ -388,8 +436,9 @@ struct Rows {
 #pragma unroll
       for (int i = 0; i < 16; ++i)
         if (!(i & h)) B::inv_bfly(v[i], v[i + h], tw_b(tw, 3 - j, blk, x.t, i >> (j + 1)), q, m2);
+      if (j == 1) reduce_wide_sums<TW>(v, q, m2);
     }
-    reduce_grown<T, 4>(v, q, m2);
+    reduce_grown<TW, T, 4>(v, q, m2);
     __syncwarp();
     x.put_contiguous(v);
     __syncwarp();
@@ -400,8 +449,9 @@ struct Rows {
 #pragma unroll
       for (int i = 0; i < 16; ++i)
         if (!(i & h)) B::inv_bfly(v[i], v[i + h], tw_a(tw, 3 - j, blk, i >> (j + 1)), q, m2);
+      if (j == 1) reduce_wide_sums<TW>(v, q, m2);
     }
-    reduce_grown<T, 4>(v, q, m2);
+    reduce_grown<TW, T, 4>(v, q, m2);
   }
 };
 
@@ -565,20 +615,42 @@ constexpr size_t ks_columns_smem(bool split) {
   return ColGeom<T, LOGN>::smem_bytes() * (split && ColGeom<T, LOGN>::kPasses <= 2 ? 2 : 1);
 }
 
+struct WideRowSource {
+  const uint64_t* in;
+  double q;
+  template <int C>
+  __device__ __forceinline__ void column(int m, int stride, double (&x)[C]) const {
+#pragma unroll
+    for (int k = 0; k < C; ++k) x[k] = Word<double>::from_word_minus(in[k * stride + m], q);
+  }
+};
+struct WideExtSource {
+  ExtSource<uint64_t> ext;
+  double q;
+  template <int C>
+  __device__ __forceinline__ void column(int m, int stride, double (&x)[C]) const {
+    uint64_t w[C];
+    ext.column(m, stride, w);
+#pragma unroll
+    for (int k = 0; k < C; ++k) x[k] = Word<double>::from_word_minus(w[k], q);
+  }
+};
+
 // Launch 1, one column tile: extension of digit a of ciphertext bi to the
 // primes of FP64 rows j0, j1 (each if live) and the column stages of their
 // forward transforms.  PRE: Y already holds the extensions (tensor-core basis
 // conversion), transformed in place.
-template <int LOGN, bool PRE>
+template <int LOGN, bool PRE, bool WIDE>
 __device__ __forceinline__ void ks_columns_f64(const KsPass<uint64_t>& k, int a, int bi, int col0, int j0, int j1,
                                                bool live0, bool live1, unsigned char* smem) {
   using G = ColGeom<uint64_t, LOGN>;
-  using C = Cols<double, LOGN, TwAtQ>;
+  using TW = TwQ<WIDE>;
+  using C = Cols<double, LOGN, TW>;
   constexpr int64_t kN = int64_t(1) << LOGN;
   if (!live0 && !live1) return;
   const DigitDesc d = k.lt.digits[a];
   double* s = reinterpret_cast<double*>(smem);
-  if constexpr (!PRE && G::kPasses <= 2) {
+  if constexpr (!PRE && !WIDE && G::kPasses <= 2) {
     if (d.alpha <= 4 && d.prime0 + d.alpha <= k.f64_end) {
       ks_columns_pair<LOGN>(k, d, a, bi, col0, j0, j1, live0, live1, s);
       return;
@@ -591,8 +663,18 @@ __device__ __forceinline__ void ks_columns_f64(const KsPass<uint64_t>& k, int a,
     const double q = k.tabs64f.prime[pid].q, qinv = k.tabs64f.prime[pid].one_s;
     uint64_t* y = k.y_poly(a, bi, jrow, true, LOGN);
     ColSink<double> sink{reinterpret_cast<double*>(y)};
-    const TwAtQ tw{k.tabs64f.twv_fwd + int64_t(pid) * kN, qinv};
-    if constexpr (PRE) {
+    const TW tw{k.tabs64f.twv_fwd + int64_t(pid) * kN, qinv};
+    if constexpr (PRE && WIDE) {
+      WideRowSource src{y, q};
+      C::template fwd<0>(src, sink, s, tw, q, qinv, col0);
+    } else if constexpr (WIDE) {  // the integer extension, below 2q
+      const PrimeInfo<uint64_t>& p = k.tabs.prime[pid];
+      WideExtSource src{ExtSource<uint64_t>{k.digits + (int64_t(bi) * k.q_limbs + (d.prime0 - k.level)) * kN,
+                                            k.lt.ext + int64_t(a) * kMaxDigitWidth * k.qp0 + pid, k.qp0, d.alpha, LOGN,
+                                            p.q, p.twice_q},
+                        q};
+      C::template fwd<0>(src, sink, s, tw, q, qinv, col0);
+    } else if constexpr (PRE) {
       U64RowSource src{y};
       C::template fwd<0>(src, sink, s, tw, q, qinv, col0);
     } else {
@@ -630,8 +712,8 @@ __device__ __forceinline__ void ks_columns_int(const KsPass<T>& k, int a, int bi
 
 // One block per (digit, ciphertext, column tile, two FP64 rows or one integer
 // row), rows fastest, so the blocks in flight share the digit's words in L2.
-template <typename T, int LOGN, bool PRE, bool SPLIT>
-__global__ void __launch_bounds__(ColGeom<T, LOGN>::kThreads, col_blocks<T, LOGN>(SPLIT && !PRE))
+template <typename T, int LOGN, bool PRE, int SPLIT>
+__global__ void __launch_bounds__(ColGeom<T, LOGN>::kThreads, col_blocks<T, LOGN>(SPLIT == kNarrowF64 && !PRE))
 k_ks_columns(const __grid_constant__ KsPass<T> k) {
   using G = ColGeom<T, LOGN>;
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -648,7 +730,7 @@ k_ks_columns(const __grid_constant__ KsPass<T> k) {
     if (!is_int) {
       const DigitDesc d = k.lt.digits[a];
       const int j0 = k.f_lo + 2 * at, j1 = j0 + 1;
-      ks_columns_f64<LOGN, PRE>(k, a, bi, col0, j0, j1, !ks_own(k, d, j0),
+      ks_columns_f64<LOGN, PRE, SPLIT == kWideF64>(k, a, bi, col0, j0, j1, !ks_own(k, d, j0),
                                 2 * at + 1 < k.f_cnt && !ks_own(k, d, j1), smem_raw);
       return;
     }
@@ -679,19 +761,20 @@ __device__ __forceinline__ T inverse_pow2(T q, T neg_inv) {
 // summed in registers, and the block stages of both inverse transforms.  Half
 // a warp per (ciphertext, 256 words), ciphertexts fastest, so that the half
 // warps of a block read the same key words and twiddles.
-template <int LOGN>
+template <int LOGN, bool WIDE>
 __device__ __forceinline__ void ks_rows_f64(const KsPass<uint64_t>& k, int jrow, int bi, int blk, bool live,
                                             unsigned char* smem) {
   constexpr int64_t kN = int64_t(1) << LOGN;
   using W = Word<double>;
-  using R = Rows<double, LOGN, TwAtQ>;
+  using TW = TwQ<WIDE>;
+  using R = Rows<double, LOGN, TW>;
   const int pid = k.level + jrow;
   const PrimeInfo<double>& p = k.tabs64f.prime[pid];
   const double q = p.q, qinv = p.one_s;
   const RowX<double> x(smem);
   const int vec = blk * kBlk + 2 * x.t;  // this thread's first word, vector layout
   const uint64_t* ct3 = k.ct3 ? k.ct3 + (int64_t(bi) * k.q_limbs + jrow) * kN + vec : nullptr;
-  const TwAtQ twf{k.tabs64f.twv_fwd + int64_t(pid) * kN, qinv};
+  const TW twf{k.tabs64f.twv_fwd + int64_t(pid) * kN, qinv};
   const RowStage<double> stage(smem + kRowSlots * kBlk * sizeof(double));
   int next = 0;  // the term whose row is requested next
   auto request = [&](int a) {  // digit a's row, unless its residue is the ciphertext's own
@@ -713,8 +796,8 @@ __device__ __forceinline__ void ks_rows_f64(const KsPass<uint64_t>& k, int jrow,
 #pragma unroll
         for (int e = 0; e < 8; ++e) {
           const ulonglong2 w = __ldg(reinterpret_cast<const ulonglong2*>(ct3 + 2 * k.ct3_stride + 32 * e));
-          v[2 * e] = W::shoup_bal(W::from_word(w.x), p.rinv, p.rinv_s, q);
-          v[2 * e + 1] = W::shoup_bal(W::from_word(w.y), p.rinv, p.rinv_s, q);
+          v[2 * e] = W::shoup_bal(f64_word<WIDE>(w.x, q), p.rinv, p.rinv_s, q);
+          v[2 * e + 1] = W::shoup_bal(f64_word<WIDE>(w.y, q), p.rinv, p.rinv_s, q);
         }
         request(a + 1);
       } else {
@@ -729,13 +812,17 @@ __device__ __forceinline__ void ks_rows_f64(const KsPass<uint64_t>& k, int jrow,
       for (int e = 0; e < 8; ++e) {
         const ulonglong2 u0 = __ldg(reinterpret_cast<const ulonglong2*>(key0 + 32 * e));
         const ulonglong2 u1 = __ldg(reinterpret_cast<const ulonglong2*>(key1 + 32 * e));
-        a0[2 * e] += W::mul_qinv_bal(v[2 * e], W::from_word(u0.x), q, qinv);
-        a0[2 * e + 1] += W::mul_qinv_bal(v[2 * e + 1], W::from_word(u0.y), q, qinv);
-        a1[2 * e] += W::mul_qinv_bal(v[2 * e], W::from_word(u1.x), q, qinv);
-        a1[2 * e + 1] += W::mul_qinv_bal(v[2 * e + 1], W::from_word(u1.y), q, qinv);
+        a0[2 * e] += W::mul_qinv_bal(v[2 * e], f64_word<WIDE>(u0.x, q), q, qinv);
+        a0[2 * e + 1] += W::mul_qinv_bal(v[2 * e + 1], f64_word<WIDE>(u0.y, q), q, qinv);
+        a1[2 * e] += W::mul_qinv_bal(v[2 * e], f64_word<WIDE>(u1.x, q), q, qinv);
+        a1[2 * e + 1] += W::mul_qinv_bal(v[2 * e + 1], f64_word<WIDE>(u1.y, q), q, qinv);
+      }
+      if (WIDE && ((a & 3) == 3 || a + 1 == k.lt.num_digits)) {  // four terms of at most 0.7 q
+        reduce_wide<TW>(a0, q, qinv);
+        reduce_wide<TW>(a1, q, qinv);
       }
     }
-    if (k.terms > 1) {  // at most 17 digits a term: the sums stay below 2^48
+    if (!WIDE && k.terms > 1) {  // at most 17 digits a term: the sums stay below 2^48
 #pragma unroll
       for (int e = 0; e < 16; ++e) {
         a0[e] = W::reduce_bal(a0[e], q, qinv);
@@ -743,7 +830,7 @@ __device__ __forceinline__ void ks_rows_f64(const KsPass<uint64_t>& k, int jrow,
       }
     }
   }
-  const TwAtQ twi{k.tabs64f.twv_inv + int64_t(pid) * kN, qinv};
+  const TW twi{k.tabs64f.twv_inv + int64_t(pid) * kN, qinv};
   auto finish = [&](double (&v)[16], const uint64_t* add, uint64_t* out) {
 #pragma unroll
     for (int e = 0; e < 16; ++e) v[e] = W::reduce_bal(v[e], q, qinv);
@@ -752,9 +839,10 @@ __device__ __forceinline__ void ks_rows_f64(const KsPass<uint64_t>& k, int jrow,
 #pragma unroll
       for (int e = 0; e < 8; ++e) {
         const ulonglong2 w = __ldg(reinterpret_cast<const ulonglong2*>(add + 32 * e));
-        v[2 * e] += W::shoup_bal(W::from_word(w.x), pc.w, pc.wp, q);
-        v[2 * e + 1] += W::shoup_bal(W::from_word(w.y), pc.w, pc.wp, q);
+        v[2 * e] += W::shoup_bal(f64_word<WIDE>(w.x, q), pc.w, pc.wp, q);
+        v[2 * e + 1] += W::shoup_bal(f64_word<WIDE>(w.y, q), pc.w, pc.wp, q);
       }
+      reduce_wide<TW>(v, q, qinv);
     }
     R::vector_to_contiguous(v, x);
     R::inv(v, x, twi, q, qinv, blk);
@@ -870,7 +958,7 @@ constexpr size_t row_smem() {
   return size_t(2 * kRowSlots) * kBlk * sizeof(T);  // exchanges and the next rows
 }
 
-template <typename T, int LOGN, bool SPLIT>
+template <typename T, int LOGN, int SPLIT>
 __global__ void __launch_bounds__(kRowThreads, sizeof(T) == 8 ? 3 : 4)
 k_ks_rows(const __grid_constant__ KsPass<T> k) {
   __shared__ __align__(16) unsigned char smem[row_smem<T>()];
@@ -889,7 +977,7 @@ k_ks_rows(const __grid_constant__ KsPass<T> k) {
   if constexpr (SPLIT) {
     static_assert(sizeof(T) == 8, "FP64 rows exist in int64 chains only");
     if (!is_int) {
-      ks_rows_f64<LOGN>(k, jrow, bi, blk, live, smem);
+      ks_rows_f64<LOGN, SPLIT == kWideF64>(k, jrow, bi, blk, live, smem);
       return;
     }
   }
@@ -898,7 +986,7 @@ k_ks_rows(const __grid_constant__ KsPass<T> k) {
 
 // Launch 3: one column tile of the inverse transform of the accumulator row z
 // of prime pid, in place, to canonical coefficients.
-template <typename T, int LOGN, bool SPLIT>
+template <typename T, int LOGN, int SPLIT>
 __device__ __forceinline__ void ks_columns_inverse(T* z, int pid, bool f64, const ChainTables<T>& tabs,
                                                    const ChainTables<double>& tabs64f, int col0,
                                                    unsigned char* smem) {
@@ -908,8 +996,8 @@ __device__ __forceinline__ void ks_columns_inverse(T* z, int pid, bool f64, cons
       const PrimeInfo<double>& p = tabs64f.prime[pid];
       ColSource<double> src{reinterpret_cast<double*>(z)};
       F64InvEpilogue epi{reinterpret_cast<uint64_t*>(z), p.q, p.ninv_rinv, p.ninv_rinv_s};
-      Cols<double, LOGN, TwAtQ>::template inv<0>(src, epi, reinterpret_cast<double*>(smem),
-                                                 TwAtQ{tabs64f.twv_inv + int64_t(pid) * kN, p.one_s}, p.q, p.one_s,
+      Cols<double, LOGN, TwQ<SPLIT == kWideF64>>::template inv<0>(src, epi, reinterpret_cast<double*>(smem),
+                                                 TwQ<SPLIT == kWideF64>{tabs64f.twv_inv + int64_t(pid) * kN, p.one_s}, p.q, p.one_s,
                                                  col0);
       return;
     }
@@ -922,7 +1010,7 @@ __device__ __forceinline__ void ks_columns_inverse(T* z, int pid, bool f64, cons
 }
 
 // One block per (component, ciphertext, row, column tile).
-template <typename T, int LOGN, bool SPLIT>
+template <typename T, int LOGN, int SPLIT>
 __global__ void __launch_bounds__(ColGeom<T, LOGN>::kThreads, col_blocks<T, LOGN>(false))
 k_ks_columns_inverse(const __grid_constant__ KsPass<T> k) {
   using G = ColGeom<T, LOGN>;
@@ -959,7 +1047,7 @@ struct WordSource {  // 64-bit words of a prime below 2^42 as balanced doubles
 
 // One column tile of the forward transform of the polynomial `in` of prime
 // pid into `out` (f64: FP64 arithmetic, the intermediate in doubles).
-template <typename T, int LOGN, bool TO_MONT, bool SPLIT>
+template <typename T, int LOGN, bool TO_MONT, int SPLIT>
 __device__ __forceinline__ void ntt_columns(const T* in, T* out, int pid, bool f64, const ChainTables<T>& tabs,
                                             const ChainTables<double>& tabs64f, int col0, unsigned char* smem) {
   constexpr int64_t kN = int64_t(1) << LOGN;
@@ -983,7 +1071,7 @@ __device__ __forceinline__ void ntt_columns(const T* in, T* out, int pid, bool f
 
 // The block stages of the forward transform of row blk of `poly`, in place,
 // to lazy words in [0, 2q).  Half a warp per row of 256 words.
-template <typename T, int LOGN, bool SPLIT>
+template <typename T, int LOGN, int SPLIT>
 __device__ __forceinline__ void ntt_rows(T* poly, int pid, bool f64, const ChainTables<T>& tabs,
                                          const ChainTables<double>& tabs64f, int blk, unsigned char* smem) {
   using X = RowX<T>;
@@ -1028,7 +1116,7 @@ __device__ __forceinline__ void ntt_rows(T* poly, int pid, bool f64, const Chain
 
 // The block stages of the inverse transform of row blk, `in` to `out` (which
 // may be the same buffer).
-template <typename T, int LOGN, bool SPLIT>
+template <typename T, int LOGN, int SPLIT>
 __device__ __forceinline__ void ntt_rows_inverse(const T* in, T* out, int pid, bool f64, const ChainTables<T>& tabs,
                                                  const ChainTables<double>& tabs64f, int blk, unsigned char* smem) {
   using X = RowX<T>;
@@ -1040,16 +1128,18 @@ __device__ __forceinline__ void ntt_rows_inverse(const T* in, T* out, int pid, b
     if (f64) {
       const double q = tabs64f.prime[pid].q, qinv = tabs64f.prime[pid].one_s;
       const RowX<double> xd(smem);
-      using R = Rows<double, LOGN, TwAtQ>;
+      using TW = TwQ<SPLIT == kWideF64>;
+      using R = Rows<double, LOGN, TW>;
       double v[16];
 #pragma unroll
       for (int e = 0; e < 8; ++e) {
         const typename X::Piece w = src[16 * e];
-        v[2 * e] = Word<double>::from_word(w.v[0]);
-        v[2 * e + 1] = Word<double>::from_word(w.v[1]);
+        v[2 * e] = f64_word<TW::kWide>(w.v[0], q);
+        v[2 * e + 1] = f64_word<TW::kWide>(w.v[1], q);
       }
+      reduce_wide<TW>(v, q, qinv);
       R::vector_to_contiguous(v, xd);
-      R::inv(v, xd, TwAtQ{tabs64f.twv_inv + int64_t(pid) * kN, qinv}, q, qinv, blk);
+      R::inv(v, xd, TW{tabs64f.twv_inv + int64_t(pid) * kN, qinv}, q, qinv, blk);
 #pragma unroll
       for (int e = 0; e < 16; ++e) reinterpret_cast<double*>(dst)[16 * e] = v[e];
       return;
@@ -1084,7 +1174,7 @@ struct WordOutEpilogue {
 };
 
 // One column tile of the inverse transform, in place.
-template <typename T, int LOGN, bool SPLIT>
+template <typename T, int LOGN, int SPLIT>
 __device__ __forceinline__ void ntt_columns_inverse(T* out, int pid, bool f64, int kind, const ChainTables<T>& tabs,
                                                     const ChainTables<double>& tabs64f, int col0,
                                                     unsigned char* smem) {
@@ -1096,8 +1186,8 @@ __device__ __forceinline__ void ntt_columns_inverse(T* out, int pid, bool f64, i
       ColSource<double> src{reinterpret_cast<const double*>(out)};
       WordOutEpilogue epi{out, p.q, std_out ? p.ninv_rinv : p.ninv, std_out ? p.ninv_rinv_s : p.ninv_s,
                           kind == kInvCentered};
-      Cols<double, LOGN, TwAtQ>::template inv<0>(src, epi, reinterpret_cast<double*>(smem),
-                                                 TwAtQ{tabs64f.twv_inv + int64_t(pid) * kN, p.one_s}, p.q, p.one_s,
+      Cols<double, LOGN, TwQ<SPLIT == kWideF64>>::template inv<0>(src, epi, reinterpret_cast<double*>(smem),
+                                                 TwQ<SPLIT == kWideF64>{tabs64f.twv_inv + int64_t(pid) * kN, p.one_s}, p.q, p.one_s,
                                                  col0);
       return;
     }
@@ -1109,7 +1199,7 @@ __device__ __forceinline__ void ntt_columns_inverse(T* out, int pid, bool f64, i
                                           TwAt<T>{tabs.tw_inv + int64_t(pid) * kN}, p.q, p.twice_q, col0);
 }
 
-template <typename T, int LOGN, bool TO_MONT, bool SPLIT>
+template <typename T, int LOGN, bool TO_MONT, int SPLIT>
 __global__ void __launch_bounds__(ColGeom<T, LOGN>::kThreads, col_blocks<T, LOGN>(false))
 k_ntt_columns(const T* in, T* out, int rows, int row_start, ChainTables<T> tabs, ChainTables<double> tabs64f,
               int f64_rows) {
@@ -1121,7 +1211,7 @@ k_ntt_columns(const T* in, T* out, int rows, int row_start, ChainTables<T> tabs,
                                        int(blockIdx.x % G::kTiles) * G::kCols, smem_raw);
 }
 
-template <typename T, int LOGN, bool SPLIT>
+template <typename T, int LOGN, int SPLIT>
 __global__ void __launch_bounds__(kRowThreads, sizeof(T) == 8 ? 5 : 8)
 k_ntt_rows(T* out, int64_t slots, int rows, int row_start, ChainTables<T> tabs, ChainTables<double> tabs64f,
            int f64_rows) {
@@ -1135,7 +1225,7 @@ k_ntt_rows(T* out, int64_t slots, int rows, int row_start, ChainTables<T> tabs, 
                            smem);
 }
 
-template <typename T, int LOGN, bool SPLIT>
+template <typename T, int LOGN, int SPLIT>
 __global__ void __launch_bounds__(kRowThreads, sizeof(T) == 8 ? 5 : 8)
 k_ntt_rows_inverse(const T* in, T* out, int64_t slots, int rows, int row_start, ChainTables<T> tabs,
                    ChainTables<double> tabs64f, int f64_rows) {
@@ -1149,7 +1239,7 @@ k_ntt_rows_inverse(const T* in, T* out, int64_t slots, int rows, int row_start, 
                                    int(slot % kBlks), smem);
 }
 
-template <typename T, int LOGN, bool SPLIT>
+template <typename T, int LOGN, int SPLIT>
 __global__ void __launch_bounds__(ColGeom<T, LOGN>::kThreads, col_blocks<T, LOGN>(false))
 k_ntt_columns_inverse(T* out, int rows, int row_start, int kind, ChainTables<T> tabs, ChainTables<double> tabs64f,
                       int f64_rows) {
@@ -1172,7 +1262,7 @@ k_ntt_columns_inverse(T* out, int rows, int row_start, int kind, ChainTables<T> 
 // lines.  y: the prepared digits [D_l, B, QP_l, N].  A thread takes its 16
 // words in two halves, so that a digit's 24 loads fit the registers and can
 // all be in flight.
-template <typename T, int LOGN, bool SPLIT>
+template <typename T, int LOGN, int SPLIT>
 __global__ void __launch_bounds__(kRowThreads, sizeof(T) == 8 ? 3 : 4)
 k_apply_rows(const __grid_constant__ KsPass<T> k, uint32_t galois) {
   using X = RowX<T>;
@@ -1197,7 +1287,8 @@ k_apply_rows(const __grid_constant__ KsPass<T> k, uint32_t galois) {
   if constexpr (SPLIT) {
     if (!is_int) {
       using W = Word<double>;
-      using R = Rows<double, LOGN, TwAtQ>;
+      using TW = TwQ<SPLIT == kWideF64>;
+      using R = Rows<double, LOGN, TW>;
       const RowX<double> xd(smem);
       const double q = k.tabs64f.prime[pid].q, qinv = k.tabs64f.prime[pid].one_s;
       double a0[16], a1[16];
@@ -1216,13 +1307,17 @@ k_apply_rows(const __grid_constant__ KsPass<T> k, uint32_t galois) {
           for (int e = 0; e < 8; ++e) w[e] = __ldg(y + src[e]), k0[e] = __ldg(key0 + 16 * e), k1[e] = __ldg(key1 + 16 * e);
 #pragma unroll
           for (int e = 0; e < 8; ++e) {
-            const double v = W::from_word(w[e]);
-            a0[h + e] += W::mul_qinv_bal(v, W::from_word(k0[e]), q, qinv);
-            a1[h + e] += W::mul_qinv_bal(v, W::from_word(k1[e]), q, qinv);
+            const double v = f64_word<TW::kWide>(w[e], q);
+            a0[h + e] += W::mul_qinv_bal(v, f64_word<TW::kWide>(k0[e], q), q, qinv);
+            a1[h + e] += W::mul_qinv_bal(v, f64_word<TW::kWide>(k1[e], q), q, qinv);
+            if (TW::kWide && (a & 3) == 3) {  // four terms of at most 0.75 q
+              a0[h + e] = W::reduce_bal(a0[h + e], q, qinv);
+              a1[h + e] = W::reduce_bal(a1[h + e], q, qinv);
+            }
           }
         }
       }
-      const TwAtQ tw{k.tabs64f.twv_inv + int64_t(pid) * kN, qinv};
+      const TW tw{k.tabs64f.twv_inv + int64_t(pid) * kN, qinv};
       auto finish = [&](double (&v)[16], T* out) {
 #pragma unroll
         for (int e = 0; e < 16; ++e) v[e] = W::reduce_bal(v[e], q, qinv);

@@ -17,6 +17,17 @@ inline int f64_rows(const Context& c, int row_start, int rows) {
   return std::max(0, std::min(rows, c.f64_prime_end - row_start));
 }
 
+// FP64 form of the chain's leading Q rows, how many of them, and its tables.
+struct F64Form {
+  int form, end;
+  const ChainTables<double>* tabs;
+};
+inline F64Form f64_form(const Context& c) {
+  if (c.f64_core && c.f64_tables_ok) return {kNarrowF64, c.f64_prime_end, &c.t64f};
+  if (c.f64_core && c.wide_tables_ok) return {kWideF64, c.wide_prime_end, &c.t64w};
+  return {kNoF64, 0, &c.t64f};
+}
+
 template <typename T, int LOGN, int EPT = 0, typename... KArgs, typename... Args>
 int launch_cluster(void (*kernel)(KArgs...), int64_t polys, size_t smem, cudaStream_t stream, Args... args) {
   using G = NttGeom<T, LOGN, EPT>;
@@ -79,7 +90,7 @@ int run_forward_e(const Context& c, const void* in, void* out, int64_t polys, in
 
 // By default (no tuning value) both directions run as two launches, columns
 // then rows of 256 words or the reverse (fhb_pass.cuh), the intermediate in `out`.
-template <typename T, int LOGN, bool SPLIT>
+template <typename T, int LOGN, int SPLIT>
 int run_forward_passes(const Context& c, const void* in, void* out, int64_t polys, int rows, int row_start, bool mont,
                        int k, cudaStream_t st) {
   using G = ColGeom<T, LOGN>;
@@ -94,16 +105,16 @@ int run_forward_passes(const Context& c, const void* in, void* out, int64_t poly
                        slots, rows, row_start, tables<T>(c), c.t64f, k);
 }
 
-template <typename T, int LOGN, bool SPLIT>
+template <typename T, int LOGN, int SPLIT>
 int run_inverse_passes(const Context& c, const void* in, void* out, int64_t polys, int rows, int row_start, int kind,
-                       int k, cudaStream_t st) {
+                       int k, cudaStream_t st, const ChainTables<double>& tabs64f) {
   using G = ColGeom<T, LOGN>;
   const int64_t slots = polys << (LOGN - kBlkLog);
   const int rc = launch_blocks(k_ntt_rows_inverse<T, LOGN, SPLIT>, (slots + kRowSlots - 1) / kRowSlots, kRowThreads, 0,
-                               st, (const T*)in, (T*)out, slots, rows, row_start, tables<T>(c), c.t64f, k);
+                               st, (const T*)in, (T*)out, slots, rows, row_start, tables<T>(c), tabs64f, k);
   if (rc != 0) return rc;
   return launch_blocks(k_ntt_columns_inverse<T, LOGN, SPLIT>, polys * G::kTiles, G::kThreads, G::smem_bytes(), st,
-                       (T*)out, rows, row_start, kind, tables<T>(c), c.t64f, k);
+                       (T*)out, rows, row_start, kind, tables<T>(c), tabs64f, k);
 }
 
 template <typename T, int LOGN>
@@ -112,9 +123,9 @@ int run_forward(const Context& c, const void* in, void* out, int64_t polys, int 
   if (c.ntt_ept_fwd == 0) {
     if constexpr (sizeof(T) == 8) {
       const int k = f64_rows(c, row_start, rows);
-      if (k > 0) return run_forward_passes<T, LOGN, true>(c, in, out, polys, rows, row_start, mont, k, st);
+      if (k > 0) return run_forward_passes<T, LOGN, kNarrowF64>(c, in, out, polys, rows, row_start, mont, k, st);
     }
-    return run_forward_passes<T, LOGN, false>(c, in, out, polys, rows, row_start, mont, 0, st);
+    return run_forward_passes<T, LOGN, kNoF64>(c, in, out, polys, rows, row_start, mont, 0, st);
   }
   if (c.ntt_ept_fwd == 16) return run_forward_e<T, LOGN, 16>(c, in, out, polys, rows, row_start, mont, st);
   return run_forward_e<T, LOGN, 0>(c, in, out, polys, rows, row_start, mont, st);
@@ -139,10 +150,15 @@ int run_inverse(const Context& c, const void* in, void* out, int64_t polys, int 
                 cudaStream_t st) {
   if (c.ntt_ept_inv == 0) {
     if constexpr (sizeof(T) == 8) {
-      const int k = f64_rows(c, row_start, rows);
-      if (k > 0) return run_inverse_passes<T, LOGN, true>(c, in, out, polys, rows, row_start, kind, k, st);
+      // the wide rows' words are canonical, so they take the canonical kinds only
+      const F64Form f = f64_form(c);
+      const int k = std::max(0, std::min(rows, f.end - row_start));
+      if (k > 0 && f.form == kNarrowF64)
+        return run_inverse_passes<T, LOGN, kNarrowF64>(c, in, out, polys, rows, row_start, kind, k, st, *f.tabs);
+      if (k > 0 && f.form == kWideF64 && kind >= kInvStandard)
+        return run_inverse_passes<T, LOGN, kWideF64>(c, in, out, polys, rows, row_start, kind, k, st, *f.tabs);
     }
-    return run_inverse_passes<T, LOGN, false>(c, in, out, polys, rows, row_start, kind, 0, st);
+    return run_inverse_passes<T, LOGN, kNoF64>(c, in, out, polys, rows, row_start, kind, 0, st, c.t64f);
   }
   if (c.ntt_ept_inv == 16) return run_inverse_e<T, LOGN, 16>(c, in, out, polys, rows, row_start, kind, st);
   return run_inverse_e<T, LOGN, 0>(c, in, out, polys, rows, row_start, kind, st);
@@ -205,23 +221,24 @@ template <typename T>
 KsPass<T> ks_pass_args(const Context& c, int level) {
   KsPass<T> k = {};
   k.q_limbs = c.num_q - level, k.qp_limbs = k.q_limbs + c.num_p, k.level = level, k.qp0 = c.qp();
-  k.f_cnt = sizeof(T) == 8 ? f64_rows(c, level, k.q_limbs) : 0;
+  const F64Form f = f64_form(c);
+  k.f_cnt = sizeof(T) == 8 ? std::max(0, std::min(k.q_limbs, f.end - level)) : 0;
   k.i_lo = k.f_cnt, k.i_cnt = k.qp_limbs - k.f_cnt;
   k.terms = 1;
   k.ext_digits = c.ext64f_digits, k.f64_end = c.f64_prime_end;
   k.tabs = tables<T>(c), k.lt = level_tables<T>(c, level);
-  k.tabs64f = c.t64f, k.ext64f = c.ext64f;
+  k.tabs64f = *f.tabs, k.ext64f = c.ext64f;
   return k;
 }
 
 // The three launches of one group of rows.
-template <typename T, int LOGN, bool SPLIT>
+template <typename T, int LOGN, int SPLIT>
 int launch_ks_pass(const KsPass<T>& k, int digits, bool pre, cudaStream_t st) {
   using G = ColGeom<T, LOGN>;
   const int64_t units = (k.f_cnt + 1) / 2 + k.i_cnt, blocks = int64_t(digits) * k.batch * units * G::kTiles;
   int rc = pre ? launch_blocks(k_ks_columns<T, LOGN, true, SPLIT>, blocks, G::kThreads, G::smem_bytes(), st, k)
                : launch_blocks(k_ks_columns<T, LOGN, false, SPLIT>, blocks, G::kThreads,
-                               ks_columns_smem<T, LOGN>(SPLIT), st, k);
+                               ks_columns_smem<T, LOGN>(SPLIT == kNarrowF64), st, k);
   if (rc != 0) return rc;
   const int64_t slots = (int64_t(k.batch) << (LOGN - kBlkLog));
   rc = launch_blocks(k_ks_rows<T, LOGN, SPLIT>, (slots + kRowSlots - 1) / kRowSlots * k.rows(), kRowThreads, 0, st, k);
@@ -231,7 +248,7 @@ int launch_ks_pass(const KsPass<T>& k, int digits, bool pre, cudaStream_t st) {
 }
 
 // Launch 1 over the ciphertexts of all terms, then launches 2 and 3 over the sums.
-template <typename T, int LOGN, bool SPLIT>
+template <typename T, int LOGN, int SPLIT>
 int launch_ks_sum(KsPass<T> k, int digits, int terms, bool pre, cudaStream_t st) {
   using G = ColGeom<T, LOGN>;
   const int batch = k.batch;
@@ -239,7 +256,7 @@ int launch_ks_sum(KsPass<T> k, int digits, int terms, bool pre, cudaStream_t st)
   const int64_t units = (k.f_cnt + 1) / 2 + k.i_cnt, blocks = int64_t(digits) * k.batch * units * G::kTiles;
   int rc = pre ? launch_blocks(k_ks_columns<T, LOGN, true, SPLIT>, blocks, G::kThreads, G::smem_bytes(), st, k)
                : launch_blocks(k_ks_columns<T, LOGN, false, SPLIT>, blocks, G::kThreads,
-                               ks_columns_smem<T, LOGN>(SPLIT), st, k);
+                               ks_columns_smem<T, LOGN>(SPLIT == kNarrowF64), st, k);
   if (rc != 0) return rc;
   k.batch = batch, k.terms = terms;
   const int64_t slots = (int64_t(batch) << (LOGN - kBlkLog));
@@ -272,11 +289,13 @@ int run_ks_sum_pass(const Context& c, const void* digits, void* y, int64_t y_wor
     k.y_rows = pre ? qpl : hi - lo;
     int rc = 0;
     if constexpr (sizeof(T) == 8) {
-      rc = f64 > 0 ? launch_ks_sum<T, LOGN, true>(k, nd, terms, pre, st)
-                   : launch_ks_sum<T, LOGN, false>(k, nd, terms, pre, st);
+      const int form = f64 > 0 ? f64_form(c).form : kNoF64;
+      rc = form == kNarrowF64 ? launch_ks_sum<T, LOGN, kNarrowF64>(k, nd, terms, pre, st)
+           : form == kWideF64 ? launch_ks_sum<T, LOGN, kWideF64>(k, nd, terms, pre, st)
+                              : launch_ks_sum<T, LOGN, kNoF64>(k, nd, terms, pre, st);
     } else {
       if (pre) return fail(-7, "the tensor-core basis conversion needs an int64 context");
-      rc = launch_ks_sum<T, LOGN, false>(k, nd, terms, false, st);
+      rc = launch_ks_sum<T, LOGN, kNoF64>(k, nd, terms, false, st);
     }
     if (rc != 0) return rc;
   }
@@ -321,10 +340,13 @@ int run_ks_pass(const Context& c, const void* digits, void* y, int64_t y_words, 
       k.y_rows = pre ? qpl : hi - lo;
       int rc = 0;
       if constexpr (sizeof(T) == 8) {
-        rc = f64 > 0 ? launch_ks_pass<T, LOGN, true>(k, nd, pre, st) : launch_ks_pass<T, LOGN, false>(k, nd, pre, st);
+        const int form = f64 > 0 ? f64_form(c).form : kNoF64;
+        rc = form == kNarrowF64 ? launch_ks_pass<T, LOGN, kNarrowF64>(k, nd, pre, st)
+             : form == kWideF64 ? launch_ks_pass<T, LOGN, kWideF64>(k, nd, pre, st)
+                                : launch_ks_pass<T, LOGN, kNoF64>(k, nd, pre, st);
       } else {
         if (pre) return fail(-7, "the tensor-core basis conversion needs an int64 context");
-        rc = launch_ks_pass<T, LOGN, false>(k, nd, false, st);
+        rc = launch_ks_pass<T, LOGN, kNoF64>(k, nd, false, st);
       }
       if (rc != 0) return rc;
     }
@@ -360,6 +382,10 @@ template <typename T, int LOGN>
 int run_prepare(const Context& c, const void* digits, void* prepared, int64_t batch, int level,
                 cudaStream_t st) {
   KsPass<T> k = ks_pass_args<T>(c, level);
+  if (f64_form(c).form == kWideF64) {  // the prepared words are the integer transform's
+    k.i_lo = k.f_cnt = 0;
+    k.i_cnt = k.qp_limbs;
+  }
   const int f64 = k.f_cnt, nd = k.lt.num_digits, qpl = k.qp_limbs;
   const int64_t n = c.n(), units = (k.f_cnt + 1) / 2 + k.i_cnt, polys = int64_t(nd) * batch * qpl;
   k.by_row = 1, k.y_rows = qpl, k.y_batch = int(batch);
@@ -378,9 +404,9 @@ int run_prepare(const Context& c, const void* digits, void* prepared, int64_t ba
                          level, tables<T>(c), c.t64f, f64);
   };
   if constexpr (sizeof(T) == 8) {
-    if (f64 > 0) return run(k_ks_columns<T, LOGN, false, true>, k_ntt_rows<T, LOGN, true>, true);
+    if (f64 > 0) return run(k_ks_columns<T, LOGN, false, kNarrowF64>, k_ntt_rows<T, LOGN, kNarrowF64>, true);
   }
-  return run(k_ks_columns<T, LOGN, false, false>, k_ntt_rows<T, LOGN, false>, false);
+  return run(k_ks_columns<T, LOGN, false, kNoF64>, k_ntt_rows<T, LOGN, kNoF64>, false);
 }
 
 template <typename T, int LOGN>
@@ -407,13 +433,16 @@ int run_apply_prepared(const Context& c, const void* prepared, const void* key, 
     return 0;
   };
   if constexpr (sizeof(T) == 8) {
-    if (k.f_cnt > 0) return run(k_apply_rows<T, LOGN, true>, k_ks_columns_inverse<T, LOGN, true>);
+    if (k.f_cnt > 0)
+      return f64_form(c).form == kNarrowF64
+                 ? run(k_apply_rows<T, LOGN, kNarrowF64>, k_ks_columns_inverse<T, LOGN, kNarrowF64>)
+                 : run(k_apply_rows<T, LOGN, kWideF64>, k_ks_columns_inverse<T, LOGN, kWideF64>);
   }
-  return run(k_apply_rows<T, LOGN, false>, k_ks_columns_inverse<T, LOGN, false>);
+  return run(k_apply_rows<T, LOGN, kNoF64>, k_ks_columns_inverse<T, LOGN, kNoF64>);
 }
 
 // ---- mixed-level item stages (fhb_items.cuh) ---------------------------------
-template <typename T, int LOGN, bool SPLIT>
+template <typename T, int LOGN, int SPLIT>
 int run_items_form(const Context& c, int stage, const ItemsView& iv, const ItemUnit* un, int64_t count,
                    const ItemUnit* column_units, int64_t column_count, int max_digits, cudaStream_t st) {
   using G = ColGeom<T, LOGN>;

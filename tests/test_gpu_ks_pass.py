@@ -12,6 +12,7 @@ import torch
 from fhelium_b200 import _native as nat
 from fhelium_b200.config import CkksConfig, Preset
 from fhelium_b200.engine import CkksEngine
+from fhelium_b200.values import Ciphertext, RelinearizationKey, RotationKey
 from tests.helpers import oracle_for, random_key, reduced_ring, to_dev, to_np, uniform_residues
 
 pytestmark = pytest.mark.gpu
@@ -65,6 +66,42 @@ def test_relinearize_every_ring_and_room(preset, log_n, level, batch):
         eng.ctx.call("fhb_ckks_relinearize", nat.ptr(d_ct3), nat.ptr(d_key), nat.ptr(out), nat.ptr(scratch), room,
                      batch, level, 0, eng._stream())
         np.testing.assert_array_equal(to_np(out), want, err_msg=f"scratch {room}")
+
+
+@pytest.mark.parametrize("preset,log_n,level", [("slots8192_scale40_levels7_int64", 14, 0),
+                                                ("slots16384_scale50_levels12_int64", 15, 0),
+                                                ("slots8192_scale50_levels5_int64", 12, 0),
+                                                ("slots16384_scale25_levels29_int32", 12, 0)])
+def test_largest_words(preset, log_n, level):
+    """Every word at the top of its range, and alternating with zero: the
+    operands whose products and sums come closest to the exactness bounds of
+    the FP64 rows and of the integer rows' double-width sums."""
+    cfg, eng, orc = _engine(preset, log_n)
+    rows = orc.q_rows(level)
+    q = np.array(cfg.moduli, dtype=np.int64)
+    qp = cfg.num_q_primes + cfg.num_p_primes
+    digits = len(orc.digits_at_level(0))
+    top = np.broadcast_to((2 * q[rows] - 1)[:, None], (3, 2, len(rows), cfg.N)).copy()
+    top[:, 1, :, 1::2] = 0
+    key = np.broadcast_to((2 * q - 1)[:, None], (digits, 2, qp, cfg.N)).copy()
+    key[:, 1, :, ::2] = 0
+    want = np.stack([orc.relinearize(top[:, b], key, level) for b in range(2)], axis=1)
+    key_d = RelinearizationKey(to_dev(key, cfg))
+    got = eng.relinearize(Ciphertext(to_dev(top, cfg), level, 1.0, "ntt", "montgomery"), key_d)
+    np.testing.assert_array_equal(to_np(got.data), want)
+    ct = np.broadcast_to((q[rows] - 1)[:, None], (2, 1, len(rows), cfg.N)).copy()
+    # a hoisted rotation lifts the digits before the automorphism, so its
+    # residues are its own (the oracle has both)
+    hoisted_want = orc.rotate_hoisted(ct[:, 0], [1, 3], {1: key, 3: key}, level)
+    for step, lifted in zip((1, 3), hoisted_want):
+        rk = RotationKey(to_dev(key, cfg), step, eng.galois_element_for_step(step))
+        want = orc.rotate(ct[:, 0], step, key, level)
+        for form in eng._BASIS_FORMS if cfg.buffer_bit_length == 62 else ["cuda_cores"]:
+            eng.basis_conversion = form
+            d_ct = Ciphertext(to_dev(ct, cfg), level, 1.0)
+            np.testing.assert_array_equal(to_np(eng.rotate_with_key(d_ct, rk).data)[:, 0], want)
+            hoisted = eng.rotate_many_with_keys(d_ct, [rk, rk])[0]
+            np.testing.assert_array_equal(to_np(hoisted.data)[:, 0], lifted)
 
 
 @pytest.mark.parametrize("preset,log_n,level,batch", [CASES[2], CASES[4], CASES[10]])
