@@ -1011,86 +1011,133 @@ __global__ void k_rns_binary(const T* __restrict__ a, const T* __restrict__ b, T
 // giant accumulators held in registers.  Replaces the per-diagonal
 // plaintext product + add of the reference's BSGS evaluation
 // (fhelium/experimental/bootstrap/_linear.py:235-393).
+//
+// The products of one giant with up to kBsgsChunk babies are added double
+// width and reduced once: 16 products of words below 2q stay below 2^126
+// (60-bit primes; 2^62 for 28-bit ones) and below 4 q 2^W, so the reduction
+// by 2^W leaves less than 5q, brought below 2q; x 4 makes it a Montgomery
+// product (R = 2^(W - 2)).
+constexpr int kBsgsChunk = 16;
+constexpr int kBsgsAcc = 8;  // giants per thread and pass
+
+template <typename T>
+struct BsgsSum {
+  std::conditional_t<sizeof(T) == 8, unsigned __int128, uint64_t> s = 0;
+  __device__ __forceinline__ void add(T x, T y) { s += static_cast<decltype(s)>(x) * y; }
+  __device__ __forceinline__ T montgomery(T q, T twoq, T qi) const {  // [0, 2q)
+    constexpr int kBits = int(8 * sizeof(T));
+    const T lo = T(s) * qi;
+    T r = T(s >> kBits) + q;
+    if constexpr (sizeof(T) == 8) {
+      r -= __umul64hi(lo, q);
+    } else {
+      r -= __umulhi(lo, q);
+    }
+    r = csub(csub(r, T(2 * twoq)), twoq);
+    r = csub(T(r + r), twoq);
+    return csub(T(r + r), twoq);
+  }
+};
+
+// kBsgsAcc giants of one coefficient: rot points at its baby 0, word(b, j) is
+// its plaintext word for baby b and giant j of the group (0 where there is
+// none: no branch stands between the loads and the products).
+template <typename T, class WordOf>
+__device__ __forceinline__ void bsgs_giants(const T* __restrict__ rot, int64_t rot_stride, int live, int babies,
+                                            const PrimeInfo<T>& p, WordOf word, T* __restrict__ out,
+                                            int64_t out_stride) {
+  const T q = p.q, twoq = p.twice_q, y = T(0) - p.neg_inv, qi = y * (T(2) - q * y);
+  T acc[kBsgsAcc];
+#pragma unroll
+  for (int j = 0; j < kBsgsAcc; ++j) acc[j] = 0;
+  for (int b0 = 0; b0 < babies; b0 += kBsgsChunk) {
+    BsgsSum<T> sum[kBsgsAcc];
+    const int b1 = min(babies, b0 + kBsgsChunk);
+#pragma unroll 4
+    for (int b = b0; b < b1; ++b) {
+      const T x = __ldg(rot + b * rot_stride);
+#pragma unroll
+      for (int j = 0; j < kBsgsAcc; ++j) sum[j].add(x, word(b, j));
+    }
+#pragma unroll
+    for (int j = 0; j < kBsgsAcc; ++j) acc[j] = csub(T(acc[j] + sum[j].montgomery(q, twoq, qi)), twoq);
+  }
+#pragma unroll
+  for (int j = 0; j < kBsgsAcc; ++j)
+    if (j < live) out[j * out_stride] = acc[j];
+}
+
 template <typename T>
 __global__ void k_bsgs_inner(const T* __restrict__ rot, int64_t rot_stride, const T* __restrict__ pts,
                              int64_t pt_stride, const int* __restrict__ table, int giants, int babies,
                              T* __restrict__ out, int64_t out_stride, int64_t polys, int rows, int row_start,
                              int log_n, ChainTables<T> tabs) {
-  constexpr int kAcc = 16;
   const int64_t n = int64_t(1) << log_n;
   const int64_t per = int64_t(rows) * n;
   const int64_t total = polys * per;
   for (int64_t idx = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; idx < total;
        idx += int64_t(gridDim.x) * blockDim.x) {
     const int64_t in_poly = idx % per;  // row * N + coefficient
-    const int row = int(in_poly >> log_n);
-    const PrimeInfo<T> p = tabs.prime[row_start + row];
-    for (int g0 = 0; g0 < giants; g0 += kAcc) {
-      T acc[kAcc];
-#pragma unroll
-      for (int j = 0; j < kAcc; ++j) acc[j] = 0;
-      for (int b = 0; b < babies; ++b) {
-        const T x = rot[b * rot_stride + idx];
-#pragma unroll
-        for (int j = 0; j < kAcc; ++j) {
-          if (g0 + j >= giants) break;
-          const int e = table[(g0 + j) * babies + b];
-          if (e >= 0)
-            acc[j] = csub(acc[j] + Word<T>::mont(x, pts[e * pt_stride + in_poly], p.q, p.neg_inv), p.twice_q);
-        }
-      }
-#pragma unroll
-      for (int j = 0; j < kAcc; ++j)
-        if (g0 + j < giants) out[(g0 + j) * out_stride + idx] = acc[j];
+    const PrimeInfo<T> p = tabs.prime[row_start + int(in_poly >> log_n)];
+    for (int g0 = 0; g0 < giants; g0 += kBsgsAcc) {
+      const int live = min(kBsgsAcc, giants - g0);
+      auto word = [&](int b, int j) {
+        const int e = j < live ? table[(g0 + j) * babies + b] : -1;
+        return e >= 0 ? pts[e * pt_stride + in_poly] : T(0);
+      };
+      bsgs_giants<T>(rot + idx, rot_stride, live, babies, p, word, out + g0 * out_stride + idx, out_stride);
     }
   }
 }
 
 // Same inner products with the plaintext rows staged in shared memory, so
 // that each plaintext residue leaves HBM once however many polynomials share
-// it.  One block per (row, 32 consecutive coefficients): the block stages
-// the 32-coefficient slice of every plaintext entry (entries * 32 words),
-// then each warp takes polynomials warp, warp + 8, ... with lane = the
-// coefficient.  Requires entries * 32 * sizeof(T) of dynamic shared memory.
+// it.  One block per (row, 32 consecutive coefficients): the block stages the
+// 32-coefficient slice of every plaintext entry, a slice of zeros, and the
+// table as offsets [group of giants][baby][giant of the group] (missing
+// entries name the zeros); then its warps take (polynomial, group) pairs in
+// turn, lane = the coefficient.  bsgs_staged_bytes of dynamic shared memory.
 template <typename T>
-__global__ void __launch_bounds__(256)
+size_t bsgs_staged_bytes(int entries, int giants, int babies) {
+  const size_t groups = size_t(giants + kBsgsAcc - 1) / kBsgsAcc;
+  return size_t(entries + 1) * 32 * sizeof(T) + groups * kBsgsAcc * babies * sizeof(int);
+}
+
+template <typename T>
+__global__ void __launch_bounds__(256, 2)
 k_bsgs_inner_staged(const T* __restrict__ rot, int64_t rot_stride, const T* __restrict__ pts, int64_t pt_stride,
                     int entries, const int* __restrict__ table, int giants, int babies, T* __restrict__ out,
                     int64_t out_stride, int64_t polys, int rows, int row_start, int log_n, ChainTables<T> tabs) {
-  constexpr int kAcc = 16;
   constexpr int kTile = 32;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  T* sp = reinterpret_cast<T*>(smem_raw);  // [entries][kTile]
+  T* sp = reinterpret_cast<T*>(smem_raw);  // [entries + 1][kTile]
+  int* st = reinterpret_cast<int*>(sp + (entries + 1) * kTile);
   const int64_t n = int64_t(1) << log_n;
   const int tiles_per_row = int(n / kTile);
   const int row = blockIdx.x / tiles_per_row;
   const int64_t col0 = int64_t(blockIdx.x % tiles_per_row) * kTile;
   const int64_t in_poly0 = int64_t(row) * n + col0;  // row * N + first coefficient of the tile
-  for (int i = threadIdx.x; i < entries * kTile; i += blockDim.x)
-    sp[i] = pts[int64_t(i / kTile) * pt_stride + in_poly0 + (i % kTile)];
+  const int groups = (giants + kBsgsAcc - 1) / kBsgsAcc;
+#pragma unroll 8
+  for (int i = threadIdx.x; i < entries * kTile; i += 256)
+    sp[i] = __ldg(pts + int64_t(i / kTile) * pt_stride + in_poly0 + (i % kTile));
+  if (threadIdx.x < kTile) sp[entries * kTile + threadIdx.x] = 0;
+  for (int i = threadIdx.x; i < groups * kBsgsAcc * babies; i += 256) {
+    const int g = i / (kBsgsAcc * babies) * kBsgsAcc + i % kBsgsAcc, b = i / kBsgsAcc % babies;
+    const int e = g < giants ? table[g * babies + b] : -1;
+    st[i] = (e < 0 ? entries : e) * kTile;
+  }
   __syncthreads();
   const PrimeInfo<T> p = tabs.prime[row_start + row];
   const int lane = threadIdx.x % kTile;
   const int64_t per = int64_t(rows) * n;
-  for (int64_t poly = threadIdx.x / kTile; poly < polys; poly += blockDim.x / kTile) {
-    const int64_t idx = poly * per + in_poly0 + lane;
-    for (int g0 = 0; g0 < giants; g0 += kAcc) {
-      T acc[kAcc];
-#pragma unroll
-      for (int j = 0; j < kAcc; ++j) acc[j] = 0;
-      for (int b = 0; b < babies; ++b) {
-        const T x = rot[b * rot_stride + idx];
-#pragma unroll
-        for (int j = 0; j < kAcc; ++j) {
-          if (g0 + j >= giants) break;
-          const int e = table[(g0 + j) * babies + b];
-          if (e >= 0) acc[j] = csub(acc[j] + Word<T>::mont(x, sp[e * kTile + lane], p.q, p.neg_inv), p.twice_q);
-        }
-      }
-#pragma unroll
-      for (int j = 0; j < kAcc; ++j)
-        if (g0 + j < giants) out[(g0 + j) * out_stride + idx] = acc[j];
-    }
+  for (int64_t w = threadIdx.x / kTile; w < polys * groups; w += 256 / kTile) {
+    const int64_t idx = w / groups * per + in_poly0 + lane;
+    const int g0 = int(w % groups) * kBsgsAcc;
+    const int* off = st + g0 * babies;
+    bsgs_giants<T>(rot + idx, rot_stride, min(kBsgsAcc, giants - g0), babies, p,
+                   [&](int b, int j) { return sp[off[b * kBsgsAcc + j] + lane]; }, out + g0 * out_stride + idx,
+                   out_stride);
   }
 }
 
