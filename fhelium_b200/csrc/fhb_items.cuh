@@ -193,6 +193,7 @@ __global__ void k_items_modup(ItemsView iv, const LevelTables<T>* __restrict__ l
 template <typename T, int NP, bool SPLIT>
 __global__ void __launch_bounds__(kMdThreads, 2)
 k_items_moddown(ItemsView iv, const __grid_constant__ MdArgs<T> args, int groups) {
+  __shared__ double staged[md_staged<SPLIT>()];
   KsItem it;
   if (!items_fetch(iv, int(blockIdx.y), it)) return;
   unsigned idx = blockIdx.x;
@@ -207,7 +208,7 @@ k_items_moddown(ItemsView iv, const __grid_constant__ MdArgs<T> args, int groups
   const uint32_t gi = !add || it.galois == 1 ? 0u : galois_inverse_dev(it.galois, a.log_n);
   moddown_rows<T, NP, SPLIT>(a, static_cast<const T*>(c ? it.t1 : it.t0), add ? static_cast<const T*>(it.a) : nullptr,
                              gi, static_cast<T*>(it.out) + ((int64_t(c) * out_limbs) << a.log_n), k0,
-                             ql * g / groups, ql * (g + 1) / groups);
+                             ql * g / groups, ql * (g + 1) / groups, staged);
 }
 
 // The transform stages take their (item, row) from a work list.  Every thread

@@ -59,6 +59,8 @@ struct MdSum32 {
 template <typename T>
 using MdSum = std::conditional_t<sizeof(T) == 8, MdSum64, MdSum32>;
 
+constexpr int kMdThreads = 256;  // two coefficients each
+
 template <typename T>
 struct MdArgs {
   int log_n, level, num_q, num_p, rescale, f64_end;
@@ -66,12 +68,24 @@ struct MdArgs {
   MdTables<T> md;
 };
 
+// The FP64 rows' constants of one block in shared memory (q, 1/q, then the
+// table's): read from device memory they cost a row thirteen dependent loads,
+// more latency than its products cover.  At most kMdRows rows per block.
+constexpr int kMdRows = 96;
+constexpr int kMdStaged = kMdDoubles + 2;
+template <bool SPLIT>
+constexpr int md_staged() {
+  return SPLIT ? kMdRows * kMdStaged : 1;
+}
+
 // Rows [i0, i1) of Q_l at coefficients k0, k0 + 1 of one component: t
 // [QP_l][N], add [Q_l][N] or null (through sigma_g with inverse gi when gi is
-// not 0), out [Q_l (- 1)][N].  NP = num_p (8: any).
+// not 0), out [Q_l (- 1)][N].  NP = num_p (8: any).  `staged`: md_staged
+// doubles of shared memory; every thread of the block calls this.
 template <typename T, int NP, bool SPLIT>
 __device__ __forceinline__ void moddown_rows(const MdArgs<T>& a, const T* __restrict__ t, const T* __restrict__ add,
-                                             uint32_t gi, T* __restrict__ out, int k0, int i0, int i1) {
+                                             uint32_t gi, T* __restrict__ out, int k0, int i0, int i1,
+                                             double* staged) {
   using W = Word<T>;
   struct alignas(2 * sizeof(T)) Two {
     T v[2];
@@ -80,6 +94,19 @@ __device__ __forceinline__ void moddown_rows(const MdArgs<T>& a, const T* __rest
   auto two = [&](const T* row) {
     return *reinterpret_cast<const Two*>(row + k0);
   };
+  const int64_t base = int64_t(a.rescale ? a.level + 1 : 0) * qp0 + a.level;  // table 0: no rescale
+  const int first = i0;
+  if constexpr (SPLIT) {
+    constexpr int kUsed = 5 + 2 * NP;
+    const int rows = min(i1, a.f64_end - a.level) - first;
+    for (int w = threadIdx.x; w < rows * kUsed; w += kMdThreads) {
+      const int r = w / kUsed, c = w % kUsed, pid = a.level + first + r;
+      staged[r * kMdStaged + c] = c == 0   ? a.md.prime[pid].q
+                                  : c == 1 ? a.md.prime[pid].one_s
+                                           : a.md.f[(base + first + r) * kMdDoubles + c - 2];
+    }
+    __syncthreads();
+  }
   // Garner digits of the P part
   T e[NP][2];
 #pragma unroll
@@ -141,8 +168,7 @@ __device__ __forceinline__ void moddown_rows(const MdArgs<T>& a, const T* __rest
       }
   }
   // the balanced value, not yet canonical
-  auto row_f64 = [&](int i, const double* __restrict__ c, const double* v0, double q, double qinv, double (&r)[2]) {
-    const Two tv = two(t + (int64_t(i) << log_n));
+  auto row_f64 = [&](int i, const Two& tv, const double* c, const double* v0, double q, double qinv, double (&r)[2]) {
 #pragma unroll
     for (int z = 0; z < 2; ++z) {
       MdSumF64 s;
@@ -158,7 +184,6 @@ __device__ __forceinline__ void moddown_rows(const MdArgs<T>& a, const T* __rest
       r[z] = s.balanced(q, qinv);
     }
   };
-  const int64_t base = int64_t(a.rescale ? a.level + 1 : 0) * qp0 + a.level;  // table 0: no rescale
   T v0[2] = {0, 0};
   double v0d[2] = {0.0, 0.0};
   T bit[2] = {0, 0};
@@ -166,7 +191,7 @@ __device__ __forceinline__ void moddown_rows(const MdArgs<T>& a, const T* __rest
     if (SPLIT && a.level < a.f64_end) {
       if constexpr (SPLIT) {
         const double q = a.md.prime[a.level].q, qinv = a.md.prime[a.level].one_s;
-        row_f64(0, a.md.f + int64_t(a.level) * kMdDoubles, nullptr, q, qinv, v0d);
+        row_f64(0, two(t), a.md.f + int64_t(a.level) * kMdDoubles, nullptr, q, qinv, v0d);
 #pragma unroll
         for (int z = 0; z < 2; ++z) {
           if (v0d[z] < 0.0) v0d[z] += q;
@@ -184,11 +209,15 @@ __device__ __forceinline__ void moddown_rows(const MdArgs<T>& a, const T* __rest
   T* o = out - (a.rescale ? int64_t(1) << log_n : 0) + k0;
   int i = i0;
   if constexpr (SPLIT) {
-#pragma unroll 2
-    for (const int f1 = min(i1, a.f64_end - a.level); i < f1; ++i) {
-      const double q = a.md.prime[a.level + i].q, qinv = a.md.prime[a.level + i].one_s;
+    const int f1 = min(i1, a.f64_end - a.level);
+    Two next = i < f1 ? two(t + (int64_t(i) << log_n)) : Two{};
+    for (; i < f1; ++i) {
+      const Two tv = next;
+      if (i + 1 < f1) next = two(t + (int64_t(i + 1) << log_n));
+      const double* c = staged + (i - first) * kMdStaged;
+      const double q = c[0], qinv = c[1];
       double r[2];
-      row_f64(i, a.md.f + (base + i) * kMdDoubles, a.rescale ? v0d : nullptr, q, qinv, r);
+      row_f64(i, tv, c + 2, a.rescale ? v0d : nullptr, q, qinv, r);
       Two w;
 #pragma unroll
       for (int z = 0; z < 2; ++z) {
@@ -210,8 +239,6 @@ __device__ __forceinline__ void moddown_rows(const MdArgs<T>& a, const T* __rest
   }
 }
 
-constexpr int kMdThreads = 256;  // two coefficients each
-
 template <typename T>
 MdArgs<T> moddown_args(const Context& c, int level, int rescale) {
   const bool f64 = sizeof(T) == 8 && c.f64_core && c.f64_tables_ok;
@@ -221,10 +248,11 @@ MdArgs<T> moddown_args(const Context& c, int level, int rescale) {
 
 // Groups of rows per coefficient tile: enough for about eight blocks per SM
 // (below that a single ciphertext leaves SMs idle; each group repeats the
-// digits, about a quarter of a row's work per digit), at most one per row.
+// digits, about a quarter of a row's work per digit), at most one per row;
+// and few enough rows in each for the staged constants.
 inline int moddown_groups(int64_t tiles, int q_limbs) {
-  const int64_t g = (148 * 8 + tiles - 1) / tiles;
-  return int(std::max<int64_t>(1, std::min<int64_t>(g, q_limbs)));
+  const int64_t g = (148 * 8 + tiles - 1) / tiles, least = (q_limbs + kMdRows - 2) / (kMdRows - 1);
+  return int(std::max<int64_t>(least, std::min<int64_t>(g, q_limbs)));
 }
 
 // t0/t1: [B, QP_l, N] canonical coefficient rows; add0/add1 (nullable):
@@ -238,6 +266,7 @@ __global__ void __launch_bounds__(kMdThreads, 2)
 k_moddown(const __grid_constant__ MdArgs<T> a, const T* __restrict__ t0, const T* __restrict__ t1,
           const T* __restrict__ add0, const T* __restrict__ add1, T* __restrict__ out, int64_t out_pitch, int groups,
           uint32_t add0_ginv, const uint32_t* __restrict__ item_galois) {
+  __shared__ double staged[md_staged<SPLIT>()];
   unsigned idx = blockIdx.x;
   const int g = int(idx % unsigned(groups));
   idx /= unsigned(groups);
@@ -252,7 +281,7 @@ k_moddown(const __grid_constant__ MdArgs<T> a, const T* __restrict__ t0, const T
   moddown_rows<T, NP, SPLIT>(a, (c ? t1 : t0) + ((int64_t(bi) * (ql + a.num_p)) << a.log_n),
                              add ? add + ((int64_t(bi) * ql) << a.log_n) : nullptr, gi,
                              out + c * out_pitch + ((int64_t(bi) * (ql - (a.rescale ? 1 : 0))) << a.log_n), k0,
-                             ql * g / groups, ql * (g + 1) / groups);
+                             ql * g / groups, ql * (g + 1) / groups, staged);
 }
 
 // Standalone rescale of coefficient/standard components: in [K, L, N] ->
