@@ -92,6 +92,28 @@ uint64_t prefix_product_mod(const std::vector<uint64_t>& mods, int k, uint64_t m
   return r;
 }
 
+// The block table of a twiddle table [rows][N] (ChainTables::twr_fwd).
+template <typename E>
+std::vector<E> block_table(const std::vector<E>& tw, uint64_t n) {
+  int src[256] = {};  // offset of entry i within its stage's run for one row, and the stage's start
+  std::vector<E> out(tw.size());
+  for (int i = 1; i < 256; ++i) {
+    int s = 0;
+    while ((2 << s) <= i) ++s;
+    const int p = i - (1 << s);
+    src[i] = s < 4 ? p : ((p & 15) << (s - 4)) + (p >> 4);
+  }
+  const uint64_t blocks = n / 256;
+  for (size_t row = 0; row < tw.size() / n; ++row) {
+    const E* from = tw.data() + row * n;
+    E* to = out.data() + row * n;
+    for (uint64_t blk = 0; blk < blocks; ++blk)
+      for (int s = 0; s < 8; ++s)
+        for (int i = 1 << s; i < (2 << s); ++i) to[blk * 256 + i] = from[(blocks << s) + (blk << s) + src[i]];
+  }
+  return out;
+}
+
 // ModDown's row constants (fhb_moddown.cuh): C = 1 or q_l^{-1}, A = P^{-1} C,
 // D = -C, B_r = -M_r A.
 template <typename T>
@@ -185,6 +207,8 @@ bool build_tables(Context& c, ChainTables<T>& t, std::vector<LevelTables<T>>& le
   t.prime = upload(c, info);
   t.tw_fwd = upload(c, fwd);
   t.tw_inv = upload(c, inv);
+  t.twr_fwd = upload(c, block_table(fwd, n));
+  t.twr_inv = upload(c, block_table(inv, n));
   // FP64 tables of the rows of primes below 2^42 (int64 chains whose leading
   // Q primes are that narrow; the rows of wider primes keep the integer
   // tables): the constants and the twiddles as (c, c / q) double pairs, and
@@ -225,6 +249,8 @@ bool build_tables(Context& c, ChainTables<T>& t, std::vector<LevelTables<T>>& le
       c.t64f.tw_inv = upload(c, dinv);
       c.t64f.twv_fwd = upload(c, vfwd);
       c.t64f.twv_inv = upload(c, vinv);
+      c.t64f.twrv_fwd = upload(c, block_table(vfwd, n));
+      c.t64f.twrv_inv = upload(c, block_table(vinv, n));
     }
   }
 
@@ -256,8 +282,11 @@ bool build_tables(Context& c, ChainTables<T>& t, std::vector<LevelTables<T>>& le
       c.t64w.prime = upload(c, dinfo);
       c.t64w.twv_fwd = upload(c, vfwd);
       c.t64w.twv_inv = upload(c, vinv);
+      c.t64w.twrv_fwd = upload(c, block_table(vfwd, n));
+      c.t64w.twrv_inv = upload(c, block_table(vinv, n));
       c.t64w.p_rinv = upload(c, dp);
-      c.wide_tables_ok = c.t64w.prime && c.t64w.twv_fwd && c.t64w.twv_inv && c.t64w.p_rinv;
+      c.wide_tables_ok = c.t64w.prime && c.t64w.twv_fwd && c.t64w.twv_inv && c.t64w.twrv_fwd && c.t64w.twrv_inv &&
+                         c.t64w.p_rinv;
     }
   }
 
@@ -292,7 +321,7 @@ bool build_tables(Context& c, ChainTables<T>& t, std::vector<LevelTables<T>>& le
     }
     c.t64f.p_rinv = upload(c, dp);
     c.f64_tables_ok = c.t64f.prime && c.t64f.tw_fwd && c.t64f.tw_inv && c.t64f.twv_fwd && c.t64f.twv_inv &&
-                      c.t64f.p_rinv;
+                      c.t64f.twrv_fwd && c.t64f.twrv_inv && c.t64f.p_rinv;
   }
 
   // ---- per level: hybrid digits, Garner and extension constants, rescale --
@@ -364,7 +393,7 @@ bool build_tables(Context& c, ChainTables<T>& t, std::vector<LevelTables<T>>& le
     c.ext64f_digits = d0;
     c.f64_tables_ok = c.f64_tables_ok && c.ext64f;
   }
-  return t.prime && t.tw_fwd && t.tw_inv && t.p_garner && t.p_mix && t.p_inv && t.p_rinv && build_moddown(c, md);
+  return t.prime && t.tw_fwd && t.tw_inv && t.twr_fwd && t.twr_inv && t.p_garner && t.p_mix && t.p_inv && t.p_rinv && build_moddown(c, md);
 }
 
 }  // namespace

@@ -50,6 +50,14 @@ struct ChainTables {
   // the quotient from the product and 1/q (prime.one_s).
   T* twv_fwd = nullptr;
   T* twv_inv = nullptr;
+  // Block tables [QP][N / 256][256] of the last eight stages (fhb_pass.cuh):
+  // entry 2^s + p of row blk is the twiddle m of stage log N - 8 + s, m = p
+  // for s < 4 and m = 2^(s - 4) (p mod 16) + p / 16 above; pairs for the
+  // integer rows, values alone (twrv) in the FP64 tables.
+  TwPair<T>* twr_fwd = nullptr;
+  TwPair<T>* twr_inv = nullptr;
+  T* twrv_fwd = nullptr;
+  T* twrv_inv = nullptr;
 };
 
 // ModDown's constants per row (fhb_moddown.cuh): table 0 without rescale,

@@ -340,6 +340,19 @@ struct RowX {
 // The next row of 256 words on its way into shared memory (cp.async, 16 bytes
 // a thread and piece) while the current one is transformed: half a warp owns
 // 256 words here, read back in the strided layout without bank conflicts.
+// Asks L2 for 256 words (a digit ahead of their use; one thread of a half warp).
+template <typename T>
+__device__ __forceinline__ void prefetch_row(const T* row) {
+  asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(row), "r"(int(kBlk * sizeof(T))) : "memory");
+}
+// A 16-byte load that stays where it is written: issued ahead of the stages
+// that run while it is under way.
+__device__ __forceinline__ uint4 load_ahead(const void* p) {
+  uint4 r;
+  asm volatile("ld.global.nc.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w) : "l"(p));
+  return r;
+}
+
 template <typename T>
 struct RowStage {
   unsigned char* w;
@@ -378,16 +391,21 @@ struct Rows {
 
   // Twiddle j of row blk's stage b of the strided layout's four (a) and of
   // thread t's stage b of the contiguous layout's four (b); the inverse
-  // stages mirror them (b = 3 first).
+  // stages mirror them (b = 3 first).  From the block tables (ChainTables::
+  // twr_*), where a row's 255 twiddles lie together and those of the
+  // contiguous layout's stages have the thread fastest: a load is one or two
+  // whole lines (in bit-reversed order a thread's twiddles lie together, and
+  // a load touches up to eight lines).
   __device__ __forceinline__ static TwPair<T> tw_a(const TW& tw, int b, int blk, int j) {
-    return tw.at((1 << (kA + b)) + (blk << b) + j);
+    return tw.at(blk * kBlk + (1 << b) + j);
   }
   __device__ __forceinline__ static TwPair<T> tw_b(const TW& tw, int b, int blk, int t, int j) {
-    return tw.at((1 << (kA + 4 + b)) + ((blk * 16 + t) << b) + j);
+    return tw.at(blk * kBlk + (16 << b) + 16 * j + t);
   }
 
-  // strided -> contiguous
-  __device__ __forceinline__ static void fwd(T (&v)[16], const RowX<T>& x, const TW& tw, T q, T m2, int blk) {
+  // strided -> contiguous: the strided layout's stages and the exchange, then
+  // the contiguous layout's stages
+  __device__ __forceinline__ static void fwd_a(T (&v)[16], const RowX<T>& x, const TW& tw, T q, T m2, int blk) {
 #pragma unroll
     for (int b = 0; b < 4; ++b) {
       const int h = 8 >> b;
@@ -400,6 +418,8 @@ struct Rows {
     x.put_strided(v);
     __syncwarp();
     x.get_contiguous(v);
+  }
+  __device__ __forceinline__ static void fwd_b(T (&v)[16], const RowX<T>& x, const TW& tw, T q, T m2, int blk) {
 #pragma unroll
     for (int b = 0; b < 4; ++b) {
       const int h = 8 >> b;
@@ -408,6 +428,10 @@ struct Rows {
         if (!(i & h)) B::fwd_bfly(v[i], v[i + h], tw_b(tw, b, blk, x.t, i >> (4 - b)), q, m2);
     }
     reduce_wide<TW>(v, q, m2);
+  }
+  __device__ __forceinline__ static void fwd(T (&v)[16], const RowX<T>& x, const TW& tw, T q, T m2, int blk) {
+    fwd_a(v, x, tw, q, m2, blk);
+    fwd_b(v, x, tw, q, m2, blk);
   }
   __device__ __forceinline__ static void contiguous_to_vector(T (&v)[16], const RowX<T>& x) {
     __syncwarp();
@@ -774,11 +798,17 @@ __device__ __forceinline__ void ks_rows_f64(const KsPass<uint64_t>& k, int jrow,
   const RowX<double> x(smem);
   const int vec = blk * kBlk + 2 * x.t;  // this thread's first word, vector layout
   const uint64_t* ct3 = k.ct3 ? k.ct3 + (int64_t(bi) * k.q_limbs + jrow) * kN + vec : nullptr;
-  const TW twf{k.tabs64f.twv_fwd + int64_t(pid) * kN, qinv};
+  const TW twf{k.tabs64f.twrv_fwd + int64_t(pid) * kN, qinv};
   const RowStage<double> stage(smem + kRowSlots * kBlk * sizeof(double));
   int next = 0;  // the term whose row is requested next
   auto request = [&](int a) {  // digit a's row, unless its residue is the ciphertext's own
     if (a == k.lt.num_digits && ++next < k.terms) a = 0;
+    if (a < k.lt.num_digits && x.t == 0) {  // and its keys
+      const uint64_t* key = k.item_keys ? reinterpret_cast<const uint64_t*>(k.item_keys[k.terms > 1 ? next : bi]) : k.key;
+      key += (int64_t(k.lt.digits[a].key_digit) * 2 * k.qp0 + pid) * kN + blk * kBlk;
+      prefetch_row(key);
+      prefetch_row(key + k.qp0 * kN);
+    }
     if (a < k.lt.num_digits && !ks_own(k, k.lt.digits[a], jrow))
       stage.request(reinterpret_cast<const double*>(k.y_poly(a, next * k.batch + bi, jrow, true, LOGN)) + blk * kBlk);
   };
@@ -791,8 +821,18 @@ __device__ __forceinline__ void ks_rows_f64(const KsPass<uint64_t>& k, int jrow,
 #pragma unroll 1
     for (int a = 0; a < k.lt.num_digits; ++a) {
       const DigitDesc d = k.lt.digits[a];
+      const uint64_t* key0 = key + ((int64_t(d.key_digit) * 2) * k.qp0 + pid) * kN + vec;
+      const uint64_t* key1 = key0 + k.qp0 * kN;
       double v[16];
+      uint4 u[8];  // the first component's key words, then the second's, loaded ahead
+      auto load = [&](const uint64_t* key) {
+#pragma unroll
+        for (int e = 0; e < 8; ++e) u[e] = load_ahead(key + 32 * e);
+      };
+      auto lo = [&](const uint4& w) { return f64_word<WIDE>(uint64_t(w.y) << 32 | w.x, q); };
+      auto hi = [&](const uint4& w) { return f64_word<WIDE>(uint64_t(w.w) << 32 | w.z, q); };
       if (ks_own(k, d, jrow)) {
+        load(key0);
 #pragma unroll
         for (int e = 0; e < 8; ++e) {
           const ulonglong2 w = __ldg(reinterpret_cast<const ulonglong2*>(ct3 + 2 * k.ct3_stride + 32 * e));
@@ -803,19 +843,21 @@ __device__ __forceinline__ void ks_rows_f64(const KsPass<uint64_t>& k, int jrow,
       } else {
         stage.take(v);
         request(a + 1);
-        R::fwd(v, x, twf, q, qinv, blk);
+        R::fwd_a(v, x, twf, q, qinv, blk);
+        load(key0);
+        R::fwd_b(v, x, twf, q, qinv, blk);
         R::contiguous_to_vector(v, x);
       }
-      const uint64_t* key0 = key + ((int64_t(d.key_digit) * 2) * k.qp0 + pid) * kN + vec;
-      const uint64_t* key1 = key0 + k.qp0 * kN;
 #pragma unroll
       for (int e = 0; e < 8; ++e) {
-        const ulonglong2 u0 = __ldg(reinterpret_cast<const ulonglong2*>(key0 + 32 * e));
-        const ulonglong2 u1 = __ldg(reinterpret_cast<const ulonglong2*>(key1 + 32 * e));
-        a0[2 * e] += W::mul_qinv_bal(v[2 * e], f64_word<WIDE>(u0.x, q), q, qinv);
-        a0[2 * e + 1] += W::mul_qinv_bal(v[2 * e + 1], f64_word<WIDE>(u0.y, q), q, qinv);
-        a1[2 * e] += W::mul_qinv_bal(v[2 * e], f64_word<WIDE>(u1.x, q), q, qinv);
-        a1[2 * e + 1] += W::mul_qinv_bal(v[2 * e + 1], f64_word<WIDE>(u1.y, q), q, qinv);
+        a0[2 * e] += W::mul_qinv_bal(v[2 * e], lo(u[e]), q, qinv);
+        a0[2 * e + 1] += W::mul_qinv_bal(v[2 * e + 1], hi(u[e]), q, qinv);
+        u[e] = load_ahead(key1 + 32 * e);
+      }
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        a1[2 * e] += W::mul_qinv_bal(v[2 * e], lo(u[e]), q, qinv);
+        a1[2 * e + 1] += W::mul_qinv_bal(v[2 * e + 1], hi(u[e]), q, qinv);
       }
       if (WIDE && ((a & 3) == 3 || a + 1 == k.lt.num_digits)) {  // four terms of at most 0.7 q
         reduce_wide<TW>(a0, q, qinv);
@@ -830,7 +872,7 @@ __device__ __forceinline__ void ks_rows_f64(const KsPass<uint64_t>& k, int jrow,
       }
     }
   }
-  const TW twi{k.tabs64f.twv_inv + int64_t(pid) * kN, qinv};
+  const TW twi{k.tabs64f.twrv_inv + int64_t(pid) * kN, qinv};
   auto finish = [&](double (&v)[16], const uint64_t* add, uint64_t* out) {
 #pragma unroll
     for (int e = 0; e < 16; ++e) v[e] = W::reduce_bal(v[e], q, qinv);
@@ -875,11 +917,17 @@ __device__ __forceinline__ void ks_rows_int(const KsPass<T>& k, int jrow, int bi
     *reinterpret_cast<uint4*>(r.v) = __ldg(reinterpret_cast<const uint4*>(at));
     return r;
   };
-  const TwAt<T> twf{k.tabs.tw_fwd + int64_t(pid) * kN};
+  const TwAt<T> twf{k.tabs.twr_fwd + int64_t(pid) * kN};
   const RowStage<T> stage(smem + kRowSlots * kBlk * sizeof(T));
   int next = 0;
   auto request = [&](int a) {
     if (a == k.lt.num_digits && ++next < k.terms) a = 0;
+    if (a < k.lt.num_digits && x.t == 0) {
+      const T* key = k.item_keys ? reinterpret_cast<const T*>(k.item_keys[k.terms > 1 ? next : bi]) : k.key;
+      key += (int64_t(k.lt.digits[a].key_digit) * 2 * k.qp0 + pid) * kN + blk * kBlk;
+      prefetch_row(key);
+      prefetch_row(key + k.qp0 * kN);
+    }
     if (a < k.lt.num_digits && !ks_own(k, k.lt.digits[a], jrow))
       stage.request(k.y_poly(a, next * k.batch + bi, jrow, false, LOGN) + blk * kBlk);
   };
@@ -922,7 +970,7 @@ __device__ __forceinline__ void ks_rows_int(const KsPass<T>& k, int jrow, int bi
       }
     }
   }
-  const TwAt<T> twi{k.tabs.tw_inv + int64_t(pid) * kN};
+  const TwAt<T> twi{k.tabs.twr_inv + int64_t(pid) * kN};
   auto finish = [&](T (&v)[16], const T* add, T* out) {
 #pragma unroll
     for (int e = 0; e < 16; ++e) {  // x 4: the products were reduced by 2^W, not by R = 2^(W - 2)
@@ -1088,7 +1136,7 @@ __device__ __forceinline__ void ntt_rows(T* poly, int pid, bool f64, const Chain
       double v[16];
 #pragma unroll
       for (int e = 0; e < 16; ++e) v[e] = src[16 * e];
-      R::fwd(v, xd, TwAtQ{tabs64f.twv_fwd + int64_t(pid) * kN, qinv}, q, qinv, blk);
+      R::fwd(v, xd, TwAtQ{tabs64f.twrv_fwd + int64_t(pid) * kN, qinv}, q, qinv, blk);
       R::contiguous_to_vector(v, xd);
 #pragma unroll
       for (int e = 0; e < 8; ++e)
@@ -1103,7 +1151,7 @@ __device__ __forceinline__ void ntt_rows(T* poly, int pid, bool f64, const Chain
   T v[16];
 #pragma unroll
   for (int e = 0; e < 16; ++e) v[e] = at[x.t + 16 * e];
-  R::fwd(v, x, TwAt<T>{tabs.tw_fwd + int64_t(pid) * kN}, q, twoq, blk);
+  R::fwd(v, x, TwAt<T>{tabs.twr_fwd + int64_t(pid) * kN}, q, twoq, blk);
   R::contiguous_to_vector(v, x);
 #pragma unroll
   for (int e = 0; e < X::kVec; ++e) {
@@ -1139,7 +1187,7 @@ __device__ __forceinline__ void ntt_rows_inverse(const T* in, T* out, int pid, b
       }
       reduce_wide<TW>(v, q, qinv);
       R::vector_to_contiguous(v, xd);
-      R::inv(v, xd, TW{tabs64f.twv_inv + int64_t(pid) * kN, qinv}, q, qinv, blk);
+      R::inv(v, xd, TW{tabs64f.twrv_inv + int64_t(pid) * kN, qinv}, q, qinv, blk);
 #pragma unroll
       for (int e = 0; e < 16; ++e) reinterpret_cast<double*>(dst)[16 * e] = v[e];
       return;
@@ -1154,7 +1202,7 @@ __device__ __forceinline__ void ntt_rows_inverse(const T* in, T* out, int pid, b
     for (int i = 0; i < X::V; ++i) v[e * X::V + i] = w.v[i];
   }
   R::vector_to_contiguous(v, x);
-  R::inv(v, x, TwAt<T>{tabs.tw_inv + int64_t(pid) * kN}, tabs.prime[pid].q, tabs.prime[pid].twice_q, blk);
+  R::inv(v, x, TwAt<T>{tabs.twr_inv + int64_t(pid) * kN}, tabs.prime[pid].q, tabs.prime[pid].twice_q, blk);
 #pragma unroll
   for (int e = 0; e < 16; ++e) dst[16 * e] = v[e];
 }
@@ -1317,7 +1365,7 @@ k_apply_rows(const __grid_constant__ KsPass<T> k, uint32_t galois) {
           }
         }
       }
-      const TW tw{k.tabs64f.twv_inv + int64_t(pid) * kN, qinv};
+      const TW tw{k.tabs64f.twrv_inv + int64_t(pid) * kN, qinv};
       auto finish = [&](double (&v)[16], T* out) {
 #pragma unroll
         for (int e = 0; e < 16; ++e) v[e] = W::reduce_bal(v[e], q, qinv);
@@ -1355,7 +1403,7 @@ k_apply_rows(const __grid_constant__ KsPass<T> k, uint32_t galois) {
       }
     }
   }
-  const TwAt<T> tw{k.tabs.tw_inv + int64_t(pid) * kN};
+  const TwAt<T> tw{k.tabs.twr_inv + int64_t(pid) * kN};
   auto finish = [&](T (&v)[16], T* out) {
 #pragma unroll
     for (int e = 0; e < 16; ++e) {  // x 4, as in ks_rows_int
