@@ -344,6 +344,7 @@ struct ItemsCore {
     k.ct3 = it.kind == 0 ? static_cast<const T*>(it.coef) : nullptr;
     k.ct3_stride = int64_t(k.q_limbs) * n;
     k.batch = k.y_batch = k.by_row = k.terms = 1;
+    k.keys_by_term = 0;
     k.y_rows = k.qp_limbs;
     k.f_lo = k.f_cnt = k.i_lo = k.i_cnt = 0;
     k.ext_digits = ext_digits, k.f64_end = f64_end;

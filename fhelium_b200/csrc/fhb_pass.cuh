@@ -500,6 +500,7 @@ struct KsPass {
   int f_lo, f_cnt, i_lo, i_cnt;
   int terms;            // > 1: accumulator bi sums the key switches of ciphertexts g batch + bi of Y
                         // (g < terms), each with the key item_keys[g]
+  int keys_by_term;     // item_keys holds one key per term (also a single one) instead of one per ciphertext
   ChainTables<T> tabs;
   LevelTables<T> lt;
   ChainTables<double> tabs64f;
@@ -804,7 +805,7 @@ __device__ __forceinline__ void ks_rows_f64(const KsPass<uint64_t>& k, int jrow,
   auto request = [&](int a) {  // digit a's row, unless its residue is the ciphertext's own
     if (a == k.lt.num_digits && ++next < k.terms) a = 0;
     if (a < k.lt.num_digits && x.t == 0) {  // and its keys
-      const uint64_t* key = k.item_keys ? reinterpret_cast<const uint64_t*>(k.item_keys[k.terms > 1 ? next : bi]) : k.key;
+      const uint64_t* key = k.item_keys ? reinterpret_cast<const uint64_t*>(k.item_keys[k.keys_by_term ? next : bi]) : k.key;
       key += (int64_t(k.lt.digits[a].key_digit) * 2 * k.qp0 + pid) * kN + blk * kBlk;
       prefetch_row(key);
       prefetch_row(key + k.qp0 * kN);
@@ -817,7 +818,7 @@ __device__ __forceinline__ void ks_rows_f64(const KsPass<uint64_t>& k, int jrow,
 #pragma unroll
   for (int e = 0; e < 16; ++e) a0[e] = a1[e] = 0.0;
   for (int g = 0; g < k.terms; ++g) {
-    const uint64_t* key = k.item_keys ? reinterpret_cast<const uint64_t*>(k.item_keys[k.terms > 1 ? g : bi]) : k.key;
+    const uint64_t* key = k.item_keys ? reinterpret_cast<const uint64_t*>(k.item_keys[k.keys_by_term ? g : bi]) : k.key;
 #pragma unroll 1
     for (int a = 0; a < k.lt.num_digits; ++a) {
       const DigitDesc d = k.lt.digits[a];
@@ -923,7 +924,7 @@ __device__ __forceinline__ void ks_rows_int(const KsPass<T>& k, int jrow, int bi
   auto request = [&](int a) {
     if (a == k.lt.num_digits && ++next < k.terms) a = 0;
     if (a < k.lt.num_digits && x.t == 0) {
-      const T* key = k.item_keys ? reinterpret_cast<const T*>(k.item_keys[k.terms > 1 ? next : bi]) : k.key;
+      const T* key = k.item_keys ? reinterpret_cast<const T*>(k.item_keys[k.keys_by_term ? next : bi]) : k.key;
       key += (int64_t(k.lt.digits[a].key_digit) * 2 * k.qp0 + pid) * kN + blk * kBlk;
       prefetch_row(key);
       prefetch_row(key + k.qp0 * kN);
@@ -937,7 +938,7 @@ __device__ __forceinline__ void ks_rows_int(const KsPass<T>& k, int jrow, int bi
 #pragma unroll
   for (int e = 0; e < 16; ++e) a0[e] = a1[e] = 0;
   for (int g = 0; g < k.terms; ++g) {
-    const T* key = k.item_keys ? reinterpret_cast<const T*>(k.item_keys[k.terms > 1 ? g : bi]) : k.key;
+    const T* key = k.item_keys ? reinterpret_cast<const T*>(k.item_keys[k.keys_by_term ? g : bi]) : k.key;
 #pragma unroll 1
     for (int a = 0; a < k.lt.num_digits; ++a) {
       const DigitDesc d = k.lt.digits[a];

@@ -278,6 +278,7 @@ int run_ks_sum_pass(const Context& c, const void* digits, void* y, int64_t y_wor
   k.digits = static_cast<const T*>(digits);
   k.y = static_cast<T*>(y);
   k.item_keys = reinterpret_cast<const unsigned long long*>(key_ptrs);
+  k.keys_by_term = 1;
   k.acc0 = static_cast<T*>(acc0), k.acc1 = static_cast<T*>(acc1);
   k.by_row = pre, k.batch = int(batch), k.y_batch = int(batch) * terms;
   const int step = pre ? qpl : int(std::min<int64_t>(qpl, y_words / per_row));

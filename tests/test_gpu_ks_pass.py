@@ -143,6 +143,10 @@ def test_workspace_holds_the_required_scratch():
     ("slots8192_scale40_levels7_int64", 12, 2, 3, 5),
     ("slots16384_scale50_levels12_int64", 15, 9, 1, 3),
     ("slots8192_scale25_levels14_int32", 14, 11, 2, 2),
+    # one term: its key serves every ciphertext of the batch
+    ("slots8192_scale40_levels7_int64", 12, 2, 3, 1),
+    ("slots16384_scale50_levels12_int64", 12, 9, 2, 1),
+    ("slots8192_scale25_levels14_int32", 12, 11, 5, 1),
 ])
 def test_key_switch_sum_equals_the_cluster_kernel(preset, log_n, level, batch, giants, form):
     """Whole numbers: the canonical sums of the launches over a work buffer
