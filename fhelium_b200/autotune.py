@@ -17,9 +17,8 @@ The knobs a run can change without recompiling:
   scratch limit of a chunk of items (fewer, larger chunks launch fewer
   times but hold more scratch);
 * ``ntt_forward_ept`` / ``ntt_inverse_ept`` (FHB_TUNE_NTT_{FORWARD,INVERSE}_EPT):
-  residues per thread of the standalone transforms, i.e. the NTT's register
-  radix and tile: 8 residues (radix-8 passes, 1024 threads per CTA at
-  N = 2^16) or 16 (radix-16 passes, 512 threads).
+  how the standalone transforms run: 8 as column and block launches, 16 as
+  one cluster per polynomial with 16 residues per thread.
 
 The cluster width (CTAs per polynomial) is fixed per ring degree when the
 library is compiled; every runtime knob above is picked here by timing the

@@ -819,12 +819,17 @@ static int keyswitch_tail(const Context& c, const fhb::Scratch& s, const void* k
   return FHB_WORD(fhb::moddown, c, s.t0, s.t1, add0, add1, out, batch, level, add0_galois, rescale, st);
 }
 
-// Relinearisation of an NTT-domain ct3 (coefficient-domain c2 already in
-// s.t0): ModUp of c2, the key-switch core with c0, c1 folded in as P c_k
+// Where c2's coefficients go before ModUp: with digits of one prime (one P
+// prime) they are the digits, so ModUp has nothing to do (4 us of 96 for one
+// ciphertext of N = 2^14); otherwise t0, free until the core.
+static char* relinearize_c2(const Context& c, const fhb::Scratch& s) { return c.num_p == 1 ? s.digits : s.t0; }
+
+// Relinearisation of an NTT-domain ct3 (canonical coefficient-domain c2
+// already in relinearize_c2): ModUp of c2, the key-switch core with c0, c1 folded in as P c_k
 // (NTT domain) and c2's own-digit rows reused, ModDown (+ rescale).
 static int relinearize_tail(const Context& c, const fhb::Scratch& s, const void* key, const void* ct3, void* out,
                             int64_t batch, int level, int rescale, cudaStream_t st) {
-  TRY(FHB_WORD(fhb::modup, c, s.t0, s.digits, batch, level, 1u, st));
+  if (c.num_p != 1) TRY(FHB_WORD(fhb::modup, c, s.t0, s.digits, batch, level, 1u, st));
   TRY(ks_core_from_digits(c, s, key, batch, level, st, nullptr, ct3));
   return FHB_WORD(fhb::moddown, c, s.t0, s.t1, nullptr, nullptr, out, batch, level, 1u, rescale, st);
 }
@@ -842,7 +847,7 @@ int fhb_ckks_relinearize(const fhb_context* ctx, const void* ct3, const void* ke
   const int limbs = c.num_q - level;
   const fhb::Scratch s = fhb::carve(c, scratch, batch, level, scratch_bytes);
   const int64_t comp = batch * limbs * c.n() * fhb::word_bytes(c);
-  TRY(fhb::inverse(c, static_cast<const char*>(ct3) + 2 * comp, s.t0, batch * limbs, limbs, level,
+  TRY(fhb::inverse(c, static_cast<const char*>(ct3) + 2 * comp, relinearize_c2(c, s), batch * limbs, limbs, level,
                    fhb::kInvStandard, st));
   return relinearize_tail(c, s, key, ct3, out, batch, level, rescale, st);
 }
@@ -989,7 +994,7 @@ int fhb_ckks_multiply_relinearize(const fhb_context* ctx, const void* a, const v
   // ct3 = a x b into the scratch (elementwise, every SM), then the
   // relinearisation of an NTT-domain ct3
   TRY(FHB_WORD(fhb::mul_ntt, c, a, b, s.coef, batch, level, st));
-  TRY(fhb::inverse(c, s.coef + 2 * comp, s.t0, batch * limbs, limbs, level, fhb::kInvStandard, st));
+  TRY(fhb::inverse(c, s.coef + 2 * comp, relinearize_c2(c, s), batch * limbs, limbs, level, fhb::kInvStandard, st));
   return relinearize_tail(c, s, key, s.coef, out, batch, level, rescale, st);
 }
 

@@ -121,8 +121,8 @@ struct Context {
   LevelTables<uint32_t>* lv32_dev = nullptr;
   std::vector<void*> allocations;
   int ks_order = 2;  // tuning: work order of the key-switch clusters (see ks_work)
-  int ntt_ept_fwd = 0;  // tuning: residues per thread of the standalone forward NTT (0 = default)
-  int ntt_ept_inv = 0;  // tuning: same for the inverse NTT and the fused HMult -> inverse NTT
+  int ntt_ept_fwd = 0;  // tuning: 16 = the standalone forward NTT as one cluster per polynomial (else two launches)
+  int ntt_ept_inv = 0;  // tuning: same for the inverse NTT; residues per thread of the fused HMult -> inverse NTT
   TcNttTables* tc = nullptr;  // tensor-core NTT tables (null until prepared)
   std::mutex tc_mutex;
   // tuning: basis conversion of the key switch on the CUDA cores (0) or the

@@ -19,7 +19,10 @@
 // (primes below 2^42) split the digits, which reach 60 bits, into 30-bit
 // halves with their own constants and add every product exactly on top of
 // 1.5 2^88 (ext_chain in fhb_pass.cuh): at most 19 products of less than
-// 2^84 (three of them) or 2^72 stay below 2^87.
+// 2^84 (three of them) or 2^72 stay below 2^87.  With a reduction per product
+// the kernel was bound by those: 1.93 -> 0.80 ms with the rescale for 32
+// ciphertexts of 35 + 4 rows at N = 2^16 (1.02 ms before the FP64 constants
+// were staged in shared memory).
 #pragma once
 #include <algorithm>
 #include <type_traits>
@@ -289,7 +292,7 @@ k_moddown(const __grid_constant__ MdArgs<T> a, const T* __restrict__ t0, const T
 // (v_i - v_0) C (+ 1) with C = q_0^{-1}.  A thread takes two coefficients of
 // up to kRescaleRows rows, so v_0 and its rounding are read and formed once
 // for them.  Blocks (row group, coefficients, polynomial).  Bound by HBM:
-// 73 us -> 25 us at its rate for 2 x 3 x 29 rows of N = 2^16.
+// 73 -> 36 us for 2 x 3 x 29 rows of N = 2^16, 25 us at the copy rate.
 constexpr int kRescaleRows = 6;
 
 template <typename T, bool SPLIT>

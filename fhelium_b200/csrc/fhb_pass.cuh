@@ -12,9 +12,11 @@
 // per block, meets a cluster barrier before and after its cross-block stages,
 // and leaves 28 of the 148 SMs without a cluster.  Measured on the key-switch
 // core at N = 2^16, L = 35 + 4, 32 ciphertexts: cluster core 20.4 ms (FP64
-// pipe 33 % busy, long scoreboard and barriers), these launches 10.9 ms
-// (FP64 pipe 52-56 % busy: columns 5.1, rows 5.2, inverse columns 0.65 ms);
-// at N = 2^14, one ciphertext, 6 rows: 217 -> 117 us for the whole HMult.
+// pipe 33 % busy, long scoreboard and barriers), these launches 8.9 ms
+// (columns 3.9, rows 4.4, inverse columns 0.64 ms; FP64 pipe 65-73 % busy
+// over the FP64 rows, 46-54 % with the five integer rows); at N = 2^14, one ciphertext: 217 -> 69 us for the whole
+// HMult.  The standalone transforms: 0.86 -> 0.39 ms forward for 12 x 2 x 35
+// int64 rows of N = 2^16, 1.72 -> 0.66 ms inverse for 48 x 2 x 25 int32 rows.
 //
 // Butterflies, twiddles and ranges are those of fhb_ntt.cuh: integer words
 // see the same operations in the same order, so even lazy results are the
@@ -265,6 +267,7 @@ struct ColSink {
 // 16-byte pieces so that every access below is free of bank conflicts.
 constexpr int kRowThreads = 128;                 // four warps, eight half warps
 constexpr int kRowSlots = kRowThreads / 16;
+constexpr int kRowWarps = kRowThreads / 32;
 
 template <typename T>
 constexpr size_t exchange_smem() {
@@ -481,9 +484,10 @@ struct Rows {
 
 // ---------------------------------------------------------------------------
 // Key switch.  The rows in flight are f_cnt FP64 rows from f_lo and i_cnt
-// integer rows from i_lo, dealt out evenly over the blocks (row_at), so that
-// blocks of both kinds share the SMs: the FP64 and the integer pipe then work
-// side by side.  Y holds, per (digit a, ciphertext b, row), the polynomial
+// integer rows from i_lo, the integer ones spread evenly among the others
+// (ks_unit).  In the columns launch neighbouring blocks are of both kinds, so
+// that the FP64 and the integer pipe work side by side; the rows launch takes
+// row after row.  Y holds, per (digit a, ciphertext b, row), the polynomial
 // between the launches: Y[(a y_batch + b) y_rows + slot][N], slot the row
 // itself (by_row: Y covers every row) or its place among the rows in flight.
 template <typename T>
@@ -786,7 +790,7 @@ __device__ __forceinline__ T inverse_pow2(T q, T neg_inv) {
 // summed in registers, and the block stages of both inverse transforms.  Half
 // a warp per (ciphertext, 256 words), ciphertexts fastest, so that the half
 // warps of a block read the same key words and twiddles.
-template <int LOGN, bool WIDE>
+template <int LOGN, bool WIDE, bool SHARED>
 __device__ __forceinline__ void ks_rows_f64(const KsPass<uint64_t>& k, int jrow, int bi, int blk, bool live,
                                             unsigned char* smem) {
   constexpr int64_t kN = int64_t(1) << LOGN;
@@ -803,7 +807,7 @@ __device__ __forceinline__ void ks_rows_f64(const KsPass<uint64_t>& k, int jrow,
   const RowStage<double> stage(smem + kRowSlots * kBlk * sizeof(double));
   int next = 0;  // the term whose row is requested next
   auto request = [&](int a) {  // digit a's row, unless its residue is the ciphertext's own
-    if (a == k.lt.num_digits && ++next < k.terms) a = 0;
+    if (!SHARED && a == k.lt.num_digits && ++next < k.terms) a = 0;
     if (a < k.lt.num_digits && x.t == 0) {  // and its keys
       const uint64_t* key = k.item_keys ? reinterpret_cast<const uint64_t*>(k.item_keys[k.keys_by_term ? next : bi]) : k.key;
       key += (int64_t(k.lt.digits[a].key_digit) * 2 * k.qp0 + pid) * kN + blk * kBlk;
@@ -813,14 +817,15 @@ __device__ __forceinline__ void ks_rows_f64(const KsPass<uint64_t>& k, int jrow,
     if (a < k.lt.num_digits && !ks_own(k, k.lt.digits[a], jrow))
       stage.request(reinterpret_cast<const double*>(k.y_poly(a, next * k.batch + bi, jrow, true, LOGN)) + blk * kBlk);
   };
-  request(0);
+  const int warp = int(threadIdx.x >> 5), a_first = SHARED ? warp : 0, a_step = SHARED ? kRowWarps : 1;
+  request(a_first);
   double a0[16], a1[16];
 #pragma unroll
   for (int e = 0; e < 16; ++e) a0[e] = a1[e] = 0.0;
   for (int g = 0; g < k.terms; ++g) {
     const uint64_t* key = k.item_keys ? reinterpret_cast<const uint64_t*>(k.item_keys[k.keys_by_term ? g : bi]) : k.key;
 #pragma unroll 1
-    for (int a = 0; a < k.lt.num_digits; ++a) {
+    for (int a = a_first; a < k.lt.num_digits; a += a_step) {
       const DigitDesc d = k.lt.digits[a];
       const uint64_t* key0 = key + ((int64_t(d.key_digit) * 2) * k.qp0 + pid) * kN + vec;
       const uint64_t* key1 = key0 + k.qp0 * kN;
@@ -840,10 +845,10 @@ __device__ __forceinline__ void ks_rows_f64(const KsPass<uint64_t>& k, int jrow,
           v[2 * e] = W::shoup_bal(f64_word<WIDE>(w.x, q), p.rinv, p.rinv_s, q);
           v[2 * e + 1] = W::shoup_bal(f64_word<WIDE>(w.y, q), p.rinv, p.rinv_s, q);
         }
-        request(a + 1);
+        request(a + a_step);
       } else {
         stage.take(v);
-        request(a + 1);
+        request(a + a_step);
         R::fwd_a(v, x, twf, q, qinv, blk);
         load(key0);
         R::fwd_b(v, x, twf, q, qinv, blk);
@@ -860,7 +865,7 @@ __device__ __forceinline__ void ks_rows_f64(const KsPass<uint64_t>& k, int jrow,
         a1[2 * e] += W::mul_qinv_bal(v[2 * e], lo(u[e]), q, qinv);
         a1[2 * e + 1] += W::mul_qinv_bal(v[2 * e + 1], hi(u[e]), q, qinv);
       }
-      if (WIDE && ((a & 3) == 3 || a + 1 == k.lt.num_digits)) {  // four terms of at most 0.7 q
+      if (WIDE && (SHARED || (a & 3) == 3 || a + 1 == k.lt.num_digits)) {  // at most four terms of 0.7 q
         reduce_wide<TW>(a0, q, qinv);
         reduce_wide<TW>(a1, q, qinv);
       }
@@ -895,11 +900,30 @@ __device__ __forceinline__ void ks_rows_f64(const KsPass<uint64_t>& k, int jrow,
       for (int e = 0; e < 16; ++e) o[16 * e] = v[e];
     }
   };
-  finish(a0, ct3, k.acc0);
-  finish(a1, ct3 ? ct3 + k.ct3_stride : nullptr, k.acc1);
+  if constexpr (SHARED) {  // the warps' partial sums: warp 0 takes component 0, warp 1 component 1
+    double* part = reinterpret_cast<double*>(smem);
+    constexpr int kWarpWords = 2 * kBlk;
+    const int lane = int(threadIdx.x & 31), mine = warp & 1;
+    __syncthreads();
+#pragma unroll
+    for (int e = 0; e < 16; ++e) {
+      part[(warp * 2) * kWarpWords + e * 32 + lane] = a0[e];
+      part[(warp * 2 + 1) * kWarpWords + e * 32 + lane] = a1[e];
+      a0[e] = 0;
+    }
+    __syncthreads();
+    for (int w = 0; w < kRowWarps; ++w)
+#pragma unroll
+      for (int e = 0; e < 16; ++e) a0[e] += part[(w * 2 + mine) * kWarpWords + e * 32 + lane];
+    __syncthreads();
+    if (warp < 2) finish(a0, mine && ct3 ? ct3 + k.ct3_stride : ct3, mine ? k.acc1 : k.acc0);
+  } else {
+    finish(a0, ct3, k.acc0);
+    finish(a1, ct3 ? ct3 + k.ct3_stride : nullptr, k.acc1);
+  }
 }
 
-template <typename T, int LOGN>
+template <typename T, int LOGN, bool SHARED>
 __device__ __forceinline__ void ks_rows_int(const KsPass<T>& k, int jrow, int bi, int blk, bool live,
                                             unsigned char* smem) {
   constexpr int64_t kN = int64_t(1) << LOGN;
@@ -922,7 +946,7 @@ __device__ __forceinline__ void ks_rows_int(const KsPass<T>& k, int jrow, int bi
   const RowStage<T> stage(smem + kRowSlots * kBlk * sizeof(T));
   int next = 0;
   auto request = [&](int a) {
-    if (a == k.lt.num_digits && ++next < k.terms) a = 0;
+    if (!SHARED && a == k.lt.num_digits && ++next < k.terms) a = 0;
     if (a < k.lt.num_digits && x.t == 0) {
       const T* key = k.item_keys ? reinterpret_cast<const T*>(k.item_keys[k.keys_by_term ? next : bi]) : k.key;
       key += (int64_t(k.lt.digits[a].key_digit) * 2 * k.qp0 + pid) * kN + blk * kBlk;
@@ -932,7 +956,8 @@ __device__ __forceinline__ void ks_rows_int(const KsPass<T>& k, int jrow, int bi
     if (a < k.lt.num_digits && !ks_own(k, k.lt.digits[a], jrow))
       stage.request(k.y_poly(a, next * k.batch + bi, jrow, false, LOGN) + blk * kBlk);
   };
-  request(0);
+  const int warp = int(threadIdx.x >> 5), a_first = SHARED ? warp : 0, a_step = SHARED ? kRowWarps : 1;
+  request(a_first);
   const T qi = inverse_pow2(q, ni);
   T a0[16], a1[16];
 #pragma unroll
@@ -940,7 +965,7 @@ __device__ __forceinline__ void ks_rows_int(const KsPass<T>& k, int jrow, int bi
   for (int g = 0; g < k.terms; ++g) {
     const T* key = k.item_keys ? reinterpret_cast<const T*>(k.item_keys[k.keys_by_term ? g : bi]) : k.key;
 #pragma unroll 1
-    for (int a = 0; a < k.lt.num_digits; ++a) {
+    for (int a = a_first; a < k.lt.num_digits; a += a_step) {
       const DigitDesc d = k.lt.digits[a];
       T v[16];
       if (ks_own(k, d, jrow)) {
@@ -950,10 +975,10 @@ __device__ __forceinline__ void ks_rows_int(const KsPass<T>& k, int jrow, int bi
 #pragma unroll
           for (int i = 0; i < X::V; ++i) v[e * X::V + i] = W::shoup(w.v[i], p.rinv, p.rinv_s, q);
         }
-        request(a + 1);
+        request(a + a_step);
       } else {
         stage.take(v);
-        request(a + 1);
+        request(a + a_step);
         R::fwd(v, x, twf, q, twoq, blk);
         R::contiguous_to_vector(v, x);
       }
@@ -998,8 +1023,27 @@ __device__ __forceinline__ void ks_rows_int(const KsPass<T>& k, int jrow, int bi
       for (int e = 0; e < 16; ++e) o[16 * e] = v[e];
     }
   };
-  finish(a0, ct3, k.acc0);
-  finish(a1, ct3 ? ct3 + k.ct3_stride : nullptr, k.acc1);
+  if constexpr (SHARED) {  // the warps' partial sums: warp 0 takes component 0, warp 1 component 1
+    T* part = reinterpret_cast<T*>(smem);
+    constexpr int kWarpWords = 2 * kBlk;
+    const int lane = int(threadIdx.x & 31), mine = warp & 1;
+    __syncthreads();
+#pragma unroll
+    for (int e = 0; e < 16; ++e) {
+      part[(warp * 2) * kWarpWords + e * 32 + lane] = a0[e];
+      part[(warp * 2 + 1) * kWarpWords + e * 32 + lane] = a1[e];
+      a0[e] = 0;
+    }
+    __syncthreads();
+    for (int w = 0; w < kRowWarps; ++w)
+#pragma unroll
+      for (int e = 0; e < 16; ++e) a0[e] = csub(a0[e] + part[(w * 2 + mine) * kWarpWords + e * 32 + lane], twoq);
+    __syncthreads();
+    if (warp < 2) finish(a0, mine && ct3 ? ct3 + k.ct3_stride : ct3, mine ? k.acc1 : k.acc0);
+  } else {
+    finish(a0, ct3, k.acc0);
+    finish(a1, ct3 ? ct3 + k.ct3_stride : nullptr, k.acc1);
+  }
 }
 
 template <typename T>
@@ -1007,30 +1051,37 @@ constexpr size_t row_smem() {
   return size_t(2 * kRowSlots) * kBlk * sizeof(T);  // exchanges and the next rows
 }
 
-template <typename T, int LOGN, int SPLIT>
+// SHARED: a block takes the rows of one warp only and deals the digits to its
+// four warps, whose sums meet in shared memory; two warps then finish a
+// component each.  For launches that do not fill the GPU: the
+// digits are a serial chain of loads and exchanges otherwise (N = 2^14, one
+// ciphertext: 47.9 -> 25.6 us).
+template <typename T, int LOGN, int SPLIT, bool SHARED>
 __global__ void __launch_bounds__(kRowThreads, sizeof(T) == 8 ? 3 : 4)
 k_ks_rows(const __grid_constant__ KsPass<T> k) {
   __shared__ __align__(16) unsigned char smem[row_smem<T>()];
   constexpr int kBlks = 1 << (LOGN - kBlkLog);
   const unsigned slots = unsigned(kBlks) * unsigned(k.batch);
-  // rows one after the other: the blocks in flight share a row's keys and
-  // twiddles (all rows side by side measured 6 % slower)
-  const unsigned per_row = (slots + kRowSlots - 1) / kRowSlots;
+  // Rows one after the other: the blocks in flight share a row's keys and
+  // twiddles, and an SM runs one of the two bodies at a time (integer blocks
+  // dealt out among the FP64 ones measured 25 % slower: the bodies evict each
+  // other from the instruction caches).
+  const unsigned per_block = SHARED ? 2 : kRowSlots, per_row = (slots + per_block - 1) / per_block;
   int at;
   const bool is_int = ks_unit(int(blockIdx.x / per_row), k.rows(), k.i_cnt, at);
   const int jrow = at + (is_int ? k.i_lo : k.f_lo);
-  unsigned slot = blockIdx.x % per_row * kRowSlots + (threadIdx.x >> 4);
+  unsigned slot = blockIdx.x % per_row * per_block + ((threadIdx.x >> 4) & (per_block - 1));
   const bool live = slot < slots;
   if (!live) slot = slots - 1;  // the last block's spare half warps repeat a row and store nothing
   const int bi = int(slot % unsigned(k.batch)), blk = int(slot / unsigned(k.batch));
   if constexpr (SPLIT) {
     static_assert(sizeof(T) == 8, "FP64 rows exist in int64 chains only");
     if (!is_int) {
-      ks_rows_f64<LOGN, SPLIT == kWideF64>(k, jrow, bi, blk, live, smem);
+      ks_rows_f64<LOGN, SPLIT == kWideF64, SHARED>(k, jrow, bi, blk, live, smem);
       return;
     }
   }
-  ks_rows_int<T, LOGN>(k, jrow, bi, blk, live, smem);
+  ks_rows_int<T, LOGN, SHARED>(k, jrow, bi, blk, live, smem);
 }
 
 // Launch 3: one column tile of the inverse transform of the accumulator row z
@@ -1310,7 +1361,10 @@ k_ntt_columns_inverse(T* out, int rows, int row_start, int kind, ChainTables<T> 
 // in the strided layout the gathers, like the key loads, are whole 128-byte
 // lines.  y: the prepared digits [D_l, B, QP_l, N].  A thread takes its 16
 // words in two halves, so that a digit's 24 loads fit the registers and can
-// all be in flight.
+// all be in flight (33 rows, three ciphertexts, 8 digits at N = 2^16:
+// 350 -> 287 us a step).  Bound by the loads' latency: four blocks per SM
+// spill (333 us), asking the next digit's lines into L2 adds instructions and
+// no overlap (371 us).
 template <typename T, int LOGN, int SPLIT>
 __global__ void __launch_bounds__(kRowThreads, sizeof(T) == 8 ? 3 : 4)
 k_apply_rows(const __grid_constant__ KsPass<T> k, uint32_t galois) {

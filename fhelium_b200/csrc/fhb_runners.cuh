@@ -69,9 +69,11 @@ constexpr size_t ntt_smem() {
 }
 
 // ---- per (T, LOGN) launchers --------------------------------------------
-// The standalone transforms exist with 8 and 16 residues per thread (radix-8
-// passes over 1024 threads or radix-16 passes over 512 for N = 2^16); the
-// context's tuning values pick one per direction (0 = the ring's default).
+// The standalone transforms run as two launches (fhb_pass.cuh) unless the
+// context's tuning value for the direction is 16: one cluster per polynomial
+// with 16 residues per thread.  (0.40 against 0.86 ms forward for 12 x 2 x 35
+// int64 rows of N = 2^16, 0.69 against 1.72 ms inverse for 48 x 2 x 25 int32
+// rows; the autotuner times both.)
 template <typename T, int LOGN, int EPT>
 int run_forward_e(const Context& c, const void* in, void* out, int64_t polys, int rows, int row_start, bool mont,
                   cudaStream_t st) {
@@ -88,8 +90,7 @@ int run_forward_e(const Context& c, const void* in, void* out, int64_t polys, in
   return mont ? launch(k_ntt_forward<T, LOGN, false, EPT>) : launch(k_ntt_forward<T, LOGN, true, EPT>);
 }
 
-// By default (no tuning value) both directions run as two launches, columns
-// then rows of 256 words or the reverse (fhb_pass.cuh), the intermediate in `out`.
+// Columns then rows of 256 words, or the reverse, the intermediate in `out`.
 template <typename T, int LOGN, int SPLIT>
 int run_forward_passes(const Context& c, const void* in, void* out, int64_t polys, int rows, int row_start, bool mont,
                        int k, cudaStream_t st) {
@@ -120,15 +121,14 @@ int run_inverse_passes(const Context& c, const void* in, void* out, int64_t poly
 template <typename T, int LOGN>
 int run_forward(const Context& c, const void* in, void* out, int64_t polys, int rows, int row_start,
                 bool mont, cudaStream_t st) {
-  if (c.ntt_ept_fwd == 0) {
+  if (c.ntt_ept_fwd != 16) {
     if constexpr (sizeof(T) == 8) {
       const int k = f64_rows(c, row_start, rows);
       if (k > 0) return run_forward_passes<T, LOGN, kNarrowF64>(c, in, out, polys, rows, row_start, mont, k, st);
     }
     return run_forward_passes<T, LOGN, kNoF64>(c, in, out, polys, rows, row_start, mont, 0, st);
   }
-  if (c.ntt_ept_fwd == 16) return run_forward_e<T, LOGN, 16>(c, in, out, polys, rows, row_start, mont, st);
-  return run_forward_e<T, LOGN, 0>(c, in, out, polys, rows, row_start, mont, st);
+  return run_forward_e<T, LOGN, 16>(c, in, out, polys, rows, row_start, mont, st);
 }
 
 template <typename T, int LOGN, int EPT>
@@ -148,7 +148,7 @@ int run_inverse_e(const Context& c, const void* in, void* out, int64_t polys, in
 template <typename T, int LOGN>
 int run_inverse(const Context& c, const void* in, void* out, int64_t polys, int rows, int row_start, int kind,
                 cudaStream_t st) {
-  if (c.ntt_ept_inv == 0) {
+  if (c.ntt_ept_inv != 16) {
     if constexpr (sizeof(T) == 8) {
       // the wide rows' words are canonical, so they take the canonical kinds only
       const F64Form f = f64_form(c);
@@ -160,8 +160,7 @@ int run_inverse(const Context& c, const void* in, void* out, int64_t polys, int 
     }
     return run_inverse_passes<T, LOGN, kNoF64>(c, in, out, polys, rows, row_start, kind, 0, st, c.t64f);
   }
-  if (c.ntt_ept_inv == 16) return run_inverse_e<T, LOGN, 16>(c, in, out, polys, rows, row_start, kind, st);
-  return run_inverse_e<T, LOGN, 0>(c, in, out, polys, rows, row_start, kind, st);
+  return run_inverse_e<T, LOGN, 16>(c, in, out, polys, rows, row_start, kind, st);
 }
 
 template <typename T, int LOGN>
@@ -231,6 +230,23 @@ KsPass<T> ks_pass_args(const Context& c, int level) {
   return k;
 }
 
+// Whether the rows launch shares a row's digits among a block's warps (k_ks_rows,
+// SHARED): with three digits or more and at most as many half warps as fill
+// the GPU once without sharing (half as many 32-bit ones).  Below that line
+// warps would be missing; above it the sharing costs its exchange.  Whole
+// HMult, without / with (us), by half warps: N = 2^14 (9 rows) 576 105/74,
+// 1728 155/121, 2880 177/155, 4608 210/217; N = 2^16, one ciphertext, four
+// digits, 3328 193/182, 4096 221/228, two digits, 2048 117/124; 32-bit words
+// of N = 2^15 (12 rows) 1536 61/59, 3072 83/87.
+template <typename T>
+bool shared_rows(int64_t half_warps, int digits) {
+  return digits > 2 && half_warps <= 148 * (sizeof(T) == 8 ? 3 : 2) * kRowSlots;
+}
+inline int64_t rows_blocks(int64_t slots, int rows, bool shared) {
+  const int64_t per = shared ? 2 : kRowSlots;
+  return (slots + per - 1) / per * rows;
+}
+
 // The three launches of one group of rows.
 template <typename T, int LOGN, int SPLIT>
 int launch_ks_pass(const KsPass<T>& k, int digits, bool pre, cudaStream_t st) {
@@ -241,7 +257,9 @@ int launch_ks_pass(const KsPass<T>& k, int digits, bool pre, cudaStream_t st) {
                                ks_columns_smem<T, LOGN>(SPLIT == kNarrowF64), st, k);
   if (rc != 0) return rc;
   const int64_t slots = (int64_t(k.batch) << (LOGN - kBlkLog));
-  rc = launch_blocks(k_ks_rows<T, LOGN, SPLIT>, (slots + kRowSlots - 1) / kRowSlots * k.rows(), kRowThreads, 0, st, k);
+  const bool shared = shared_rows<T>(slots * k.rows(), digits);
+  rc = launch_blocks(shared ? k_ks_rows<T, LOGN, SPLIT, true> : k_ks_rows<T, LOGN, SPLIT, false>,
+                     rows_blocks(slots, k.rows(), shared), kRowThreads, 0, st, k);
   if (rc != 0) return rc;
   return launch_blocks(k_ks_columns_inverse<T, LOGN, SPLIT>, int64_t(2) * k.batch * k.rows() * G::kTiles, G::kThreads,
                        G::smem_bytes(), st, k);
@@ -260,7 +278,9 @@ int launch_ks_sum(KsPass<T> k, int digits, int terms, bool pre, cudaStream_t st)
   if (rc != 0) return rc;
   k.batch = batch, k.terms = terms;
   const int64_t slots = (int64_t(batch) << (LOGN - kBlkLog));
-  rc = launch_blocks(k_ks_rows<T, LOGN, SPLIT>, (slots + kRowSlots - 1) / kRowSlots * k.rows(), kRowThreads, 0, st, k);
+  const bool shared = terms == 1 && shared_rows<T>(slots * k.rows(), digits);
+  rc = launch_blocks(shared ? k_ks_rows<T, LOGN, SPLIT, true> : k_ks_rows<T, LOGN, SPLIT, false>,
+                     rows_blocks(slots, k.rows(), shared), kRowThreads, 0, st, k);
   if (rc != 0) return rc;
   return launch_blocks(k_ks_columns_inverse<T, LOGN, SPLIT>, int64_t(2) * batch * k.rows() * G::kTiles, G::kThreads,
                        G::smem_bytes(), st, k);
@@ -274,6 +294,7 @@ int run_ks_sum_pass(const Context& c, const void* digits, void* y, int64_t y_wor
   KsPass<T> k = ks_pass_args<T>(c, level);
   const int qpl = k.qp_limbs, nd = k.lt.num_digits, f64 = k.f_cnt, ints = k.i_cnt;
   const int64_t per_row = int64_t(nd) * terms * batch * c.n();
+  if (batch <= 0) return 0;
   if (batch * terms > kMaxPassGroup) return fail(-6, "too many ciphertexts for one launch");
   k.digits = static_cast<const T*>(digits);
   k.y = static_cast<T*>(y);
@@ -307,6 +328,7 @@ template <typename T, int LOGN>
 int run_ks_pass(const Context& c, const void* digits, void* y, int64_t y_words, const void* key, void* acc0,
                 void* acc1, int64_t batch, int level, cudaStream_t st, const uint64_t* item_keys, const void* ct3,
                 bool pre, int64_t ct3_pitch) {
+  if (batch <= 0) return 0;
   KsPass<T> k = ks_pass_args<T>(c, level);
   const int ql = k.q_limbs, qpl = k.qp_limbs, nd = k.lt.num_digits, f64 = k.f_cnt, ints = k.i_cnt;
   const int64_t n = c.n();

@@ -70,13 +70,14 @@ int fhb_context_destroy(fhb_context* ctx);
 int fhb_context_root(const fhb_context* ctx, int prime_id, uint64_t* psi);
 
 /* Launch tuning of a context (set by the autotuner, fhelium_b200/autotune.py).
- * FHB_TUNE_KS_ORDER: work order of the key-switch clusters, 0 = the rows of
+ * FHB_TUNE_KS_ORDER: work order of the key-switch clusters (of calls without
+ * workspace, and of the mixed-level items' work lists), 0 = the rows of
  * one ciphertext back to back, 1 = one row across the batch back to back,
  * 2 = one row across a group of four ciphertexts, group by group (default).
- * FHB_TUNE_NTT_FORWARD_EPT / FHB_TUNE_NTT_INVERSE_EPT: residues per thread of
- * the standalone forward / inverse NTT (and of the fused HMult -> inverse
- * NTT): 8 = radix-8 register passes, 16 = radix-16 passes over half the
- * threads, 0 = the ring's default.
+ * FHB_TUNE_NTT_FORWARD_EPT / FHB_TUNE_NTT_INVERSE_EPT: the standalone forward
+ * / inverse NTT as column and block launches (0, the default, or 8) or as one
+ * cluster per polynomial with 16 residues per thread (16); of the fused HMult
+ * -> inverse NTT, residues per thread of its cluster (0 and 8: 8).
  * FHB_TUNE_BASIS_CONVERSION: 0 = the key switch's exact basis extension on
  * the CUDA cores, fused into the key-switch core (the context's default; the
  * Python engine's "auto" keeps it on chains with FP64 rows and sets 1 on

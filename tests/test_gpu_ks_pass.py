@@ -33,6 +33,10 @@ CASES = [
     ("slots16384_scale25_levels29_int32", 15, 26, 7),
     ("slots32768_scale25_levels24_int32", 16, 22, 3),
     ("slots65536_scale25_levels14_int32", 17, 12, 1),
+    # few rows of many digits: the digits dealt to a block's warps
+    ("slots16384_scale50_levels12_int64", 12, 0, 1),
+    ("slots16384_scale25_levels29_int32", 13, 0, 1),
+    ("slots32768_scale40_levels34_int64", 12, 0, 3),
 ]
 
 
@@ -176,3 +180,21 @@ def test_key_switch_sum_equals_the_cluster_kernel(preset, log_n, level, batch, g
     with pytest.raises(nat.NativeCallError):
         eng.ctx.call("fhb_ckks_keyswitch_sum_work", nat.ptr(digits), nat.ptr(ptrs), nat.ptr(got[0]), nat.ptr(got[1]),
                      nat.ptr(work), rooms[0] - 16, giants, batch, level, eng._stream())
+
+
+def test_empty_batches_are_accepted():
+    cfg, eng, _ = _engine("slots8192_scale40_levels7_int64", 14)
+    x = torch.zeros(4096, dtype=torch.int64, device="cuda")
+    st = eng._stream()
+    for room in _rooms(eng, cfg, 0, 1):
+        scratch = torch.empty(room, dtype=torch.uint8, device="cuda")
+        eng.ctx.call("fhb_ckks_relinearize", nat.ptr(x), nat.ptr(x), nat.ptr(x), nat.ptr(scratch), room, 0, 0, 1, st)
+        eng.ctx.call("fhb_ckks_rotate", nat.ptr(x), nat.ptr(x), nat.ptr(x), nat.ptr(scratch), room, 0, 0, 5, st)
+    eng.ctx.call("fhb_ckks_prepare_rotation", nat.ptr(x), nat.ptr(x), 0, 0, st)
+    eng.ctx.call("fhb_ckks_apply_prepared_rotation", nat.ptr(x), nat.ptr(x), nat.ptr(x), nat.ptr(x), 0, 0, 5, st)
+    eng.ctx.call("fhb_ckks_moddown", nat.ptr(x), nat.ptr(x), None, None, nat.ptr(x), 0, 0, 1, 0, st)
+    eng.ctx.call("fhb_ckks_rescale", nat.ptr(x), nat.ptr(x), 0, 0, 1, st)
+    eng.ctx.call("fhb_forward_ntt", nat.ptr(x), nat.ptr(x), 0, 1, 0, 0, st)
+    eng.ctx.call("fhb_inverse_ntt", nat.ptr(x), nat.ptr(x), 0, 1, 0, 2, st)
+    torch.cuda.synchronize()
+    assert not x.any()
