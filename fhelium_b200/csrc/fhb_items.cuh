@@ -353,6 +353,24 @@ struct ItemsCore {
   }
 };
 
+// The item of a block's unit as key-switch arguments in shared memory (every
+// thread of a block works on one unit: a polynomial has a multiple of
+// kRowSlots rows of 256 words).  One thread fetches and checks the
+// descriptor; null (status raised) for a unit that is not the plan's.
+template <typename T>
+__device__ __forceinline__ const KsPass<T>* items_core_pass(const ItemsView& iv, int item, int row, int rows_named,
+                                                            const ItemsCore<T>& core, int64_t n) {
+  __shared__ __align__(16) unsigned char held[sizeof(KsPass<T>)];
+  __shared__ bool ok;
+  if (threadIdx.x == 0) {
+    KsItem it;
+    ok = items_core_unit(iv, item, row, rows_named, core.num_q, core.num_p, it);
+    if (ok) *reinterpret_cast<KsPass<T>*>(held) = core.pass(it, n);
+  }
+  __syncthreads();
+  return ok ? reinterpret_cast<const KsPass<T>*>(held) : nullptr;
+}
+
 // Blocks (unit, column tile, digit), digits fastest; digits past an item's level return.
 template <typename T, int LOGN, bool SPLIT>
 __global__ void __launch_bounds__(ColGeom<T, LOGN>::kThreads, col_blocks<T, LOGN>(SPLIT))
@@ -367,13 +385,13 @@ k_items_core_columns(ItemsView iv, const ItemUnit* __restrict__ units, int max_d
   const ItemUnit u = units[idx / G::kTiles];
   if (u.item == kItemNone && u.row == kItemNone) return;
   const int named = u.row >= kItemPair ? 2 : 1, j0 = u.row >= kItemPair ? u.row - kItemPair : u.row;
-  KsItem it;
-  if (!items_core_unit(iv, u.item, j0, named, core.num_q, core.num_p, it)) return;
-  const KsPass<T> k = core.pass(it, int64_t(1) << LOGN);
+  const KsPass<T>* held = items_core_pass(iv, u.item, j0, named, core, int64_t(1) << LOGN);
+  if (!held) return;
+  const KsPass<T>& k = *held;
   if (a >= k.lt.num_digits) return;
   if constexpr (SPLIT) {
-    if (it.level + j0 < core.f64_end) {
-      const bool two = named == 2 && it.level + j0 + 1 < core.f64_end;
+    if (k.level + j0 < core.f64_end) {
+      const bool two = named == 2 && k.level + j0 + 1 < core.f64_end;
       const DigitDesc d = k.lt.digits[a];
       ks_columns_f64<LOGN, false, false>(k, a, 0, col0, j0, j0 + 1, !ks_own(k, d, j0), two && !ks_own(k, d, j0 + 1),
                                   smem_raw);
@@ -392,15 +410,16 @@ k_items_core_rows(ItemsView iv, const ItemUnit* __restrict__ units, int64_t slot
                   const __grid_constant__ ItemsCore<T> core) {
   constexpr int kBlks = 1 << (LOGN - kBlkLog);
   __shared__ __align__(16) unsigned char smem[row_smem<T>()];
+  static_assert(kBlks % kRowSlots == 0, "a block's rows belong to one unit");
   const int64_t slot = int64_t(blockIdx.x) * kRowSlots + (threadIdx.x >> 4);
-  if (slot >= slots) return;
+  if (slot >= slots) return;  // whole blocks
   const ItemUnit u = units[slot / kBlks];
   const int blk = int(slot % kBlks);
-  KsItem it;
-  if (!items_core_unit(iv, u.item, u.row, 1, core.num_q, core.num_p, it)) return;
-  const KsPass<T> k = core.pass(it, int64_t(1) << LOGN);
+  const KsPass<T>* held = items_core_pass(iv, u.item, u.row, 1, core, int64_t(1) << LOGN);
+  if (!held) return;
+  const KsPass<T>& k = *held;
   if constexpr (SPLIT) {
-    if (it.level + u.row < core.f64_end) {
+    if (k.level + u.row < core.f64_end) {
       ks_rows_f64<LOGN, false, false>(k, u.row, 0, blk, true, smem);
       return;
     }
