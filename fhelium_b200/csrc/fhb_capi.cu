@@ -147,12 +147,24 @@ int modup(const Context& c, const void* comp, void* digits, int64_t batch, int l
   constexpr int V = 16 / sizeof(T);
   const bool vec = aligned16(comp) && aligned16(digits);
   const dim3 g = row_grid(c.n(), vec ? V : 1, lt.num_digits, batch);
+  auto run = [&](auto kern) {
+    kern<<<g, kEwThreads, 0, st>>>((const T*)comp, (T*)digits, batch, limbs, c.log_n, level, ginv, item_galois,
+                                   tables<T>(c), lt);
+  };
+  auto width = [&](auto v) {
+    constexpr int VW = decltype(v)::value;
+    switch (c.num_p) {
+      case 1: return run(k_modup_digits<T, VW, 1>);
+      case 2: return run(k_modup_digits<T, VW, 2>);
+      case 3:
+      case 4: return run(k_modup_digits<T, VW, 4>);
+      default: return run(k_modup_digits<T, VW, kMaxDigitWidth>);
+    }
+  };
   if (vec)
-    k_modup_digits<T, V><<<g, kEwThreads, 0, st>>>((const T*)comp, (T*)digits, batch, limbs, c.log_n, level, ginv,
-                                                  item_galois, tables<T>(c), lt);
+    width(std::integral_constant<int, V>{});
   else
-    k_modup_digits<T, 1><<<g, kEwThreads, 0, st>>>((const T*)comp, (T*)digits, batch, limbs, c.log_n, level, ginv,
-                                                  item_galois, tables<T>(c), lt);
+    width(std::integral_constant<int, 1>{});
   return cuda_status(cudaGetLastError(), "k_modup_digits");
 }
 

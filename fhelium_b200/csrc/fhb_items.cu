@@ -149,8 +149,17 @@ int run_elementwise(const Context& c, const char* plan, const PlanLayout& l, con
     rc = run_stage(c, 1, iv, plan + l.inv_off, info.inverse_units, st);
     if (rc) return rc;
   }
-  k_items_modup<T, V><<<dim3(xb, unsigned(info.max_digits), unsigned(info.items)), kEwThreads, 0, st>>>(
-      iv, level_tables_dev<T>(c), c.num_q, c.log_n, tables<T>(c));
+  auto modup = [&](auto kern) {
+    kern<<<dim3(xb, unsigned(info.max_digits), unsigned(info.items)), kEwThreads, 0, st>>>(
+        iv, level_tables_dev<T>(c), c.num_q, c.log_n, tables<T>(c));
+  };
+  switch (c.num_p) {
+    case 1: modup(k_items_modup<T, V, 1>); break;
+    case 2: modup(k_items_modup<T, V, 2>); break;
+    case 3:
+    case 4: modup(k_items_modup<T, V, 4>); break;
+    default: modup(k_items_modup<T, V, kMaxDigitWidth>);
+  }
   if (int e = cuda_status(cudaGetLastError(), "k_items_modup")) return e;
   if (int rc = run_stage(c, 2, iv, plan + l.core_off, info.core_units, st, plan + l.pair_off, l.pairs,
                          info.max_digits))

@@ -135,7 +135,7 @@ __global__ void k_items_mul(ItemsView iv, const int32_t* __restrict__ hmult, int
 // ModUp digits of every item (k_modup_digits per item): the source is d2 in
 // the coefficient domain (t0) for HMult, c1 through sigma_g for a rotation.
 // Grid (N / (256 V), digits, items), digits past an item's level return.
-template <typename T, int V>
+template <typename T, int V, int WIDTH>
 __global__ void k_items_modup(ItemsView iv, const LevelTables<T>* __restrict__ levels, int num_q, int log_n,
                               ChainTables<T> tabs) {
   KsItem it;
@@ -152,8 +152,10 @@ __global__ void k_items_modup(ItemsView iv, const LevelTables<T>* __restrict__ l
   const uint32_t gi = (it.kind == 0 || it.galois == 1) ? 0u : galois_inverse_dev(it.galois, log_n);
   const T* src = it.kind == 0 ? static_cast<const T*>(it.t0) : static_cast<const T*>(it.a) + int64_t(limbs) * n;
   T* dst = static_cast<T*>(it.digits);
-  EwVec<T, V> dig[kMaxDigitWidth];
-  for (int r = 0; r < d.alpha; ++r) {
+  EwVec<T, V> dig[WIDTH];
+#pragma unroll
+  for (int r = 0; r < WIDTH; ++r) {
+    if (r >= d.alpha) break;
     const int row = d.prime0 - it.level + r;
     const T q = tabs.prime[d.prime0 + r].q;
     EwVec<T, V> x;
@@ -175,6 +177,7 @@ __global__ void k_items_modup(ItemsView iv, const LevelTables<T>* __restrict__ l
 #pragma unroll
       for (int e = 0; e < V; ++e) {
         T acc = 0;
+#pragma unroll
         for (int i = 0; i < r; ++i) {
           const TwPair<T> c = g[r * kMaxDigitWidth + i];
           acc = csub(acc + csub(W::shoup(dig[i].v[e], c.w, c.wp, q), q), q);

@@ -349,7 +349,9 @@ __device__ __forceinline__ int galois_ntt_source(int k, int log_n, uint32_t g) {
 // coefficient/standard (canonical or lazy [0, 2q)); digits: [B, L, N],
 // row r holds the mixed-radix digit of the prime in row r.  When ginv != 0
 // the input is first mapped through sigma_g (rotation).
-template <typename T, int V>
+// WIDTH: at least the digits' primes (the P count, or 8), so that the digits
+// stay in registers.
+template <typename T, int V, int WIDTH>
 __global__ void k_modup_digits(const T* __restrict__ comp, T* __restrict__ digits, int64_t batch,
                                int limbs, int log_n, int level, uint32_t ginv,
                                const uint32_t* __restrict__ item_galois, ChainTables<T> tabs, LevelTables<T> lt) {
@@ -365,8 +367,10 @@ __global__ void k_modup_digits(const T* __restrict__ comp, T* __restrict__ digit
     const uint32_t gi = item_galois ? (item_galois[bi] == 1 ? 0u : galois_inverse_dev(item_galois[bi], log_n)) : ginv;
     const T* src = comp + bi * limbs * n;
     T* dst = digits + bi * limbs * n;
-    EwVec<T, V> dig[kMaxDigitWidth];
-    for (int r = 0; r < d.alpha; ++r) {
+    EwVec<T, V> dig[WIDTH];
+#pragma unroll
+    for (int r = 0; r < WIDTH; ++r) {
+      if (r >= d.alpha) break;
       const int row = d.prime0 - level + r;
       const T q = tabs.prime[d.prime0 + r].q;
       EwVec<T, V> x;
@@ -388,6 +392,7 @@ __global__ void k_modup_digits(const T* __restrict__ comp, T* __restrict__ digit
 #pragma unroll
         for (int e = 0; e < V; ++e) {
           T acc = 0;
+#pragma unroll
           for (int i = 0; i < r; ++i) {
             const TwPair<T> c = g[r * kMaxDigitWidth + i];
             acc = csub(acc + csub(W::shoup(dig[i].v[e], c.w, c.wp, q), q), q);
@@ -1007,8 +1012,8 @@ __global__ void k_rns_binary(const T* __restrict__ a, const T* __restrict__ b, T
 //   out[k] = sum_b rot[b] (.) pts[table[k][b]]      (NTT/Montgomery, lazy)
 // rot: [babies][polys][rows][N] baby rotations; pts: [entries][rows][N]
 // diagonal plaintexts shared by every poly; table: [giants][babies] entry
-// index or -1.  Each baby residue is read once and multiplied into up to 16
-// giant accumulators held in registers.  Replaces the per-diagonal
+// index or -1.  A thread multiplies a baby residue into the accumulators of
+// kBsgsAcc giants, held in registers.  Replaces the per-diagonal
 // plaintext product + add of the reference's BSGS evaluation
 // (fhelium/experimental/bootstrap/_linear.py:235-393).
 //
@@ -1016,7 +1021,9 @@ __global__ void k_rns_binary(const T* __restrict__ a, const T* __restrict__ b, T
 // width and reduced once: 16 products of words below 2q stay below 2^126
 // (60-bit primes; 2^62 for 28-bit ones) and below 4 q 2^W, so the reduction
 // by 2^W leaves less than 5q, brought below 2q; x 4 makes it a Montgomery
-// product (R = 2^(W - 2)).
+// product (R = 2^(W - 2)).  A reduction per product bound the kernel:
+// 5.2 -> 1.8 ms a launch in the full-slot bootstrap of two ciphertexts of
+// N = 2^16.
 constexpr int kBsgsChunk = 16;
 constexpr int kBsgsAcc = 8;  // giants per thread and pass
 
