@@ -51,19 +51,9 @@ ROOT = os.path.dirname(os.path.abspath(__file__))
 sys.path.insert(0, ROOT)
 
 PRESET = "slots32768_scale40_levels34_int64"
-KS_TRAFFIC_BYTES_BATCH32 = 12741399552 + 2934590720  # ncu dram read + write, k_keyswitch_core, batch 32 (profiles/)
-# same for the key-switch core of the tensor-core form: captured at batch 8 (3094038784 + 705889536 bytes,
-# 2.01x the batch-4 capture) and scaled by the ciphertexts processed
-KS_EXT_TRAFFIC_BYTES_BATCH32 = 4 * (3094038784 + 705889536)
-# the CUDA-core form's core with its FP64 rows (k_keyswitch_core_split<false>, the extension computed in FP64 in
-# the core, the default for this chain): captured at batch 8 (3810678272 + 360568320 bytes; every destination row
-# re-reads its group's digit rows and the group's key rows, so the traffic grows with the batch) and scaled by the
-# ciphertexts processed
-KS_SPLIT_TRAFFIC_BYTES_BATCH32 = 4 * (3810678272 + 360568320)
-# the tensor-core form's core with its FP64 rows (k_keyswitch_core_split<PRE>): captured at batch 8 (3085136640 + 355092224
-# bytes; the key and digit rows are re-read per group of four ciphertexts, so the traffic grows with the batch)
-# and scaled by the ciphertexts processed
-KS_F64_TRAFFIC_BYTES_BATCH32 = 4 * (3085136640 + 355092224)
+# ncu dram read + write of the key-switch core's three launches over all rows, captured at batch 4 and scaled by the
+# ciphertexts processed (columns 0.76 GB, rows 1.59 GB, inverse columns 0.27 GB); see profiles/
+KS_TRAFFIC_BYTES_BATCH4 = 2616626000
 METRIC = "hmult_relin_rescale_ops_per_s_logN16_L35"
 UNIT = "ops/s"
 CONFIG = {
@@ -757,15 +747,19 @@ def main() -> int:
     ms = _max_over_ranks(ms, ws, dev)
     from fhelium_b200 import ranks
     value = ranks.job_rate(B, ws, ms)
-    # tensor product, INTT of c2, ModUp digits, (tensor-core basis extension,) key-switch core, ModDown+rescale
-    # (the tensor-core form's core is two launches when its Q rows run in FP64:
-    # the P rows stay on the integer kernel)
     f64_core = bool(eng.ctx.get_tuning(nat.TUNE_F64_CORE))
-    # tensor product, inverse NTT of d2, ModUp digits, (tensor-core extension,) core, ModDown; the FP64 rows of
-    # the NTT and of the core share their launches with the integer rows
-    # per chunk of the overlapped call (batches of 16 or more run in up to FHB_TUNE_OVERLAP_CHUNKS chunks)
-    chunks_per_step = max(1, min(int(eng.ctx.get_tuning(nat.TUNE_OVERLAP_CHUNKS)), B // 8))
-    launches_per_step = (6 if form == "tensor_cores" else 5) * (chunks_per_step if chunks_per_step > 1 else 1)
+    # kernels of one step: tensor product, inverse NTT of d2 (two launches), ModUp digits, (tensor-core extension,)
+    # the key-switch core (columns, rows, inverse columns, once per group of rows that the workspace's room holds;
+    # the tensor-core form takes all rows at once), ModDown + rescale
+    lib, h = eng.ctx.lib, eng.ctx.handle
+    qp_rows = cfg.num_q_primes + cfg.num_p_primes
+    row_groups = 1
+    if form != "tensor_cores":
+        room = (int(lib.fhb_ckks_keyswitch_workspace_bytes(h, B, 0))
+                - int(lib.fhb_ckks_keyswitch_scratch_bytes(h, B, 0)))
+        per_row = len(eng.level_digits[0]) * B * cfg.N * 8
+        row_groups = -(-qp_rows // min(qp_rows, room // per_row))
+    launches_per_step = 5 + (1 if form == "tensor_cores" else 0) + 3 * row_groups
 
     # ---- end to end through the public API with host buffers -------------
     host_a = ca.data.cpu().pin_memory()
@@ -810,18 +804,21 @@ def main() -> int:
     d2h = out_host.numel() * 8
 
     # ---- dominant kernel alone: fused key-switch core --------------------
-    lib, h = eng.ctx.lib, eng.ctx.handle
     L = cfg.num_q_primes
     coef = torch.empty((3, B, L, cfg.N), dtype=torch.int64, device=dev)
     digits = torch.empty((B, L, cfg.N), dtype=torch.int64, device=dev)
     t = torch.empty((2, B, L + cfg.num_p_primes, cfg.N), dtype=torch.int64, device=dev)
     s = stream.cuda_stream
+    key_ptr = torch.tensor([rlk.data.data_ptr()], dtype=torch.int64, device=dev)
+    work = torch.empty(int(lib.fhb_ckks_keyswitch_sum_workspace_bytes(h, 1, B, 0)), dtype=torch.uint8, device=dev)
     kernels = {
         "mul_to_coefficient": lambda: lib.fhb_ckks_multiply_to_coefficient(h, nat.ptr(ca.data), nat.ptr(cb.data),
                                                                              nat.ptr(coef), B, 0, s),
         "modup_digits": lambda: lib.fhb_ckks_modup_digits(h, nat.ptr(coef[2]), nat.ptr(digits), B, 0, 1, s),
-        "keyswitch_core": lambda: lib.fhb_ckks_keyswitch_core(h, nat.ptr(digits), nat.ptr(rlk.data), nat.ptr(t[0]),
-                                                              nat.ptr(t[1]), B, 0, s),
+        # one term: the key switch of the batch over a work buffer, as the fused step runs it
+        "keyswitch_core": lambda: lib.fhb_ckks_keyswitch_sum_work(h, nat.ptr(digits), nat.ptr(key_ptr), nat.ptr(t[0]),
+                                                                  nat.ptr(t[1]), nat.ptr(work), work.numel(), 1, B,
+                                                                  0, s),
         "moddown_rescale": lambda: lib.fhb_ckks_moddown(h, nat.ptr(t[0]), nat.ptr(t[1]), nat.ptr(coef[0]),
                                                         nat.ptr(coef[1]), nat.ptr(state["out"].data), B, 0, 1, 1, s),
         # the two launches the fused step uses before ModUp: NTT-domain tensor
@@ -831,11 +828,9 @@ def main() -> int:
     }
     ext = None
     if form == "tensor_cores":
-        # the tensor-core form's two key-switch kernels
+        # the tensor-core form's extension alone (keyswitch_core includes it)
         ext = torch.empty(int(lib.fhb_tc_basis_extend_words(h, B, 0)), dtype=torch.int64, device=dev)
         kernels["tc_basis_extend"] = lambda: lib.fhb_tc_basis_extend(h, nat.ptr(digits), nat.ptr(ext), B, 0, s)
-        kernels["keyswitch_core_extended"] = lambda: lib.fhb_ckks_keyswitch_core_extended(
-            h, nat.ptr(ext), nat.ptr(rlk.data), nat.ptr(t[0]), nat.ptr(t[1]), B, 0, s)
     per_kernel = {}
     for name, fn in kernels.items():
         fn()
@@ -893,7 +888,7 @@ def main() -> int:
     ks_peak = mixed_peak(f64_rows / (L + cfg.num_p_primes))
     # kernels whose rows of primes below 2^42 run in FP64, and their FP64 share
     f64_share = {"inverse_ntt_d2": f64_rows / L, "keyswitch_core": f64_rows / (L + cfg.num_p_primes),
-                 "keyswitch_core_extended": f64_rows / (L + cfg.num_p_primes)}
+                 "moddown_rescale": f64_rows / L}
     modmul_achieved = ks_modmul / (per_kernel["keyswitch_core"] / 1000.0)
     step_bytes = B * (4 * L + 2 * (L - 1)) * limb + 10 * 2 * (L + cfg.num_p_primes) * limb
     # every step kernel against its roofs: algorithmic bytes (each operand row
@@ -921,8 +916,6 @@ def main() -> int:
         int8_ops["tc_basis_extend"] = nd_ * B * (n_ // 128) * sum(2 * 128 * ((c + 15) // 16 * 16) * 32
                                                                   for c in chunk_n)
         kroof["tc_basis_extend"] = (rows(L) + rows(ext_rows), 0)
-        kroof["keyswitch_core_extended"] = (rows(ext_rows) + rows(2 * (L + P_)) + 2 * dnum_ * (L + P_) * limb,
-                                            ks_modmul - B * qp_ * L * n_)
     int8_peak, int8_src = _int8_peak_tops()
     kernel_roofline = {}
     for name, (nbytes, nmul) in kroof.items():
@@ -937,26 +930,13 @@ def main() -> int:
             entry.update({"int8_ops": int8_ops[name], "int8_tops": int8_ops[name] / sec / 1e12,
                           "int8_frac": int8_ops[name] / sec / 1e12 / int8_peak, "int8_peak_source": int8_src})
         kernel_roofline[name] = entry
-    # DRAM bytes of one k_keyswitch_core launch: 15.7 GB measured by ncu
-    # (dram__bytes_read.sum + dram__bytes_write.sum) on the batch-32 launch of
-    # this command, work order 2 (groups of four ciphertexts share the key
-    # rows); every destination row re-reads the digit rows of its group, so
-    # the traffic grows with the batch and is scaled by the units processed.
-    traffic = KS_TRAFFIC_BYTES_BATCH32 * B / 32 if cfg.logN == 16 and L == 35 else None
-    # the dominant kernel of the headline form
-    dom = "keyswitch_core_extended" if ext is not None else "keyswitch_core"
-    dom_kernel = {"keyswitch_core": ("k_keyswitch_core_split<false> (FP64 rows for the primes below 2^42 with the "
-                                     "extension computed in FP64, int64 rows for the base prime and P)"
-                                     if f64_core else "k_keyswitch_core"),
-                  "keyswitch_core_extended": ("k_keyswitch_core_split<PRE> (FP64 rows for the primes below 2^42, "
-                                              "int64 rows for the base prime and P)"
-                                              if f64_core else "k_keyswitch_core<PRE>")}[dom]
-    if dom == "keyswitch_core_extended":
-        ext_traffic = KS_F64_TRAFFIC_BYTES_BATCH32 if f64_core else KS_EXT_TRAFFIC_BYTES_BATCH32
-        traffic = ext_traffic * B / 32 if ext_traffic and cfg.logN == 16 and L == 35 else None
-    elif f64_core:
-        traffic = (KS_SPLIT_TRAFFIC_BYTES_BATCH32 * B / 32
-                   if KS_SPLIT_TRAFFIC_BYTES_BATCH32 and cfg.logN == 16 and L == 35 else None)
+    # DRAM bytes of the key-switch core's launches (the intermediate crosses
+    # device memory between them), scaled by the ciphertexts processed
+    traffic = KS_TRAFFIC_BYTES_BATCH4 * B / 4 if cfg.logN == 16 and L == 35 and form == "cuda_cores" else None
+    dom = "keyswitch_core"
+    dom_kernel = ("k_ks_columns + k_ks_rows + k_ks_columns_inverse "
+                  + ("(FP64 rows for the primes below 2^42, int64 rows for the base prime and P)" if f64_core
+                     else "(int64 rows)"))
     dom_bytes, dom_modmul = kroof[dom]
     achieved = dom_bytes / (per_kernel[dom] / 1000.0) / 1e9
     modmul_achieved = dom_modmul / (per_kernel[dom] / 1000.0)

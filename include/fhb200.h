@@ -415,12 +415,12 @@ int fhb_ckks_keyswitch_sum_work(const fhb_context* ctx, const void* digits, cons
  * its own Galois element with its own key (kind 1).  fhb_ckks_items_plan_info
  * (host only) validates the items and returns the plan and scratch sizes;
  * fhb_ckks_items_plan writes the device plan (item descriptors with their
- * scratch regions resolved, and the work lists of the cluster stages) into
+ * scratch regions resolved, and the work lists of the transform stages) into
  * `plan` with a blocking copy, binding it to `scratch`; fhb_ckks_items_run
- * then issues six launches over all items - forward NTT of the HMult
- * operands, tensor product, inverse NTT of d2, ModUp digits, key-switch
- * core, ModDown with the rescale or with sigma_g(c0) - with no host call, so
- * it can be captured in a CUDA graph and replayed (the plan, scratch, inputs
+ * then issues ten launches over all items - forward NTT of the HMult
+ * operands (two), tensor product, inverse NTT of d2 (two), ModUp digits,
+ * key-switch core (three), ModDown with the rescale or with sigma_g(c0) -
+ * with no host call, so it can be captured in a CUDA graph and replayed (the plan, scratch, inputs
  * and outputs must stay allocated).  Results are integer-equal to the
  * per-level calls (fhb_ckks_multiply_relinearize with rescale after a
  * forward NTT of the operands, fhb_ckks_rotate).  Replaces the reference's
