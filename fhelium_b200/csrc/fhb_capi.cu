@@ -273,9 +273,8 @@ template <typename T>
 int bsgs_inner(const Context& c, const void* rot, int64_t rot_stride, const void* pts, int64_t pt_stride,
                int entries, const int* table, int giants, int babies, void* out, int64_t out_stride, int64_t polys,
                int rows, int row_start, cudaStream_t st) {
-  const size_t staged = bsgs_staged_bytes<T>(entries, giants, babies);
-  // staged whenever two blocks fit an SM: the plaintexts are most of the bytes
-  if (entries > 0 && staged <= 100 * 1024) {
+  if (bsgs_staged<T>(entries, giants, babies, polys)) {
+    const size_t staged = bsgs_staged_bytes<T>(entries, giants, babies);
     const int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(k_bsgs_inner_staged<T>), int(staged));
     if (rc != 0) return rc;
     const int64_t blocks = (int64_t(rows) << c.log_n) / 32;

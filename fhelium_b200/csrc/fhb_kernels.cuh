@@ -1012,18 +1012,58 @@ __global__ void k_rns_binary(const T* __restrict__ a, const T* __restrict__ b, T
 //   out[k] = sum_b rot[b] (.) pts[table[k][b]]      (NTT/Montgomery, lazy)
 // rot: [babies][polys][rows][N] baby rotations; pts: [entries][rows][N]
 // diagonal plaintexts shared by every poly; table: [giants][babies] entry
-// index or -1.  A thread multiplies a baby residue into the accumulators of
-// kBsgsAcc giants, held in registers.  Replaces the per-diagonal
-// plaintext product + add of the reference's BSGS evaluation
-// (fhelium/experimental/bootstrap/_linear.py:235-393).
+// index or -1.  Replaces the per-diagonal plaintext product + add of the
+// reference's BSGS evaluation
+// (fhelium/experimental/bootstrap/_linear.py:235-393).  Two forms, chosen by
+// bsgs_staged.
 //
-// The products of one giant with up to kBsgsChunk babies are added double
-// width and reduced once: 16 products of words below 2q stay below 2^126
-// (60-bit primes; 2^62 for 28-bit ones) and below 4 q 2^W, so the reduction
-// by 2^W leaves less than 5q, brought below 2q; x 4 makes it a Montgomery
-// product (R = 2^(W - 2)).  A reduction per product bound the kernel:
-// 5.2 -> 1.8 ms a launch in the full-slot bootstrap of two ciphertexts of
-// N = 2^16.
+// k_bsgs_inner, one thread per residue: a baby residue is read once and
+// multiplied into the accumulators of 16 giants, one Montgomery reduction per
+// product; missing entries cost nothing, and every polynomial reads the
+// plaintexts itself.
+template <typename T>
+__global__ void k_bsgs_inner(const T* __restrict__ rot, int64_t rot_stride, const T* __restrict__ pts,
+                             int64_t pt_stride, const int* __restrict__ table, int giants, int babies,
+                             T* __restrict__ out, int64_t out_stride, int64_t polys, int rows, int row_start,
+                             int log_n, ChainTables<T> tabs) {
+  constexpr int kAcc = 16;
+  const int64_t n = int64_t(1) << log_n;
+  const int64_t per = int64_t(rows) * n;
+  const int64_t total = polys * per;
+  for (int64_t idx = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; idx < total;
+       idx += int64_t(gridDim.x) * blockDim.x) {
+    const int64_t in_poly = idx % per;  // row * N + coefficient
+    const int row = int(in_poly >> log_n);
+    const PrimeInfo<T> p = tabs.prime[row_start + row];
+    for (int g0 = 0; g0 < giants; g0 += kAcc) {
+      T acc[kAcc];
+#pragma unroll
+      for (int j = 0; j < kAcc; ++j) acc[j] = 0;
+      for (int b = 0; b < babies; ++b) {
+        const T x = rot[b * rot_stride + idx];
+#pragma unroll
+        for (int j = 0; j < kAcc; ++j) {
+          if (g0 + j >= giants) break;
+          const int e = table[(g0 + j) * babies + b];
+          if (e >= 0)
+            acc[j] = csub(acc[j] + Word<T>::mont(x, pts[e * pt_stride + in_poly], p.q, p.neg_inv), p.twice_q);
+        }
+      }
+#pragma unroll
+      for (int j = 0; j < kAcc; ++j)
+        if (g0 + j < giants) out[(g0 + j) * out_stride + idx] = acc[j];
+    }
+  }
+}
+
+// k_bsgs_inner_staged, plaintext slices in shared memory, so that each
+// plaintext residue leaves HBM once however many polynomials share it.  The
+// products of one giant with up to kBsgsChunk babies are added double width
+// and reduced once: 16 products of words below 2q stay below 2^126 (60-bit
+// primes; 2^62 for 28-bit ones) and below 4 q 2^W, so the reduction by 2^W
+// leaves less than 5q, brought below 2q; x 4 makes it a Montgomery product
+// (R = 2^(W - 2)).  A reduction per product bound the kernel: 5.2 -> 1.8 ms a
+// launch in the full-slot bootstrap of two ciphertexts of N = 2^16.
 constexpr int kBsgsChunk = 16;
 constexpr int kBsgsAcc = 8;  // giants per thread and pass
 
@@ -1074,32 +1114,7 @@ __device__ __forceinline__ void bsgs_giants(const T* __restrict__ rot, int64_t r
     if (j < live) out[j * out_stride] = acc[j];
 }
 
-template <typename T>
-__global__ void k_bsgs_inner(const T* __restrict__ rot, int64_t rot_stride, const T* __restrict__ pts,
-                             int64_t pt_stride, const int* __restrict__ table, int giants, int babies,
-                             T* __restrict__ out, int64_t out_stride, int64_t polys, int rows, int row_start,
-                             int log_n, ChainTables<T> tabs) {
-  const int64_t n = int64_t(1) << log_n;
-  const int64_t per = int64_t(rows) * n;
-  const int64_t total = polys * per;
-  for (int64_t idx = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; idx < total;
-       idx += int64_t(gridDim.x) * blockDim.x) {
-    const int64_t in_poly = idx % per;  // row * N + coefficient
-    const PrimeInfo<T> p = tabs.prime[row_start + int(in_poly >> log_n)];
-    for (int g0 = 0; g0 < giants; g0 += kBsgsAcc) {
-      const int live = min(kBsgsAcc, giants - g0);
-      auto word = [&](int b, int j) {
-        const int e = j < live ? table[(g0 + j) * babies + b] : -1;
-        return e >= 0 ? pts[e * pt_stride + in_poly] : T(0);
-      };
-      bsgs_giants<T>(rot + idx, rot_stride, live, babies, p, word, out + g0 * out_stride + idx, out_stride);
-    }
-  }
-}
-
-// Same inner products with the plaintext rows staged in shared memory, so
-// that each plaintext residue leaves HBM once however many polynomials share
-// it.  One block per (row, 32 consecutive coefficients): the block stages the
+// One block per (row, 32 consecutive coefficients): the block stages the
 // 32-coefficient slice of every plaintext entry, a slice of zeros, and the
 // table as offsets [group of giants][baby][giant of the group] (missing
 // entries name the zeros); then its warps take (polynomial, group) pairs in
@@ -1108,6 +1123,29 @@ template <typename T>
 size_t bsgs_staged_bytes(int entries, int giants, int babies) {
   const size_t groups = size_t(giants + kBsgsAcc - 1) / kBsgsAcc;
   return size_t(entries + 1) * 32 * sizeof(T) + groups * kBsgsAcc * babies * sizeof(int);
+}
+
+// Whether a call takes the staged form: by the work of both on one tile of 32
+// coefficients, in products of the direct form.  Direct: one per (polynomial,
+// entry).  Staged: half a product to stage an entry, 64 for the block; then
+// its eight warps take the (polynomial, group of eight giants) pairs in
+// rounds, every baby's eight products together cost one (missing entries
+// included) and two for the round's latency; 1.5 to reduce and store an
+// output.  Measured, direct / staged (us): 3 rows of N = 2^16, 50-bit primes,
+// 4 polynomials, 16 babies x 16 giants, all entries 939/273, half of them
+// 521/248; 16 x 1 68/164; 1 polynomial, 16 x 4 84/138, 16 x 16 312/208; 18
+// polynomials, 2 x 1 51/172, 32 x 8 3790/1007; 32-bit words, 12 rows of N =
+// 2^16, 8 polynomials, 16 x 16, half of the entries 2402/883.  Over 982 shapes
+// (1 to 18 polynomials, 1 to 32 babies and giants, both words) the choice is
+// on average 2 % from the faster form (worst: 3 x 16 of 32-bit words, 1.3).
+// Above 100 KB one block fits an SM and needs work for all of its eight warps
+// (16 x 32, 4 polynomials 1868/835; 1 polynomial, 6 rows 943/1190).
+template <typename T>
+bool bsgs_staged(int entries, int giants, int babies, int64_t polys) {
+  const int64_t groups = (int64_t(giants) + kBsgsAcc - 1) / kBsgsAcc, rounds = (polys * groups + 7) / 8;
+  const size_t bytes = bsgs_staged_bytes<T>(entries, giants, babies);
+  if (entries < 1 || bytes > (polys * groups < 8 ? 100 : 200) * 1024) return false;
+  return 2 * polys * entries > entries + 4 * rounds * babies + 2 * polys * groups * babies + 128 + 3 * polys * giants;
 }
 
 template <typename T>

@@ -65,3 +65,33 @@ class _RingView:
 
     def __getattr__(self, name):
         return getattr(self._cfg, name)
+
+
+def captured_kernels(call) -> list[tuple[str, tuple[int, int, int]]]:
+    """(mangled name, grid) of every kernel that `call` launches on the current
+    torch stream, in launch order, read from a stream capture of it (nothing
+    runs).  Call it once before, so that no kernel attribute is first set here."""
+    from cuda.bindings import driver
+
+    def ok(result):
+        assert result[0] == driver.CUresult.CUDA_SUCCESS, result[0]
+        return result[1]
+
+    graph = torch.cuda.CUDAGraph(keep_graph=True)
+    torch.cuda.synchronize()
+    with torch.cuda.graph(graph, stream=torch.cuda.Stream()):
+        call()
+    raw = driver.CUgraph(graph.raw_cuda_graph())
+    status, _, count = driver.cuGraphGetNodes(raw, 0)
+    assert status == driver.CUresult.CUDA_SUCCESS
+    status, nodes, count = driver.cuGraphGetNodes(raw, count)
+    assert status == driver.CUresult.CUDA_SUCCESS
+    out = []
+    for node in nodes[:count]:
+        if ok(driver.cuGraphNodeGetType(node)) != driver.CUgraphNodeType.CU_GRAPH_NODE_TYPE_KERNEL:
+            continue
+        params = ok(driver.cuGraphKernelNodeGetParams(node))
+        name = ok(driver.cuFuncGetName(params.func)) if int(params.func) else ok(driver.cuKernelGetName(params.kern))
+        out.append((name.decode() if isinstance(name, bytes) else str(name),
+                    (params.gridDimX, params.gridDimY, params.gridDimZ)))
+    return out

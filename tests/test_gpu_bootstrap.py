@@ -66,7 +66,7 @@ def test_bootstrap_reference_preset_reference_input():
     assert -math.log2(float(err.max())) > 8
 
 
-@pytest.mark.parametrize("batch", [1, 2, 9])  # direct kernel below 8 polynomials, staged from 8
+@pytest.mark.parametrize("batch", [1, 2, 9])
 def test_bsgs_inner_product_matches_plaintext_products(batch):
     """fhb_ckks_bsgs_inner_product against the per-diagonal plaintext product
     and addition it replaces (equal modulo q)."""
@@ -96,6 +96,74 @@ def test_bsgs_inner_product_matches_plaintext_products(batch):
             want = term if want is None else eng.add(want, term)
         qd = q.cuda()
         assert torch.equal(out[k] % qd, want.data % qd)
+
+
+# (scale bits, word bits, polynomials, babies, giants, entries, staged): a
+# second chunk of babies (17, 33), a partial second group of giants (9), more
+# slices than two blocks of an SM hold, more than one block holds (forces the
+# direct form), no rounds for some warps, and either form of small calls
+BSGS_SHAPES = [
+    (50, 62, 1, 1, 1, 1, False), (50, 62, 18, 1, 1, 1, False), (50, 62, 1, 17, 9, 150, False),
+    (50, 62, 4, 17, 9, 153, True), (50, 62, 9, 33, 9, 290, True), (50, 62, 4, 32, 16, 512, True),
+    (50, 62, 4, 32, 32, 1000, False), (50, 62, 1, 16, 32, 500, False), (50, 62, 3, 16, 8, 40, False),
+    (25, 30, 2, 17, 9, 153, True), (25, 30, 9, 16, 8, 128, True), (25, 30, 4, 33, 17, 30, False),
+    (25, 30, 8, 32, 33, 1056, True),
+]
+
+
+@pytest.mark.parametrize("bits,word,polys,babies,giants,entries,staged", BSGS_SHAPES)
+@pytest.mark.parametrize("top", [False, True])
+def test_bsgs_inner_product_forms(bits, word, polys, babies, giants, entries, staged, top):
+    """Both forms against exact sums of Montgomery products, whole numbers
+    modulo q; `top`: every operand 2q - 1, on a chain with a 60-bit row (int64),
+    the largest sums of double-width products.  And the form a call takes:
+    the staged one only where many products share a slice (its block
+    stages every entry and multiplies every missing one)."""
+    import numpy as np
+    from fhelium_b200 import _native as nat
+    from tests.helpers import captured_kernels
+    preset = Preset.slots8192_scale50_levels5_int64 if word == 62 else Preset.slots8192_scale25_levels14_int32
+    eng = CkksEngine(preset, rng_seed=9)
+    row_start, limbs = (eng.num_q - 1, 1) if top else (0, 2)
+    q = torch.tensor([eng.moduli[row_start + i] for i in range(limbs)], dtype=torch.int64, device="cuda").view(limbs, 1)
+    if top and word == 62:
+        assert int(q.max()) > 1 << 55
+    g = torch.Generator(device="cuda").manual_seed(polys * 1000 + entries)
+
+    def words(*prefix):
+        if top:
+            return (2 * q - 1).expand(*prefix, limbs, eng.n).to(eng.dtype).contiguous()
+        return (torch.randint(0, 1 << 62, (*prefix, limbs, eng.n), generator=g, device="cuda") % (2 * q)).to(eng.dtype)
+
+    rot, pts = words(babies, polys), words(entries)
+    table = torch.full((giants * babies,), -1, dtype=torch.int32, device="cuda")
+    at = torch.randperm(giants * babies, generator=g, device="cuda")[:entries]
+    table[at] = torch.arange(at.numel(), dtype=torch.int32, device="cuda")
+    out = torch.full((giants, polys, limbs, eng.n), -1, dtype=eng.dtype, device="cuda")
+
+    def call():
+        eng.ctx.call("fhb_ckks_bsgs_inner_product", nat.ptr(rot), rot[0].numel(), nat.ptr(pts), pts[0].numel(),
+                     entries, nat.ptr(table), giants, babies, nat.ptr(out), out[0].numel(), polys, limbs, row_start,
+                     eng._stream())
+
+    call()
+    names = [name for name, _ in captured_kernels(call)]
+    assert len(names) == 1 and ("staged" in names[0]) == staged, names
+    cols = [0, 1, 31, 32, eng.n // 2 + 5, eng.n - 1]
+    got = out[..., cols].cpu().numpy().astype(object)
+    x, y = rot[..., cols].cpu().numpy().astype(object), pts[..., cols].cpu().numpy().astype(object)
+    t = table.cpu().numpy().reshape(giants, babies)
+    for j in range(limbs):
+        p = int(eng.moduli[row_start + j])
+        rinv = pow(1 << word, -1, p)
+        for k in range(giants):
+            want = sum((x[b, :, j] * y[t[k, b], j] for b in range(babies) if t[k, b] >= 0),
+                       np.zeros((polys, len(cols)), dtype=object))
+            lazy = got[k, :, j]
+            assert (lazy >= 0).all() and (lazy < 2 * p).all()
+            assert ((lazy - want * rinv) % p == 0).all(), (k, j)
+    whole = out.long()
+    assert bool(((whole >= 0) & (whole < 2 * q)).all())
 
 
 def test_rotate_and_sum_close_to_separate_rotations():
