@@ -802,11 +802,28 @@ static int check_scratch(const fhb_context* ctx, int64_t batch, int level, int64
   return 0;
 }
 
-// Whether the caller's buffer has room for the key-switch core's column and
-// block launches; without it (exactly fhb_ckks_keyswitch_scratch_bytes) the
-// one-launch cluster core runs.
-static bool ks_passes(const Context& c, const fhb::Scratch& s, int level) {
-  return c.basis_tc || s.y_words >= fhb::ks_pass_min_words(c, level);
+// Whether the key-switch core runs as column and block launches, in the groups
+// of rows (and of ciphertexts) that the caller's room holds, or as the
+// one-launch cluster core (always with exactly fhb_ckks_keyswitch_scratch_bytes).
+// A group is three launches, so unless one group takes everything, groups must
+// be large enough to pay for theirs: on average 2^14 transforms of 256 words
+// (a row of a ciphertext has N / 256 for each digit and two for the sums).
+// Whole relinearisations over 225 shapes (rings 2^14 to 2^16, both words, 1 to
+// 40 ciphertexts, 1 to 15 digits) and 1671 rooms, launches / cluster core: one
+// group 0.24 to 1.01; several at or above the line 0.44 to 1.04; below it 0.33
+// to 20 (N = 2^14, 9 rows of 8 digits, 5 ciphertexts, cluster core 250 us: one
+// ciphertext's row a group 991, one row 248, three rows 170, all rows 130; 3
+// rows of 2 digits, 40 ciphertexts, 204 against 4028).
+static bool ks_passes(const Context& c, const fhb::Scratch& s, int64_t batch, int level) {
+  const int64_t per_row = fhb::ks_pass_min_words(c, level), room = s.y_words / per_row;
+  if (c.basis_tc || batch == 0) return true;  // extensions of their own, or nothing to do
+  if (room < 1) return false;
+  const int64_t rows = c.num_q - level + c.num_p;
+  const int64_t cts = std::min(batch, room), row_step = std::min(rows, room / cts);
+  const int64_t groups = (batch + cts - 1) / cts * ((rows + row_step - 1) / row_step);
+  if (groups == 1) return true;
+  const int64_t per_ct = rows * (int64_t(c.level_digits[level].size()) + 2) * (c.n() >> 8);
+  return per_ct * batch >= groups << 14;
 }
 
 // Key-switch core on the ModUp digits in s.digits: with the tensor-core
@@ -818,7 +835,7 @@ static int ks_core_from_digits(const Context& c, const fhb::Scratch& s, const vo
     TRY(fhb::tc_extend(const_cast<Context&>(c), s.digits, s.ext, batch, level, ct3 != nullptr, st));
     return fhb::ks_pass(c, s.digits, s.ext, 0, key, s.t0, s.t1, batch, level, st, item_keys, ct3, true);
   }
-  if (ks_passes(c, s, level))
+  if (ks_passes(c, s, batch, level))
     return fhb::ks_pass(c, s.digits, s.y, s.y_words, key, s.t0, s.t1, batch, level, st, item_keys, ct3, false);
   return fhb::ks_core(c, s.digits, key, s.t0, s.t1, batch, level, st, item_keys, ct3);
 }
@@ -997,7 +1014,7 @@ int fhb_ckks_multiply_relinearize(const fhb_context* ctx, const void* a, const v
   const int64_t out_bytes = 2 * batch * (limbs - (rescale ? 1 : 0)) * c.n() * fhb::word_bytes(c);
   const bool alias = ranges_overlap(out, out_bytes, a, in_bytes) || ranges_overlap(out, out_bytes, b, in_bytes);
   const fhb::Scratch s = fhb::carve(c, scratch, batch, level, scratch_bytes);
-  if (k > 1 && cap == cudaStreamCaptureStatusNone && !ks_passes(c, s, level) && !alias)
+  if (k > 1 && cap == cudaStreamCaptureStatusNone && !ks_passes(c, s, batch, level) && !alias)
     return multiply_relinearize_chunked(ctx, static_cast<const char*>(a), static_cast<const char*>(b), key,
                                         static_cast<char*>(out), static_cast<char*>(scratch), batch, level, rescale,
                                         st, k);
@@ -1206,7 +1223,7 @@ int fhb_ckks_rotate(const fhb_context* ctx, const void* ct, const void* key, voi
   TRY(fhb::cuda_status(cudaStreamIsCapturing(st, &cap), "capture status"));
   const int64_t ct_bytes = 2 * batch * limbs * c.n() * fhb::word_bytes(c);
   const fhb::Scratch s = fhb::carve(c, scratch, batch, level, scratch_bytes);
-  if (k > 1 && cap == cudaStreamCaptureStatusNone && !ks_passes(c, s, level) &&
+  if (k > 1 && cap == cudaStreamCaptureStatusNone && !ks_passes(c, s, batch, level) &&
       !ranges_overlap(out, ct_bytes, ct, ct_bytes))
     return rotate_chunked(ctx, static_cast<const char*>(ct), key, static_cast<char*>(out),
                           static_cast<char*>(scratch), batch, level, galois, st, k);

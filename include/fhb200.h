@@ -332,7 +332,8 @@ int64_t fhb_ckks_keyswitch_scratch_bytes(const fhb_context* ctx, int64_t batch, 
  * plus room (at most 1 GiB) for the intermediate of the key-switch core's
  * transforms, which then run as column and block launches on every SM.  With
  * less (down to fhb_ckks_keyswitch_scratch_bytes) the calls give the same
- * results through smaller groups of rows or the one-launch cluster core.
+ * results, through groups of rows where the surplus holds groups that are
+ * worth their launches, otherwise through the one-launch cluster core.
  * -1 for an invalid batch or level. */
 int64_t fhb_ckks_keyswitch_workspace_bytes(const fhb_context* ctx, int64_t batch, int level);
 

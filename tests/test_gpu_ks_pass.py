@@ -1,9 +1,8 @@
 """The key-switch core as column and block launches (fhb_pass.cuh), against the
 oracle, at every ring degree (each has its own split of the stages), with
-every amount of scratch the calls accept: exactly the required size (the
-one-launch cluster core), room for one ciphertext's digits of one row (groups
-of one ciphertext and one row), room for a few rows (an uneven last group)
-and the recommended size.  Whole numbers, no tolerance."""
+every amount of scratch the calls accept: exactly the required size and small
+surpluses (the one-launch cluster core), room for groups of rows and of
+ciphertexts, and the recommended size.  Whole numbers, no tolerance."""
 
 import numpy as np
 import pytest
@@ -13,7 +12,7 @@ from fhelium_b200 import _native as nat
 from fhelium_b200.config import CkksConfig, Preset
 from fhelium_b200.engine import CkksEngine
 from fhelium_b200.values import Ciphertext, RelinearizationKey, RotationKey
-from tests.helpers import oracle_for, random_key, reduced_ring, to_dev, to_np, uniform_residues
+from tests.helpers import captured_kernels, oracle_for, random_key, reduced_ring, to_dev, to_np, uniform_residues
 
 pytestmark = pytest.mark.gpu
 
@@ -126,6 +125,96 @@ def test_rotations_with_their_own_keys_every_room(preset, log_n, level, batch):
         eng.ctx.call("fhb_ckks_rotate_multi", nat.ptr(d_ct), nat.ptr(ptrs), nat.ptr(galois), nat.ptr(out),
                      nat.ptr(scratch), room, batch, level, eng._stream())
         np.testing.assert_array_equal(to_np(out), want, err_msg=f"scratch {room}")
+
+
+def _relinearize(eng, cfg, ct3, key, room, batch, level):
+    """(result, names of the launched kernels) with `room` bytes of scratch."""
+    out = torch.full((2, *ct3.shape[1:]), -1, dtype=cfg.torch_dtype, device="cuda")
+    scratch = torch.empty(room, dtype=torch.uint8, device="cuda")
+
+    def call():
+        eng.ctx.call("fhb_ckks_relinearize", nat.ptr(ct3), nat.ptr(key), nat.ptr(out), nat.ptr(scratch), room, batch,
+                     level, 0, eng._stream())
+
+    call()
+    names = [name for name, _ in captured_kernels(call)]
+    torch.cuda.synchronize()
+    return out, names
+
+
+def _groups(names):
+    """Launch groups of the key-switch core, 0 for the cluster core."""
+    rows = sum("k_ks_rows" in n for n in names)
+    assert (rows > 0) != any("k_keyswitch_core" in n for n in names), names
+    return rows
+
+
+# (preset, level, batch, room in rows of one ciphertext, groups): groups of
+# rows (an uneven last one; FP64, wide FP64, integer and int32 rows), of
+# ciphertexts (one row at a time, a smaller last one), one group; and rooms
+# whose groups would be too small to pay for their launches
+GROUPS = [
+    ("slots8192_scale40_levels7_int64", 0, 18, 4 * 18, 3),
+    ("slots16384_scale50_levels12_int64", 0, 6, 9 * 6 + 5, 2),
+    ("slots32768_scale40_levels34_int64", 20, 5, 8 * 5, 3),
+    ("slots32768_scale25_levels24_int32", 10, 6, 7 * 6, 3),
+    ("slots32768_scale40_levels34_int64", 33, 33, 17, 12),
+    ("slots32768_scale25_levels24_int32", 22, 40, 25, 14),
+    ("slots8192_scale40_levels7_int64", 0, 1, 9, 1),
+    ("slots8192_scale40_levels7_int64", 0, 1, 8, 0),
+    ("slots8192_scale40_levels7_int64", 0, 5, 1, 0),
+    ("slots8192_scale40_levels7_int64", 6, 18, 2 * 18, 0),
+    ("slots32768_scale25_levels24_int32", 6, 1, 3, 0),
+]
+
+
+@pytest.mark.parametrize("preset,level,batch,room,groups", GROUPS)
+def test_groups_that_the_room_holds(preset, level, batch, room, groups):
+    """The launches run in as many groups as the surplus asks for when each is
+    worth its launches, the cluster core otherwise, with one result."""
+    cfg = CkksConfig.parse(Preset[preset])
+    eng = CkksEngine(cfg, basis_conversion="cuda_cores")
+    rng = np.random.default_rng(batch)
+    rows = range(level, eng.num_q)
+    ct3 = to_dev(uniform_residues(rng, cfg.moduli, rows, (3, batch), cfg.N, lazy=True), cfg)
+    key = to_dev(random_key(rng, cfg, cfg.N), cfg)
+    need = int(eng.ctx.lib.fhb_ckks_keyswitch_scratch_bytes(eng.ctx.handle, batch, level))
+    row = len(eng.level_digits[level]) * cfg.N * ct3.element_size()
+    want, names = _relinearize(eng, cfg, ct3, key, need, batch, level)
+    assert _groups(names) == 0
+    got, names = _relinearize(eng, cfg, ct3, key, need + room * row, batch, level)
+    assert _groups(names) == groups
+    assert torch.equal(got, want)
+
+
+@pytest.mark.parametrize("preset", ["slots8192_scale40_levels7_int64", "slots8192_scale25_levels14_int32",
+                                    "slots16384_scale40_levels16_int64", "slots32768_scale25_levels24_int32"])
+def test_noalloc_takes_few_launches(preset):
+    """fhb_ckks_relinearize_noalloc's fixed scratch leaves every batch another
+    surplus: the core is one launch, or groups of at least 2^14 transforms of
+    256 words (a row of a ciphertext has N / 256 for each digit and sum)."""
+    cfg = CkksConfig.parse(Preset[preset])
+    eng = CkksEngine(cfg, basis_conversion="cuda_cores")
+    lib, st = eng.ctx.lib, eng._stream
+    most = int(lib.fhb_ckks_relinearize_noalloc_max_scratch_bytes())
+    key = torch.zeros((eng.key_digit_count, 2, eng.num_q + eng.num_p, cfg.N), dtype=cfg.torch_dtype, device="cuda")
+    seen = set()
+    for level in range(eng.num_q):
+        per_ct = int(lib.fhb_ckks_keyswitch_scratch_bytes(eng.ctx.handle, 1, level))
+        work = (eng.num_q - level + eng.num_p) * (len(eng.level_digits[level]) + 2) * cfg.N // 256
+        for batch in range(1, most // per_ct + 1):
+            ct3 = torch.zeros((3, batch, eng.num_q - level, cfg.N), dtype=cfg.torch_dtype, device="cuda")
+            out = torch.empty_like(ct3[:2])
+
+            def call():
+                eng.ctx.call("fhb_ckks_relinearize_noalloc", nat.ptr(ct3), nat.ptr(key), nat.ptr(out), batch, level, 0,
+                             st())
+
+            call()
+            groups = _groups([name for name, _ in captured_kernels(call)])
+            assert groups <= 1 or work * batch >= groups << 14, (level, batch, groups)
+            seen.add(min(groups, 1))
+    assert seen == {0, 1}
 
 
 def test_workspace_holds_the_required_scratch():
