@@ -249,13 +249,21 @@ MdArgs<T> moddown_args(const Context& c, int level, int rescale) {
                    md_tables<T>(c)};
 }
 
-// Groups of rows per coefficient tile: enough for about eight blocks per SM
-// (below that a single ciphertext leaves SMs idle; each group repeats the
-// digits, about a quarter of a row's work per digit), at most one per row;
-// and few enough rows in each for the staged constants.
-inline int moddown_groups(int64_t tiles, int q_limbs) {
-  const int64_t g = (148 * 8 + tiles - 1) / tiles, least = (q_limbs + kMdRows - 2) / (kMdRows - 1);
-  return int(std::max<int64_t>(least, std::min<int64_t>(g, q_limbs)));
+// Groups of rows per coefficient tile, so that a few ciphertexts fill the GPU:
+// as many as give two blocks per SM, which hide one another's loads.  More cost
+// more than they give, since each group forms the digits (and v_0) again: about
+// num_p / 2 rows' work, so a group has at least 1 + num_p / 2 rows.  Measured
+// without rescale, by groups (us): N = 2^16, 35 + 4 rows, 1 ciphertext (256
+// tiles) 1: 49.5, 2: 52.7, 4: 58.4; N = 2^14, 8 + 1 rows, 1 ciphertext (64
+// tiles) 1: 6.4, 2: 4.7, 4: 4.2, 8: 5.2; 16 ciphertexts of 2 + 1 rows (1024
+// tiles) 1: 11.6, 2: 14.2 (one group for all rows and both components, before
+// the sums of products: 10.5).  Over 292 calls the choice is within 0.2 % of
+// the best on average, 14 % at most.  And few enough rows in each for the
+// staged constants.
+inline int moddown_groups(int64_t tiles, int q_limbs, int num_p) {
+  const int64_t fill = 2 * 148 / tiles, most = q_limbs / (1 + num_p / 2);
+  const int64_t least = (q_limbs + kMdRows - 2) / (kMdRows - 1);
+  return int(std::max({least, int64_t(1), std::min(fill, most)}));
 }
 
 // t0/t1: [B, QP_l, N] canonical coefficient rows; add0/add1 (nullable):
@@ -263,7 +271,7 @@ inline int moddown_groups(int64_t tiles, int q_limbs) {
 // c0); out: [2, B, Q_l (- 1), N] canonical, components out_pitch words apart.
 // Blocks (coefficients, component, ciphertext, group of rows), groups
 // fastest: they share the P rows in L2.  Every group forms the digits (and
-// v_0) itself; there are as many groups as it takes to fill the GPU.
+// v_0) itself.
 template <typename T, int NP, bool SPLIT>
 __global__ void __launch_bounds__(kMdThreads, 2)
 k_moddown(const __grid_constant__ MdArgs<T> a, const T* __restrict__ t0, const T* __restrict__ t1,

@@ -271,6 +271,60 @@ def test_key_switch_sum_equals_the_cluster_kernel(preset, log_n, level, batch, g
                      nat.ptr(work), rooms[0] - 16, giants, batch, level, eng._stream())
 
 
+# blocks of ModDown: the coefficient tiles (N / 512, two components, the batch)
+# times the groups of rows
+@pytest.mark.parametrize("preset,log_n,level,batch,groups", [
+    ("slots8192_scale40_levels7_int64", 14, 6, 16, 1),
+    ("slots8192_scale40_levels7_int64", 14, 0, 1, 4),
+    ("slots8192_scale40_levels7_int64", 12, 7, 1, 1),
+    ("slots32768_scale40_levels34_int64", 16, 0, 1, 1),
+    ("slots32768_scale40_levels34_int64", 12, 0, 1, 11),
+    ("slots16384_scale25_levels29_int32", 12, 0, 3, 6),
+    ("slots65536_scale40_levels72_int64", 12, 0, 1, 18),
+])
+@pytest.mark.parametrize("rescale", [0, 1])
+def test_moddown_groups(preset, log_n, level, batch, groups, rescale):
+    """Groups for two blocks per SM, none below 1 + P / 2 rows (each forms the
+    digits again), every split with the oracle's residues."""
+    cfg, eng, orc = _engine(preset, log_n)
+    limbs = eng.num_q - level
+    if rescale and limbs == 1:
+        pytest.skip("no rescale at the last level")
+    rng = np.random.default_rng(limbs)
+    ids = list(range(level, eng.num_q + eng.num_p))
+    t = uniform_residues(rng, cfg.moduli, ids, (2, batch), cfg.N)
+    add = uniform_residues(rng, cfg.moduli, ids[:limbs], (2, batch), cfg.N)
+    t_d, add_d = to_dev(t, cfg), to_dev(add, cfg)
+    out = torch.full((2, batch, limbs - rescale, cfg.N), -1, dtype=cfg.torch_dtype, device="cuda")
+
+    def call():
+        eng.ctx.call("fhb_ckks_moddown", nat.ptr(t_d[0]), nat.ptr(t_d[1]), nat.ptr(add_d[0]), nat.ptr(add_d[1]),
+                     nat.ptr(out), batch, level, 1, rescale, eng._stream())
+
+    call()
+    (name, grid), = captured_kernels(call)
+    assert "k_moddown" in name and grid[0] == cfg.N // 512 * 2 * batch * groups
+    assert groups == 1 or grid[0] <= 2 * 148
+    q = np.array([cfg.moduli[i] for i in ids[:limbs]], dtype=object).reshape(-1, 1)
+    cols = [0, 1, 255, 256, cfg.N // 2 + 7, cfg.N - 1]
+    p_all = 1
+    for r in range(eng.num_p):
+        p_all *= int(cfg.moduli[eng.num_q + r])
+    got = to_np(out)[..., cols]
+    for c in range(2):
+        for b in range(batch):
+            x = t[c, b][:, cols].astype(object)
+            tail = sum(x[limbs + r] * (p_all // p) * pow(p_all // p, -1, p)
+                       for r, p in enumerate(int(cfg.moduli[eng.num_q + r]) for r in range(eng.num_p))) % p_all
+            v = np.stack([((x[i] - tail) * pow(p_all, -1, int(q[i, 0])) + add[c, b][i, cols].astype(object))
+                          % int(q[i, 0]) for i in range(limbs)])
+            if rescale:
+                half = (v[0] > int(q[0, 0]) // 2).astype(object)
+                v = np.stack([((v[i] - v[0]) * pow(int(q[0, 0]), -1, int(q[i, 0])) + half) % int(q[i, 0])
+                              for i in range(1, limbs)])
+            assert (got[c, b] == v).all(), (c, b)
+
+
 def test_empty_batches_are_accepted():
     cfg, eng, _ = _engine("slots8192_scale40_levels7_int64", 14)
     x = torch.zeros(4096, dtype=torch.int64, device="cuda")
