@@ -18,13 +18,15 @@ inline int f64_rows(const Context& c, int row_start, int rows) {
 }
 
 // FP64 form of the chain's leading Q rows, how many of them, and its tables.
+// FHB_TUNE_F64_CORE is the narrow rows' switch: it reads 0 on chains without
+// them, and a caller that puts back what it read must change nothing there.
 struct F64Form {
   int form, end;
   const ChainTables<double>* tabs;
 };
 inline F64Form f64_form(const Context& c) {
   if (c.f64_core && c.f64_tables_ok) return {kNarrowF64, c.f64_prime_end, &c.t64f};
-  if (c.f64_core && c.wide_tables_ok) return {kWideF64, c.wide_prime_end, &c.t64w};
+  if (c.wide_tables_ok) return {kWideF64, c.wide_prime_end, &c.t64w};
   return {kNoF64, 0, &c.t64f};
 }
 

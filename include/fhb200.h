@@ -102,10 +102,13 @@ int fhb_context_root(const fhb_context* ctx, int prime_id, uint64_t* psi);
  * 8192-word span (1), or in three (0, default: faster on B200).
  * FHB_TUNE_F64_CORE (int64 chains): 1 = the rows of primes below 2^42 run in
  * exact FP64 arithmetic (integers held in doubles, balanced residues,
- * products on the FP64 pipe; default) in the forward / inverse NTTs and, for
- * N <= 2^16, in the key-switch core (both basis-conversion forms), the
- * hoisted-rotation kernels and the mixed-level items stages; 0 = on the
- * integer pipe.  Reads back 0 where the chain has no such primes.
+ * products on the FP64 pipe; default) in the forward / inverse NTTs, the
+ * key-switch core (both basis-conversion forms; its cluster form for N <= 2^16),
+ * the hoisted-rotation kernels, ModDown, the rescale and the mixed-level items
+ * stages; 0 = on the integer pipe.  Reads back 0, and changes nothing, where
+ * the chain has no such primes.  (The rows of primes below 1.1 2^50 of those
+ * chains run in FP64 arithmetic in the core's launches, the application of
+ * hoisted rotations and the inverse NTT to standard words, whatever its value.)
  * FHB_TUNE_OVERLAP_CHUNKS (1..8, default 4): fhb_ckks_multiply_relinearize
  * and fhb_ckks_rotate cut a batch of at least 16 ciphertexts into at most
  * this many chunks and run one chunk's element-wise stages (tensor product,

@@ -252,7 +252,7 @@ def test_f64_core_matches_integer_core(family, log_n, level, batch, form):
 
 
 def test_f64_core_unavailable_for_wide_primes():
-    """50-bit Q primes: no FP64 tables, the switch reads back 0, results unchanged."""
+    """50-bit Q primes: no rows of primes below 2^42, their switch reads back 0; one result in both forms."""
     eng = CkksEngine(Preset.slots8192_scale50_levels5_int64)
     eng.basis_conversion = "tensor_cores"
     assert eng.ctx.get_tuning(nat.TUNE_F64_CORE) == 0
@@ -262,3 +262,22 @@ def test_f64_core_unavailable_for_wide_primes():
     got = eng.multiply_relinearize_rescale(a, b)
     eng.basis_conversion = "cuda_cores"
     assert torch.equal(got.data, eng.multiply_relinearize_rescale(a, b).data)
+
+
+def test_f64_core_switch_leaves_wide_primes_alone():
+    """The switch belongs to the rows of primes below 2^42: on a 50-bit chain,
+    where it reads 0, putting back what was read (or setting either value)
+    keeps the core's FP64 rows (form 2 of k_ks_rows)."""
+    from tests.helpers import captured_kernels
+    eng = CkksEngine(Preset.slots8192_scale50_levels5_int64, basis_conversion="cuda_cores")
+    rng = np.random.default_rng(5)
+    a = eng.coefficient_domain_to_ntt_domain(eng.encrypt_message(rng.uniform(-0.05, 0.05, eng.num_slots)))
+    want = eng.multiply_relinearize_rescale(a, a).data
+    before = eng.ctx.get_tuning(nat.TUNE_F64_CORE)
+    assert before == 0
+    for value in (before, 1, 0):
+        eng.ctx.set_tuning(nat.TUNE_F64_CORE, value)
+        assert eng.ctx.get_tuning(nat.TUNE_F64_CORE) == 0
+        assert torch.equal(eng.multiply_relinearize_rescale(a, a).data, want)
+        names = [n for n, _ in captured_kernels(lambda: eng.multiply_relinearize_rescale(a, a)) if "k_ks_rows" in n]
+        assert names and all("k_ks_rowsImLi14ELi2E" in n for n in names), (value, names)
