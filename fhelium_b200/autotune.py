@@ -40,6 +40,12 @@ import torch
 
 _LOCK = threading.Lock()
 
+# Part of every key: counted up when a saved value comes to mean something else
+# or the kernels it was timed with are others (2: 8 residues per thread names
+# the column and block launches; items hold the core's intermediate in their
+# scratch), so that an older file's entries are searched again.
+_REVISION = 2
+
 
 def default_cache_path() -> str:
     env = os.environ.get("FHB200_AUTOTUNE_CACHE")
@@ -74,7 +80,7 @@ def workload_key(engine, executor) -> str:
     digest = hashlib.sha256(json.dumps(shape).encode()).hexdigest()[:16]
     chain = hashlib.sha256(json.dumps([int(m) for m in engine.moduli]).encode()).hexdigest()[:12]
     dev = torch.cuda.get_device_name(engine.device)
-    return f"{dev}|logN={engine.log_n}|q={engine.num_q}|p={engine.num_p}|chain={chain}|mixed={digest}"
+    return f"{dev}|r{_REVISION}|logN={engine.log_n}|q={engine.num_q}|p={engine.num_p}|chain={chain}|mixed={digest}"
 
 
 def time_replays(run, device, *, warmup: int = 1, repeats: int = 3) -> float:
@@ -98,7 +104,8 @@ def time_replays(run, device, *, warmup: int = 1, repeats: int = 3) -> float:
 
 def tune_ntt(ctx, x: torch.Tensor, rows: int, row_start: int = 0, *, candidates: Iterable[int] = (8, 16),
              repeats: int = 5, cache_path: str | None = None, use_cache: bool = True) -> dict:
-    """Pick residues per thread of the forward and of the inverse NTT for
+    """Pick the form of the forward and of the inverse NTT (8: column and block
+    launches; 16: one cluster per polynomial, 16 residues per thread) for
     polynomials shaped like `x` ([..., rows, N] residues of prime ids
     [row_start, row_start + rows) on ctx's device) and leave `ctx` set to the
     winners.  Returns ``{"forward_ept", "inverse_ept", "forward_ms", ...}``."""
@@ -108,7 +115,8 @@ def tune_ntt(ctx, x: torch.Tensor, rows: int, row_start: int = 0, *, candidates:
     batch = x.numel() // (rows * n)
     dev = x.device
     bits = 32 if x.element_size() == 4 else 64
-    key = f"{torch.cuda.get_device_name(dev)}|ntt|bits={bits}|N={n}|rows={rows}|row_start={row_start}|batch={batch}"
+    key = (f"{torch.cuda.get_device_name(dev)}|r{_REVISION}|ntt|bits={bits}|N={n}|rows={rows}|row_start={row_start}"
+           f"|batch={batch}")
     if use_cache:
         hit = _load(cache_path).get(key)
         if hit and {"forward_ept", "inverse_ept"} <= set(hit):
@@ -168,7 +176,7 @@ def items_workload_key(engine, ciphertexts, ops) -> str:
     digest = hashlib.sha256(json.dumps(shape).encode()).hexdigest()[:16]
     chain = hashlib.sha256(json.dumps([int(m) for m in engine.moduli]).encode()).hexdigest()[:12]
     dev = torch.cuda.get_device_name(engine.device)
-    return f"{dev}|logN={engine.log_n}|q={engine.num_q}|p={engine.num_p}|chain={chain}|items={digest}"
+    return f"{dev}|r{_REVISION}|logN={engine.log_n}|q={engine.num_q}|p={engine.num_p}|chain={chain}|items={digest}"
 
 
 def tune_items(engine, ciphertexts, ops, *, ks_orders: Iterable[int] = (0, 2),
