@@ -185,11 +185,26 @@ class MixedBatchExecutor:
             loads[s] += g.cost(eng.num_p)
         while len(self._streams) < self.streams:
             self._streams.append(torch.cuda.Stream(eng.device))
-        need = [0] * self.streams
-        for g in self.groups:
-            nb = int(eng.ctx.lib.fhb_ckks_keyswitch_workspace_bytes(eng.ctx.handle, g.items, g.level))
-            need[g.stream] = max(need[g.stream], nb)
-        self._scratch = [torch.empty(max(nb, 16), dtype=torch.uint8, device=eng.device) for nb in need]
+        lib, handle = eng.ctx.lib, eng.ctx.handle
+
+        def per_stream(size) -> list[int]:
+            need = [16] * self.streams
+            for g in self.groups:
+                need[g.stream] = max(need[g.stream], int(size(handle, g.items, g.level)))
+            return need
+
+        def allocate(sizes: list[int]) -> list[torch.Tensor]:
+            return [torch.empty(nb, dtype=torch.uint8, device=eng.device) for nb in sizes]
+
+        # what the calls run fastest with (up to 1 GiB more per stream), or what
+        # they need where the device has no room for that
+        self._scratch = []
+        try:
+            self._scratch = allocate(per_stream(lib.fhb_ckks_keyswitch_workspace_bytes))
+        except torch.cuda.OutOfMemoryError:
+            pass
+        if not self._scratch:  # past the handler, which would keep the first streams' buffers alive
+            self._scratch = allocate(per_stream(lib.fhb_ckks_keyswitch_scratch_bytes))
 
     # ---------------------------------------------------------------- run
     def _issue_group(self, g: _Group, stream: torch.cuda.Stream, scratch: torch.Tensor) -> None:

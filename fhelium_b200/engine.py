@@ -83,6 +83,7 @@ class CkksEngine:
         self._relinearization_key: RelinearizationKey | None = None
         self._rotation_keys = RotationKeySet()
         self._scratch: torch.Tensor | None = None
+        self._scratch_refused = math.inf  # scratch bytes that the device could not give
         self.level_digits = self._digit_layout()
         self.basis_conversion = basis_conversion
 
@@ -152,10 +153,26 @@ class CkksEngine:
         return torch.empty(shape, dtype=self.dtype, device=self.device)
 
     def _scratch_for(self, batch: int, level: int) -> tuple[torch.Tensor, int]:
-        nbytes = int(self.ctx.lib.fhb_ckks_keyswitch_workspace_bytes(self.ctx.handle, batch, level))
-        if self._scratch is None or self._scratch.numel() < nbytes:
-            self._scratch = torch.empty(nbytes, dtype=torch.uint8, device=self.device)
-        return self._scratch, nbytes
+        """Scratch of a key-switch call and its bytes, kept for later calls: as
+        much as the call runs fastest with (up to 1 GiB above what it needs),
+        or, where the device has no room for that, what it needs.  The larger
+        size is asked for again when the scratch has to be made anew."""
+        lib, handle = self.ctx.lib, self.ctx.handle
+        nbytes = int(lib.fhb_ckks_keyswitch_workspace_bytes(handle, batch, level))
+        held = -1 if self._scratch is None else self._scratch.numel()
+        if held >= nbytes:
+            return self._scratch, nbytes
+        need = int(lib.fhb_ckks_keyswitch_scratch_bytes(handle, batch, level))
+        if held < need or nbytes < self._scratch_refused:
+            try:
+                self._scratch = torch.empty(nbytes, dtype=torch.uint8, device=self.device)
+                return self._scratch, nbytes
+            except torch.cuda.OutOfMemoryError:
+                self._scratch_refused = nbytes
+        if held < need:
+            self._scratch = None
+            self._scratch = torch.empty(need, dtype=torch.uint8, device=self.device)
+        return self._scratch, self._scratch.numel()
 
     def _check_ct(self, ct: Ciphertext) -> None:
         if ct.data.device != self.device or ct.data.dtype != self.dtype:
@@ -547,10 +564,16 @@ class CkksEngine:
             self.ctx.call("fhb_ckks_modup_digits", nat.ptr(ct.c1), nat.ptr(digits[i]), b, level, key.galois_element, st)
         key_ptrs = torch.tensor([k.data.data_ptr() for k in keys], dtype=torch.int64, device=self.device)
         t = self._empty(2, b, limbs + self.num_p, self.n)
-        # (a batch beyond the work buffer's launches takes the cluster kernel)
+        # a batch beyond the work buffer's launches, or without memory for the
+        # buffer, takes the cluster kernel
+        work = None
         if len(cts) * b <= 4096:
             nbytes = int(self.ctx.lib.fhb_ckks_keyswitch_sum_workspace_bytes(self.ctx.handle, len(cts), b, level))
-            work = torch.empty(nbytes, dtype=torch.uint8, device=self.device)
+            try:
+                work = torch.empty(nbytes, dtype=torch.uint8, device=self.device)
+            except torch.cuda.OutOfMemoryError:
+                pass
+        if work is not None:
             self.ctx.call("fhb_ckks_keyswitch_sum_work", nat.ptr(digits), nat.ptr(key_ptrs), nat.ptr(t[0]),
                           nat.ptr(t[1]), nat.ptr(work), nbytes, len(cts), b, level, st)
         else:

@@ -4,6 +4,8 @@ every amount of scratch the calls accept: exactly the required size and small
 surpluses (the one-launch cluster core), room for groups of rows and of
 ciphertexts, and the recommended size.  Whole numbers, no tolerance."""
 
+import weakref
+
 import numpy as np
 import pytest
 import torch
@@ -229,6 +231,85 @@ def test_workspace_holds_the_required_scratch():
             assert need <= full <= need + (1 << 30)
     assert int(lib.fhb_ckks_keyswitch_workspace_bytes(eng.ctx.handle, -1, 0)) == -1
     assert int(lib.fhb_ckks_keyswitch_workspace_bytes(eng.ctx.handle, 1, eng.num_q)) == -1
+
+
+@pytest.fixture
+def refuse(monkeypatch):
+    """refuse(sizes): torch.empty has no memory for byte buffers of these sizes;
+    returns the list that collects what it was asked for: (bytes, weak
+    reference to the buffer or None)."""
+    empty = torch.empty
+
+    def start(sizes):
+        asked = []
+
+        def fake(*shape, **kwargs):
+            if kwargs.get("dtype") is not torch.uint8:
+                return empty(*shape, **kwargs)
+            if shape[0] in sizes:
+                asked.append((shape[0], None))
+                raise torch.cuda.OutOfMemoryError("refused")
+            out = empty(*shape, **kwargs)
+            asked.append((shape[0], weakref.ref(out)))
+            return out
+
+        monkeypatch.setattr(torch, "empty", fake)
+        return asked
+
+    return start
+
+
+def test_calls_run_where_only_the_required_scratch_fits(refuse):
+    """Without memory for the recommended scratch the same calls run with the
+    required one, with one result; the larger size is not asked for on every
+    call, and again when the scratch is made anew."""
+    from fhelium_b200.batch import ROTATE, MixedBatchExecutor, MixedOp
+    cfg = CkksConfig.parse(Preset.slots8192_scale40_levels7_int64)
+    eng = CkksEngine(cfg, rng_seed=2)
+    rng = np.random.default_rng(8)
+    batch, rows = 16, range(eng.num_q)
+    key = RelinearizationKey(to_dev(random_key(rng, cfg, cfg.N), cfg))
+    rk = RotationKey(to_dev(random_key(rng, cfg, cfg.N), cfg), 3, eng.galois_element_for_step(3))
+    eng.set_rotation_key(rk)
+    ct3 = Ciphertext(to_dev(uniform_residues(rng, cfg.moduli, rows, (3, batch), cfg.N), cfg), 0, 1.0, "ntt",
+                     "montgomery")
+    ct = Ciphertext(to_dev(uniform_residues(rng, cfg.moduli, rows, (2, batch), cfg.N), cfg), 0, 1.0)
+    singles = [Ciphertext(ct.data[:, i:i + 1].contiguous(), 0, 1.0) for i in range(batch // 2)]
+    singles += [Ciphertext(c.data[..., 1:, :].contiguous(), 1, 1.0) for c in singles[1:]]
+    ops = [MixedOp(ROTATE, i, step=3) for i in range(len(singles))]
+    lib, handle = eng.ctx.lib, eng.ctx.handle
+
+    def sizes(b, level):
+        return (int(lib.fhb_ckks_keyswitch_workspace_bytes(handle, b, level)),
+                int(lib.fhb_ckks_keyswitch_scratch_bytes(handle, b, level)))
+
+    def mixed():  # two groups on two streams, at levels 0 and 1
+        ex = MixedBatchExecutor(eng, singles, ops, streams=2, use_graph=False)
+        ex.run()
+        return [r.data for r in ex.results()], [s.numel() for s in ex._scratch]
+
+    full, need = sizes(batch, 0)
+    groups = [sizes(8, 0), sizes(7, 1)]
+    work = int(lib.fhb_ckks_keyswitch_sum_workspace_bytes(handle, 2, batch, 0))
+    assert full > need and len({full, need, work, *groups[0], *groups[1]}) == 7
+    want = eng.relinearize(ct3, key).data
+    want_sum = eng.rotate_and_sum([ct, ct], [rk, rk]).data
+    want_mixed, held = mixed()
+    assert eng._scratch.numel() == full and held == [g[0] for g in groups]
+    eng._scratch = None
+    asked = refuse({full, work, groups[1][0]})
+    for _ in range(2):
+        assert torch.equal(eng.relinearize(ct3, key).data, want)
+    assert [a[0] for a in asked] == [full, need] and eng._scratch.numel() == need
+    assert torch.equal(eng.rotate_and_sum([ct, ct], [rk, rk]).data, want_sum)
+    assert [a[0] for a in asked[2:]] == [work]
+    got, held = mixed()
+    assert all(torch.equal(x, y) for x, y in zip(got, want_mixed)) and held == [g[1] for g in groups]
+    assert [a[0] for a in asked[3:]] == [groups[0][0], groups[1][0], groups[0][1], groups[1][1]]
+    assert asked[3][1]() is None  # the first stream's larger buffer is given back
+    refuse(set())
+    eng._scratch = None
+    assert torch.equal(eng.relinearize(ct3, key).data, want) and eng._scratch.numel() == full
 
 
 @pytest.mark.parametrize("form", ["cuda_cores", "tensor_cores"])
