@@ -788,7 +788,8 @@ int64_t fhb_ckks_keyswitch_workspace_bytes(const fhb_context* ctx, int64_t batch
   const int64_t row = fhb::ks_pass_min_words(c, level) * fhb::word_bytes(c);
   const int64_t rows = c.num_q - level + c.num_p;
   const int64_t all = batch > INT64_MAX / (row * rows) ? INT64_MAX : row * rows * batch;
-  return need + std::min(all, std::max(row, fhb::kKsPassRoom));
+  const int64_t room = std::min(all, std::max(row, fhb::kKsPassRoom));
+  return need > INT64_MAX - room ? need : need + room;
 }
 
 // Scratch check shared by the entry points that take a caller scratch buffer:
@@ -1043,9 +1044,9 @@ int64_t fhb_ckks_keyswitch_sum_workspace_bytes(const fhb_context* ctx, int giant
   const Context& c = *ctx->impl;
   if (batch > INT64_MAX / giants) return -1;
   const int64_t cts = batch * giants, word = fhb::word_bytes(c);
-  if (c.basis_tc) return fhb::tc_ext_words(c, cts, level) * word;
   const int64_t one = fhb::ks_pass_min_words(c, level) * word, rows = c.num_q - level + c.num_p;
   if (cts > INT64_MAX / (one * rows)) return -1;
+  if (c.basis_tc) return fhb::tc_ext_words(c, cts, level) * word;
   return std::min(one * rows * cts, std::max(one * cts, fhb::kKsPassRoom));
 }
 
@@ -1061,6 +1062,8 @@ int fhb_ckks_keyswitch_sum_work(const fhb_context* ctx, const void* digits, cons
   if (!key_ptrs) return fail(-2, "key_ptrs is NULL");
   if (giants < 1 || batch < 0) return fail(-2, "need giants >= 1 and batch >= 0");
   if (batch == 0) return 0;
+  if (fhb_ckks_keyswitch_sum_workspace_bytes(ctx, giants, batch, level) < 0)
+    return fail(-4, "the work size of this batch overflows 64 bits");
   const int64_t cts = batch * giants, words = work_bytes / fhb::word_bytes(c);
   if (words < (c.basis_tc ? fhb::tc_ext_words(c, cts, level) : fhb::ks_pass_min_words(c, level) * cts))
     return fail(-8, "work buffer too small");

@@ -352,6 +352,25 @@ def test_key_switch_sum_equals_the_cluster_kernel(preset, log_n, level, batch, g
                      nat.ptr(work), rooms[0] - 16, giants, batch, level, eng._stream())
 
 
+def test_sums_whose_sizes_overflow_are_refused():
+    """batch x giants ciphertexts beyond 64 bits: an error, before any
+    arithmetic on their product."""
+    _, eng, _ = _engine("slots8192_scale40_levels7_int64", 12)
+    x = torch.zeros(4096, dtype=torch.int64, device="cuda")
+    p = nat.ptr(x)
+    for form in ("tensor_cores", "cuda_cores"):
+        eng.basis_conversion = form
+        for giants, batch in ((4, 1 << 62), (2, 1 << 62), (1, 1 << 62), (1, 1 << 50), (7, (1 << 61) + 3)):
+            assert int(eng.ctx.lib.fhb_ckks_keyswitch_sum_workspace_bytes(eng.ctx.handle, giants, batch, 0)) == -1
+            with pytest.raises(nat.NativeCallError, match="overflows"):
+                eng.ctx.call("fhb_ckks_keyswitch_sum_work", p, p, p, p, p, 1 << 40, giants, batch, 0, eng._stream())
+    largest = int(eng.ctx.lib.fhb_ckks_keyswitch_scratch_bytes(eng.ctx.handle, 1, 0))
+    largest = ((1 << 63) - 1) // largest
+    need, full = (int(size(eng.ctx.handle, largest, 0)) for size in (
+        eng.ctx.lib.fhb_ckks_keyswitch_scratch_bytes, eng.ctx.lib.fhb_ckks_keyswitch_workspace_bytes))
+    assert 0 < need <= full
+
+
 # blocks of ModDown: the coefficient tiles (N / 512, two components, the batch)
 # times the groups of rows
 @pytest.mark.parametrize("preset,log_n,level,batch,groups", [
