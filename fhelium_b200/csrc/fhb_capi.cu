@@ -178,7 +178,7 @@ int moddown(const Context& c, const void* t0, const void* t1, const void* a0, co
     if (c.basis_tc && c.tc_moddown)  // P -> Q conversion on the int8 tensor cores
       return tc_moddown(const_cast<Context&>(c), t0, t1, a0, a1, out, batch, level, ginv, item_galois, rescale, st);
   }
-  if (batch == 0) return 0;
+  if (batch <= 0) return 0;
   if (out_pitch <= 0) out_pitch = batch * (c.num_q - level - (rescale ? 1 : 0)) * c.n();
   const MdArgs<T> args = moddown_args<T>(c, level, rescale);
   const int64_t tiles = (int64_t(c.n()) >> 9) * 2 * batch;

@@ -441,3 +441,18 @@ def test_empty_batches_are_accepted():
     eng.ctx.call("fhb_inverse_ntt", nat.ptr(x), nat.ptr(x), 0, 1, 0, 2, st)
     torch.cuda.synchronize()
     assert not x.any()
+
+
+@pytest.mark.parametrize("preset", ["slots8192_scale40_levels7_int64", "slots8192_scale25_levels14_int32"])
+def test_negative_batches_do_nothing(preset):
+    """The element-wise stages take a negative batch as an empty one."""
+    cfg, eng, _ = _engine(preset, 14)
+    x = torch.zeros(4096, dtype=cfg.torch_dtype, device="cuda")
+    p, st = nat.ptr(x), eng._stream()
+    for batch in (-1, -7):
+        for rescale in (0, 1):
+            eng.ctx.call("fhb_ckks_moddown", p, p, p, p, p, batch, 0, 5, rescale, st)
+        eng.ctx.call("fhb_ckks_rescale", p, p, batch, 0, 1, st)
+        eng.ctx.call("fhb_ckks_apply_prepared_rotation", p, p, p, p, batch, 0, 5, st)
+    torch.cuda.synchronize()
+    assert not x.any()
