@@ -73,6 +73,7 @@ SIGNATURES: dict[str, tuple] = {
     "fhb_rns_lift_signed": (_I, [_P, _P, _P, _I64, _I, _I, _P]),
     "fhb_ckks_keyswitch_scratch_bytes": (_I64, [_P, _I64, _I]),
     "fhb_ckks_keyswitch_workspace_bytes": (_I64, [_P, _I64, _I]),
+    "fhb_ckks_keyswitch_core_launches": (_I64, [_P, _I64, _I, _I64]),
     "fhb_ckks_relinearize": (_I, [_P, _P, _P, _P, _P, _I64, _I64, _I, _I, _P]),
     "fhb_ckks_multiply_relinearize": (_I, [_P, _P, _P, _P, _P, _P, _I64, _I64, _I, _I, _P]),
     "fhb_ckks_rotate": (_I, [_P, _P, _P, _P, _P, _I64, _I64, _I, _U32, _P]),

@@ -263,10 +263,21 @@ class MixedBatchExecutor:
             self.capture()
         self._graph.replay()
 
+    def _core_launches(self, g: _Group) -> int:
+        eng = self.engine
+        return int(eng.ctx.lib.fhb_ckks_keyswitch_core_launches(eng.ctx.handle, g.items, g.level,
+                                                               self._scratch[g.stream].numel()))
+
     @property
     def launches_per_run(self) -> int:
-        """Library kernels one run launches (excluding the input gathers)."""
-        return sum(5 if g.kind == HMULT else 3 for g in self.groups)
+        """Library kernels one captured run launches (excluding the input
+        gathers): per group the key-switch core in as many as its scratch
+        gives, ModUp (HMult with one P prime has none) and ModDown, and for
+        HMult the forward NTT, the product and the inverse NTT of d2."""
+        ctx = self.engine.ctx
+        ntts = sum(1 if ctx.get_tuning(p) == 16 else 2 for p in (nat.TUNE_NTT_FORWARD_EPT, nat.TUNE_NTT_INVERSE_EPT))
+        hmult = ntts + 2 + (self.engine.num_p != 1)
+        return sum(self._core_launches(g) + (hmult if g.kind == HMULT else 2) for g in self.groups)
 
     # ---------------------------------------------------------------- results
     def result_view(self, op_index: int) -> torch.Tensor:

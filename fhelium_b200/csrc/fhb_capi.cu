@@ -803,9 +803,9 @@ static int check_scratch(const fhb_context* ctx, int64_t batch, int level, int64
   return 0;
 }
 
-// Whether the key-switch core runs as column and block launches, in the groups
-// of rows (and of ciphertexts) that the caller's room holds, or as the
-// one-launch cluster core (always with exactly fhb_ckks_keyswitch_scratch_bytes).
+// The groups of rows (and of ciphertexts) of the key-switch core's column and
+// block launches in the caller's room, or 0 for the one-launch cluster core
+// (always with exactly fhb_ckks_keyswitch_scratch_bytes).
 // A group is three launches, so unless one group takes everything, groups must
 // be large enough to pay for theirs: on average 2^14 transforms of 256 words
 // (a row of a ciphertext has N / 256 for each digit and two for the sums).
@@ -815,16 +815,25 @@ static int check_scratch(const fhb_context* ctx, int64_t batch, int level, int64
 // to 20 (N = 2^14, 9 rows of 8 digits, 5 ciphertexts, cluster core 250 us: one
 // ciphertext's row a group 991, one row 248, three rows 170, all rows 130; 3
 // rows of 2 digits, 40 ciphertexts, 204 against 4028).
-static bool ks_passes(const Context& c, const fhb::Scratch& s, int64_t batch, int level) {
+static int64_t ks_pass_groups(const Context& c, const fhb::Scratch& s, int64_t batch, int level) {
   const int64_t per_row = fhb::ks_pass_min_words(c, level), room = s.y_words / per_row;
-  if (c.basis_tc || batch == 0) return true;  // extensions of their own, or nothing to do
-  if (room < 1) return false;
+  // extensions of their own, or nothing to do
+  if (c.basis_tc || batch == 0) return std::max<int64_t>(1, (batch + fhb::kMaxPassGroup - 1) / fhb::kMaxPassGroup);
+  if (room < 1) return 0;
   const int64_t rows = c.num_q - level + c.num_p;
-  const int64_t cts = std::min(batch, room), row_step = std::min(rows, room / cts);
-  const int64_t groups = (batch + cts - 1) / cts * ((rows + row_step - 1) / row_step);
-  if (groups == 1) return true;
+  const int64_t cts = std::min(std::min(batch, fhb::kMaxPassGroup), room), last = (batch - 1) % cts + 1;
+  auto row_groups = [&](int64_t n) {
+    const int64_t step = std::min(rows, room / n);
+    return (rows + step - 1) / step;
+  };
+  const int64_t groups = (batch - last) / cts * row_groups(cts) + row_groups(last);
+  if (groups == 1) return 1;
   const int64_t per_ct = rows * (int64_t(c.level_digits[level].size()) + 2) * (c.n() >> 8);
-  return per_ct * batch >= groups << 14;
+  return per_ct * batch >= groups << 14 ? groups : 0;
+}
+
+static bool ks_passes(const Context& c, const fhb::Scratch& s, int64_t batch, int level) {
+  return ks_pass_groups(c, s, batch, level) > 0;
 }
 
 // Key-switch core on the ModUp digits in s.digits: with the tensor-core
@@ -861,6 +870,15 @@ static int relinearize_tail(const Context& c, const fhb::Scratch& s, const void*
   if (c.num_p != 1) TRY(FHB_WORD(fhb::modup, c, s.t0, s.digits, batch, level, 1u, st));
   TRY(ks_core_from_digits(c, s, key, batch, level, st, nullptr, ct3));
   return FHB_WORD(fhb::moddown, c, s.t0, s.t1, nullptr, nullptr, out, batch, level, 1u, rescale, st);
+}
+
+int64_t fhb_ckks_keyswitch_core_launches(const fhb_context* ctx, int64_t batch, int level, int64_t scratch_bytes) {
+  const int64_t need = fhb_ckks_keyswitch_scratch_bytes(ctx, batch, level);
+  if (need < 0 || scratch_bytes < need) return -1;
+  const Context& c = *ctx->impl;
+  const int64_t groups = ks_pass_groups(c, fhb::carve(c, nullptr, batch, level, scratch_bytes), batch, level);
+  if (batch == 0) return 0;
+  return (c.basis_tc ? 1 : 0) + (groups > 0 ? 3 * groups : 1);
 }
 
 int fhb_ckks_relinearize(const fhb_context* ctx, const void* ct3, const void* key, void* out, void* scratch,

@@ -19,6 +19,7 @@ constexpr int kMdDoubles = 3 + 2 * kMaxDigitWidth;
 // Room for the key-switch core's intermediate that fhb_ckks_keyswitch_workspace_bytes
 // asks for at most (rows are processed in groups that fit it).
 constexpr int64_t kKsPassRoom = int64_t{1} << 30;
+constexpr int64_t kMaxPassGroup = 4096;  // ciphertexts per launch of it (grid limit)
 constexpr uint64_t kWidePrimeEnd = (uint64_t{1} << 50) / 10 * 11;  // 1.1 2^50
 constexpr int kMaxOverlapChunks = 8;  // chunks of the overlapped fused HMult
 

@@ -215,8 +215,6 @@ int run_ks_core(const Context& c, const void* digits, const void* key, void* acc
   return launch_int(k_keyswitch_core<T, LOGN>);
 }
 
-constexpr int64_t kMaxPassGroup = 4096;  // ciphertexts per launch (grid limit)
-
 // What the pass kernels of one level share; all rows in flight.
 template <typename T>
 KsPass<T> ks_pass_args(const Context& c, int level) {

@@ -340,6 +340,12 @@ int64_t fhb_ckks_keyswitch_scratch_bytes(const fhb_context* ctx, int64_t batch, 
  * -1 for an invalid batch or level. */
 int64_t fhb_ckks_keyswitch_workspace_bytes(const fhb_context* ctx, int64_t batch, int level);
 
+/* Kernels that the key-switch core of such a call launches with this much
+ * scratch: three per group of rows, or one (the cluster core); with the
+ * tensor-core basis conversion one more for the extension.  0 for an empty
+ * batch; -1 for invalid sizes. */
+int64_t fhb_ckks_keyswitch_core_launches(const fhb_context* ctx, int64_t batch, int level, int64_t scratch_bytes);
+
 /* HMult-result relinearisation (optionally fused with the rescale):
  * ct3 [3, batch, L, N] NTT/Montgomery -> out [2, batch, L (- 1), N]
  * coefficient/standard canonical.  Replaces CkksEngine.relinearize

@@ -278,6 +278,27 @@ def test_autotune_picks_and_caches(small, tmp_path):
         assert torch.equal(ex.result(i).data, w.data)
 
 
+@pytest.mark.parametrize("form", ["cuda_cores", "tensor_cores"])
+@pytest.mark.parametrize("preset", ["slots8192_scale40_levels7_int64", "slots16384_scale40_levels16_int64"])
+@pytest.mark.parametrize("scratch", ["recommended", "required"])
+def test_launches_per_run_is_what_a_run_launches(preset, form, scratch, monkeypatch):
+    """Against the kernels of a stream capture: one P prime and more, both
+    basis-conversion forms, the launches and (largest group of a stream) the
+    cluster core."""
+    from tests.helpers import captured_kernels
+    eng = CkksEngine(Preset[preset], rng_seed=3, basis_conversion=form)
+    if scratch == "required":
+        monkeypatch.setattr(eng.ctx.lib, "fhb_ckks_keyswitch_workspace_bytes",
+                            eng.ctx.lib.fhb_ckks_keyswitch_scratch_bytes)
+    cts, ops = _workload(eng, 24, seed=5, max_step=8)
+    ex = MixedBatchExecutor(eng, cts, ops, streams=2, use_graph=False)
+    ex.run()
+    names = [n for n, _ in captured_kernels(ex.run) if n.startswith("_ZN3fhb")]
+    assert ex.launches_per_run == len(names)
+    if scratch == "required" and form == "cuda_cores":
+        assert any("k_keyswitch_core" in n for n in names)
+
+
 def test_ntt_autotune_sets_and_caches(tmp_path):
     from fhelium_b200 import _native as nat
     eng = CkksEngine(Preset.slots8192_scale40_levels7_int64, rng_seed=2)
