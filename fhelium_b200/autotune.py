@@ -3,7 +3,8 @@
 The knobs a run can change without recompiling:
 
 * ``ks_order`` (FHB_TUNE_KS_ORDER): the work order of the key-switch
-  clusters, 0 = the limbs of one ciphertext back to back (the digits of one
+  clusters, which run where a call's scratch has no room for the column and
+  block launches (the engine's and the executors' has), 0 = the limbs of one ciphertext back to back (the digits of one
   ciphertext stay in L2 while its limbs are processed), 1 = one limb across
   the batch back to back (the key rows of one prime are shared by the whole
   batch, which pays when every item uses the same key), 2 = one limb across
@@ -145,7 +146,8 @@ def tune_ntt(ctx, x: torch.Tensor, rows: int, row_start: int = 0, *, candidates:
 
 def tune_mixed_batch(engine, executor, *, ks_orders: Iterable[int] = (0, 1, 2), streams: Iterable[int] = (1, 2, 3, 4),
                      repeats: int = 3, cache_path: str | None = None, use_cache: bool = True) -> dict:
-    """Pick (ks_order, streams) for `executor` by timing graph replays.
+    """Pick (ks_order, streams) for `executor` by timing graph replays; one
+    order only where no group's key-switch core follows it (usually).
 
     Leaves the executor configured with the winner and returns
     ``{"ks_order", "streams", "ms", "candidates": [...], "cached": bool}``.
@@ -158,7 +160,8 @@ def tune_mixed_batch(engine, executor, *, ks_orders: Iterable[int] = (0, 1, 2), 
             executor.configure(streams=int(hit["streams"]), ks_order=int(hit["ks_order"]))
             return dict(hit, cached=True)
     results = []
-    for order in ks_orders:
+    orders = list(ks_orders)
+    for order in orders if executor.follows_ks_order else orders[:1]:
         for s in streams:
             executor.configure(streams=s, ks_order=order)
             ms = time_replays(executor.run, engine.device, repeats=repeats)

@@ -279,6 +279,12 @@ class MixedBatchExecutor:
         hmult = ntts + 2 + (self.engine.num_p != 1)
         return sum(self._core_launches(g) + (hmult if g.kind == HMULT else 2) for g in self.groups)
 
+    @property
+    def follows_ks_order(self) -> bool:
+        """Whether any group's key-switch core is the cluster kernel, whose work
+        order ``ks_order`` sets (its scratch then has no room for launches)."""
+        return self.engine.basis_conversion == "cuda_cores" and any(self._core_launches(g) == 1 for g in self.groups)
+
     # ---------------------------------------------------------------- results
     def result_view(self, op_index: int) -> torch.Tensor:
         """[2, limbs, N] view of op `op_index`'s result inside its group arena."""

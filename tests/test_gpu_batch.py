@@ -266,8 +266,8 @@ def test_autotune_picks_and_caches(small, tmp_path):
     ex = MixedBatchExecutor(eng, cts, ops, streams=1)
     path = str(tmp_path / "tune.json")
     first = autotune.tune_mixed_batch(eng, ex, streams=(1, 2), repeats=1, cache_path=path)
-    # three key-switch work orders x two branch counts
-    assert not first["cached"] and len(first["candidates"]) == 6
+    # the launches follow no work order: one, x two branch counts
+    assert not first["cached"] and len(first["candidates"]) == 2 and not ex.follows_ks_order
     assert (ex.streams, ex.ks_order) == (first["streams"], first["ks_order"])
     with open(path) as f:
         assert autotune.workload_key(eng, ex) in json.load(f)
@@ -276,6 +276,26 @@ def test_autotune_picks_and_caches(small, tmp_path):
     ex.run()
     for i, w in enumerate(want):
         assert torch.equal(ex.result(i).data, w.data)
+
+
+def test_autotune_orders_of_the_cluster_core(small, tmp_path, monkeypatch):
+    """An executor with only the required scratch runs the cluster core, whose
+    work order is timed too: three orders x two branch counts, one result."""
+    eng, cts, ops, want = small
+    lib = eng.ctx.lib
+    required = lib.fhb_ckks_keyswitch_scratch_bytes
+    monkeypatch.setattr(lib, "fhb_ckks_keyswitch_workspace_bytes", required)
+    # one group, so that no larger group's scratch leaves it a surplus
+    level = next(c.level for c in cts)
+    some = [op for op in ops if cts[op.index].level == level and op.kind == ROTATE][:1] or [MixedOp(ROTATE, 0, step=3)]
+    ex = MixedBatchExecutor(eng, cts, some, streams=1)
+    assert ex.follows_ks_order
+    path = str(tmp_path / "tune.json")
+    first = autotune.tune_mixed_batch(eng, ex, streams=(1, 2), repeats=1, cache_path=path)
+    assert len(first["candidates"]) == 6
+    assert (ex.streams, ex.ks_order) == (first["streams"], first["ks_order"])
+    ex.run()
+    assert torch.equal(ex.result(0).data, run_per_ciphertext(eng, cts, some)[0].data)
 
 
 @pytest.mark.parametrize("form", ["cuda_cores", "tensor_cores"])
