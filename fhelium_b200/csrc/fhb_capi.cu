@@ -1022,9 +1022,8 @@ int fhb_ckks_multiply_relinearize(const fhb_context* ctx, const void* a, const v
   TRY(check_scratch(ctx, batch, level, scratch_bytes));
   if (rescale && level + 1 >= c.num_q) return fail(-4, "cannot rescale at the last level");
   const int limbs = c.num_q - level;
-  // a batch of at least two chunks of 8: chunks overlapped (not under stream
-  // capture, and not with ModDown on the tensor cores, which writes whole
-  // batches)
+  // a batch of at least two chunks of 8 on the cluster core: chunks overlapped
+  // (not under stream capture)
   const int k = int(std::min<int64_t>(c.overlap_chunks, batch / 8));
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
   TRY(fhb::cuda_status(cudaStreamIsCapturing(st, &cap), "capture status"));

@@ -109,13 +109,14 @@ int fhb_context_root(const fhb_context* ctx, int prime_id, uint64_t* psi);
  * the chain has no such primes.  (The rows of primes below 1.1 2^50 of those
  * chains run in FP64 arithmetic in the core's launches, the application of
  * hoisted rotations and the inverse NTT to standard words, whatever its value.)
- * FHB_TUNE_OVERLAP_CHUNKS (1..8, default 4): fhb_ckks_multiply_relinearize
- * and fhb_ckks_rotate cut a batch of at least 16 ciphertexts into at most
- * this many chunks and run one chunk's element-wise stages (tensor product,
- * ModUp digits, ModDown) on low-priority streams beside another chunk's
- * key-switch core, whose 8-CTA clusters leave SMs idle; 1 = one pass over
- * the batch.  The streams belong to the context and are forked from and
- * joined back into the caller's stream.  Under stream capture, or when the
+ * FHB_TUNE_OVERLAP_CHUNKS (1..8, default 4): where the key-switch core is the
+ * cluster kernel (CUDA-core form, scratch without room for its launches),
+ * fhb_ckks_multiply_relinearize and fhb_ckks_rotate cut a batch of at least 16
+ * ciphertexts into at most this many chunks and run one chunk's element-wise
+ * stages (tensor product, ModUp digits, ModDown) on low-priority streams
+ * beside another chunk's core, whose 8-CTA clusters leave SMs idle; 1 = one
+ * pass over the batch.  The streams belong to the context and are forked from
+ * and joined back into the caller's stream.  Under stream capture, or when the
  * output overlaps an input, the call runs in one pass.
  * Results do not depend on any of these (stall aside).  No counterpart in the reference
  * (its launch shapes and arithmetic units are fixed). */

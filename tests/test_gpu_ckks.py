@@ -16,7 +16,8 @@ from fhelium_b200.config import Preset
 from fhelium_b200.engine import CkksEngine
 from fhelium_b200.values import Ciphertext, RelinearizationKey, RotationKey
 from oracle import oracle as orc_mod
-from tests.helpers import CONFIGS, canon, oracle_for, random_key, reduced_ring, to_dev, to_np, uniform_residues
+from tests.helpers import (CONFIGS, canon, captured_kernels, oracle_for, random_key, reduced_ring, to_dev, to_np,
+                           uniform_residues)
 
 pytestmark = pytest.mark.gpu
 
@@ -68,19 +69,30 @@ def test_relinearize_matches_oracle(family, log_n, level):
 
 @pytest.mark.parametrize("family,log_n,level", CASES[:2])
 def test_keyswitch_work_orders_agree(family, log_n, level):
-    """Every key-switch work order (rows of one ciphertext, one row across the
-    batch, one row across groups of four) gives the same result; batch 6
-    leaves a partial group for order 2."""
+    """Every work order of the cluster core, which runs with exactly the
+    required scratch (rows of one ciphertext, one row across the batch, one row
+    across groups of four), gives the same result; batch 6 leaves a partial
+    group for order 2."""
     cfg, eng, orc, rng = _setup(family, log_n, level, 4)
+    eng.basis_conversion = "cuda_cores"
     rows = orc.q_rows(level)
     ct3 = uniform_residues(rng, cfg.moduli, rows, (3, 6), cfg.N, lazy=True)
     key = random_key(rng, cfg, cfg.N)
-    rlk = RelinearizationKey(to_dev(key, cfg))
+    d_ct3, d_key = to_dev(ct3, cfg), to_dev(key, cfg)
+    need = int(eng.ctx.lib.fhb_ckks_keyswitch_scratch_bytes(eng.ctx.handle, 6, level))
+    scratch = torch.empty(need, dtype=torch.uint8, device="cuda")
     outs = []
     for order in (0, 1, 2):
         eng.ctx.set_tuning(nat.TUNE_KS_ORDER, order)
-        got = eng.relinearize(Ciphertext(to_dev(ct3, cfg), level, 1.0, "ntt", "montgomery"), rlk)
-        outs.append(to_np(got.data))
+        out = torch.full((2, 6, len(rows), cfg.N), -1, dtype=cfg.torch_dtype, device="cuda")
+
+        def call():
+            eng.ctx.call("fhb_ckks_relinearize", nat.ptr(d_ct3), nat.ptr(d_key), nat.ptr(out), nat.ptr(scratch), need,
+                         6, level, 0, eng._stream())
+
+        call()
+        assert any("k_keyswitch_core" in name for name, _ in captured_kernels(call))
+        outs.append(to_np(out))
     eng.ctx.set_tuning(nat.TUNE_KS_ORDER, 0)
     np.testing.assert_array_equal(outs[0][:, 5], orc.relinearize(ct3[:, 5], key, level))
     np.testing.assert_array_equal(outs[1], outs[0])
@@ -187,28 +199,51 @@ def test_automorphism_and_add_match_oracle():
     np.testing.assert_array_equal(to_np(out).reshape(2, len(rows), cfg.N), want)
 
 
-@pytest.mark.parametrize("preset,batch,level", [(Preset.slots8192_scale40_levels7_int64, 26, 1),
-                                                (Preset.slots32768_scale40_levels34_int64, 16, 20)])
-@pytest.mark.parametrize("form", ["cuda_cores", "tensor_cores"])
-def test_fused_hmult_overlapped_chunks_bit_identical(preset, batch, level, form):
-    """fhb_ckks_multiply_relinearize cuts a batch of >= 16 into chunks whose
-    element-wise stages run beside the other chunks' key-switch cores on
-    their own streams: every chunk count gives the one-pass residues (uneven
-    last chunk included)."""
-    eng = CkksEngine(preset, rng_seed=5, basis_conversion=form)
-    rng = np.random.default_rng(batch)
-    msgs = [rng.uniform(-0.05, 0.05, (batch, eng.num_slots)) for _ in range(2)]
-    ca, cb = (eng.coefficient_domain_to_ntt_domain(eng.encrypt_message(m, level=level)) for m in msgs)
-    got = {}
+def _chunk_counts(eng, form, batch, level, call):
+    """`call(scratch, bytes)` -> result with exactly the required scratch for
+    every chunk count, and that the chunks ran: they lay the scratch out chunk
+    by chunk.  (The tensor-core form has launches of its own and no chunks.)"""
+    need = int(eng.ctx.lib.fhb_ckks_keyswitch_scratch_bytes(eng.ctx.handle, batch, level))
+    got, left = {}, {}
     try:
         for chunks in (1, 2, 3, 4):
             eng.ctx.set_tuning(nat.TUNE_OVERLAP_CHUNKS, chunks)
-            got[chunks] = eng.multiply_relinearize_rescale(ca, cb).data.clone()
+            scratch = torch.zeros(need, dtype=torch.uint8, device="cuda")
+            got[chunks] = call(scratch, need)
+            left[chunks] = scratch
     finally:
         eng.ctx.set_tuning(nat.TUNE_OVERLAP_CHUNKS, 4)
     for chunks in (2, 3, 4):
         assert torch.equal(got[chunks], got[1]), chunks
-    got = np.asarray(eng.decrypt_message(eng.multiply_relinearize_rescale(ca, cb)))
+        assert torch.equal(left[chunks], left[1]) == (form == "tensor_cores"), chunks
+    return got[1]
+
+
+@pytest.mark.parametrize("preset,batch,level", [(Preset.slots8192_scale40_levels7_int64, 26, 1),
+                                                (Preset.slots32768_scale40_levels34_int64, 16, 20)])
+@pytest.mark.parametrize("form", ["cuda_cores", "tensor_cores"])
+def test_fused_hmult_overlapped_chunks_bit_identical(preset, batch, level, form):
+    """With exactly the required scratch fhb_ckks_multiply_relinearize cuts a
+    batch of >= 16 into chunks whose element-wise stages run beside the other
+    chunks' key-switch cores on their own streams: every chunk count gives the
+    one-pass residues (uneven last chunk included), which are those of the
+    column and block launches."""
+    eng = CkksEngine(preset, rng_seed=5, basis_conversion=form)
+    rng = np.random.default_rng(batch)
+    msgs = [rng.uniform(-0.05, 0.05, (batch, eng.num_slots)) for _ in range(2)]
+    ca, cb = (eng.coefficient_domain_to_ntt_domain(eng.encrypt_message(m, level=level)) for m in msgs)
+    key = eng.relinearization_key
+
+    def call(scratch, need):
+        out = torch.full((2, batch, eng.num_q - level - 1, eng.n), -1, dtype=eng.dtype, device="cuda")
+        eng.ctx.call("fhb_ckks_multiply_relinearize", nat.ptr(ca.data), nat.ptr(cb.data), nat.ptr(key.data),
+                     nat.ptr(out), nat.ptr(scratch), need, batch, level, 1, eng._stream())
+        return out
+
+    got = _chunk_counts(eng, form, batch, level, call)
+    product = eng.multiply_relinearize_rescale(ca, cb)
+    assert torch.equal(got, product.data)
+    got = np.asarray(eng.decrypt_message(product))
     assert float(np.abs(got - msgs[0] * msgs[1]).max()) < 3e-5
 
 
@@ -217,20 +252,20 @@ def test_fused_hmult_overlapped_chunks_bit_identical(preset, batch, level, form)
 @pytest.mark.parametrize("form", ["cuda_cores", "tensor_cores"])
 def test_rotation_overlapped_chunks_bit_identical(preset, batch, level, form):
     """fhb_ckks_rotate overlaps its chunks like the fused HMult: every chunk
-    count gives the one-pass residues."""
+    count gives the one-pass residues, those of the launches."""
     eng = CkksEngine(preset, rng_seed=6, basis_conversion=form)
     rng = np.random.default_rng(batch + 1)
     msg = rng.uniform(-0.05, 0.05, (batch, eng.num_slots))
     ct = eng.encrypt_message(msg, level=level)
-    eng.generate_rotation_keys([3])
-    got = {}
-    try:
-        for chunks in (1, 2, 3, 4):
-            eng.ctx.set_tuning(nat.TUNE_OVERLAP_CHUNKS, chunks)
-            got[chunks] = eng.rotate_by_step(ct, 3).data.clone()
-    finally:
-        eng.ctx.set_tuning(nat.TUNE_OVERLAP_CHUNKS, 4)
-    for chunks in (2, 3, 4):
-        assert torch.equal(got[chunks], got[1]), chunks
+    key = eng.rotation_key(3)
+
+    def call(scratch, need):
+        out = torch.full_like(ct.data, -1)
+        eng.ctx.call("fhb_ckks_rotate", nat.ptr(ct.data), nat.ptr(key.data), nat.ptr(out), nat.ptr(scratch), need,
+                     batch, level, key.galois_element, eng._stream())
+        return out
+
+    got = _chunk_counts(eng, form, batch, level, call)
+    assert torch.equal(got, eng.rotate_by_step(ct, 3).data)
     dec = np.asarray(eng.decrypt_message(eng.rotate_by_step(ct, 3)))
     assert float(np.abs(dec - np.roll(msg, 3, axis=1)).max()) < 2e-5
