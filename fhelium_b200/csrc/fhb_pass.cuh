@@ -51,14 +51,15 @@ using TwAtQ = TwQ<false>;
 // Forms of the FP64 rows (the kernels' FORM): none; narrow, primes below
 // 2^42; or wide, primes below 1.1 2^50 (kWidePrimeEnd), on chains without
 // narrow rows (the 50-bit chains).  Wide rows use the same butterfly with
-// twiddles balanced to (-q/2, q/2) and keep less headroom: a product of x by
-// such a twiddle has a quotient below |x| / 2, whose estimate is off by at most
-// |x / q| / 8 besides the rounding, so it leaves (0.5 + |x / q| / 8) q, and
-// every value stays exact below 2^53 = 7.2 q as long as each pass of at most
-// four stages starts from reduced words: forward from 1.0 q, 1.63, 2.33, 3.1
-// to 4.0 q; inverse from 0.51 q, sums double, so the words that were sums
-// twice are reduced after two stages (2.0 q) and reach 3.0 q after four.
-// Operands stay below 3.1 q, quotients below 1.55 q < 2^51.  Words enter as
+// twiddles balanced to (-q/2, q/2) and keep less headroom.  The quotient of a
+// product x w comes from the rounded product and the rounded 1/q, each off by
+// 2^-53 of it, besides the rounding to an integer; with q < 1.1 2^50 and |w| <=
+// q/2 that is at most (1.1/8) |x/q|, so a product leaves (0.5 + 0.1375 |x/q|) q.
+// Every value stays exact below 2^53 = 7.2 q as long as each pass of at most
+// four stages starts from reduced words: forward from 1.0 q, 1.64, 2.37, 3.19
+// to 4.13 q; inverse from 0.51 q, sums double, so the words that were sums
+// twice are reduced after two stages (2.04 q) and reach 3.12 q after four.
+// Operands stay below 3.2 q, quotients below 1.6 q < 2^51.  Words enter as
 // u - q (lazy words below 2q, so |x| <= q).
 constexpr int kNoF64 = 0, kNarrowF64 = 1, kWideF64 = 2;
 
@@ -865,7 +866,7 @@ __device__ __forceinline__ void ks_rows_f64(const KsPass<uint64_t>& k, int jrow,
         a1[2 * e] += W::mul_qinv_bal(v[2 * e], lo(u[e]), q, qinv);
         a1[2 * e + 1] += W::mul_qinv_bal(v[2 * e + 1], hi(u[e]), q, qinv);
       }
-      if (WIDE && (SHARED || (a & 3) == 3 || a + 1 == k.lt.num_digits)) {  // at most four terms of 0.7 q
+      if (WIDE && (SHARED || (a & 3) == 3 || a + 1 == k.lt.num_digits)) {  // at most four terms of 0.68 q
         reduce_wide<TW>(a0, q, qinv);
         reduce_wide<TW>(a1, q, qinv);
       }
@@ -1417,7 +1418,7 @@ k_apply_rows(const __grid_constant__ KsPass<T> k, uint32_t galois) {
             const double v = f64_word<TW::kWide>(w[e], q);
             a0[h + e] += W::mul_qinv_bal(v, f64_word<TW::kWide>(k0[e], q), q, qinv);
             a1[h + e] += W::mul_qinv_bal(v, f64_word<TW::kWide>(k1[e], q), q, qinv);
-            if (TW::kWide && (a & 3) == 3) {  // four terms of at most 0.75 q
+            if (TW::kWide && (a & 3) == 3) {  // four terms of at most 0.78 q
               a0[h + e] = W::reduce_bal(a0[h + e], q, qinv);
               a1[h + e] = W::reduce_bal(a1[h + e], q, qinv);
             }

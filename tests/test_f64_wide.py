@@ -36,6 +36,13 @@ def _product(x: int, w: int, q: int) -> int:
     return r
 
 
+def _by_constant(x: int, w: int, q: int) -> int:
+    """A product by a constant kept with w / q (0 <= w < q)."""
+    r = x * w - _rounded(x, w / q) * q
+    assert abs(r) < 1 << 53
+    return r
+
+
 def _reduce(x: int, q: int) -> int:
     assert abs(x) < 1 << 53
     r = x - _rounded(x, 1.0 / q) * q
@@ -53,18 +60,20 @@ def _twiddles(q: int, rng) -> list[int]:
     return [half, -half, half - 1, 1, -1] + [int(v) for v in rng.integers(-half, half, 6)]
 
 
-@pytest.mark.parametrize("start", [1.0, 0.51])
-def test_forward_pass_of_four_stages(start):
+@pytest.mark.parametrize("start,stated", [(1.0, (1.64, 2.37, 3.19, 4.13)), (0.51, (1.09, 1.74, 2.48, 3.33))])
+def test_forward_pass_of_four_stages(start, stated):
+    """`stated`: the bounds after each stage, over q, of the largest modulus."""
     rng = np.random.default_rng(3)
     for q in _primes():
         bound = start
-        for _ in range(4):
+        for after in stated:
+            assert bound + 0.5 + bound * 1.1 / 8 <= after
             xs, top = _worst(bound, q, rng), 0
             for y in xs:
                 for w in _twiddles(q, rng):
                     top = max(top, abs(_product(y, w, q)))
             assert top <= (0.5 + bound * 1.1 / 8 + 1e-3) * q
-            bound += top / q
+            bound = min(after, bound + 0.5 + bound * 1.1 / 8)
             assert bound * q < 1 << 53
         for x in _worst(bound, q, rng):
             _reduce(x, q)
@@ -85,6 +94,7 @@ def test_inverse_pass_of_four_stages():
                 top = max(abs(_product(d, w, q)) for d in _worst(total, q, rng)[:6] for w in _twiddles(q, rng)[:5])
                 nxt[i], nxt[j] = total, max(top / q, 0.5 + total * 1.1 / 8)
             grown = nxt
+            assert max(grown) <= (1.02, 2.04, 1.57, 3.13)[stage]
             if stage == 1:
                 grown = [0.51 if (i & 3) < 2 else g for i, g in enumerate(grown)]
         for g in grown:
@@ -93,10 +103,17 @@ def test_inverse_pass_of_four_stages():
 
 
 def test_key_products_and_their_sums():
-    """Reduced words and u - q words times key words less q; four terms on a
-    reduced sum, then the addend."""
+    """Key words enter as u - q.  The rows launch multiplies reduced words, or
+    own-digit words (a product by R^-1 of a word u - q, 0.64 q at most): four
+    terms of 0.68 q on a reduced sum.  The application of hoisted rotations
+    multiplies words u - q themselves: four terms of 0.78 q."""
     rng = np.random.default_rng(5)
     for q in _primes():
-        top = max(abs(_product(x, k, q)) for x in _worst(1.0, q, rng) for k in [q - 1, -q, 1 - q, q // 3])
-        assert 0.51 * q + 4 * top < 1 << 53
-        assert 0.51 * q + top < 1 << 53
+        keys = [q - 1, -q, 1 - q, q // 3]
+        own = max(abs(_by_constant(x, w, q)) for x in _worst(1.0, q, rng)
+                  for w in [q - 1, q - 2, q // 2, 1] + [int(v) for v in rng.integers(0, q, 12)])
+        assert own <= 0.64 * q
+        for start, term in ((0.64, 0.68), (1.0, 0.78)):
+            top = max(abs(_product(x, k, q)) for x in _worst(start, q, rng) for k in keys)
+            assert top <= (0.5 + start * 1.1 / 4 + 1e-3) * q <= term * q
+            assert (0.51 + 4 * term) * q < 1 << 53
