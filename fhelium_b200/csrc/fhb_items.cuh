@@ -423,11 +423,11 @@ k_items_core_rows(ItemsView iv, const ItemUnit* __restrict__ units, int64_t slot
   const KsPass<T>& k = *held;
   if constexpr (SPLIT) {
     if (k.level + u.row < core.f64_end) {
-      ks_rows_f64<LOGN, false, false>(k, u.row, 0, blk, true, smem);
+      ks_rows_f64<LOGN, false, false>(k, u.row, 0, blk, smem);
       return;
     }
   }
-  ks_rows_int<T, LOGN, false>(k, u.row, 0, blk, true, smem);
+  ks_rows_int<T, LOGN, false>(k, u.row, 0, blk, smem);
 }
 
 // Blocks (unit, component, column tile).

@@ -792,7 +792,7 @@ __device__ __forceinline__ T inverse_pow2(T q, T neg_inv) {
 // a warp per (ciphertext, 256 words), ciphertexts fastest, so that the half
 // warps of a block read the same key words and twiddles.
 template <int LOGN, bool WIDE, bool SHARED>
-__device__ __forceinline__ void ks_rows_f64(const KsPass<uint64_t>& k, int jrow, int bi, int blk, bool live,
+__device__ __forceinline__ void ks_rows_f64(const KsPass<uint64_t>& k, int jrow, int bi, int blk,
                                             unsigned char* smem) {
   constexpr int64_t kN = int64_t(1) << LOGN;
   using W = Word<double>;
@@ -896,10 +896,8 @@ __device__ __forceinline__ void ks_rows_f64(const KsPass<uint64_t>& k, int jrow,
     R::vector_to_contiguous(v, x);
     R::inv(v, x, twi, q, qinv, blk);
     double* o = reinterpret_cast<double*>(out) + (int64_t(bi) * k.qp_limbs + jrow) * kN + blk * kBlk + x.t;
-    if (live) {
 #pragma unroll
-      for (int e = 0; e < 16; ++e) o[16 * e] = v[e];
-    }
+    for (int e = 0; e < 16; ++e) o[16 * e] = v[e];
   };
   if constexpr (SHARED) {  // the warps' partial sums: warp 0 takes component 0, warp 1 component 1
     double* part = reinterpret_cast<double*>(smem);
@@ -925,7 +923,7 @@ __device__ __forceinline__ void ks_rows_f64(const KsPass<uint64_t>& k, int jrow,
 }
 
 template <typename T, int LOGN, bool SHARED>
-__device__ __forceinline__ void ks_rows_int(const KsPass<T>& k, int jrow, int bi, int blk, bool live,
+__device__ __forceinline__ void ks_rows_int(const KsPass<T>& k, int jrow, int bi, int blk,
                                             unsigned char* smem) {
   constexpr int64_t kN = int64_t(1) << LOGN;
   using W = Word<T>;
@@ -1019,10 +1017,8 @@ __device__ __forceinline__ void ks_rows_int(const KsPass<T>& k, int jrow, int bi
     R::vector_to_contiguous(v, x);
     R::inv(v, x, twi, q, twoq, blk);
     T* o = out + (int64_t(bi) * k.qp_limbs + jrow) * kN + blk * kBlk + x.t;
-    if (live) {
 #pragma unroll
-      for (int e = 0; e < 16; ++e) o[16 * e] = v[e];
-    }
+    for (int e = 0; e < 16; ++e) o[16 * e] = v[e];
   };
   if constexpr (SHARED) {  // the warps' partial sums: warp 0 takes component 0, warp 1 component 1
     T* part = reinterpret_cast<T*>(smem);
@@ -1071,22 +1067,21 @@ k_ks_rows(const __grid_constant__ KsPass<T> k) {
   // twiddles, and an SM runs one of the two bodies at a time (integer blocks
   // dealt out among the FP64 ones measured 25 % slower: the bodies evict each
   // other from the instruction caches).
-  const unsigned per_block = SHARED ? 2 : kRowSlots, per_row = (slots + per_block - 1) / per_block;
+  static_assert(kBlks % kRowSlots == 0, "a block's half warps all have a row");
+  const unsigned per_block = SHARED ? 2 : kRowSlots, per_row = slots / per_block;
   int at;
   const bool is_int = ks_unit(int(blockIdx.x / per_row), k.rows(), k.i_cnt, at);
   const int jrow = at + (is_int ? k.i_lo : k.f_lo);
-  unsigned slot = blockIdx.x % per_row * per_block + ((threadIdx.x >> 4) & (per_block - 1));
-  const bool live = slot < slots;
-  if (!live) slot = slots - 1;  // the last block's spare half warps repeat a row and store nothing
+  const unsigned slot = blockIdx.x % per_row * per_block + ((threadIdx.x >> 4) & (per_block - 1));
   const int bi = int(slot % unsigned(k.batch)), blk = int(slot / unsigned(k.batch));
   if constexpr (SPLIT) {
     static_assert(sizeof(T) == 8, "FP64 rows exist in int64 chains only");
     if (!is_int) {
-      ks_rows_f64<LOGN, SPLIT == kWideF64, SHARED>(k, jrow, bi, blk, live, smem);
+      ks_rows_f64<LOGN, SPLIT == kWideF64, SHARED>(k, jrow, bi, blk, smem);
       return;
     }
   }
-  ks_rows_int<T, LOGN, SHARED>(k, jrow, bi, blk, live, smem);
+  ks_rows_int<T, LOGN, SHARED>(k, jrow, bi, blk, smem);
 }
 
 // Launch 3: one column tile of the inverse transform of the accumulator row z

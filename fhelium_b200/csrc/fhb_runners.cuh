@@ -243,8 +243,7 @@ bool shared_rows(int64_t half_warps, int digits) {
   return digits > 2 && half_warps <= 148 * (sizeof(T) == 8 ? 3 : 2) * kRowSlots;
 }
 inline int64_t rows_blocks(int64_t slots, int rows, bool shared) {
-  const int64_t per = shared ? 2 : kRowSlots;
-  return (slots + per - 1) / per * rows;
+  return slots / (shared ? 2 : kRowSlots) * rows;  // (a polynomial has a multiple of kRowSlots rows of 256 words)
 }
 
 // The three launches of one group of rows.

@@ -19,7 +19,7 @@ from tests.helpers import captured_kernels, oracle_for, random_key, reduced_ring
 pytestmark = pytest.mark.gpu
 
 # (preset, logN, level, batch): FP64 + integer rows, integer rows only, int32;
-# odd batches leave spare half warps in the last block
+# batches that are no multiple of a block's half warps
 CASES = [
     ("slots8192_scale40_levels7_int64", 12, 4, 3),
     ("slots8192_scale40_levels7_int64", 13, 0, 1),
