@@ -51,9 +51,9 @@ ROOT = os.path.dirname(os.path.abspath(__file__))
 sys.path.insert(0, ROOT)
 
 PRESET = "slots32768_scale40_levels34_int64"
-# ncu dram read + write of the key-switch core's three launches over all rows, captured at batch 4 and scaled by the
-# ciphertexts processed (columns 0.76 GB, rows 1.59 GB, inverse columns 0.27 GB); see profiles/
-KS_TRAFFIC_BYTES_BATCH4 = 2616626000
+# ncu dram read + write of the key-switch core's launches as the keyswitch_core leg runs them, by batch (captured at
+# these batches only: one group of rows at 4, seven groups at 32); see profiles/
+KS_TRAFFIC_BYTES = {4: 2530229408, 32: 20619080424}
 METRIC = "hmult_relin_rescale_ops_per_s_logN16_L35"
 UNIT = "ops/s"
 CONFIG = {
@@ -748,18 +748,12 @@ def main() -> int:
     from fhelium_b200 import ranks
     value = ranks.job_rate(B, ws, ms)
     f64_core = bool(eng.ctx.get_tuning(nat.TUNE_F64_CORE))
-    # kernels of one step: tensor product, inverse NTT of d2 (two launches), ModUp digits, (tensor-core extension,)
-    # the key-switch core (columns, rows, inverse columns, once per group of rows that the workspace's room holds;
-    # the tensor-core form takes all rows at once), ModDown + rescale
+    # kernels of one step: tensor product, inverse NTT of d2 (two launches), ModUp digits, the key-switch core (columns,
+    # rows, inverse columns for every group of rows that the engine's scratch holds, in the tensor-core form the
+    # extension and one group) and ModDown + rescale
     lib, h = eng.ctx.lib, eng.ctx.handle
-    qp_rows = cfg.num_q_primes + cfg.num_p_primes
-    row_groups = 1
-    if form != "tensor_cores":
-        room = (int(lib.fhb_ckks_keyswitch_workspace_bytes(h, B, 0))
-                - int(lib.fhb_ckks_keyswitch_scratch_bytes(h, B, 0)))
-        per_row = len(eng.level_digits[0]) * B * cfg.N * 8
-        row_groups = -(-qp_rows // min(qp_rows, room // per_row))
-    launches_per_step = 5 + (1 if form == "tensor_cores" else 0) + 3 * row_groups
+    core_launches = int(lib.fhb_ckks_keyswitch_core_launches(h, B, 0, eng._scratch_for(B, 0)[1]))
+    launches_per_step = 5 + core_launches
 
     # ---- end to end through the public API with host buffers -------------
     host_a = ca.data.cpu().pin_memory()
@@ -815,7 +809,8 @@ def main() -> int:
         "mul_to_coefficient": lambda: lib.fhb_ckks_multiply_to_coefficient(h, nat.ptr(ca.data), nat.ptr(cb.data),
                                                                              nat.ptr(coef), B, 0, s),
         "modup_digits": lambda: lib.fhb_ckks_modup_digits(h, nat.ptr(coef[2]), nat.ptr(digits), B, 0, 1, s),
-        # one term: the key switch of the batch over a work buffer, as the fused step runs it
+        # the core's launches over a work buffer, as the sum of one term: every digit row is transformed and nothing is
+        # added (the fused step takes own-digit rows, L of the dnum (L + P), from d2 and adds P d0, P d1)
         "keyswitch_core": lambda: lib.fhb_ckks_keyswitch_sum_work(h, nat.ptr(digits), nat.ptr(key_ptr), nat.ptr(t[0]),
                                                                   nat.ptr(t[1]), nat.ptr(work), work.numel(), 1, B,
                                                                   0, s),
@@ -930,9 +925,8 @@ def main() -> int:
             entry.update({"int8_ops": int8_ops[name], "int8_tops": int8_ops[name] / sec / 1e12,
                           "int8_frac": int8_ops[name] / sec / 1e12 / int8_peak, "int8_peak_source": int8_src})
         kernel_roofline[name] = entry
-    # DRAM bytes of the key-switch core's launches (the intermediate crosses
-    # device memory between them), scaled by the ciphertexts processed
-    traffic = KS_TRAFFIC_BYTES_BATCH4 * B / 4 if cfg.logN == 16 and L == 35 and form == "cuda_cores" else None
+    # DRAM bytes of the leg's launches (the intermediate crosses device memory between them)
+    traffic = KS_TRAFFIC_BYTES.get(B) if cfg.logN == 16 and L == 35 and form == "cuda_cores" else None
     dom = "keyswitch_core"
     dom_kernel = ("k_ks_columns + k_ks_rows + k_ks_columns_inverse "
                   + ("(FP64 rows for the primes below 2^42, int64 rows for the base prime and P)" if f64_core
@@ -1039,7 +1033,8 @@ def main() -> int:
         "kernel_ms": per_kernel,
         "kernel_roofline": kernel_roofline,
         "kernel_ms_note": "each public entry point timed alone on the same inputs; the fused step runs the "
-                          "HMult->INTT for d2 only and folds d0, d1 into the key-switch accumulators",
+                          "HMult->INTT for d2 only, folds d0, d1 into the key-switch accumulators and reuses d2 for "
+                          "the own-digit rows that the keyswitch_core leg transforms",
         "step_algorithmic_gbs": step_bytes / (ms / 1000.0) / 1e9,
         "clocks": csum,
         "cpu_baseline": cpu,
