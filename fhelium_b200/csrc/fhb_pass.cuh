@@ -15,8 +15,8 @@
 // pipe 33 % busy, long scoreboard and barriers), these launches 8.9 ms
 // (columns 3.9, rows 4.4, inverse columns 0.64 ms; FP64 pipe 65-73 % busy
 // over the FP64 rows, 46-54 % with the five integer rows); at N = 2^14, one ciphertext: 217 -> 69 us for the whole
-// HMult.  The standalone transforms: 0.86 -> 0.39 ms forward for 12 x 2 x 35
-// int64 rows of N = 2^16, 1.72 -> 0.66 ms inverse for 48 x 2 x 25 int32 rows.
+// HMult.  The standalone transforms: 0.86 -> 0.40 ms forward for 12 x 2 x 35
+// int64 rows of N = 2^16, 1.72 -> 0.68 ms inverse for 48 x 2 x 25 int32 rows.
 //
 // Butterflies, twiddles and ranges are those of fhb_ntt.cuh: integer words
 // see the same operations in the same order, so even lazy results are the

@@ -74,7 +74,7 @@ constexpr size_t ntt_smem() {
 // The standalone transforms run as two launches (fhb_pass.cuh) unless the
 // context's tuning value for the direction is 16: one cluster per polynomial
 // with 16 residues per thread.  (0.40 against 0.86 ms forward for 12 x 2 x 35
-// int64 rows of N = 2^16, 0.69 against 1.72 ms inverse for 48 x 2 x 25 int32
+// int64 rows of N = 2^16, 0.68 against 1.72 ms inverse for 48 x 2 x 25 int32
 // rows; the autotuner times both.)
 template <typename T, int LOGN, int EPT>
 int run_forward_e(const Context& c, const void* in, void* out, int64_t polys, int rows, int row_start, bool mont,

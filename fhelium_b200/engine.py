@@ -316,7 +316,8 @@ class CkksEngine:
                                      relinearization_key: RelinearizationKey | None = None,
                                      *, rescale: bool = True) -> Ciphertext:
         """multiply -> relinearize -> rescale_to_next_level in one fused
-        pipeline (four kernel launches); bit-identical to the three calls."""
+        pipeline (five launches and the key-switch core's, three for each group
+        of rows that its scratch holds); bit-identical to the three calls."""
         lhs.assert_state(polynomial_domain="ntt", residue_representation="montgomery", components=2)
         self._assert_same_layout(lhs, rhs)
         key = relinearization_key or self.relinearization_key
