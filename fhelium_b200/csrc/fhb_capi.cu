@@ -182,7 +182,7 @@ int moddown(const Context& c, const void* t0, const void* t1, const void* a0, co
   if (out_pitch <= 0) out_pitch = batch * (c.num_q - level - (rescale ? 1 : 0)) * c.n();
   const MdArgs<T> args = moddown_args<T>(c, level, rescale);
   const int64_t tiles = (int64_t(c.n()) >> 9) * 2 * batch;
-  const int groups = moddown_groups(tiles, c.num_q - level, c.num_p);
+  const int groups = moddown_groups(tiles, c.num_q - level, c.num_p, rescale);
   if (tiles * groups > 0x7fffffffLL) return fail(-6, "too many blocks for one launch");
   auto run = [&](auto kern) {
     kern<<<unsigned(tiles * groups), kMdThreads, 0, st>>>(args, (const T*)t0, (const T*)t1, (const T*)a0,

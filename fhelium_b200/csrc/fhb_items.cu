@@ -166,7 +166,7 @@ int run_elementwise(const Context& c, const char* plan, const PlanLayout& l, con
     return rc;
   const MdArgs<T> args = moddown_args<T>(c, 0, 0);
   const int64_t tiles = (n >> 9) * 2;
-  const int groups = moddown_groups(tiles * info.items, info.max_limbs, c.num_p);
+  const int groups = moddown_groups(tiles * info.items, info.max_limbs, c.num_p, info.hmult_items > 0);
   auto run = [&](auto kern) {
     kern<<<dim3(unsigned(tiles * groups), unsigned(info.items)), kMdThreads, 0, st>>>(iv, args, groups);
     return cuda_status(cudaGetLastError(), "k_items_moddown");

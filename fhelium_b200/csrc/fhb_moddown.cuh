@@ -249,21 +249,28 @@ MdArgs<T> moddown_args(const Context& c, int level, int rescale) {
                    md_tables<T>(c)};
 }
 
-// Groups of rows per coefficient tile, so that a few ciphertexts fill the GPU:
-// as many as give two blocks per SM, which hide one another's loads.  More cost
-// more than they give, since each group forms the digits (and v_0) again: about
-// num_p / 2 rows' work, so a group has at least 1 + num_p / 2 rows.  Measured
-// without rescale, by groups (us): N = 2^16, 35 + 4 rows, 1 ciphertext (256
-// tiles) 1: 49.5, 2: 52.7, 4: 58.4; N = 2^14, 8 + 1 rows, 1 ciphertext (64
-// tiles) 1: 6.4, 2: 4.7, 4: 4.2, 8: 5.2; 16 ciphertexts of 2 + 1 rows (1024
-// tiles) 1: 11.6, 2: 14.2 (one group for all rows and both components, before
-// the sums of products: 10.5).  Over 292 calls the choice is within 0.2 % of
-// the best on average, 14 % at most.  And few enough rows in each for the
-// staged constants.
-inline int moddown_groups(int64_t tiles, int q_limbs, int num_p) {
-  const int64_t fill = 2 * 148 / tiles, most = q_limbs / (1 + num_p / 2);
+// Groups of rows per coefficient tile, so that a few ciphertexts fill the GPU.
+// Each group forms the digits (and v_0) again, about num_p / 2 rows' work:
+// * as many as give two blocks per SM, which hide one another's loads, with at
+//   least 1 + num_p / 2 rows each;
+// * up to fourteen blocks per SM where the rows are many (2 + 2 num_p, 6 more
+//   with the rescale, whose v_0 is a row's sum that nothing hides): shorter
+//   blocks leave a smaller last wave.
+// Measured, by groups (us): N = 2^14, 8 + 1 rows, 1 ciphertext (64 tiles) 1:
+// 6.4, 2: 4.7, 4: 4.2, 8: 5.2; 16 ciphertexts of 2 + 1 rows (1024 tiles) 1: 11.6,
+// 2: 14.2 (one group for all rows and both components, before the sums of
+// products: 10.5); N = 2^16, 29 + 4 rows through sigma_g, 3 ciphertexts (768
+// tiles) 1: 106.6, 2: 100.9, 3: 110.0, 4 of them 1: 132.1, 2: 134.4; 32-bit words
+// of N = 2^15, 30 + 2 rows, 7 ciphertexts (896 tiles) 1: 49.7, 2: 42.8, 3: 42.1,
+// with the rescale 44.9, 40.7, 41.3.  Over 1041 calls (1 to 24 ciphertexts, both
+// words, with and without addends and rescale) the choice is 0.9 % from the best
+// on average, 16 % at most.  And few enough rows in each for the staged
+// constants.
+inline int moddown_groups(int64_t tiles, int q_limbs, int num_p, int rescale) {
+  const int64_t fill = std::min<int64_t>(2 * 148 / tiles, q_limbs / (1 + num_p / 2));
+  const int64_t tail = std::min<int64_t>(14 * 148 / tiles, q_limbs / (2 + 2 * num_p + (rescale ? 6 : 0)));
   const int64_t least = (q_limbs + kMdRows - 2) / (kMdRows - 1);
-  return int(std::max({least, int64_t(1), std::min(fill, most)}));
+  return int(std::max({least, int64_t(1), fill, tail}));
 }
 
 // t0/t1: [B, QP_l, N] canonical coefficient rows; add0/add1 (nullable):

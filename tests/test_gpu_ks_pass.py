@@ -372,20 +372,24 @@ def test_sums_whose_sizes_overflow_are_refused():
 
 
 # blocks of ModDown: the coefficient tiles (N / 512, two components, the batch)
-# times the groups of rows
+# times the groups of rows, without and with the rescale
 @pytest.mark.parametrize("preset,log_n,level,batch,groups", [
-    ("slots8192_scale40_levels7_int64", 14, 6, 16, 1),
-    ("slots8192_scale40_levels7_int64", 14, 0, 1, 4),
-    ("slots8192_scale40_levels7_int64", 12, 7, 1, 1),
-    ("slots32768_scale40_levels34_int64", 16, 0, 1, 1),
-    ("slots32768_scale40_levels34_int64", 12, 0, 1, 11),
-    ("slots16384_scale25_levels29_int32", 12, 0, 3, 6),
-    ("slots65536_scale40_levels72_int64", 12, 0, 1, 18),
+    ("slots8192_scale40_levels7_int64", 14, 6, 16, (1, 1)),
+    ("slots8192_scale40_levels7_int64", 14, 0, 1, (4, 4)),
+    ("slots8192_scale40_levels7_int64", 12, 7, 1, (1, 1)),
+    ("slots32768_scale40_levels34_int64", 16, 0, 1, (3, 2)),
+    ("slots32768_scale40_levels34_int64", 16, 6, 3, (2, 1)),
+    ("slots32768_scale40_levels34_int64", 12, 0, 1, (11, 11)),
+    ("slots16384_scale25_levels29_int32", 12, 0, 3, (6, 6)),
+    ("slots16384_scale25_levels29_int32", 15, 0, 7, (2, 2)),
+    ("slots65536_scale40_levels72_int64", 12, 0, 1, (18, 18)),
 ])
 @pytest.mark.parametrize("rescale", [0, 1])
 def test_moddown_groups(preset, log_n, level, batch, groups, rescale):
-    """Groups for two blocks per SM, none below 1 + P / 2 rows (each forms the
-    digits again), every split with the oracle's residues."""
+    """Groups of rows for two blocks per SM, none too short for the digits that
+    each forms again, and up to fourteen blocks of long groups; every split
+    with the exact residues."""
+    groups = groups[rescale]
     cfg, eng, orc = _engine(preset, log_n)
     limbs = eng.num_q - level
     if rescale and limbs == 1:
@@ -404,7 +408,7 @@ def test_moddown_groups(preset, log_n, level, batch, groups, rescale):
     call()
     (name, grid), = captured_kernels(call)
     assert "k_moddown" in name and grid[0] == cfg.N // 512 * 2 * batch * groups
-    assert groups == 1 or grid[0] <= 2 * 148
+    assert groups == 1 or grid[0] <= 14 * 148
     q = np.array([cfg.moduli[i] for i in ids[:limbs]], dtype=object).reshape(-1, 1)
     cols = [0, 1, 255, 256, cfg.N // 2 + 7, cfg.N - 1]
     p_all = 1
